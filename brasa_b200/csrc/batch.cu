@@ -19,7 +19,7 @@
 using namespace brasa_dev;
 
 int32_t brasa_sample_batched_launch(brasa_cmd *cmd, const float *logits, uint32_t n, uint32_t count, float temperature, uint32_t top_k, float top_p,
-                                    unsigned long long *rng, float *scratch, uint32_t *out);
+                                    unsigned long long *rng, uint32_t *out);
 
 namespace {
 
@@ -549,11 +549,11 @@ __global__ void spread_shard_kernel(const float *shard, float *full, uint32_t n,
 // Next token of `count` rows of logits (row stride = this rank's lm_head rows). A tensor-parallel shard holds only its
 // rows of the vocabulary: a greedy choice exchanges each row's best (value, index) pair between the ranks, a sampled one the rows.
 int32_t choose_tokens(brasa_batch *b, brasa_cmd *cmd, brasa_buf *logits, uint32_t count, brasa_sampling_params params, unsigned long long *rng,
-                      float *scratch, brasa_buf *out, uint64_t out_index) {
+                      brasa_buf *out, uint64_t out_index) {
     brasa_model *m = b->m;
     const uint32_t rows = m->cfg.head_rows;
     if (!m->tp || (params.temperature > 0.0f && rows == m->cfg.vocab))  // (a one-rank group holds the whole vocabulary)
-        return brasa_sample_batched_launch(cmd, F(logits), rows, count, params.temperature, params.top_k, params.top_p, rng, scratch,
+        return brasa_sample_batched_launch(cmd, F(logits), rows, count, params.temperature, params.top_k, params.top_p, rng,
                                            (uint32_t *)out->ptr + out_index);
     if (params.temperature <= 0.0f) {
         for (uint32_t r = 0; r < count; ++r)
@@ -576,7 +576,7 @@ int32_t choose_tokens(brasa_batch *b, brasa_cmd *cmd, brasa_buf *logits, uint32_
         BRASA_TRY(brasa_post_launch(cmd, "spread_shard"));
         BRASA_TRY(brasa_k_tp_allreduce_add(cmd, m->tp, A(b->tp_pad), brasa_arg{nullptr, 0}, A(b->tp_full), tot));
         BRASA_TRY(brasa_sample_batched_launch(cmd, F(b->tp_full), vocab, n, params.temperature, params.top_k, params.top_p, rng + 2 * (size_t)r0,
-                                              scratch + (size_t)r0 * 2 * vocab, (uint32_t *)out->ptr + out_index + r0));
+                                              (uint32_t *)out->ptr + out_index + r0));
     }
     return BRASA_OK;
 }
@@ -888,6 +888,7 @@ int32_t brasa_batch_create(brasa_model *m, uint32_t max_seqs, uint32_t num_pages
     BRASA_TRY(balloc(b.get(), (uint64_t)max_seqs * 16, &b->rng));
     BRASA_TRY(balloc(b.get(), (uint64_t)max_seqs * m->cfg.head_rows * 4, &b->logits));
     BRASA_TRY(balloc(b.get(), (uint64_t)max_seqs * m->cfg.heads * b->max_chunks * 130 * 4, &b->partials));
+    // (part of the planned bytes; the sampler itself keeps nothing in device memory)
     BRASA_TRY(balloc(b.get(), (uint64_t)max_seqs * 2 * m->cfg.vocab * 4, &b->scratch));
     if (m->cfg.head_rows < m->cfg.vocab) {
         BRASA_TRY(balloc(b.get(), (uint64_t)max_seqs * m->cfg.vocab * 4, &b->tp_pad));
@@ -1021,8 +1022,7 @@ int32_t brasa_batch_add_sequence(brasa_batch *b, const uint32_t *ids, uint32_t n
     BRASA_TRY(brasa_cmd_begin(ctx, &cmd));
     int32_t rc = copy_rows_to_pages(b, cmd, seq, matched, total - matched);
     if (rc == BRASA_OK)
-        rc = choose_tokens(b, cmd, m->logits, 1, params, (unsigned long long *)b->rng->ptr + 2 * seq, F(b->scratch) + (size_t)seq * 2 * m->cfg.vocab,
-                           b->ids, seq);
+        rc = choose_tokens(b, cmd, m->logits, 1, params, (unsigned long long *)b->rng->ptr + 2 * seq, b->ids, seq);
     int32_t rc2 = brasa_cmd_wait(cmd, nullptr);
     BRASA_TRY(rc);
     BRASA_TRY(rc2);
@@ -1057,7 +1057,7 @@ int32_t brasa_batch_decode(brasa_batch *b, uint32_t steps, brasa_sampling_params
     for (uint32_t s = 0; s < steps && rc == BRASA_OK; ++s) {
         rc = encode_step(b, cmd, n);
         if (rc != BRASA_OK) break;
-        rc = choose_tokens(b, cmd, b->logits, n, params, (unsigned long long *)b->rng->ptr, F(b->scratch), b->out, 0);
+        rc = choose_tokens(b, cmd, b->logits, n, params, (unsigned long long *)b->rng->ptr, b->out, 0);
         if (rc != BRASA_OK) break;
         gather_ids_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>((uint32_t *)b->ids->ptr, (const uint32_t *)b->out->ptr, n);
         rc = brasa_post_launch(cmd, "next_ids");

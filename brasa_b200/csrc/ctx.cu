@@ -93,7 +93,6 @@ void brasa_ctx_destroy(brasa_ctx *ctx) {
     cudaFree(ctx->gemm_part);
     cudaFree(ctx->kv_expand);
     cudaFree(ctx->gemm_counters);
-    cudaFree(ctx->sample_scratch);
     cudaFree(ctx->gemv_trace);
     cudaFree(ctx->status);
     cudaStreamDestroy(ctx->stream);

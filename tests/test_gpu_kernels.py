@@ -765,6 +765,50 @@ def test_sampler_for_many_rows_follows_the_reference_sampler(B, ctx, K, n):
             assert agree >= 0.97 * total, (agree, total)
 
 
+@pytest.mark.parametrize("n", [1, 2, 9, 513, 4097, 60_000])
+@pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.9), (7, 1.0), (30, 0.8)])
+def test_device_sampler_against_64_bits(B, ctx, K, n, top_k, top_p):
+    """The one-row sampler where its split can go wrong (fewer candidates than blocks or threads, every eighth one longer than the last;
+    many equal logits on either side of each cut; masked candidates; a maximum that stands alone) against the same walk in 64 bits. A
+    draw or a cut within 1e-5 of a candidate's boundary, the rounding of an f32 exp, may fall to either side and is left out."""
+    rng = np.random.default_rng(n * 31 + top_k)
+    out, checked = ctx.buffer(4), 0
+    state = ctx.buffer_from(B.pcg32_state(n))
+    for case in range(8):
+        l = (rng.standard_normal(n) * 3.0).astype(np.float32)
+        if case & 1:
+            l = np.round(l)  # a handful of values
+        if case & 2:
+            l[rng.random(n) < 0.4] = -np.inf
+        if case & 4:
+            l[rng.integers(0, n)] = 20.0
+        if not np.isfinite(l.max()):
+            l[0] = 0.0
+        old, inc = (int(v) for v in state.download(np.uint64, 2))
+        x, rot = ((((old >> 18) ^ old) >> 27) & 0xffffffff), old >> 59
+        u24 = (((x >> rot) | (x << ((32 - rot) & 31))) & 0xffffffff) >> 8
+        g = ctx.buffer_from(l)
+        run(ctx, lambda c: K.sample_top_p(c, g, n, 0.8, top_k, top_p, state, out))
+        got = int(out.download(np.uint32, 1)[0])
+        assert int(state.download(np.uint64, 2)[0]) == (old * 6364136223846793005 + inc) % 2 ** 64
+        order = np.lexsort((np.arange(n), -l.astype(np.float64)))
+        if top_k:
+            order = order[:top_k]
+        cum = np.cumsum(np.exp((l[order].astype(np.float64) - float(l.max())) / np.float64(np.float32(0.8))))
+        cut = len(order) - 1
+        if top_p < 1.0:
+            p = float(np.float32(top_p)) * cum[-1]
+            cut = int(np.searchsorted(cum, p))
+            if np.min(np.abs(cum - p)) <= 1e-5 * cum[-1]:
+                continue
+        r = u24 / 2.0 ** 24 * cum[cut]
+        if np.min(np.abs(cum[:cut + 1] - r)) <= 1e-5 * cum[-1]:
+            continue
+        checked += 1
+        assert got == int(order[np.searchsorted(cum[:cut + 1], r)]), (case, u24)
+    assert checked >= 4 or n <= 9
+
+
 def test_device_sampler_frequency_and_greedy(B, ctx, K):
     """The reference's frequency check (sampler.rs:252-267): logits (0, ln 3) at temperature 1 pick token 1 three
     times out of four; temperature 0 is the greedy argmax."""
