@@ -10,6 +10,7 @@
 #include "brasa_internal.h"
 
 bool brasa_gemm_tc_supported(const brasa_qmatrix &w, uint32_t tokens);
+bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool glu);
 bool brasa_gemm_tc_few_tokens(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens);
 int32_t brasa_gemm_tc_add_norm(brasa_cmd *cmd, const brasa_qmatrix &w, const __half *x, float *acc, const float *norm_w, __half *out, uint32_t tokens,
                                float eps);
@@ -186,7 +187,8 @@ bool tc_enabled() {
 // True when brasa_k_gemm_swiglu runs as one tensor-core launch for these matrices and token count (given an output that
 // does not overlap the input). The model then hands it a separate output buffer.
 bool brasa_gemm_swiglu_fuses(const brasa_qmatrix &wg, const brasa_qmatrix &wu, uint32_t tokens) {
-    return tc_enabled() && tokens >= 128 && wg.rows == wu.rows && wg.cols == wu.cols && wg.qtype == BRASA_Q4_0 && wu.qtype == BRASA_Q4_0 &&
+    const brasa_qmatrix both[2] = {wg, wu};
+    return tc_enabled() && (tokens >= 128 || brasa_gemm_pair_takes(both, 2, tokens, true)) && wg.rows == wu.rows && wg.cols == wu.cols && wg.qtype == BRASA_Q4_0 && wu.qtype == BRASA_Q4_0 &&
            qm_fits(wg) && qm_fits(wu) && brasa_gemm_tc_supported(wg, tokens) && brasa_gemm_tc_supported(wu, tokens);
 }
 

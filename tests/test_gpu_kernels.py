@@ -667,6 +667,41 @@ def test_gemm_tensor_core_token_counts(B, ctx, K, rows, cols):
         assert np.max(np.abs(got - want16) / s16) <= 1e-5, tokens
 
 
+@pytest.mark.parametrize("tokens", [65, 96, 97, 256, 257, 513, 900])
+@pytest.mark.parametrize("rows,cols", [((256,), 256), ((512, 256, 256), 2560), ((2560,), 1024), ((20480,), 256)])
+def test_gemm_cta_pairs(B, ctx, K, rows, cols, tokens):
+    """The CTA-pair GEMM at the edges of its token tiles (as many as hold the tokens, 32 to 256 each), fewer units than pairs, runs that
+    share a tile among many, that begin and end inside tiles and that hold several whole ones, one and three matrices; each against the
+    oracle's sum within the bound of the reference's GEMM test. The SwiGLU form over the same matrices, and one with the residual."""
+    rng = O.Rng(tokens + cols)
+    raws = [rng.qmatrix(O.Q4_0, r, cols) for r in rows]
+    ws = [tiled(B, ctx, K, "q4_0", raw, r, cols)[0] for raw, r in zip(raws, rows)]
+    x = rng.vec(tokens * cols, 1.0)
+    gx = ctx.buffer_from(x.astype(np.float16))
+    ys = [ctx.buffer(tokens * r * 4) for r in rows]
+    for y in ys:
+        y.fill(0xFF)
+    run(ctx, lambda c: K.gemm_multi(c, ws, gx, ys, tokens, B.PrefillPrecision.F16))
+    got = [y.download(np.float32).reshape(tokens, r) for y, r in zip(ys, rows)]
+    want = [O.matmul(O.Q4_0, raw, r, cols, x, f16_inputs=True) for raw, r in zip(raws, rows)]
+    for g, (w, s) in zip(got, want):
+        assert np.max(np.abs(g - w) / s) <= 1e-5
+    acc0 = rng.vec(tokens * rows[0], 2.0)
+    ga, gs = ctx.buffer_from(acc0), ctx.buffer(tokens * rows[0] * 4)
+    run(ctx, lambda c: K.gemm_add(c, ws[0], gx, ga, gs, tokens))
+    w, s = want[0]
+    d = np.abs(ga.download(np.float32).reshape(tokens, -1) - (w + acc0.reshape(tokens, -1)))
+    assert np.all(d <= 1e-5 * s + 2.0 ** -23 * (np.abs(w) + np.abs(acc0.reshape(tokens, -1))))
+    uraw = rng.qmatrix(O.Q4_0, rows[0], cols)
+    up = tiled(B, ctx, K, "q4_0", uraw, rows[0], cols)[0]
+    gg, gu, go = (ctx.buffer(tokens * rows[0] * 4) for _ in range(3))
+    run(ctx, lambda c: K.gemm_swiglu(c, ws[0], up, gx, gg, gu, go, tokens))
+    wu, su = O.matmul(O.Q4_0, uraw, rows[0], cols, x, f16_inputs=True)
+    o = O.swiglu(w, wu).reshape(tokens, -1)
+    got = go.download(np.uint16, tokens * rows[0]).view(np.float16).astype(np.float32).reshape(tokens, -1)
+    assert np.all(np.abs(got - o) <= 1e-5 * (np.abs(wu) * 1.1 * s + np.abs(w) * su) + np.abs(o) * 2.0 ** -10 + 1e-7)
+
+
 @pytest.mark.parametrize("kv", ["F16", "Q8_0"])
 @pytest.mark.parametrize("tokens,pos0", [(512, 0), (300, 77), (129, 255), (200, 1500)])
 def test_flash_attention_tensor_core_many_query_tiles(B, ctx, K, tokens, pos0, kv):
