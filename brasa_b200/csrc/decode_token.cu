@@ -572,208 +572,287 @@ __device__ __forceinline__ void gemv_epilogue(const TokCtx &c, const TokOp &op, 
 }
 
 // ---- attention of this token over the cache, new row included ----
+// Eight dims of a cached row as they lie there (segment seg of 0..15), and as floats; a q8_0 row's are its codes, whose scale
+// goes with the dot product (with the probability) instead.
+template <int KV> struct KvSeg;
+template <> struct KvSeg<BRASA_KV_F16> {
+    uint4 w;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t seg) { w = __ldcg(reinterpret_cast<const uint4 *>(row) + seg); }
+    __device__ __forceinline__ void load_shared(const uint8_t *row, uint32_t seg) { w = reinterpret_cast<const uint4 *>(row)[seg]; }
+    __device__ __forceinline__ float scale() const { return 1.0f; }
+    __device__ __forceinline__ void four(int i, float v[4]) const {  // values 4 i .. 4 i + 3
+        const uint32_t lo = i ? w.z : w.x, hi = i ? w.w : w.y;
+        const float2 a = __half22float2(*reinterpret_cast<const __half2 *>(&lo)), b = __half22float2(*reinterpret_cast<const __half2 *>(&hi));
+        v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
+    }
+};
+template <> struct KvSeg<BRASA_KV_F32> {
+    float4 w[2];
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t seg) {
+        w[0] = __ldcg(reinterpret_cast<const float4 *>(row) + 2 * seg);
+        w[1] = __ldcg(reinterpret_cast<const float4 *>(row) + 2 * seg + 1);
+    }
+    __device__ __forceinline__ void load_shared(const uint8_t *row, uint32_t seg) {
+        w[0] = reinterpret_cast<const float4 *>(row)[2 * seg];
+        w[1] = reinterpret_cast<const float4 *>(row)[2 * seg + 1];
+    }
+    __device__ __forceinline__ float scale() const { return 1.0f; }
+    __device__ __forceinline__ void four(int i, float v[4]) const { v[0] = w[i].x; v[1] = w[i].y; v[2] = w[i].z; v[3] = w[i].w; }
+};
+template <> struct KvSeg<BRASA_KV_Q8_0> {
+    uint2 w;
+    unsigned short d;
+    __device__ __forceinline__ void load(const uint8_t *row, uint32_t seg) {
+        w = __ldcg(reinterpret_cast<const uint2 *>(row) + seg);
+        d = __ldcg(reinterpret_cast<const unsigned short *>(row + 128) + (seg >> 2));
+    }
+    __device__ __forceinline__ void load_shared(const uint8_t *row, uint32_t seg) {
+        w = reinterpret_cast<const uint2 *>(row)[seg];
+        d = reinterpret_cast<const unsigned short *>(row + 128)[seg >> 2];
+    }
+    __device__ __forceinline__ float scale() const { return __half2float(__ushort_as_half(d)); }
+    __device__ __forceinline__ void four(int i, float v[4]) const {
+        const uint32_t c = (i ? w.y : w.x) ^ 0x80808080u;  // code + 128
+        // the float 2^23 + byte, minus 2^23 + 128: exact, and two instructions where a conversion takes a quarter-rate one
+        v[0] = __uint_as_float(__byte_perm(c, 0x4B000000u, 0x7440)) - 8388736.0f;
+        v[1] = __uint_as_float(__byte_perm(c, 0x4B000000u, 0x7441)) - 8388736.0f;
+        v[2] = __uint_as_float(__byte_perm(c, 0x4B000000u, 0x7442)) - 8388736.0f;
+        v[3] = __uint_as_float(__byte_perm(c, 0x4B000000u, 0x7443)) - 8388736.0f;
+    }
+};
+
+// Every warp walks keys of its own, four at a time, with a running maximum, sum and output in registers: sixteen lanes hold two keys, a
+// lane 8 dims of them for four heads. Nothing is shared until a group of keys is done, so an item has two block barriers where a tile
+// form (K and V tiles in shared memory, 64 keys between barriers) had four per 64 keys, and the next keys' rows are on their
+// way while these are worked on. The bound is the multiply-adds (1 024 per key for four heads, 512 lanes): ATTN_MEASURED
 template <int KV>
 __device__ __forceinline__ void attention_op(const TokCtx &c, const TokOp &op, uint32_t oi, uint32_t epoch, uint32_t heads,
                                           uint32_t kv_heads, uint32_t max_chunks, const float *cos_t, const float *sin_t,
                                           unsigned long long *partials, float attn_scale) {
-    constexpr int RB = KvRow<KV>::BYTES, RS = KvRow<KV>::STRIDE;
-    constexpr uint32_t C = KV == BRASA_KV_F32 ? 32 : 64;  // keys per work item
-    constexpr int KPW = C / TK_WARPS, LPK = 32 / KPW, DPL = 128 / LPK;  // keys per warp, lanes per key, dims per lane
-    // q in shared memory: 16-float segments 20 floats apart, so the lanes of a key (one segment or half segment each)
-    // read conflict-free
-    constexpr int QS_SEG = 20, QS_HEAD = 8 * QS_SEG;
+    constexpr int RB = KvRow<KV>::BYTES;
+    constexpr uint32_t C = KV == BRASA_KV_F32 ? 32 : 64;  // keys a group is cut by
+    constexpr bool AHEAD = KV != BRASA_KV_F32;            // the next keys' rows fit the registers
+    constexpr int QS_HEAD = 128;  // q of a head in shared memory: the first four values of every segment, then the other four
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t Gq = heads / kv_heads, pos = c.pos;
     const uint32_t lk = pos + 1, nchunks = (lk + C - 1) / C;
-    uint8_t *kt = c.xfb, *vt = c.xfb + C * RS;
-    float *qs = reinterpret_cast<float *>(vt + C * RS);  // [8][QS_HEAD]
-    float *ps = qs + 8 * QS_HEAD;                        // [8][C]
-    float *red = c.red;
-    // A work item is (kv head, group of consecutive chunks). While the chunks are few there is one chunk per group;
-    // a long cache has more chunks than the grid has blocks per kv head, and a block then walks its group's chunks with
-    // a running maximum and sum, so that a head is merged from a dozen partial results instead of hundreds.
+    float *osum = reinterpret_cast<float *>(c.xfb);               // [16 warps][4 heads][128]
+    float *wm = osum + TK_WARPS * 512, *wl = wm + TK_WARPS * 4;   // [16 warps][4 heads]: running maximum and sum
+    float *qs = wl + TK_WARPS * 4;                                // [8][QS_HEAD]
+    uint8_t *krow = reinterpret_cast<uint8_t *>(qs + 8 * QS_HEAD), *vrow = krow + 512;  // this token's rows, in the cache's type
+    const uint32_t kgrp = lane >> 4, seg = lane & 15;
+    // A work item is (kv head, group of consecutive chunks): a dozen or so partial results per head to merge, however long the cache
     const uint32_t groups_max = max(1u, c.G / kv_heads);
     const uint32_t cpg = (nchunks + groups_max - 1) / groups_max, ngroups = (nchunks + cpg - 1) / cpg;
     const uint32_t nitems = kv_heads * ngroups;
 #pragma unroll 1
     for (uint32_t item = c.b; item < nitems; item += c.G) {
         const uint32_t kh = item / ngroups, gi = item - kh * ngroups;
-        const uint32_t ch_lo = gi * cpg, ch_hi = min(nchunks, ch_lo + cpg);
-        float run[8][2];  // this thread's share (its key class) of an output element pair of every head
-#pragma unroll
-        for (int g = 0; g < 8; ++g) run[g][0] = run[g][1] = 0.0f;
-        if (tid < 8) { red[16 + tid] = -INFINITY; red[24 + tid] = 0.0f; }  // running maximum and sum per head
-        // The cached rows of chunk ch2 into a tile, one copy group per tile. K of the next chunk is asked for as soon as the
-        // scores of this one are out, V as soon as P V is done, so a block that walks several chunks (a long cache) waits
-        // for neither; groups complete in the order K(ch), V(ch), K(ch + 1), .., and every wait below leaves one pending.
-        auto load_tile = [&](uint8_t *tile, const uint8_t *cache, uint32_t ch2) {
-            if (ch2 < ch_hi) {
-                constexpr int VEC = KV == BRASA_KV_Q8_0 ? 8 : 16, PER_ROW = RB / VEC;
-                const uint32_t k0 = ch2 * C, nk = min(C, lk - k0), n = ch2 == nchunks - 1 ? nk - 1 : nk;  // the new row is not in the cache yet
+        const uint32_t k_lo = gi * cpg * C, k_hi = min(lk, k_lo + cpg * C);
+        const uint32_t cached = min(k_hi, pos);  // the new row is not in the cache yet
+        const uint8_t *kbase = op.kc + (size_t)kh * RB, *vbase = op.vc + (size_t)kh * RB;
+        const size_t pitch = (size_t)kv_heads * RB;
 #pragma unroll 1
-                for (uint32_t i = tid; i < n * PER_ROW; i += TK_THREADS) {
-                    const uint32_t r = i / PER_ROW, v = i % PER_ROW;
-                    const size_t goff = ((size_t)(k0 + r) * kv_heads + kh) * RB + (size_t)v * VEC;
-                    if (KV == BRASA_KV_Q8_0) cp_async8(tile + r * RS + v * VEC, cache + goff);
-                    else cp_async16(tile + r * RS + v * VEC, cache + goff);
+        for (uint32_t g0 = 0; g0 < Gq; g0 += 4) {
+            KvSeg<KV> kw[2]{}, vw[2]{};
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const uint32_t key = k_lo + 4 * warp + 2 * u + kgrp;
+                if (key < cached) {  // (does not wait for this token's q)
+                    kw[u].load(kbase + key * pitch, seg);
+                    vw[u].load(vbase + key * pitch, seg);
                 }
             }
-            asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        load_tile(kt, op.kc, ch_lo);
-        load_tile(vt, op.vc, ch_lo);
-#pragma unroll 1
-        for (uint32_t ch = ch_lo; ch < ch_hi; ++ch) {
-        const uint32_t key0 = ch * C, nkeys = min(C, lk - key0);
-        const bool has_new = ch == nchunks - 1;
-        if ((uint32_t)warp < Gq + 2 && (((uint32_t)warp < Gq && ch == ch_lo) || ((uint32_t)warp >= Gq && has_new))) {
-            // warps 0 .. Gq-1: a query head (once per item); warp Gq: the new key row; warp Gq + 1: the new value row
-            const uint32_t g = warp;
-            const uint32_t *src = op.in + c.par_cur + (g < Gq ? (size_t)(kh * Gq + g) * 128 : (size_t)(heads + (g - Gq) * kv_heads + kh) * 128);
-            float xv[4], y[4], wv[4], cs[2], sn[2];
-            {   // what does not depend on this token's q, k, v first: norm weight, cos and sin of this position
-                const float *nw = g < Gq ? op.q_norm : op.k_norm;
-                for (int j = 0; j < 4; ++j) wv[j] = nw[lane + 32 * j];
-                for (int j = 0; j < 2; ++j) {
-                    cs[j] = cos_t[(size_t)pos * 64 + lane + 32 * j];
-                    sn[j] = sin_t[(size_t)pos * 64 + lane + 32 * j];
+            if (g0 == 0 && ((uint32_t)warp < Gq || ((uint32_t)warp < Gq + 2 && k_hi == lk))) {
+                // warps 0 .. Gq-1: a query head (once per item); warp Gq: the new key row; warp Gq + 1: the new value row
+                const uint32_t g = warp;
+                const uint32_t *src = op.in + c.par_cur + (g < Gq ? (size_t)(kh * Gq + g) * 128 : (size_t)(heads + (g - Gq) * kv_heads + kh) * 128);
+                float xv[4], y[4], wv[4], cs[2], sn[2];
+                {   // what does not depend on this token's q, k, v first: norm weight, cos and sin of this position
+                    const float *nw = g < Gq ? op.q_norm : op.k_norm;
+                    for (int j = 0; j < 4; ++j) wv[j] = nw[lane + 32 * j];
+                    for (int j = 0; j < 2; ++j) {
+                        cs[j] = cos_t[(size_t)pos * 64 + lane + 32 * j];
+                        sn[j] = sin_t[(size_t)pos * 64 + lane + 32 * j];
+                    }
+                    uint32_t raw[4];
+                    vs_wait4(c, src + lane, src + lane + 32, src + lane + 64, src + lane + 96, raw);
+                    for (int j = 0; j < 4; ++j) xv[j] = __uint_as_float(raw[j]);
                 }
-                uint32_t raw[4];
-                vs_wait4(c, src + lane, src + lane + 32, src + lane + 64, src + lane + 96, raw);
-                for (int j = 0; j < 4; ++j) xv[j] = __uint_as_float(raw[j]);
+                if (g <= Gq) norm_rope_regs(xv, wv, cs, sn, op.eps, y);
+                if (g < Gq) {
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t e = lane + 32 * j;
+                        qs[g * QS_HEAD + ((e >> 2) & 1) * 64 + (e >> 3) * 4 + (e & 3)] = y[j];
+                    }
+                } else {
+                    const size_t grow = ((size_t)pos * kv_heads + kh) * RB;
+                    if (g == Gq) put_row<KV>(op.kc + grow, krow, y, lane);
+                    else put_row<KV>(op.vc + grow, vrow, xv, lane);
+                }
             }
-            if (g <= Gq) norm_rope_regs(xv, wv, cs, sn, op.eps, y);
-            if (g < Gq) {
-                for (int j = 0; j < 4; ++j) qs[g * QS_HEAD + ((lane + 32 * j) >> 4) * QS_SEG + ((lane + 32 * j) & 15)] = y[j];
-            } else {
-                const size_t grow = ((size_t)pos * kv_heads + kh) * RB;
-                if (g == Gq) put_row<KV>(op.kc + grow, kt + (nkeys - 1) * RS, y, lane);
-                else put_row<KV>(op.vc + grow, vt + (nkeys - 1) * RS, xv, lane);
-            }
-        }
-        TRACE(1);
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // K of this chunk
-        __syncthreads();
-        TRACE(2);
-        {   // scores: KPW keys per warp, LPK lanes share a key
-            const uint32_t key = warp * KPW + lane / LPK;
-            const int d0 = (lane % LPK) * DPL;
-            float kv[DPL];
-            const uint8_t *row = kt + min(key, nkeys - 1) * RS;
+            TRACE(1);
+            __syncthreads();
+            TRACE(2);
+            const float *q0 = qs + g0 * QS_HEAD + 4 * seg;
+            float acc[4][8];
 #pragma unroll
-            for (int d = 0; d < DPL; d += 8) tile_load8<KV>(row, d0 + d, kv + d);
+            for (int g = 0; g < 4; ++g)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) acc[g][i] = 0.0f;
+            float m = -INFINITY, l = 0.0f;  // of head g0 + (seg / 2) % 4, over this half warp's keys
 #pragma unroll 1
-            for (uint32_t g0 = 0; g0 < Gq; g0 += 4) {  // four heads side by side: four independent chains (qs has eight head slots)
-                float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            for (uint32_t k0 = k_lo + 4 * warp; k0 < k_hi; k0 += 4 * TK_WARPS) {
+                const uint32_t key0 = k0 + kgrp, next0 = key0 + 4 * TK_WARPS;  // this half warp's keys: key0, key0 + 2
+                KvSeg<KV> kn[2]{}, vn[2]{};
 #pragma unroll
-                for (int d = 0; d < DPL; d += 4) {
-#pragma unroll
-                    for (int gg = 0; gg < 4; ++gg) {
-                        const float4 qa = *reinterpret_cast<const float4 *>(qs + (g0 + gg) * QS_HEAD + (d0 >> 4) * QS_SEG + ((d0 + d) & 15));
-                        a[gg] = fmaf(qa.x, kv[d], a[gg]); a[gg] = fmaf(qa.y, kv[d + 1], a[gg]);
-                        a[gg] = fmaf(qa.z, kv[d + 2], a[gg]); a[gg] = fmaf(qa.w, kv[d + 3], a[gg]);
+                for (int u = 0; u < 2; ++u) {
+                    if (AHEAD && next0 + 2 * u < cached) {
+                        kn[u].load(kbase + (next0 + 2 * u) * pitch, seg);
+                        vn[u].load(vbase + (next0 + 2 * u) * pitch, seg);
+                    }
+                    if (key0 + 2 * u == pos && pos < k_hi) {
+                        kw[u].load_shared(krow, seg);
+                        vw[u].load_shared(vrow, seg);
                     }
                 }
-                for (int o = LPK / 2; o > 0; o >>= 1) {
+                float s[2][4] = {};
 #pragma unroll
-                    for (int gg = 0; gg < 4; ++gg) a[gg] += __shfl_xor_sync(0xffffffffu, a[gg], o);
-                }
-                if (lane % LPK == 0) {
+                for (int i = 0; i < 2; ++i) {
+                    float kf[2][4];
+                    kw[0].four(i, kf[0]);
+                    kw[1].four(i, kf[1]);
 #pragma unroll
-                    for (int gg = 0; gg < 4; ++gg)
-                        if (g0 + gg < Gq) ps[key * 8 + g0 + gg] = key < nkeys ? a[gg] * attn_scale : -INFINITY;
-                }
-            }
-        }
-        __syncthreads();
-        load_tile(kt, op.kc, ch + 1);
-        TRACE(3);
-        if ((uint32_t)warp < Gq) {  // softmax numerators of this chunk against the running maximum, head = warp; ps is [key][8 heads]
-            const uint32_t g = warp;
-            float v0 = ps[lane * 8 + g], v1 = C == 64 ? ps[(lane + 32) * 8 + g] : -INFINITY;
-            float m = fmaxf(v0, v1);
-            for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-            const float m_old = red[16 + g], m_new = fmaxf(m_old, m);
-            v0 = expf(v0 - m_new);
-            v1 = C == 64 ? expf(v1 - m_new) : 0.0f;
-            ps[lane * 8 + g] = v0;
-            if (C == 64) ps[(lane + 32) * 8 + g] = v1;
-            float l = v0 + v1;
-            for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-            if (lane == 0) {
-                const float keep = m_old == -INFINITY ? 0.0f : expf(m_old - m_new);  // what the earlier chunks still weigh
-                red[32 + g] = keep;
-                red[24 + g] = red[24 + g] * keep + l;
-                red[16 + g] = m_new;
-            }
-        }
-        asm volatile("cp.async.wait_group 1;" ::: "memory");  // V of this chunk (K of the next one may still be on its way)
-        __syncthreads();
-        TRACE(4);
-        {   // P V. Warp w owns output elements 8w .. 8w + 7 of every head; its lanes are 4 element pairs x 8 key classes
-            // (keys ks, ks + 8, ..): a value pair is read once for all heads, the key's probabilities come as one
-            // broadcast vector, and no two lanes of a load share a bank. The key classes meet at the end of the item.
-            const float *pt = ps;
-            const int d = warp * 8 + 2 * (lane & 3);
-            float acc[8][2];
+                    for (int g = 0; g < 4; ++g) {
+                        const float4 qa = *reinterpret_cast<const float4 *>(q0 + g * QS_HEAD + 64 * i);
 #pragma unroll
-            for (int g = 0; g < 8; ++g) acc[g][0] = acc[g][1] = 0.0f;
-#pragma unroll 2
-            for (uint32_t j = lane >> 2; j < nkeys; j += 8) {
-                const float2 v = tile_at2<KV>(vt + j * RS, d);
-                const float4 p0 = *reinterpret_cast<const float4 *>(pt + j * 8);
-                acc[0][0] = fmaf(p0.x, v.x, acc[0][0]); acc[0][1] = fmaf(p0.x, v.y, acc[0][1]);
-                acc[1][0] = fmaf(p0.y, v.x, acc[1][0]); acc[1][1] = fmaf(p0.y, v.y, acc[1][1]);
-                acc[2][0] = fmaf(p0.z, v.x, acc[2][0]); acc[2][1] = fmaf(p0.z, v.y, acc[2][1]);
-                acc[3][0] = fmaf(p0.w, v.x, acc[3][0]); acc[3][1] = fmaf(p0.w, v.y, acc[3][1]);
-                if (Gq > 4) {
-                    const float4 p1 = *reinterpret_cast<const float4 *>(pt + j * 8 + 4);
-                    acc[4][0] = fmaf(p1.x, v.x, acc[4][0]); acc[4][1] = fmaf(p1.x, v.y, acc[4][1]);
-                    acc[5][0] = fmaf(p1.y, v.x, acc[5][0]); acc[5][1] = fmaf(p1.y, v.y, acc[5][1]);
-                    acc[6][0] = fmaf(p1.z, v.x, acc[6][0]); acc[6][1] = fmaf(p1.z, v.y, acc[6][1]);
-                    acc[7][0] = fmaf(p1.w, v.x, acc[7][0]); acc[7][1] = fmaf(p1.w, v.y, acc[7][1]);
-                }
-            }
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                if ((uint32_t)g < Gq) {  // heads past Gq multiplied whatever lay in their column: never used
-                    const float keep = red[32 + g];
-                    run[g][0] = run[g][0] * keep + acc[g][0];
-                    run[g][1] = run[g][1] * keep + acc[g][1];
-                }
-            }
-        }
-        __syncthreads();
-        load_tile(vt, op.vc, ch + 1);
-        }  // chunks of the group
-        {   // the key classes of an output element meet (lanes 4 apart), lanes 0-3 of the warp send the element pair out
-            const uint32_t d = warp * 8 + 2 * (lane & 3);
-#pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                if ((uint32_t)g < Gq) {
-                    float r0 = run[g][0], r1 = run[g][1];
-                    for (int o = 4; o < 32; o <<= 1) {
-                        r0 += __shfl_xor_sync(0xffffffffu, r0, o);
-                        r1 += __shfl_xor_sync(0xffffffffu, r1, o);
-                    }
-                    if (lane < 4) {
-                        const uint32_t head = kh * Gq + g;
-                        if (ngroups == 1) {
-                            const float l = red[24 + g];
-                            uint32_t *o0 = op.out + (size_t)head * 128 + d;
-                            vs_store(o0 + c.par_cur, o0 + c.par_alt, __float_as_uint(r0 / l));
-                            vs_store(o0 + c.par_cur + 1, o0 + c.par_alt + 1, __float_as_uint(r1 / l));
-                        } else {
-                            unsigned long long *pp = partials + ((size_t)head * max_chunks + gi) * 130;
-                            ll_store(pp + 2 + d, __float_as_uint(r0), epoch);
-                            ll_store(pp + 3 + d, __float_as_uint(r1), epoch);
-                            if (d == 0) { ll_store(pp, __float_as_uint(red[16 + g]), epoch); ll_store(pp + 1, __float_as_uint(red[24 + g]), epoch); }
+                        for (int u = 0; u < 2; ++u) {
+                            s[u][g] = fmaf(qa.x, kf[u][0], s[u][g]); s[u][g] = fmaf(qa.y, kf[u][1], s[u][g]);
+                            s[u][g] = fmaf(qa.z, kf[u][2], s[u][g]); s[u][g] = fmaf(qa.w, kf[u][3], s[u][g]);
                         }
                     }
                 }
+                if (KV == BRASA_KV_Q8_0) {
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const float d = kw[u].scale();
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) s[u][g] *= d;
+                    }
+                }
+                // the sixteen lanes' shares meet: lane seg ends with key key0 + 2 (seg / 8), head (seg / 2) % 4 (each twice)
+                const uint32_t mu = seg >> 3;
+                float b[4];
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    b[g] = mu ? s[1][g] : s[0][g];
+                    b[g] += __shfl_xor_sync(0xffffffffu, mu ? s[0][g] : s[1][g], 8);
+                }
+                float a0 = (seg & 4) ? b[2] : b[0], a1 = (seg & 4) ? b[3] : b[1];
+                a0 += __shfl_xor_sync(0xffffffffu, (seg & 4) ? b[0] : b[2], 4);
+                a1 += __shfl_xor_sync(0xffffffffu, (seg & 4) ? b[1] : b[3], 4);
+                float sc = (seg & 2) ? a1 : a0;
+                sc += __shfl_xor_sync(0xffffffffu, (seg & 2) ? a0 : a1, 2);
+                sc += __shfl_xor_sync(0xffffffffu, sc, 1);
+                const bool seen = key0 + 2 * mu < k_hi;
+                sc = seen ? sc * attn_scale : -INFINITY;
+                const float mn = fmaxf(m, fmaxf(sc, __shfl_xor_sync(0xffffffffu, sc, 8)));
+                const float keep = m == -INFINITY ? 0.0f : expf(m - mn), pr = seen ? expf(sc - mn) : 0.0f;
+                const bool moved = mn != m;
+                l = l * keep + pr;
+                m = mn;
+                if (__any_sync(0xffffffffu, moved)) {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        const float kg = __shfl_sync(0xffffffffu, keep, (lane & 16) + 2 * g);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) acc[g][i] *= kg;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    float pg[4];
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        pg[g] = __shfl_sync(0xffffffffu, pr, (lane & 16) + 8 * u + 2 * g);
+                        if (KV == BRASA_KV_Q8_0) pg[g] *= vw[u].scale();
+                    }
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        float vf[4];
+                        vw[u].four(i, vf);
+#pragma unroll
+                        for (int g = 0; g < 4; ++g)
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) acc[g][4 * i + e] = fmaf(pg[g], vf[e], acc[g][4 * i + e]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    if (AHEAD) {
+                        kw[u] = kn[u];
+                        vw[u] = vn[u];
+                    } else if (next0 + 2 * u < cached) {
+                        kw[u].load(kbase + (next0 + 2 * u) * pitch, seg);
+                        vw[u].load(vbase + (next0 + 2 * u) * pitch, seg);
+                    }
+                }
             }
+            TRACE(3);
+            {   // the warp's halves meet: lane (kgrp, seg) ends with dims 8 seg .. of heads g0 + 2 kgrp and the next
+                l += __shfl_xor_sync(0xffffffffu, l, 8);
+                const float mw = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16)), f = m == -INFINITY ? 0.0f : expf(m - mw);
+                l *= f;
+                l += __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    const float fg = __shfl_sync(0xffffffffu, f, (lane & 16) + 2 * g);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) acc[g][i] *= fg;
+                }
+#pragma unroll
+                for (int g = 0; g < 2; ++g) {
+                    float4 *dst = reinterpret_cast<float4 *>(osum + (warp * 4 + 2 * kgrp + g) * 128 + 8 * seg);
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float mine = kgrp ? acc[2 + g][i] : acc[g][i];
+                        acc[g][i] = mine + __shfl_xor_sync(0xffffffffu, kgrp ? acc[g][i] : acc[2 + g][i], 16);
+                    }
+                    dst[0] = make_float4(acc[g][0], acc[g][1], acc[g][2], acc[g][3]);
+                    dst[1] = make_float4(acc[g][4], acc[g][5], acc[g][6], acc[g][7]);
+                }
+                if (kgrp == 0 && (seg & 9) == 0) {
+                    wm[warp * 4 + (seg >> 1)] = mw;
+                    wl[warp * 4 + (seg >> 1)] = l;
+                }
+            }
+            __syncthreads();
+            TRACE(4);
+            {   // the warps meet: thread = (head, dim)
+                const uint32_t hd = tid >> 7, d = tid & 127;
+                const float mw = wm[(lane & 15) * 4 + hd];
+                float M = mw;
+                for (int o = 8; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+                const float f = mw == -INFINITY ? 0.0f : expf(mw - M);
+                float L = wl[(lane & 15) * 4 + hd] * f;
+                for (int o = 8; o > 0; o >>= 1) L += __shfl_xor_sync(0xffffffffu, L, o);
+                float a = 0.0f;
+#pragma unroll
+                for (int w = 0; w < TK_WARPS; ++w) a = fmaf(osum[(w * 4 + hd) * 128 + d], __shfl_sync(0xffffffffu, f, w), a);
+                if (g0 + hd < Gq) {
+                    const uint32_t head = kh * Gq + g0 + hd;
+                    if (ngroups == 1) {
+                        uint32_t *o0 = op.out + (size_t)head * 128 + d;
+                        vs_store(o0 + c.par_cur, o0 + c.par_alt, __float_as_uint(a / L));
+                    } else {
+                        unsigned long long *pp = partials + ((size_t)head * max_chunks + gi) * 130;
+                        ll_store(pp + 2 + d, __float_as_uint(a), epoch);
+                        if (d == 0) { ll_store(pp, __float_as_uint(M), epoch); ll_store(pp + 1, __float_as_uint(L), epoch); }
+                    }
+                }
+            }
+            if (g0 + 4 < Gq || item + c.G < nitems) __syncthreads();  // the next pass writes the same shared memory
         }
-        __syncthreads();
     }
     TRACE(5);
     if (ngroups > 1) {
@@ -1031,7 +1110,6 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
 }
 
 uint32_t attn_chunk(int32_t kv) { return kv == BRASA_KV_F32 ? 32u : 64u; }
-uint32_t attn_row_stride(int32_t kv) { return kv == BRASA_KV_F32 ? 528u : (kv == BRASA_KV_F16 ? 272u : 144u); }
 
 // Column slices and active half blocks per lane for a GEMV of this width; false when the kernel does not take it.
 bool gemv_shape(int qtype, uint32_t cols, uint32_t *S_out, uint32_t *nact_out) {
@@ -1245,7 +1323,7 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
     p.block_ops = (const uint4 *)d_bops;
 
     // ---- shared memory ----
-    const size_t attn_bytes = (size_t)2 * C * attn_row_stride(m.kv) + (8 * 160 + 8 * C + 2 * max_chunks) * 4;
+    const size_t attn_bytes = (size_t)(TK_WARPS * (512 + 8) + 8 * 128) * 4 + 2 * 512;  // see attention_op
     p.xf_bytes = (uint32_t)((std::max<size_t>((size_t)max_cols / 16 * 16 * (m.kv == BRASA_KV_F32 ? XRec<3>::CHUNKS : XRec<2>::CHUNKS), attn_bytes) + 127) / 128 * 128);
     p.part_floats = (part_floats + 3) & ~3u;
     p.resid_floats = ((H + G - 1) / G + 4) & ~3u;
