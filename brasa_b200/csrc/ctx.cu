@@ -91,6 +91,7 @@ void brasa_ctx_destroy(brasa_ctx *ctx) {
     cudaFree(ctx->gemv_counters);
     cudaFree(ctx->argmax_scratch);
     cudaFree(ctx->gemm_part);
+    cudaFree(ctx->flash_part);
     cudaFree(ctx->kv_expand);
     cudaFree(ctx->gemm_counters);
     cudaFree(ctx->gemv_trace);

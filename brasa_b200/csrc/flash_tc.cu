@@ -13,8 +13,11 @@
 // (N = dim is contiguous), P as a K-major A operand (row = query, K = key).
 // Every wait is bounded; a wait that runs out raises the context's status word and the CTA leaves.
 #include <cuda.h>
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
+
+#include <algorithm>
 
 #include "attn_device.cuh"
 #include "brasa_internal.h"
@@ -60,6 +63,29 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t da, uint64_t db, 
         "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate)
         : "memory");
+}
+// the A operand out of tensor memory
+__device__ __forceinline__ void umma_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+// true in one lane of the (converged) warp
+__device__ __forceinline__ bool elect_one() {
+    uint32_t pred;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "elect.sync _|P, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(pred));
+    return pred != 0;
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t v[8]) {  // (the caller waits for its stores)
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]),
+                 "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -926,6 +952,432 @@ __global__ void __launch_bounds__(32 * (FLASH_SW + 1), 1) flash_tc_f16_kernel(co
     }
 }
 
+// Two query tiles of one KV head per CTA (two heads of its group over the same 128 queries, or, when the group is odd, one head's
+// tiles 2 i and 2 i + 1), so that K and V arrive once for both and the tensor core works for one tile while the other's
+// probabilities are formed. What bounds it: the tensor core, 3 products of 128^3 per tile of keys (5 with SPLITKV: 1 540 and 2 560
+// cycles), and beside it the 6 instructions a score costs. The one-tile kernel above wrote probabilities to shared memory, out of
+// which the tensor core read them back (a 128 x 128 product out of two shared operands alone fills its 128 bytes per clock),
+// and one block barrier per tile joined everyone: 4 700 (7 100) cycles a tile. Here
+//   * P is the A operand out of TENSOR memory, hi and lo over the columns S had: no shared memory written, none read for it;
+//   * two threads hold a row, 64 scores each, in registers: warps 0-7 tile A, 8-15 tile B (one thread per row, and 128 scores, took
+//     3 100 cycles from S to P, more than the 2 000 that the other tile keeps the tensor core busy). Warp 16 issues the products, warp
+//     17 the copies; every hand-over is a barrier of its own;
+//   * the issue order is P V of A, S of A's next keys, P V of B, S of B's next: S overwrites the columns of the P that the product
+//     before it read. K and V tiles (hi, lo) go through a ring of five 32 KB slots in the order in which they are needed: with
+//     SPLITKV four are in use at a time, and the fifth covers the copies because the lo terms are needed last;
+//   * the work is a line of items and key tiles, cut into one run per SM where that ends sooner (see the launch): 448 items over 148 SMs
+//     would leave 144 SMs idle for the last four. A run's parts of items go to a workspace and are merged by a dependent kernel.
+// Measured (32 query heads over 8; us, one-tile kernel in brackets): f16 cache, 1 024 queries behind 4 096 keys 132 (195), 3 584 behind 12 800
+// 1 122 (1 775), 3 584 behind none 179 (298); q8_0 cache 207 (285), 1 855 (2 540), 267 (414). Tensor pipe active 63 % (f16) and 68 % (q8_0) of
+// a busy SM's cycles at 1 024 queries before the row threads were doubled; what is left is the way from S to P of one tile (16 MUFU.EX2
+// lanes a clock: 1 024 cycles a tile) where the other tile's products are shorter.
+constexpr uint32_t FL2_SLOTS = 5;
+constexpr uint32_t FL2_START = 2;
+constexpr uint32_t FL2_TILE = 128 * 128 + 2 * 128;  // floats of one query tile's partial result: O [dims / 4][row][4], then m and l by row
+
+struct FlashTwoParams {
+    FlashTcParams a;
+    uint32_t pairs, nq;     // items: query tiles (pairs of tiles) x pairs of heads (heads)
+    uint32_t units, whole;  // length of the line below; whole: run b is item b
+    float *part;            // [2 x runs][2 tiles][FL2_TILE]: slot 2 b is run b's item that began before it, 2 b + 1 the one it leaves open
+};
+
+// The launch's work in a line: items (one KV head, two query tiles) from the longest to the shortest, each as FL2_START units for its set-up
+// (Q, the first copies, the output: about as long as that many key tiles) and one per key tile. Runs are equal pieces of the line; a cut
+// among an item's set-up units is a cut before its first key tile.
+struct FlashPlace {
+    uint32_t q, pair, nkt, first, j;  // query tile (pair of tiles), pair of heads (head), the item's key tiles, its first unit, key tile
+};
+__device__ __forceinline__ uint32_t flash_item_tiles(const FlashTwoParams &p, uint32_t q) {
+    const uint32_t span = p.a.hq / p.a.hkv % 2 == 0 ? 128 : 256;
+    return (p.a.pos0 + min(span * (q + 1), p.a.tokens) - 1) / 128 + 1;
+}
+__device__ __forceinline__ FlashPlace flash_run_begin(const FlashTwoParams &p, uint32_t b, uint32_t runs) {
+    FlashPlace f{};
+    if (p.whole) {
+        f.q = p.nq - 1 - b / p.pairs;
+        f.pair = b % p.pairs;
+        f.nkt = flash_item_tiles(p, f.q);
+        f.first = b;
+        return f;
+    }
+    const uint32_t unit = (uint32_t)((uint64_t)b * p.units / runs);
+    f.q = p.nq - 1;
+    f.nkt = flash_item_tiles(p, f.q);
+    while (f.q > 0 && unit >= f.first + (f.nkt + FL2_START) * p.pairs) {
+        f.first += (f.nkt + FL2_START) * p.pairs;
+        f.nkt = flash_item_tiles(p, --f.q);
+    }
+    f.pair = (unit - f.first) / (f.nkt + FL2_START);  // (p.pairs behind the last item: nothing begins there)
+    f.first += f.pair * (f.nkt + FL2_START);
+    f.j = unit - f.first > FL2_START ? unit - f.first - FL2_START : 0u;
+    return f;
+}
+
+template <bool SPLITKV>
+__global__ void __launch_bounds__(576, 1) flash_tc_two_kernel(const __grid_constant__ FlashF16Maps maps, const __grid_constant__ FlashTwoParams fp) {
+    const FlashTcParams &p = fp.a;
+    constexpr uint32_t NL = SPLITKV ? 4 : 2, VL = NL / 2;  // loads per key tile: K (hi, lo), V (hi, lo); V's first
+    extern __shared__ __align__(1024) uint8_t smem_raw[];
+    uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
+    uint8_t *ring = smem + 2 * TILE_BYTES;
+    __shared__ uint64_t full[FL2_SLOTS], freed[FL2_SLOTS], s_ready[2], p_ready[2], o_done[2];
+    __shared__ uint32_t tmem_base_s, abort_s;
+    __shared__ __half pair[2][2][128];  // [tile][half of the keys][row]: largest score (f16: a reference need only be the same for the row's threads)
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const uint32_t group = p.hq / p.hkv;
+    const bool heads = group % 2 == 0;
+
+    if (tid == 0) {
+        for (uint32_t i = 0; i < FL2_SLOTS; ++i) {
+            mbar_init(&full[i], 1);
+            mbar_init(&freed[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&s_ready[i], 1);
+            mbar_init(&p_ready[i], 8);  // one arrival per softmax warp
+            mbar_init(&o_done[i], 1);
+        }
+        abort_s = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 16) {  // tensor memory: S (then, per 64 keys, P hi and P lo) of A in [0, 128), of B in [128, 256); O of A in [256, 384), of B in [384, 512)
+        const uint32_t ncols = 512;
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(ncols) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    // launched as a programmatic dependent: what the kernels before this one wrote (q, the cache) is touched after the wait
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t tmem = tmem_base_s;
+    volatile uint32_t *abort_flag = &abort_s;
+    auto wait = [&](uint64_t *bar, uint32_t parity) -> bool {
+        for (uint32_t it = 0; it < FA_WAIT_LIMIT; ++it) {
+            if (fa_mbar_try(bar, parity)) return true;
+            if (*abort_flag) return false;
+        }
+        atomicExch(p.status, 5u);
+        *abort_flag = 1;
+        return false;
+    };
+
+    // ---- the run: items and parts of items; barrier phases and ring slots go on from one to the next ----
+    FlashPlace item = flash_run_begin(fp, blockIdx.x, gridDim.x);
+    uint32_t end_first = item.first + 1, end_j = 0;
+    if (!fp.whole) {
+        const FlashPlace e = flash_run_begin(fp, blockIdx.x + 1, gridDim.x);
+        end_first = e.first;
+        end_j = e.j;
+    }
+    uint32_t it0 = 0, seg = 0;  // key tiles, items begun so far
+#pragma unroll 1
+    while (item.first < end_first || (item.first == end_first && item.j < end_j)) {
+        const uint32_t j0 = item.j, j1 = item.first == end_first ? end_j : item.nkt, len = j1 - j0;
+        auto head_of = [&](uint32_t x) { return heads ? 2 * item.pair + x : item.pair; };
+        auto query_of = [&](uint32_t x) { return heads ? 128 * item.q : 128 * (2 * item.q + x); };
+        const uint32_t kh = head_of(0) / group;
+        // K and V tiles: rows [128 j, 128 j + 128) of this KV head, two boxes of 64 dims each; load n of the run goes to slot n % 5
+        uint32_t n = it0 * NL;
+        const uint32_t n_end = (it0 + len) * NL;
+        auto load = [&]() -> bool {
+            const uint32_t s = n % FL2_SLOTS, i = n % NL, j = j0 + n / NL - it0;
+            if (n >= FL2_SLOTS && !wait(&freed[s], ((n / FL2_SLOTS) - 1) & 1)) return false;
+            const CUtensorMap *map = i == 0 ? &maps.k : (i == VL ? &maps.v : (i == 1 ? &maps.klo : &maps.vlo));
+            mbar_expect_tx(&full[s], TILE_BYTES);
+#pragma unroll
+            for (int half = 0; half < 2; ++half)
+                asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                                 smem_u32(ring + (size_t)s * TILE_BYTES + half * 16384)),
+                             "l"(map), "r"(half * 64), "r"((int)kh), "r"((int)(j * 128)), "r"(smem_u32(&full[s]))
+                             : "memory");
+            ++n;
+            return true;
+        };
+        if (warp == 17) {  // (every slot is free here: the item before has used them all up)
+            if (lane == 0)
+                for (uint32_t k = 0; k < FL2_SLOTS && n < n_end && load(); ++k) {}
+        } else if (warp < 16) {
+            // Q tiles: scale, round to f16, swizzled K-major; rows past the last query are zeros
+#pragma unroll 1
+            for (uint32_t i0 = tid; i0 < 2 * 128 * 16; i0 += 4 * 512) {
+                float4 v[4][2];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t i = i0 + 512 * k, x = i >> 11, qq = query_of(x) + ((i >> 4) & 127);
+                    v[k][0] = v[k][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if (qq < p.tokens) {
+                        const float4 *src = reinterpret_cast<const float4 *>(p.q + ((size_t)qq * p.hq + head_of(x)) * 128 + (i & 15) * 8);
+                        v[k][0] = src[0];
+                        v[k][1] = src[1];
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint32_t i = i0 + 512 * k;
+                    const float4 a = v[k][0], b = v[k][1];
+                    const __half2 h0 = __floats2half2_rn(a.x * p.scale, a.y * p.scale), h1 = __floats2half2_rn(a.z * p.scale, a.w * p.scale);
+                    const __half2 h2 = __floats2half2_rn(b.x * p.scale, b.y * p.scale), h3 = __floats2half2_rn(b.z * p.scale, b.w * p.scale);
+                    *reinterpret_cast<uint4 *>(smem + (i >> 11) * TILE_BYTES + tile_chunk((i >> 4) & 127, (i & 15) * 8)) =
+                        make_uint4(*reinterpret_cast<const uint32_t *>(&h0), *reinterpret_cast<const uint32_t *>(&h1), *reinterpret_cast<const uint32_t *>(&h2),
+                                   *reinterpret_cast<const uint32_t *>(&h3));
+                }
+            }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncthreads();
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+
+        if (warp == 17) {
+            if (lane == 0) {  // ---- the other copies ----
+                while (n < n_end && load()) {}
+                if (*abort_flag) {  // leaving early: let the copies in flight land before the CTA's shared memory is handed on
+                    for (uint32_t k = n > FL2_SLOTS ? n - FL2_SLOTS : 0; k < n; ++k)
+                        for (uint32_t it = 0; it < FA_WAIT_LIMIT && !fa_mbar_try(&full[k % FL2_SLOTS], (k / FL2_SLOTS) & 1); ++it) {}
+                }
+            }
+        } else if (warp == 16) {  // ---- products: the warp waits, one lane issues ----
+            const uint32_t idesc_s = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+            const uint32_t idesc_o = idesc_s | (1u << 16);  // V is an MN-major B operand
+            auto all_wait = [&](uint64_t *bar, uint32_t parity) { return __all_sync(0xffffffffu, wait(bar, parity)) != 0; };
+            auto landed = [&](uint32_t m) { return all_wait(&full[m % FL2_SLOTS], (m / FL2_SLOTS) & 1); };
+            auto slot = [&](uint32_t m) { return smem_u32(ring + (size_t)(m % FL2_SLOTS) * TILE_BYTES); };
+            bool ok = true;
+            for (uint32_t j = 0; j <= len && ok; ++j) {
+#pragma unroll
+                for (uint32_t x = 0; x < 2; ++x) {
+                    if (j > 0) {  // O += P V of the tile before
+                        const uint32_t m = (it0 + j - 1) * NL + VL;
+                        const uint32_t o = tmem + 256 + 128 * x, ph = tmem + 128 * x;
+                        ok = ok && all_wait(&p_ready[x], (it0 + j - 1) & 1) && landed(m);
+                        if (!ok) break;
+                        if (elect_one()) {
+                            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                            const uint32_t v = slot(m);
+#pragma unroll
+                            for (uint32_t ks = 0; ks < 8; ++ks) {  // 64 keys: 32 columns of P hi, 32 of P lo
+                                const uint32_t a = ph + 64 * (ks >> 2) + 8 * (ks & 3);
+                                umma_ta(o, a, desc_mnmajor(v + ks * 2048), idesc_o, (j > 1 || ks > 0) ? 1u : 0u);
+                                umma_ta(o, a + 32, desc_mnmajor(v + ks * 2048), idesc_o, 1u);
+                            }
+                            if (x == 1) umma_commit(&freed[m % FL2_SLOTS]);
+                        }
+                        __syncwarp();
+                        if (SPLITKV && !(ok = landed(m + 1))) break;
+                        if (elect_one()) {
+                            if (SPLITKV) {  // lo x lo is below 2^-22
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                const uint32_t v = slot(m + 1);
+#pragma unroll
+                                for (uint32_t ks = 0; ks < 8; ++ks) umma_ta(o, ph + 64 * (ks >> 2) + 8 * (ks & 3), desc_mnmajor(v + ks * 2048), idesc_o, 1u);
+                            }
+                            if (SPLITKV && x == 1) umma_commit(&freed[(m + 1) % FL2_SLOTS]);
+                            if (j == len) umma_commit(&o_done[x]);
+                        }
+                        __syncwarp();
+                    }
+                    if (j < len) {  // S = Q K^T of this tile, over the columns of the P just read
+                        const uint32_t m = (it0 + j) * NL, q = smem_u32(smem + x * TILE_BYTES);
+#pragma unroll
+                        for (uint32_t t = 0; t < VL; ++t) {  // K hi, K lo
+                            if (!(ok = landed(m + t))) break;
+                            if (elect_one()) {
+                                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                                const uint32_t k = slot(m + t);
+#pragma unroll
+                                for (uint32_t ks = 0; ks < 8; ++ks) {
+                                    const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
+                                    umma(tmem + 128 * x, desc_kmajor(q + off), desc_kmajor(k + off), idesc_s, (t > 0 || ks > 0) ? 1u : 0u);
+                                }
+                                if (x == 1) umma_commit(&freed[(m + t) % FL2_SLOTS]);
+                                if (t + 1 == VL) umma_commit(&s_ready[x]);
+                            }
+                            __syncwarp();
+                        }
+                        if (!ok) break;
+                    }
+                }
+            }
+        } else {  // ---- softmax: two threads per query row, 64 keys of every tile each ----
+            constexpr float LOG2E = 1.4426950408889634f;
+            const uint32_t x = warp >> 3, h = (warp >> 2) & 1, row = (warp & 3) * 32 + lane, q0 = query_of(x), qpos = p.pos0 + q0 + row;
+            const uint32_t nfree = (p.pos0 + q0 + 1) / 128;  // tiles [0, nfree) lie wholly at or below every row's own position
+            const uint32_t trow = ((warp & 3) * 32u) << 16, ts = tmem + 128 * x + 64 * h + trow, to = tmem + 256 + 128 * x + 64 * h + trow;
+            const uint32_t both = 1 + 4 * x + (warp & 3);  // named barrier of the two warps that hold these rows
+            float m = -INFINITY, mneg = 0.0f, l0 = 0.0f, l1 = 0.0f;
+            bool ok = true;
+            for (uint32_t j = j0; j < j1; ++j) {
+                ok = wait(&s_ready[x], (it0 + j - j0) & 1);  // S of this tile, and with it every product issued before: P V of the tile before
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                uint32_t v[2][32];
+                tmem_ld32(ts, v[0]);
+                tmem_ld32(ts + 32, v[1]);
+                if (j >= nfree) {
+                    const int seen = (int)qpos + 1 - (int)(j * 128 + 64 * h);  // of this thread's keys, those the row sees
+#pragma unroll
+                    for (int i = 0; i < 64; ++i)
+                        if (i >= seen) v[i >> 5][i & 31] = 0xff800000u;  // -inf: exp2 gives 0
+                }
+                float t[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                for (int i = 0; i < 64; ++i) t[i & 3] = fmaxf(t[i & 3], __uint_as_float(v[i >> 5][i & 31]));
+                float tmax = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
+                pair[x][h][row] = __float2half_rn(tmax);
+                asm volatile("bar.sync %0, 64;" ::"r"(both) : "memory");
+                tmax = fmaxf(__half2float(pair[x][0][row]), __half2float(pair[x][1][row]));
+                float rescale = 1.0f;
+                bool move = false;
+                if (tmax > m + ONEPASS_SLACK || (m == -INFINITY && tmax != -INFINITY)) {
+                    move = m != -INFINITY;
+                    rescale = move ? ex2_approx((m - tmax) * LOG2E) : 1.0f;
+                    l0 *= rescale;
+                    l1 *= rescale;
+                    m = tmax;
+                    mneg = -m * LOG2E;
+                }
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {  // 16 keys: 8 columns of P hi, 8 of P lo (all of this thread's scores are in registers by now)
+                    uint32_t hi[8], lo[8];
+#pragma unroll
+                    for (int i = 0; i < 16; i += 2) {
+                        const int k = 16 * c + i;
+                        const float p0 = ex2_approx(fmaf(__uint_as_float(v[k >> 5][k & 31]), LOG2E, mneg));
+                        const float p1 = ex2_approx(fmaf(__uint_as_float(v[k >> 5][(k & 31) + 1]), LOG2E, mneg));
+                        l0 += p0;
+                        l1 += p1;
+                        split_pair(p0, p1, hi[i >> 1], lo[i >> 1]);
+                    }
+                    tmem_st8(ts + 8 * c, hi);
+                    tmem_st8(ts + 32 + 8 * c, lo);
+                }
+                if (__any_sync(0xffffffffu, move)) {  // what O holds for the row was accumulated against the old reference
+#pragma unroll 1
+                    for (uint32_t c = 0; c < 64; c += 32) {
+                        uint32_t o[32];
+                        tmem_ld32(to + c, o);
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
+                        tmem_st32(to + c, o);
+                    }
+                }
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&p_ready[x])) : "memory");
+            }
+            // ---- output: O / l, rounded to f16; a part of the item's keys: O, m and l as they are ----
+            ok = ok && wait(&o_done[x], seg & 1);
+            ok = __all_sync(0xffffffffu, ok);
+            float *sums = reinterpret_cast<float *>(smem + x * TILE_BYTES);  // [half][row], over the Q tile: its products are done
+            if (ok) sums[h * 128 + row] = l0 + l1;
+            asm volatile("bar.sync %0, 64;" ::"r"(both) : "memory");
+            if (ok && len < item.nkt) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                float *dst = fp.part + ((size_t)(2 * blockIdx.x + (j0 == 0)) * 2 + x) * FL2_TILE;
+                if (h == 0) {
+                    dst[128 * 128 + row] = m;
+                    dst[128 * 128 + 128 + row] = sums[row] + sums[128 + row];
+                }
+#pragma unroll 1
+                for (uint32_t c = 0; c < 2; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(to + 32 * c, o);
+#pragma unroll
+                    for (int g = 0; g < 8; ++g)
+                        reinterpret_cast<uint4 *>(dst)[(16 * h + 8 * c + g) * 128 + row] = make_uint4(o[4 * g], o[4 * g + 1], o[4 * g + 2], o[4 * g + 3]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            } else if (ok) {
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const float inv = 1.0f / (sums[row] + sums[128 + row]);
+                const bool live = q0 + row < p.tokens;
+                uint4 *dst = reinterpret_cast<uint4 *>(p.o + ((size_t)(q0 + row) * p.hq + head_of(x)) * 128 + 64 * h);
+#pragma unroll 1
+                for (uint32_t c = 0; c < 2; ++c) {
+                    uint32_t o[32];
+                    tmem_ld32(to + 32 * c, o);
+                    uint32_t packed[16];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        const __half2 hh = __floats2half2_rn(__uint_as_float(o[i]) * inv, __uint_as_float(o[i + 1]) * inv);
+                        packed[i >> 1] = *reinterpret_cast<const uint32_t *>(&hh);
+                    }
+#pragma unroll
+                    for (int g = 0; g < 4; ++g)
+                        if (live) dst[4 * c + g] = make_uint4(packed[4 * g], packed[4 * g + 1], packed[4 * g + 2], packed[4 * g + 3]);
+                }
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            }
+        }
+        it0 += len;
+        ++seg;
+        if (item.first < end_first) {
+            item.first += fp.whole ? 1u : item.nkt + FL2_START;
+            item.j = 0;
+            if (++item.pair == fp.pairs) {
+                item.pair = 0;
+                item.nkt = item.q > 0 ? flash_item_tiles(fp, --item.q) : 0u;
+            }
+        } else {
+            item.j = j1;
+        }
+        if (__syncthreads_or(*abort_flag)) break;  // Q, the row sums and O are free again
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 16) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t ncols = 512;
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(ncols) : "memory");
+    }
+}
+
+// The items that several runs worked on: block (i, y) takes the one that run i + 1 goes on with, when that run is the first to do so, and
+// of it 32 rows of one query tile. out = f16(sum of exp(m - M) O / sum of exp(m - M) l) over the parts, in key order.
+__global__ void __launch_bounds__(256) flash_tc_merge_kernel(const __grid_constant__ FlashTwoParams fp, uint32_t runs) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const uint32_t b = blockIdx.x + 1;
+    const FlashPlace item = flash_run_begin(fp, b, runs), before = flash_run_begin(fp, b - 1, runs);
+    if (item.j == 0 || (before.first == item.first && before.j > 0)) return;
+    uint32_t end = b;  // runs [b - 1, end) hold parts of the item
+    for (FlashPlace e = item; e.first == item.first && e.j < item.nkt && end < runs;) e = flash_run_begin(fp, ++end, runs);
+    const uint32_t x = blockIdx.y >> 2, row = (blockIdx.y & 3) * 32 + (threadIdx.x & 31), group = fp.a.hq / fp.a.hkv;
+    const uint32_t head = group % 2 == 0 ? 2 * item.pair + x : item.pair, q = (group % 2 == 0 ? 128 * item.q : 128 * (2 * item.q + x)) + row;
+    auto part = [&](uint32_t z) { return fp.part + ((size_t)(z < b ? 2 * z + 1 : 2 * z) * 2 + x) * FL2_TILE; };
+    float M = -INFINITY, l = 0.0f;
+    for (uint32_t z = b - 1; z < end; ++z) M = fmaxf(M, __ldcg(part(z) + 128 * 128 + row));
+    float4 o[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t z = b - 1; z < end; ++z) {
+        const float *src = part(z);
+        const float m = __ldcg(src + 128 * 128 + row), w = m == -INFINITY ? 0.0f : expf(m - M);
+        l = fmaf(w, __ldcg(src + 128 * 128 + 128 + row), l);
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(src) + ((threadIdx.x >> 5) + 8 * k) * 128 + row);
+            o[k].x = fmaf(w, v.x, o[k].x);
+            o[k].y = fmaf(w, v.y, o[k].y);
+            o[k].z = fmaf(w, v.z, o[k].z);
+            o[k].w = fmaf(w, v.w, o[k].w);
+        }
+    }
+    if (q >= fp.a.tokens) return;
+    const float inv = 1.0f / l;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const __half2 lo = __floats2half2_rn(o[k].x * inv, o[k].y * inv), hi = __floats2half2_rn(o[k].z * inv, o[k].w * inv);
+        *reinterpret_cast<uint2 *>(fp.a.o + ((size_t)q * fp.a.hq + head) * 128 + 4 * ((threadIdx.x >> 5) + 8 * k)) =
+            make_uint2(*reinterpret_cast<const uint32_t *>(&lo), *reinterpret_cast<const uint32_t *>(&hi));
+    }
+}
+
 }  // namespace
 
 // F16 prefill precision over a cache of type kv; q, k, v, o as for brasa_k_flash_attention_with (already validated there).
@@ -984,15 +1436,57 @@ int32_t brasa_flash_tc_launch(brasa_cmd *cmd, int32_t kv, const float *q, const 
         CUresult r1 = enc(&maps.k, kh), r2 = enc(&maps.v, vh), r3 = split ? enc(&maps.klo, kl) : CUDA_SUCCESS, r4 = split ? enc(&maps.vlo, vl) : CUDA_SUCCESS;
         if (r1 != CUDA_SUCCESS || r2 != CUDA_SUCCESS || r3 != CUDA_SUCCESS || r4 != CUDA_SUCCESS)
             return brasa_fail(ctx, BRASA_ECUDA, "cuTensorMapEncodeTiled failed for the KV cache (%d, %d, %d, %d)", (int)r1, (int)r2, (int)r3, (int)r4);
-        const size_t smem = 7 * TILE_BYTES + 1024;
-        if (split) {
-            BRASA_TRY(brasa_smem_optin(ctx, (const void *)flash_tc_f16_kernel<true>, smem));
-            flash_tc_f16_kernel<true><<<grid, 32 * (FLASH_SW + 1), smem, ctx->stream>>>(maps, p);
-        } else {
-            BRASA_TRY(brasa_smem_optin(ctx, (const void *)flash_tc_f16_kernel<false>, smem));
-            flash_tc_f16_kernel<false><<<grid, 32 * (FLASH_SW + 1), smem, ctx->stream>>>(maps, p);
+        FlashTwoParams fp{p, 0, 0, 0, 0, nullptr};
+        const bool by_heads = sh.hq / sh.hkv % 2 == 0;
+        fp.pairs = by_heads ? sh.hq / 2 : sh.hq;
+        fp.nq = by_heads ? (sh.tokens + 127) / 128 : (sh.tokens + 255) / 256;
+        uint64_t units = 0;
+        uint32_t longest = 0, shortest = 0;
+        for (uint32_t i = 0; i < fp.nq; ++i) {
+            longest = (sh.pos0 + std::min((by_heads ? 128u : 256u) * (i + 1), sh.tokens) - 1) / 128 + 1;
+            if (i == 0) shortest = longest;
+            units += (uint64_t)fp.pairs * (longest + FL2_START);
         }
-        return brasa_post_launch(cmd, "flash_tc_f16");
+        // An item per block, handed out as blocks end, or equal runs of the line: which is shorter, in key tiles. Blocks that end apart leave
+        // up to the shortest item's time idle in the last wave; a run begins and ends inside items, which costs the parts' way through
+        // memory, the merge (6 tiles' time) and another set-up per item. 3 584 queries behind 12 800 keys (448 items on 148 SMs): 1 371 us
+        // whole, 1 122 cut; behind none 179 and 221; 1 024 behind none 39 and 46; 100 behind 1 024 40 and 30; 512 behind 2 048 74 and 54.
+        const double sms = ctx->sm_count, items = (double)fp.pairs * fp.nq, each = units / sms, waves = items / sms;
+        const double whole = waves <= 1.0 ? longest + FL2_START : each + (shortest + FL2_START) * (1.0 - (waves - floor(waves)));
+        const bool cut = units < (1ull << 31) && each + 6.0 + FL2_START * (waves + 1.0) < whole;
+        // short prompts whose one-tile CTAs fit the SMs at once: 512 queries behind none 23.5 us, 26.3 in pairs of tiles
+        const bool one_tile = !cut && grid.x * grid.y <= (uint32_t)ctx->sm_count;
+        if (one_tile) {
+            const size_t smem = 7 * TILE_BYTES + 1024;
+            auto kernel = split ? flash_tc_f16_kernel<true> : flash_tc_f16_kernel<false>;
+            BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernel, smem));
+            kernel<<<grid, 32 * (FLASH_SW + 1), smem, ctx->stream>>>(maps, p);
+            return brasa_post_launch(cmd, "flash_tc_f16");
+        }
+        fp.units = (uint32_t)units;
+        uint32_t runs = std::min<uint32_t>((uint32_t)ctx->sm_count, std::max(1u, fp.units / 2));
+        const size_t need = (size_t)runs * 4 * FL2_TILE * sizeof(float);
+        if (cut && ctx->flash_part_bytes < need && !ctx->capturing) {
+            BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+            if (ctx->flash_part) cudaFree(ctx->flash_part);
+            ctx->flash_part = nullptr;
+            ctx->flash_part_bytes = 0;
+            if (cudaMalloc((void **)&ctx->flash_part, need) == cudaSuccess) ctx->flash_part_bytes = need;
+            else cudaGetLastError();
+        }
+        if (cut && ctx->flash_part_bytes >= need) fp.part = ctx->flash_part;
+        else {  // (or no workspace: a graph is being recorded, no memory is left)
+            fp.whole = 1;
+            runs = fp.pairs * fp.nq;
+        }
+        const size_t smem = (2 + FL2_SLOTS) * TILE_BYTES + 1024;
+        auto kernel = split ? flash_tc_two_kernel<true> : flash_tc_two_kernel<false>;
+        BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernel, smem));
+        BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernel, dim3(runs), dim3(576), smem, maps, fp));
+        BRASA_TRY(brasa_post_launch(cmd, "flash_tc_two"));
+        if (fp.whole || runs == 1) return BRASA_OK;
+        BRASA_CUDA(ctx, brasa_launch_dependent(ctx, flash_tc_merge_kernel, dim3(runs - 1, 8), dim3(256), 0, fp, runs));
+        return brasa_post_launch(cmd, "flash_tc_merge");
     }
 #define LAUNCH_FTC(KVT, TILES)                                                                                              \
     do {                                                                                                                   \

@@ -703,6 +703,27 @@ def test_gemm_cta_pairs(B, ctx, K, rows, cols, tokens):
 
 
 @pytest.mark.parametrize("kv", ["F16", "Q8_0"])
+@pytest.mark.parametrize("hq,hkv,tokens,pos0", [(8, 2, 130, 3000), (3, 1, 300, 2100), (5, 5, 1, 1400), (32, 8, 700, 0), (32, 32, 333, 50), (6, 2, 257, 1000), (2, 1, 40, 5000)])
+def test_flash_attention_query_tile_pairs(B, ctx, K, kv, hq, hkv, tokens, pos0):
+    """The attention that takes two query tiles at once: two heads of a group or, in groups of odd size, one head's neighbouring tiles (the
+    last without a neighbour); an item per block, and runs that cut items at any key tile, among them parts in which a row sees no key
+    at all, items shared by many runs and runs that hold several items. Bound of the reference's attention test."""
+    rng = O.Rng(tokens + pos0)
+    dim, lk = 128, pos0 + tokens
+    cap = (lk + 63) // 64 * 64
+    q = rng.vec(tokens * hq * dim, 2.0)
+    kvt = getattr(B.KvType, kv)
+    gk, gv, k, v = make_cache(B, ctx, kvt, rng.vec(cap * hkv * dim, 2.0), rng.vec(cap * hkv * dim, 3.0))
+    want16, vmax = O.attention(q, k, v, tokens, hq, hkv, dim, pos0, q16=True)
+    gq, goh = ctx.buffer_from(q), ctx.buffer(q.size * 2)
+    goh.fill(0xFF)
+    run(ctx, lambda c: K.flash_attention(c, gq, gk, gv, goh, B.AttnShape(tokens, hq, hkv, dim, pos0, kvt)))
+    oh = goh.download(np.float16).astype(np.float32)
+    d = np.maximum(np.abs(oh - want16) - np.abs(want16) * 2.0 ** -11, 0.0)  # the output's own f16 rounding is discounted
+    assert float(np.max(d / np.maximum(vmax, 1e-30))) <= 1e-5
+
+
+@pytest.mark.parametrize("kv", ["F16", "Q8_0"])
 @pytest.mark.parametrize("tokens,pos0", [(512, 0), (300, 77), (129, 255), (200, 1500)])
 def test_flash_attention_tensor_core_many_query_tiles(B, ctx, K, tokens, pos0, kv):
     """The tcgen05 prefill attention (F16 precision over an f16 cache, and over a q8_0 cache expanded to hi + lo f16
