@@ -49,7 +49,7 @@ enum { EPI_SCALE = 0, EPI_SWIGLU = 1, EPI_RESID = 2, EPI_LOGITS = 3 };
 struct SlotDesc {
     const uint8_t *src;
     uint32_t bytes;
-    uint32_t pad;
+    uint32_t part;  // 0: the bytes as they lie; else columns of a half row | rows << 16 | half << 24 (see issue_slot)
 };
 
 struct TokOp {
@@ -60,7 +60,7 @@ struct TokOp {
     float eps;
     uint32_t xchg;  // tensor parallel: 1 + index of this residual add among the token's exchanges (0: no exchange)
     uint32_t fast;  // every lane's half blocks before its last iteration lie inside the row (see gemv_rows)
-    uint32_t pad1[1];
+    uint32_t halves;  // 2: rows too wide for a slot and a lane's registers, taken as two halves of `cols` columns one after the other
     const uint8_t *w[3];
     const float *normw;
     const uint32_t *in;  // first copy; the second one lies TokParams::par_words further
@@ -272,11 +272,22 @@ __device__ __forceinline__ bool slot_wait(const TokCtx &c, uint64_t *bar, uint32
     return false;
 }
 
-// a slot descriptor {address lo, address hi, bytes, -} -> ring[s]
+// a slot descriptor {address lo, address hi, bytes, part} -> ring[s]
 __device__ __forceinline__ void issue_slot(const TokCtx &c, uint4 d, uint32_t s) {
     const uint8_t *src = reinterpret_cast<const uint8_t *>(((unsigned long long)d.y << 32) | d.x);
+    uint8_t *dst = c.ring + (size_t)s * SLOT_CAP;
     mbar_expect_tx(&c.full[s], d.z);
-    bulk_g2s(c.ring + (size_t)s * SLOT_CAP, src, d.z, &c.full[s]);
+    if (d.w == 0) {
+        bulk_g2s(dst, src, d.z, &c.full[s]);
+        return;
+    }
+    // half rows: a row's codes and scales of these columns, laid together as a row of that many columns is
+    const uint32_t cols = d.w & 0xffffu, n = (d.w >> 16) & 0xffu, half = d.w >> 24, cb = cols / 2, sb = cols / 16;
+#pragma unroll 1
+    for (uint32_t r = 0; r < n; ++r, src += 2 * (cb + sb), dst += cb + sb) {
+        bulk_g2s(dst, src + half * cb, cb, &c.full[s]);
+        bulk_g2s(dst + cb, src + 2 * cb + half * sb, sb, &c.full[s]);
+    }
 }
 
 // ---- GEMV, phase 1: wait for the input, fold the norm weight, convert to fixed point. A thread takes one quad of four
@@ -342,11 +353,11 @@ __device__ __forceinline__ void quad_to_fixed(const TokCtx &c, const TokOp &op, 
 }
 
 template <int P>
-__device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, const uint8_t *embed, uint32_t vocab) {
+__device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, const uint8_t *embed, uint32_t vocab, uint32_t half) {
     const int tid = threadIdx.x;
     const uint32_t cols = op.cols, nq = cols / 4;  // a multiple of 64: a warp is inside or outside as a whole
     uint32_t *xw = reinterpret_cast<uint32_t *>(c.xfb);
-    const uint32_t *in = op.in + c.par_cur;
+    const uint32_t *in = op.in + c.par_cur + half * cols;
     float ssq = 0.0f;
     if (op.in_kind == IN_EMBED) {
 #pragma unroll 1
@@ -388,7 +399,7 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
 // of the last iteration lie inside the row (TokOp::fast): loads at addresses worked out once (row_pair_dot_at).
 // NACT = 0: any shape the kernel takes, addresses worked out per half block.
 template <int QT, int P, int NACT>
-__device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, const uint32_t *bo, uint32_t gslot, const WarpRing wr) {
+__device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, const uint32_t *bo, uint32_t gslot, uint32_t half, const WarpRing wr) {
     constexpr int NX = NACT > 0 ? NACT : NMAX;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t cols = op.cols, nhb = cols / 16, lS = op.log2S, S = 1u << lS, nact = op.nact;
@@ -398,6 +409,7 @@ __device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, 
     const uint32_t sl0 = (rows0 + RPS - 1) >> lRPS, sl1 = sl0 + ((rows1 + RPS - 1) >> lRPS), total_slots = sl1 + ((rows2 + RPS - 1) >> lRPS);
     const uint4 *xf = reinterpret_cast<const uint4 *>(c.xfb);
     const uint32_t slice = warp & (S - 1), rwl = (warp >> lS) & (half_w - 1);
+    const uint32_t lP = lS + op.halves - 1, sum = slice + (half << lS);  // this warp's place among a row's partial sums
     XFixed<P> xr[NX];
 #pragma unroll
     for (int i = 0; i < NX; ++i) {
@@ -451,13 +463,13 @@ __device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, 
                 const uint8_t *row_a = row0 + (size_t)r * row_bytes;
                 z = row_pair_dot<QT, NX>(row_a, row_a + row_bytes, xr, slice, nhb, hi_off, sc_off, lane, (int)nact);
             }
-            if ((lane & 23) == 0) c.part[((sg_before + (ks << lRPS) + in_slot + r + (lane >> 3)) << lS) + slice] = z;
+            if ((lane & 23) == 0) c.part[((sg_before + (ks << lRPS) + in_slot + r + (lane >> 3)) << lP) + sum] = z;
         }
         if (r < nv) {  // an odd row on its own: half the work of a pair (short last slots are shared out one row per warp)
             float z;
             if (NACT > 0) z = row_single_dot_at<QT, NX, P>(row0_32 + r * row_bytes, lo, xr);
             else z = row_single_dot<QT, NX>(row0 + (size_t)r * row_bytes, xr, slice, nhb, hi_off, sc_off, lane, (int)nact);
-            if (lane == 0) c.part[((sg_before + (ks << lRPS) + in_slot + r) << lS) + slice] = z;
+            if (lane == 0) c.part[((sg_before + (ks << lRPS) + in_slot + r) << lP) + sum] = z;
         }
         __syncwarp();
         if (lane == 0 && kk + c.nslot < c.my_slots) {
@@ -482,7 +494,7 @@ __device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, 
 __device__ __forceinline__ void gemv_epilogue(const TokCtx &c, const TokOp &op, const uint32_t *bo, float scale, uint32_t epoch, float *logits,
                                            unsigned long long *cand, const TokParams &p) {
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const uint32_t lS = op.log2S, S = 1u << lS;
+    const uint32_t lS = op.log2S + op.halves - 1, S = 1u << lS;
     const bool swiglu = op.epilogue == EPI_SWIGLU;
     const uint32_t r0 = bo[0], rows0 = bo[1] & 0xffffu, rows1 = bo[1] >> 16, rows2 = bo[2];
     const uint32_t nr = swiglu ? rows0 : rows0 + rows1 + rows2;  // segments follow one another in part[] and in the output
@@ -919,11 +931,11 @@ __device__ __forceinline__ void attention_op(const TokCtx &c, const TokOp &op, u
     }
 }
 
-template <int KV>
+// PLANES: byte planes of the fixed-point input of the GEMVs (gemv_device.cuh). An f32 cache keeps the f32 accuracy class of the kernel-
+// per-operation path; f16 and q8_0 caches, whose own rounding is orders of magnitude larger, take two. Models whose feed-forward goes in
+// halves keep three for every cache: they had the 22 bits of the kernel-per-operation path before they came here.
+template <int KV, int PLANES>
 __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
-    // byte planes of the fixed-point input of the GEMVs (gemv_device.cuh): an f32 cache keeps the f32 accuracy class of
-    // the kernel-per-operation path; f16 and q8_0 caches, whose own rounding is orders of magnitude larger, take two
-    constexpr int PLANES = KV == BRASA_KV_F32 ? 3 : 2;
     extern __shared__ __align__(128) uint8_t smem[];
     TokCtx c;
     c.ring = smem;
@@ -1009,37 +1021,40 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
         if (op.type == OP_GEMV) {
             const uint32_t lRPS = 4 - op.log2S, RPS = 1u << lRPS;
             const uint32_t total_slots = (((bo[1] & 0xffffu) + RPS - 1) >> lRPS) + (((bo[1] >> 16) + RPS - 1) >> lRPS) + ((bo[2] + RPS - 1) >> lRPS);
-            // the descriptors this operation's refills and L2 requests will need, fetched by the threads that poll least
-            for (uint32_t i = TK_THREADS - 1 - tid; i < total_slots; i += TK_THREADS) {
-                const uint32_t k = gslot + p.nslot + i;
-                c.sdesc[i] = k < c.my_slots ? c.myslots[k] : make_uint4(0, 0, 0, 0);
+#pragma unroll 1
+            for (uint32_t half = 0; half < op.halves; ++half) {
+                // the descriptors this operation's refills and L2 requests will need, fetched by the threads that poll least
+                for (uint32_t i = TK_THREADS - 1 - tid; i < total_slots; i += TK_THREADS) {
+                    const uint32_t k = gslot + p.nslot + i;
+                    c.sdesc[i] = k < c.my_slots ? c.myslots[k] : make_uint4(0, 0, 0, 0);
+                }
+                TRACE(1);
+                float ssq = gemv_input<PLANES>(c, op, p.embed, p.vocab, half);
+                TRACE(3);
+                TRACEB(1);
+                for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
+                if (lane == 0) c.red[warp] = ssq;
+                __syncthreads();
+                TRACE(4);
+                if (warp == TK_WARPS - 1) {  // 1 / rms of the whole input from the warps' sums, parked for the epilogue
+                    float tot = c.red[lane & (TK_WARPS - 1)];
+                    for (int o = TK_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+                    if (lane == 0) c.red[47] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
+                }
+                if (op.qtype == BRASA_Q4_0) {
+                    if (op.fast && op.nact == 5) wr = gemv_rows<BRASA_Q4_0, PLANES, 5>(c, op, bo, gslot, half, wr);
+                    else if (op.fast && op.nact == 4) wr = gemv_rows<BRASA_Q4_0, PLANES, 4>(c, op, bo, gslot, half, wr);
+                    else wr = gemv_rows<BRASA_Q4_0, PLANES, 0>(c, op, bo, gslot, half, wr);
+                } else {
+                    if (op.fast && op.nact == 5) wr = gemv_rows<BRASA_Q6_0, PLANES, 5>(c, op, bo, gslot, half, wr);
+                    else wr = gemv_rows<BRASA_Q6_0, PLANES, 0>(c, op, bo, gslot, half, wr);
+                }
+                TRACE(7);
+                TRACEB(2);
+                gslot += total_slots;
+                __syncthreads();
+                TRACE(8);
             }
-            TRACE(1);
-            float ssq = gemv_input<PLANES>(c, op, p.embed, p.vocab);
-            TRACE(3);
-            TRACEB(1);
-            for (int o = 16; o > 0; o >>= 1) ssq += __shfl_xor_sync(0xffffffffu, ssq, o);
-            if (lane == 0) c.red[warp] = ssq;
-            __syncthreads();
-            TRACE(4);
-            if (warp == TK_WARPS - 1) {  // 1 / rms of the whole input from the warps' sums, parked for the epilogue
-                float tot = c.red[lane & (TK_WARPS - 1)];
-                for (int o = TK_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-                if (lane == 0) c.red[47] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
-            }
-            if (op.qtype == BRASA_Q4_0) {
-                if (op.fast && op.nact == 5) wr = gemv_rows<BRASA_Q4_0, PLANES, 5>(c, op, bo, gslot, wr);
-                else if (op.fast && op.nact == 4) wr = gemv_rows<BRASA_Q4_0, PLANES, 4>(c, op, bo, gslot, wr);
-                else wr = gemv_rows<BRASA_Q4_0, PLANES, 0>(c, op, bo, gslot, wr);
-            } else {
-                if (op.fast && op.nact == 5) wr = gemv_rows<BRASA_Q6_0, PLANES, 5>(c, op, bo, gslot, wr);
-                else wr = gemv_rows<BRASA_Q6_0, PLANES, 0>(c, op, bo, gslot, wr);
-            }
-            TRACE(7);
-            TRACEB(2);
-            gslot += total_slots;
-            __syncthreads();
-            TRACE(8);
             gemv_epilogue(c, op, bo, c.red[47], epoch, p.logits, p.cand, p);
         } else {
             attention_op<KV>(c, op, oi, epoch, p.heads, p.kv_heads, p.max_chunks, p.cos_t, p.sin_t, p.partials, p.attn_scale);
@@ -1109,6 +1124,13 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
     }
 }
 
+typedef void (*TokenKernel)(TokParams);
+TokenKernel token_kernel(int32_t kv, int planes) {
+    if (kv == BRASA_KV_F32) return decode_token_kernel<BRASA_KV_F32, 3>;
+    if (kv == BRASA_KV_F16) return planes == 3 ? decode_token_kernel<BRASA_KV_F16, 3> : decode_token_kernel<BRASA_KV_F16, 2>;
+    return planes == 3 ? decode_token_kernel<BRASA_KV_Q8_0, 3> : decode_token_kernel<BRASA_KV_Q8_0, 2>;
+}
+
 uint32_t attn_chunk(int32_t kv) { return kv == BRASA_KV_F32 ? 32u : 64u; }
 
 // Column slices and active half blocks per lane for a GEMV of this width; false when the kernel does not take it.
@@ -1127,6 +1149,14 @@ bool gemv_shape(int qtype, uint32_t cols, uint32_t *S_out, uint32_t *nact_out) {
     return false;
 }
 
+// How many pieces a q4_0 row of `cols` columns is taken in: one where the kernel takes it whole, two where it takes half of it (20 481 to
+// 40 960 columns: the 32B architecture's 25 600 on one GPU), 0 where neither.
+uint32_t gemv_halves(uint32_t cols) {
+    uint32_t S, n;
+    if (gemv_shape(BRASA_Q4_0, cols, &S, &n)) return 1;
+    return cols % 512 == 0 && cols / 2 < 65536 && gemv_shape(BRASA_Q4_0, cols / 2, &S, &n) ? 2 : 0;
+}
+
 }  // namespace
 
 struct brasa_token_program {
@@ -1134,6 +1164,7 @@ struct brasa_token_program {
     TokParams params{};
     size_t smem = 0;
     int32_t kv = 0;
+    int planes = 2;
     uint32_t grid = 0;
     std::vector<void *> device;  // allocations owned by the program
     void *vectors = nullptr;     // both copies of the activation vectors
@@ -1148,7 +1179,7 @@ bool brasa_token_program_supported(brasa_ctx *ctx, const brasa_token_model &m) {
     if (m.head.layout != BRASA_LAYOUT_TILED || (m.head.qtype != BRASA_Q4_0 && m.head.qtype != BRASA_Q6_0)) return false;
     uint32_t S, n;
     if (!gemv_shape(m.head.qtype, m.hidden, &S, &n) || !gemv_shape(BRASA_Q4_0, m.hidden, &S, &n) ||
-        !gemv_shape(BRASA_Q4_0, m.heads * 128, &S, &n) || !gemv_shape(BRASA_Q4_0, m.ffn, &S, &n))
+        !gemv_shape(BRASA_Q4_0, m.heads * 128, &S, &n) || !gemv_halves(m.ffn))
         return false;
     for (const brasa_token_layer &l : m.layers)
         for (const brasa_qmatrix *w : {&l.wq, &l.wk, &l.wv, &l.wo, &l.gate, &l.up, &l.down})
@@ -1169,6 +1200,7 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
     std::unique_ptr<brasa_token_program, void (*)(brasa_token_program *)> prog(new brasa_token_program, brasa_token_program_free);
     prog->ctx = ctx;
     prog->kv = m.kv;
+    prog->planes = m.kv == BRASA_KV_F32 || gemv_halves(m.ffn) == 2 ? 3 : 2;
     const uint32_t G = (uint32_t)ctx->sm_count;
     prog->grid = G;
     const uint32_t H = m.hidden, QD = m.heads * 128, KD = m.kv_heads * 128, F = m.ffn;
@@ -1205,7 +1237,8 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
         TokOp o{};
         o.type = OP_GEMV;
         o.qtype = (uint32_t)w[0].qtype;
-        o.cols = w[0].cols;
+        o.halves = w[0].qtype == BRASA_Q4_0 && gemv_halves(w[0].cols) == 2 ? 2 : 1;
+        o.cols = w[0].cols / o.halves;
         o.nmat = nmat;
         o.total_rows = 0;
         for (uint32_t i = 0; i < nmat; ++i) {
@@ -1291,15 +1324,20 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
             block_ops[oi * G + b] = make_uint4(r0, nrows[0] | (nrows[1] << 16), nrows[2], 0);
             const uint32_t S = 1u << o.log2S, RPS = TK_WARPS / S * R / 2, row_bytes = tiled_row_bytes((int)o.qtype, o.cols);
             uint32_t items = 0, op_slots = 0;
-            for (int i = 0; i < 3; ++i) {
-                for (uint32_t f = 0; f < nrows[i]; f += RPS) {
-                    uint32_t n = std::min(RPS, nrows[i] - f);
-                    slots.push_back(SlotDesc{o.w[i] + (size_t)(first[i] + f) * row_bytes, n * row_bytes, 0});
-                    ++op_slots;
+            for (uint32_t half = 0; half < o.halves; ++half) {
+                op_slots = 0;
+                items = 0;
+                for (int i = 0; i < 3; ++i) {
+                    for (uint32_t f = 0; f < nrows[i]; f += RPS) {
+                        const uint32_t n = std::min(RPS, nrows[i] - f);
+                        slots.push_back(SlotDesc{o.w[i] + (size_t)(first[i] + f) * row_bytes * o.halves, n * row_bytes,
+                                                 o.halves == 2 ? o.cols | (n << 16) | (half << 24) : 0u});
+                        ++op_slots;
+                    }
+                    items += nrows[i];
                 }
-                items += nrows[i];
             }
-            part_floats = std::max(part_floats, items * S);
+            part_floats = std::max(part_floats, items * S * o.halves);
             max_cols = std::max(max_cols, o.cols);
             max_op_slots = std::max(max_op_slots, op_slots);
         }
@@ -1324,7 +1362,7 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
 
     // ---- shared memory ----
     const size_t attn_bytes = (size_t)(TK_WARPS * (512 + 8) + 8 * 128) * 4 + 2 * 512;  // see attention_op
-    p.xf_bytes = (uint32_t)((std::max<size_t>((size_t)max_cols / 16 * 16 * (m.kv == BRASA_KV_F32 ? XRec<3>::CHUNKS : XRec<2>::CHUNKS), attn_bytes) + 127) / 128 * 128);
+    p.xf_bytes = (uint32_t)((std::max<size_t>((size_t)max_cols / 16 * 16 * (prog->planes == 3 ? XRec<3>::CHUNKS : XRec<2>::CHUNKS), attn_bytes) + 127) / 128 * 128);
     p.part_floats = (part_floats + 3) & ~3u;
     p.resid_floats = ((H + G - 1) / G + 4) & ~3u;
     p.sdesc_n = max_op_slots;
@@ -1367,14 +1405,9 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
         p.trace_op = env ? (uint32_t)atoi(env) : 5;
     }
 
-#define SET_ATTR(KVT) BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_token_kernel<KVT>, prog->smem))
-    if (m.kv == BRASA_KV_F32) SET_ATTR(BRASA_KV_F32);
-    else if (m.kv == BRASA_KV_F16) SET_ATTR(BRASA_KV_F16);
-    else SET_ATTR(BRASA_KV_Q8_0);
-#undef SET_ATTR
+    const TokenKernel fn = token_kernel(m.kv, prog->planes);
+    BRASA_TRY(brasa_smem_optin(ctx, (const void *)fn, prog->smem));
     int per_sm = 0;
-    const void *fn = m.kv == BRASA_KV_F32 ? (const void *)decode_token_kernel<BRASA_KV_F32>
-                     : m.kv == BRASA_KV_F16 ? (const void *)decode_token_kernel<BRASA_KV_F16> : (const void *)decode_token_kernel<BRASA_KV_Q8_0>;
     BRASA_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, TK_THREADS, prog->smem));
     BRASA_REQUIRE(ctx, per_sm >= 1, "token program: the kernel does not fit an SM");
     *out = prog.release();
@@ -1398,8 +1431,6 @@ int32_t brasa_token_program_launch(brasa_cmd *cmd, brasa_token_program *prog) {
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    if (prog->kv == BRASA_KV_F32) BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, decode_token_kernel<BRASA_KV_F32>, prog->params));
-    else if (prog->kv == BRASA_KV_F16) BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, decode_token_kernel<BRASA_KV_F16>, prog->params));
-    else BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, decode_token_kernel<BRASA_KV_Q8_0>, prog->params));
+    BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, token_kernel(prog->kv, prog->planes), prog->params));
     return brasa_post_launch(cmd, "decode_token");
 }

@@ -352,6 +352,29 @@ def test_token_kernel_matches_kernel_per_operation_path(kv, monkeypatch, golden_
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("ffn", [20992, 25600, 22528])
+def test_token_kernel_takes_wide_feed_forward_in_halves(ffn, monkeypatch, tmp_path):
+    """A down projection too wide for a ring slot and a lane's registers goes through the whole-token kernel as two halves of its columns
+    (the first width that does, the 32B architecture's, and halves with idle lanes). Both paths keep 22 bits of the input there, so the
+    logits agree far inside the f16 tolerance of crates/models/tests/forward.rs:40-55: 2e-5 of their scale, the 22-bit rounding of a
+    few layers."""
+    import brasa_b200 as B
+    from brasa_b200 import synth
+    cfg = dict(synth.QWEN3_4B, tie_word_embeddings=True, num_hidden_layers=2, hidden_size=256, intermediate_size=ffn, num_attention_heads=2,
+               num_key_value_heads=1, vocab_size=512)
+    synth.write_synthetic_model(B.Context(0), tmp_path / "wide.brasa", cfg, seed=3)
+    runs = []
+    for mode in ("0", "1"):
+        monkeypatch.setenv("BRASA_TOKEN_KERNEL", mode)
+        ctx = B.Context(0)
+        m = B.Qwen3.load(ctx, tmp_path / "wide.brasa", B.Limits(ctx=64, max_tokens=16, max_logit_rows=1, kv=B.KvType.F16))
+        m.forward(list(range(7)), 0, want_logits=False)
+        runs.append(np.stack([m.forward([11 * i + 5], 7 + i)[0][0].copy() for i in range(6)]))
+        m.free()
+    assert np.abs(runs[0] - runs[1]).max() <= 2e-5 * np.abs(runs[0]).max()
+
+
+@pytest.mark.gpu
 def test_token_kernel_long_cache_groups_chunks(monkeypatch, golden_dir):
     """Past (SMs / kv heads) attention chunks a block of the whole-token kernel walks several chunks with a running
     maximum and sum: 2 700 positions of an f32 cache (32-key chunks, 2 kv heads) are well beyond that point. Logits must
