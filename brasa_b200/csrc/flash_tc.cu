@@ -584,6 +584,8 @@ struct FlashF16Maps {
 // A q8_0 cache for this kernel: every value d * q (f16 scale, 8-bit code) is written as two f16 terms hi + lo, which is
 // exact, into f16 arrays shaped like an f16 cache; the kernel then adds the products with the low terms.
 __global__ void __launch_bounds__(256) kv_q8_expand_kernel(const uint8_t *cache, __half *hi, __half *lo, uint64_t rows) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;  // one thread per 8 values
     if (i >= rows * 16) return;
     const uint64_t r = i >> 4;
@@ -689,6 +691,9 @@ __global__ void __launch_bounds__(32 * (FLASH_SW + 1), 1) flash_tc_f16_kernel(co
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(ncols) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
+    // launched as a programmatic dependent: what the kernels before this one wrote (q, the cache) is touched after the wait
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     // Q tile: scale, round to f16, swizzled K-major; rows past the last query are zeros
     for (uint32_t i = tid; i < 128 * 16; i += 32 * (SW + 1)) {
         const uint32_t r = i >> 4, c8 = (i & 15) * 8;
@@ -1418,9 +1423,9 @@ int32_t brasa_flash_tc_launch(brasa_cmd *cmd, int32_t kv, const float *q, const 
             }
             uint8_t *base = ctx->kv_expand;
             const uint32_t blocks = (uint32_t)((rows * 16 + 255) / 256);
-            kv_q8_expand_kernel<<<blocks, 256, 0, ctx->stream>>>(kc, (__half *)base, (__half *)(base + one), rows);
+            BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kv_q8_expand_kernel, dim3(blocks), dim3(256), 0, kc, (__half *)base, (__half *)(base + one), rows));
             BRASA_TRY(brasa_post_launch(cmd, "kv_q8_expand"));
-            kv_q8_expand_kernel<<<blocks, 256, 0, ctx->stream>>>(vc, (__half *)(base + 2 * one), (__half *)(base + 3 * one), rows);
+            BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kv_q8_expand_kernel, dim3(blocks), dim3(256), 0, vc, (__half *)(base + 2 * one), (__half *)(base + 3 * one), rows));
             BRASA_TRY(brasa_post_launch(cmd, "kv_q8_expand"));
             kh = base; kl = base + one; vh = base + 2 * one; vl = base + 3 * one;
         }
@@ -1460,7 +1465,7 @@ int32_t brasa_flash_tc_launch(brasa_cmd *cmd, int32_t kv, const float *q, const 
             const size_t smem = 7 * TILE_BYTES + 1024;
             auto kernel = split ? flash_tc_f16_kernel<true> : flash_tc_f16_kernel<false>;
             BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernel, smem));
-            kernel<<<grid, 32 * (FLASH_SW + 1), smem, ctx->stream>>>(maps, p);
+            BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernel, grid, dim3(32 * (FLASH_SW + 1)), smem, maps, p));
             return brasa_post_launch(cmd, "flash_tc_f16");
         }
         fp.units = (uint32_t)units;

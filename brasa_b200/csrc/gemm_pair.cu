@@ -8,8 +8,8 @@
 //     f16 rounds the product once), as in the few-token kernel of gemm_tc.cu;
 //   * two CTAs share one product (cta_group::2, M = 256 weight rows, N = up to 256 tokens): each holds 128 weight rows and half of
 //     the tokens' X, so a CTA fetches 16 KB of X per K stage of 64 and the tensor core reads 32 bytes per clock of it;
-//   * the launch is persistent and cut evenly: the (weight tile, token tile, K chunk of 256) units, in that order, are split into
-//     one run per pair. 152 tiles over 74 pairs are 2.05 waves, and 20 tiles (a 2 560-row matrix at 512 tokens) not even one. A
+//   * the launch is persistent and, where that is shorter, cut evenly: the (weight tile, token tile, K chunk of 256) units, in that order,
+//     are split into one run per pair. 152 tiles over 74 pairs are 2.05 waves, and 20 tiles (a 2 560-row matrix at 512 tokens) not even one. A
 //     run that holds a tile's whole K range stores Y; any other leaves a partial tile, at most two per run, and a dependent
 //     kernel adds each shared tile's parts in K order;
 //   * a thread converts the first chunk of the next tile before it drains the finished one, and frees the accumulator as soon
@@ -17,9 +17,10 @@
 // Roles: warp 0 raw weights by TMA (128 rows x (128 code + 16 scale) bytes a chunk), warp 2 X by TMA, warp 1 of the first CTA the
 // products, warps 4-11 conversion and epilogue. Gate and up share a tile (64 rows of each per CTA, lanes 0-15 of a warp gate, 16-31
 // the same rows of up): silu(gate) * up is formed with one shuffle per value.
-// Measured (4B layer: qkv, o + residual, gate / up, down + residual; us, gemm_tc.cu's kernel in brackets): 3 584 tokens 109 (139), 83 (113),
-// 324 (377), 156 (185), 1 075 (889) TFLOP/s together; 1 024 tokens 48 (52), 40 (80), 108 (145), 55 (132), 824 (505) TFLOP/s; 512 tokens 35
-// (42), 33 (47), 66 (99), 42 (66).
+// Measured (4B layer: qkv, o + residual, gate / up, down + residual; us, gemm_tc.cu's kernel in brackets): 3 584 tokens 99 (139), 70 (113),
+// 322 (377), 141 (185), 1 143 (889) TFLOP/s together; 1 024 tokens 45 (52), 39 (80), 108 (145), 51 (132), 850 (505) TFLOP/s; 512 tokens 29
+// (42), 30 (47), 66 (99), 38 (66). Tensor pipe active 78 % of the cycles in down; 55 % in gate / up, whose SwiGLU keeps the conversion
+// threads from the next tile's chunks.
 // Every wait is bounded: one that runs out raises the context's status word and a CTA-wide flag, every role leaves its loop, both
 // CTAs meet at the cluster barrier, tensor memory is freed and the kernel returns.
 #include <cuda.h>
@@ -79,6 +80,7 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// (A branch-free quotient, rcp.approx refined and corrected in fma, costs more than it saves: 367 us against 317 for gate / up at 3 584 tokens.)
 __device__ __forceinline__ float swiglu(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
@@ -514,8 +516,16 @@ int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatr
     p.resid = resid;
     p.glu = glu;
     BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x) & 15) == 0, "gemm: misaligned x");
+    // Runs of whole tiles, or even ones that cut tiles: which is shorter, in chunks. Cut tiles cost their parts' way through memory and the
+    // kernel behind: 10 chunks' time for 256 tokens a tile, 7 for 128; 4 where that kernel also takes SwiGLU off the blocks. 3 584 tokens: qkv 99 us
+    // whole, 109 cut; o 70, 83; down 141, 156; gate / up 322, 320. 512 tokens: qkv 29, 35; gate / up 73, 66.
+    const uint32_t whole = (tiles * p.ntok + pairs - 1) / pairs * cpt;
+    if (whole <= (p.units + pairs - 1) / pairs + 4 + (glu ? 0 : p.n / 42)) {
+        p.gran = cpt;
+        pairs = std::min(sm_pairs, p.units / cpt);
+    }
     bool shared = false;  // some run begins inside a tile
-    for (uint32_t b = 1; b < pairs; ++b) shared = shared || pair_begin(b, pairs, p.units, 1) % cpt != 0;
+    for (uint32_t b = 1; b < pairs; ++b) shared = shared || pair_begin(b, pairs, p.units, p.gran) % cpt != 0;
     if (shared) {
         const size_t need = (size_t)2 * pairs * p.n * 256 * sizeof(float);
         if (ctx->gemm_part_bytes < need && !ctx->capturing) {
@@ -557,6 +567,6 @@ int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatr
     BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_pair_kernel, dim3(2 * pairs), dim3(384), GP_SMEM, tmap, maps, p));
     BRASA_TRY(brasa_post_launch(cmd, "gemm_pair"));
     if (!shared) return BRASA_OK;
-    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_pair_sum_kernel, dim3(pairs - 1, 8), dim3(256), 0, p, pairs));
+    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_pair_sum_kernel, dim3(pairs - 1, 16), dim3(256), 0, p, pairs));
     return brasa_post_launch(cmd, "gemm_pair_sum");
 }

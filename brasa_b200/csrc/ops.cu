@@ -423,6 +423,8 @@ template <int KV>
 __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, const float *q_norm, const float *k_norm, const float *cos_t,
                                           const float *sin_t, uint8_t *kc, uint8_t *vc, uint32_t hq, uint32_t hkv, uint32_t pos0, float eps,
                                           uint32_t rows) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t gr = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
     if (gr >= rows) return;
@@ -672,11 +674,11 @@ int32_t brasa_k_qk_norm_rope_store(brasa_cmd *cmd, int32_t kv, const brasa_arg q
     uint32_t rows = sh.tokens * (sh.hq + 2 * sh.hkv);
     if (rows == 0) return BRASA_OK;
     unsigned grid = (rows + 3) / 4;
-#define LAUNCH_QK(KVT)                                                                                                                      \
-    qk_norm_rope_store_kernel<KVT><<<grid, 128, 0, ctx->stream>>>((float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]), (const float *)arg_ptr(qkv[2]), \
-                                                                  (const float *)arg_ptr(norms[0]), (const float *)arg_ptr(norms[1]),               \
-                                                                  (const float *)arg_ptr(cos_t), (const float *)arg_ptr(sin_t), arg_ptr(dst[0]),    \
-                                                                  arg_ptr(dst[1]), sh.hq, sh.hkv, sh.pos0, eps, rows)
+#define LAUNCH_QK(KVT)                                                                                                                              \
+    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, qk_norm_rope_store_kernel<KVT>, dim3(grid), dim3(128), 0, (float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]), \
+                                           (const float *)arg_ptr(qkv[2]), (const float *)arg_ptr(norms[0]), (const float *)arg_ptr(norms[1]),           \
+                                           (const float *)arg_ptr(cos_t), (const float *)arg_ptr(sin_t), arg_ptr(dst[0]), arg_ptr(dst[1]), sh.hq, sh.hkv, \
+                                           sh.pos0, eps, rows))
     if (kv == BRASA_KV_F32) LAUNCH_QK(BRASA_KV_F32);
     else if (kv == BRASA_KV_F16) LAUNCH_QK(BRASA_KV_F16);
     else LAUNCH_QK(BRASA_KV_Q8_0);
