@@ -1356,10 +1356,12 @@ __global__ void __launch_bounds__(256) flash_tc_merge_kernel(const __grid_consta
     const uint32_t head = group % 2 == 0 ? 2 * item.pair + x : item.pair, q = (group % 2 == 0 ? 128 * item.q : 128 * (2 * item.q + x)) + row;
     auto part = [&](uint32_t z) { return fp.part + ((size_t)(z < b ? 2 * z + 1 : 2 * z) * 2 + x) * FL2_TILE; };
     float M = -INFINITY, l = 0.0f;
+#pragma unroll 4
     for (uint32_t z = b - 1; z < end; ++z) M = fmaxf(M, __ldcg(part(z) + 128 * 128 + row));
     float4 o[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) o[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
     for (uint32_t z = b - 1; z < end; ++z) {
         const float *src = part(z);
         const float m = __ldcg(src + 128 * 128 + row), w = m == -INFINITY ? 0.0f : expf(m - M);

@@ -78,18 +78,18 @@ __global__ void advance_kernel(uint32_t *ids, const uint32_t *next, uint32_t *ou
 // The reference sorts the candidates (descending logit, f32 total order), turns them into weights
 // exp((l - max) / T), keeps the shortest prefix whose normalised mass reaches top_p and walks that prefix with one
 // PCG32 draw. Here nothing is sorted: a prefix of the sorted order is the set {key > t, or key = t and id <= i}, and the
-// three prefixes the algorithm needs (the top_k-th candidate, the top_p cut, the drawn token) are each found by five
-// histograms of the candidates' mass: 256 steps of (max - l) / T first (logits of one vocabulary share two or three
-// values of their key's top byte: a histogram over that byte is one long queue on the same word), then the four bytes of
-// the 32-bit order key among the candidates of the chosen step. A count or an ascending walk over the ids settles equal
-// logits (they keep ascending id, as in the host sampler).
+// three prefixes the algorithm needs (the top_k-th candidate, the top_p cut, the drawn token) are each found in five
+// steps: among 256 steps of (max - l) / T first (logits of one vocabulary share two or three values of their key's top byte: a
+// histogram over that byte is one long queue on the same word), then by histograms over the four bytes of the 32-bit order key among the
+// candidates of the chosen step. A count over ascending ids settles equal logits (they keep ascending id, as in the host sampler).
 // Masses are 64-bit fixed point (weight x 2^k with n 2^k <= 2^62, truncated): sums do not depend on the order of the
 // additions, and what truncation loses is below 2^-26 of the largest weight for 2^18 candidates, a quarter of one rounding
 // of the f32 sums the reference forms.
-// A row is one cluster of eight blocks: each keeps to its eighth of the ids (76 KB at 151 936, out of L1 after the first
-// pass), and the histograms meet through distributed shared memory, one cluster barrier per pass. Bound: latency, some 13
-// passes of one barrier each. A chat turn of 12 tokens drawn from 151 936 logits took 66.6 ms with one block a row that bisected
-// over the whole row (3.84 ms a token) and takes 20.7 ms.
+// A row is one cluster of eight blocks, each with an eighth of the ids; histograms meet through distributed shared memory, one cluster
+// barrier per histogram. The logits are read twice, for the maximum and for the first histogram, which also leaves every id's step as a
+// byte in shared memory; the later passes look at four steps per word and touch the few logits that match (vocabularies too long for
+// that work the step out again). Bound: latency, some ten passes of a barrier each. One row of 151 936: 79 us (3 840 with one block a row
+// that bisected over the whole row, 158 with every pass over the logits); a step of 64 rows 113 us (240 as eleven launches).
 struct Prefix {
     uint32_t t;   // candidates with key > t are in
     uint32_t id;  // candidates with key == t are in when their id <= id
@@ -131,7 +131,8 @@ struct SampleShared {
     unsigned long long wh[SM_WARPS][256];  // a histogram per warp
     unsigned long long hist[2][256];       // the block's, read by the cluster; two, so that one barrier per pass is enough
     unsigned long long word[2];            // one number per block, likewise
-    unsigned long long wtot[8], total, bound, above, hit;
+    unsigned long long mass[256], count[256];  // of the steps, over the cluster and the kept candidates
+    unsigned long long wtot[8], bound, above, hit;
     uint32_t wcnt[SM_WARPS], bin, pass;
 };
 
@@ -155,105 +156,139 @@ __device__ unsigned long long cluster_sum(SampleShared &s, unsigned long long mi
 
 struct SampleRow {
     const float *l;
-    uint32_t lo, hi;  // this block's ids
-    float mx, temperature, fix;
+    uint32_t lo, hi;    // this block's ids
+    const uint8_t *steps;  // of this block's ids, in shared memory; null: worked out again
+    float mx, temperature, per_step, fix;
     __device__ __forceinline__ unsigned long long weight(float v) const {
         const float w = expf((v - mx) / temperature) * fix;
         return w > 0.0f ? __float2ull_rz(w) : 0ull;  // (a NaN weighs nothing)
     }
     __device__ __forceinline__ uint32_t step(float v) const {  // never larger for a larger logit
-        const float x = (mx - v) / temperature * 8.0f;
+        const float x = (mx - v) * per_step;
         return x < 255.0f ? (uint32_t)x : 255u;
     }
+    // bit j: id lo + i + j (four from i, a multiple of four) belongs to this step
+    __device__ __forceinline__ uint32_t four(uint32_t i, uint32_t at) const {
+        const uint32_t n = hi - lo;
+        if (i >= n) return 0u;
+        uint32_t m = 0;
+        if (steps) {
+            const uint32_t eq = __vcmpeq4(*reinterpret_cast<const uint32_t *>(steps + i), at * 0x01010101u);
+            m = (eq & 1u) | ((eq >> 7) & 2u) | ((eq >> 14) & 4u) | ((eq >> 21) & 8u);
+        } else {
+            for (uint32_t j = 0; j < 4; ++j) m |= (i + j < n && step(l[lo + i + j]) == at ? 1u : 0u) << j;
+        }
+        return i + 4 <= n ? m : m & ((1u << (n - i)) - 1u);
+    }
 };
+
+// s.hist[buf] = the sum over the warps' histograms
+__device__ __forceinline__ void block_hist(SampleShared &s, uint32_t buf) {
+    __syncthreads();
+    if (threadIdx.x < 256) {
+        unsigned long long a = 0;
+#pragma unroll
+        for (int w = 0; w < SM_WARPS; ++w) a += s.wh[w][threadIdx.x];
+        s.hist[buf][threadIdx.x] = a;
+    }
+}
+__device__ __forceinline__ unsigned long long cluster_bin(const SampleShared &s, uint32_t buf) {  // thread < 256: its bin over the cluster
+    unsigned long long h = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < SM_CLUSTER; ++r) h += cluster_load(&s.hist[buf][threadIdx.x], r);
+    return h;
+}
+// The first bin at which `above` and the bins so far reach s.bound: into s.bin, what lies before it into s.above. h: thread's bin (thread
+// < 256). Sets s.bound first when `share` does (from the sum over the bins).
+template <typename Bound>
+__device__ __forceinline__ void pick_bin(SampleShared &s, unsigned long long h, bool first, Bound bound_of) {
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    unsigned long long v = h;
+    if (tid < 256) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long up = __shfl_up_sync(0xffffffffu, v, o);
+            if ((int)lane >= o) v += up;
+        }
+        if (lane == 31) s.wtot[warp] = v;
+    }
+    __syncthreads();
+    if (tid == 0 && first) {
+        unsigned long long total = 0;
+        for (int w = 0; w < 8; ++w) total += s.wtot[w];
+        const unsigned long long bound = bound_of(total);
+        s.bound = bound < 1 ? 1 : bound;  // (a draw of 0 takes the first candidate)
+        s.above = 0;
+    }
+    __syncthreads();
+    const unsigned long long bound = s.bound, above = s.above;
+    if (tid < 256) {
+        for (uint32_t w = 0; w < warp; ++w) v += s.wtot[w];
+        v += above;
+    }
+    __syncthreads();  // everyone has read `above`
+    if (tid < 256 && v >= bound && v - h < bound) {  // exactly one bin
+        s.bin = tid;
+        s.above = v - h;
+    }
+    __syncthreads();
+}
 
 enum SampleBound { BOUND_COUNT, BOUND_SHARE, BOUND_DRAW };
 
 // Narrows `inside` to its shortest prefix whose mass reaches the bound (top_k candidates; top_p of its mass; u24 / 2^24 of
-// its mass, at least one unit).
+// its mass, at least one unit). s.mass and s.count are those of `inside`, and of the narrowed one afterwards unless it is the draw.
 template <SampleBound KIND>
 __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix inside, uint32_t top_k, float top_p, uint32_t u24) {
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint32_t step = 0, pref = 0;
-    for (int level = 0; level < 5; ++level) {
-        const uint32_t shift = level ? 8u * (4 - level) : 0u, buf = s.pass & 1;
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, len = row.hi - row.lo;
+    pick_bin(s, tid < 256 ? (KIND == BOUND_COUNT ? s.count[tid] : s.mass[tid]) : 0ull, true, [&](unsigned long long total) -> unsigned long long {
+        if (KIND == BOUND_COUNT) return top_k;
+        if (KIND == BOUND_SHARE) {
+            const double b = ceil((double)total * (double)top_p);
+            return b >= (double)total ? total : (unsigned long long)b;
+        }
+        const unsigned long long hi64 = __umul64hi(total, (unsigned long long)u24), lo64 = total * (unsigned long long)u24;  // ceil(total u24 / 2^24)
+        return ((hi64 << 40) | (lo64 >> 24)) + ((lo64 & 0xffffffull) ? 1 : 0);
+    });
+    const uint32_t step = s.bin;
+    uint32_t pref = 0;
+    for (int shift = 24; shift >= 0; shift -= 8) {
+        const uint32_t buf = s.pass & 1;
         for (uint32_t i = tid; i < SM_WARPS * 256; i += SM_THREADS) (&s.wh[0][0])[i] = 0;
         __syncthreads();
-#pragma unroll 4
-        for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) {
-            const float v = row.l[i];
-            const uint32_t k = order_key(v);
-            if (level > 1 && (k >> (shift + 8)) != (pref >> (shift + 8))) continue;
-            if (!in_prefix(k, i, inside)) continue;
-            const uint32_t at = row.step(v);
-            if (level > 0 && at != step) continue;
-            const unsigned long long w = KIND == BOUND_COUNT ? 1ull : row.weight(v);
-            if (w) atomicAdd(&s.wh[warp][level ? 255u - ((k >> shift) & 255u) : at], w);
+        for (uint32_t i = 4 * tid; i < len; i += 4 * SM_THREADS) {
+            for (uint32_t m = row.four(i, step); m; m &= m - 1) {
+                const uint32_t id = row.lo + i + __ffs(m) - 1;
+                const float v = row.l[id];
+                const uint32_t k = order_key(v);
+                if (shift < 24 && (k >> (shift + 8)) != (pref >> (shift + 8))) continue;
+                if (!in_prefix(k, id, inside)) continue;
+                const unsigned long long w = KIND == BOUND_COUNT ? 1ull : row.weight(v);
+                if (w) atomicAdd(&s.wh[warp][255u - ((k >> shift) & 255u)], w);
+            }
         }
-        __syncthreads();
-        if (tid < 256) {
-            unsigned long long a = 0;
-#pragma unroll
-            for (int w = 0; w < SM_WARPS; ++w) a += s.wh[w][tid];
-            s.hist[buf][tid] = a;
-        }
+        block_hist(s, buf);
         cluster_sync();
-        unsigned long long h = 0, v = 0;  // the bin's mass over the cluster, and with the bins before it
-        if (tid < 256) {
-#pragma unroll
-            for (uint32_t r = 0; r < SM_CLUSTER; ++r) h += cluster_load(&s.hist[buf][tid], r);
-            v = h;
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long up = __shfl_up_sync(0xffffffffu, v, o);
-                if ((int)lane >= o) v += up;
-            }
-            if (lane == 31) s.wtot[warp] = v;
-        }
+        const unsigned long long h = tid < 256 ? cluster_bin(s, buf) : 0ull;
         __syncthreads();
-        if (tid == 0) {
-            ++s.pass;
-            if (level == 0) {
-                unsigned long long total = 0, bound;
-                for (int w = 0; w < 8; ++w) total += s.wtot[w];
-                if (KIND == BOUND_COUNT) {
-                    bound = top_k;
-                } else if (KIND == BOUND_SHARE) {
-                    const double b = ceil((double)total * (double)top_p);
-                    bound = b >= (double)total ? total : (unsigned long long)b;
-                } else {  // ceil(total u24 / 2^24)
-                    const unsigned long long hi64 = __umul64hi(total, (unsigned long long)u24), lo64 = total * (unsigned long long)u24;
-                    bound = ((hi64 << 40) | (lo64 >> 24)) + ((lo64 & 0xffffffull) ? 1 : 0);
-                }
-                s.bound = bound < 1 ? 1 : bound;  // (a draw of 0 takes the first candidate)
-                s.above = 0;
-            }
-        }
-        __syncthreads();
-        const unsigned long long bound = s.bound, above = s.above;
-        if (tid < 256) {
-            for (uint32_t w = 0; w < warp; ++w) v += s.wtot[w];
-            v += above;
-        }
-        __syncthreads();  // everyone has read `above`
-        if (tid < 256 && v >= bound && v - h < bound) {  // exactly one bin
-            s.bin = tid;
-            s.hit = v - h;
-        }
-        __syncthreads();
-        if (tid == 0) s.above = s.hit;
-        if (level == 0) step = s.bin;
-        else pref |= (255u - s.bin) << shift;
+        if (tid == 0) ++s.pass;
+        pick_bin(s, h, false, [](unsigned long long) { return 0ull; });
+        pref |= (255u - s.bin) << shift;
         __syncthreads();
     }
     // the prefix ends with the m-th, in ascending id order, of the candidates whose key is `pref`
     const unsigned long long wt = KIND == BOUND_COUNT ? 1ull : row.weight(key_value(pref)), m = (s.bound - s.above + wt - 1) / wt;
-    const uint32_t span = (row.hi - row.lo + SM_WARPS - 1) / SM_WARPS, b = min(row.hi, row.lo + warp * span), e = min(row.hi, b + span);
+    const uint32_t span = ((len + SM_WARPS - 1) / SM_WARPS + 3) & ~3u, b = min(len, warp * span), e = min(len, b + span);
+    auto equals = [&](uint32_t i) {  // of the four ids from i, those with that key
+        uint32_t has = 0;
+        for (uint32_t c = i < e ? row.four(i, step) : 0u; c; c &= c - 1) {
+            const uint32_t j = __ffs(c) - 1, id = row.lo + i + j;
+            if (order_key(row.l[id]) == pref && in_prefix(pref, id, inside)) has |= 1u << j;
+        }
+        return has;
+    };
     uint32_t cnt = 0;
-#pragma unroll 4
-    for (uint32_t i0 = b; i0 < e; i0 += 32) {
-        const uint32_t i = i0 + lane;
-        cnt += __popc(__ballot_sync(0xffffffffu, i < e && order_key(row.l[min(i, e - 1)]) == pref && in_prefix(pref, i, inside)));
-    }
+    for (uint32_t i0 = b; i0 < e; i0 += 128) cnt += __popc(equals(i0 + 4 * lane));
+    for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
     if (lane == 0) s.wcnt[warp] = cnt;
     __syncthreads();
     uint32_t mine = 0, before_warp = 0;
@@ -268,30 +303,72 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
     __syncthreads();
     if (before < m && m <= before + cnt) {  // one warp of the cluster
         uint32_t left = (uint32_t)(m - before);
-        for (uint32_t i0 = b; i0 < e; i0 += 32) {
-            const uint32_t i = i0 + lane;
-            uint32_t has = __ballot_sync(0xffffffffu, i < e && order_key(row.l[min(i, e - 1)]) == pref && in_prefix(pref, i, inside));
-            const uint32_t c = __popc(has);
-            if (left <= c) {
-                for (; left > 1; --left) has &= has - 1;
-                if (lane == 0) s.hit = i0 + __ffs(has);  // id + 1
+        for (uint32_t i0 = b; i0 < e; i0 += 128) {
+            uint32_t has = equals(i0 + 4 * lane), incl = __popc(has);
+            const uint32_t own = incl;
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t up = __shfl_up_sync(0xffffffffu, incl, o);
+                if ((int)lane >= o) incl += up;
+            }
+            const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+            if (left <= all) {
+                if (left > incl - own && left <= incl) {
+                    for (uint32_t k = left - (incl - own); k > 1; --k) has &= has - 1;
+                    s.hit = row.lo + i0 + 4 * lane + __ffs(has);  // id + 1
+                }
                 break;
             }
-            left -= c;
+            left -= all;
         }
     }
     __syncthreads();
     unsigned long long unused;
     const unsigned long long id1 = cluster_sum(s, s.hit, unused);
-    return Prefix{pref, (uint32_t)id1 - 1};
+    const Prefix cut{pref, (uint32_t)id1 - 1};
+    if (KIND != BOUND_DRAW) {  // what the narrowed prefix holds of each step
+        unsigned long long c = 0, w = 0;
+        for (uint32_t i = 4 * tid; i < len; i += 4 * SM_THREADS)
+            for (uint32_t f = row.four(i, step); f; f &= f - 1) {
+                const uint32_t id = row.lo + i + __ffs(f) - 1;
+                const float v = row.l[id];
+                if (in_prefix(order_key(v), id, cut) && in_prefix(order_key(v), id, inside)) {
+                    ++c;
+                    w += row.weight(v);
+                }
+            }
+        for (int o = 16; o > 0; o >>= 1) {
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+            w += __shfl_xor_sync(0xffffffffu, w, o);
+        }
+        __syncthreads();
+        if (lane == 0) {
+            s.wh[warp][0] = c;
+            s.wh[warp][1] = w;
+        }
+        __syncthreads();
+        c = w = 0;
+        for (int k = 0; k < SM_WARPS; ++k) {
+            c += s.wh[k][0];
+            w += s.wh[k][1];
+        }
+        c = cluster_sum(s, c, unused);
+        w = cluster_sum(s, w, unused);
+        if (tid < 256 && tid >= step) {
+            s.count[tid] = tid == step ? c : 0ull;
+            s.mass[tid] = tid == step ? w : 0ull;
+        }
+        __syncthreads();
+    }
+    return cut;
 }
 
 // Row r: logits[r n ..], the PCG32 state at rng + 2 r, the token at out + r. `lone`: what a row whose largest logit is not
 // finite yields, the last of its candidates when set (the end of the reference's walk, which no comparison with NaN stops), else
-// the first infinite one, or token 0.
-__global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS)
-    sample_kernel(const float *logits, uint32_t n, float temperature, uint32_t top_k, float top_p, float fix, bool lone, unsigned long long *rng,
-                  uint32_t *out) {
+// the first infinite one, or token 0. keep_steps: the dynamic shared memory holds a byte per id of a block.
+__global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS, 2)
+    sample_kernel(const float *logits, uint32_t n, float temperature, uint32_t top_k, float top_p, float fix, bool lone, bool keep_steps,
+                  unsigned long long *rng, uint32_t *out) {
+    extern __shared__ __align__(16) uint8_t step_bytes[];
     __shared__ SampleShared s;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.x / SM_CLUSTER, me = cluster_rank();
     const uint32_t seg = (uint32_t)(((uint64_t)n + SM_CLUSTER - 1) / SM_CLUSTER);
@@ -299,15 +376,17 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS)
     row.l = logits + (size_t)r * n;
     row.lo = (uint32_t)min((uint64_t)n, (uint64_t)me * seg);
     row.hi = (uint32_t)min((uint64_t)n, (uint64_t)row.lo + seg);
+    row.steps = keep_steps ? step_bytes : nullptr;
     row.temperature = temperature;
+    row.per_step = 8.0f / temperature;
     row.fix = fix;
     if (tid == 0) s.pass = 0;
-    // the largest key; beside it the smallest with the largest of its ids, for rows without a finite maximum
     uint32_t kmax = 0;
-#pragma unroll 4
+#pragma unroll 8
     for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) kmax = max(kmax, order_key(row.l[i]));
     for (int o = 16; o > 0; o >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
     if (lane == 0) s.wcnt[warp] = kmax;
+    for (uint32_t i = tid; i < SM_WARPS * 256; i += SM_THREADS) (&s.wh[0][0])[i] = 0;
     __syncthreads();
     for (uint32_t w = 0; w < SM_WARPS; ++w) kmax = max(kmax, s.wcnt[w]);
     if (tid == 0) s.word[0] = kmax;
@@ -334,10 +413,36 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS)
         }
         return;
     }
+    const bool counted = top_k > 0 && top_k < n;
+    // mass (and count) of every step
+#pragma unroll 4
+    for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) {
+        const float v = row.l[i];
+        const uint32_t at = row.step(v);
+        if (keep_steps) step_bytes[i - row.lo] = (uint8_t)at;
+        const unsigned long long w = row.weight(v);
+        if (w) atomicAdd(&s.wh[warp][at], w);
+    }
+    block_hist(s, 1);
+    cluster_sync();
+    if (tid < 256) s.mass[tid] = cluster_bin(s, 1);
+    __syncthreads();
+    if (tid == 0) s.pass = 2;
+    if (counted) {
+        for (uint32_t i = tid; i < SM_WARPS * 256; i += SM_THREADS) (&s.wh[0][0])[i] = 0;
+        __syncthreads();
+        for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) atomicAdd(&s.wh[warp][keep_steps ? step_bytes[i - row.lo] : row.step(row.l[i])], 1ull);
+        block_hist(s, 0);
+        cluster_sync();
+        if (tid < 256) s.count[tid] = cluster_bin(s, 0);
+        __syncthreads();
+        if (tid == 0) s.pass = 3;
+    }
+    __syncthreads();
     const uint32_t x = (uint32_t)(((old >> 18) ^ old) >> 27), rot = (uint32_t)(old >> 59);
     const uint32_t u24 = ((x >> rot) | (x << ((32 - rot) & 31))) >> 8;  // one PCG32 draw
     Prefix kept{0u, 0xffffffffu};  // everything
-    if (top_k > 0 && top_k < n) kept = select_prefix<BOUND_COUNT>(s, row, kept, top_k, 0.0f, 0u);
+    if (counted) kept = select_prefix<BOUND_COUNT>(s, row, kept, top_k, 0.0f, 0u);
     if (top_p < 1.0f) kept = select_prefix<BOUND_SHARE>(s, row, kept, 0u, top_p, 0u);
     const Prefix pick = select_prefix<BOUND_DRAW>(s, row, kept, 0u, 0.0f, u24);
     cluster_sync();  // every block has read the state, and the others' shared memory
@@ -365,9 +470,14 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *logits, 
 // Sampler::sample for `count` rows of n logits at once: row r uses the PCG32 state at rng + 2 r; out[r] receives its token.
 static int32_t sample_launch(brasa_cmd *cmd, const float *logits, uint32_t n, uint32_t count, float temperature, uint32_t top_k, float top_p, bool lone,
                              unsigned long long *rng, uint32_t *out) {
+    brasa_ctx *ctx = cmd->ctx;
     int bits = 0;
     while (bits < 32 && (1ull << bits) < n) ++bits;
-    sample_kernel<<<count * SM_CLUSTER, SM_THREADS, 0, cmd->ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), lone, rng, out);
+    const size_t bytes = (((size_t)n + SM_CLUSTER - 1) / SM_CLUSTER + 15) / 16 * 16;
+    const bool keep_steps = bytes + sizeof(SampleShared) + 4096 <= ctx->smem_optin / 2;  // (two blocks on an SM: many rows at once)
+    if (keep_steps) BRASA_TRY(brasa_smem_optin(ctx, (const void *)sample_kernel, bytes));
+    sample_kernel<<<count * SM_CLUSTER, SM_THREADS, keep_steps ? bytes : 0, ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), lone,
+                                                                                          keep_steps, rng, out);
     return brasa_post_launch(cmd, "sample_top_p");
 }
 
