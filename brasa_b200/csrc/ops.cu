@@ -99,14 +99,20 @@ __global__ void __launch_bounds__(64) rms_norm_rows_kernel(const float *x, const
 }
 
 // One block of 128 threads per row, the row in registers (n a multiple of 512, at most 512 * RMS_BLOCK_CHUNKS): one pass with
-// 16-byte loads and one block barrier. For few rows (a decode step of a batch), where the row count cannot hide latency.
+// 16-byte loads and one block barrier. What bounds it is latency: a warp per row left 512 rows of 2 560 at 3 warps an SM (9.7 us a launch of a 512-token prompt; 3.7 a
+// launch at 1 024 tokens now).
 constexpr int RMS_BLOCK_CHUNKS = 10;
 template <bool HALF_OUT>
 __global__ void __launch_bounds__(128) rms_norm_block_kernel(const float *x, const float *w, void *out, uint32_t n, float eps) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     __shared__ float red[4];
     const uint32_t t = threadIdx.x, chunks = n / 512;
+    const float4 *wr = reinterpret_cast<const float4 *>(w);
+    float4 wv[RMS_BLOCK_CHUNKS];
+#pragma unroll
+    for (int c = 0; c < RMS_BLOCK_CHUNKS; ++c)
+        if (c < (int)chunks) wv[c] = wr[c * 128 + t];  // (a constant: ahead of the wait)
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)blockIdx.x * n);
     float4 v[RMS_BLOCK_CHUNKS];
     float ss = 0.0f;
@@ -122,11 +128,10 @@ __global__ void __launch_bounds__(128) rms_norm_block_kernel(const float *x, con
     __syncthreads();
     ss = (red[0] + red[1]) + (red[2] + red[3]);
     const float scale = 1.0f / sqrtf(ss / (float)n + eps);
-    const float4 *wr = reinterpret_cast<const float4 *>(w);
 #pragma unroll
     for (int c = 0; c < RMS_BLOCK_CHUNKS; ++c) {
         if (c < (int)chunks) {
-            const float4 ww = wr[c * 128 + t];
+            const float4 ww = wv[c];
             const float a = v[c].x * scale * ww.x, b = v[c].y * scale * ww.y, cc = v[c].z * scale * ww.z, d = v[c].w * scale * ww.w;
             if (HALF_OUT) {
                 const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(cc, d);
@@ -423,21 +428,31 @@ template <int KV>
 __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, const float *q_norm, const float *k_norm, const float *cos_t,
                                           const float *sin_t, uint8_t *kc, uint8_t *vc, uint32_t hq, uint32_t hkv, uint32_t pos0, float eps,
                                           uint32_t rows) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     uint32_t gr = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     int lane = threadIdx.x & 31;
-    if (gr >= rows) return;
     uint32_t per_tok = hq + 2 * hkv, t = gr / per_tok, r = gr % per_tok;
+    bool is_q = r < hq;
+    float wv[4], c[2], s[2];
+    if (gr < rows && r < hq + hkv) {  // constants: ahead of the wait
+        const float *w = is_q ? q_norm : k_norm;
+        for (int j = 0; j < 4; ++j) wv[j] = w[lane + 32 * j];
+        for (int j = 0; j < 2; ++j) {
+            c[j] = cos_t[(size_t)(pos0 + t) * 64 + lane + 32 * j];
+            s[j] = sin_t[(size_t)(pos0 + t) * 64 + lane + 32 * j];
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    if (gr >= rows) return;
     if (r >= hq + hkv) {
         size_t vh = (size_t)t * hkv + (r - hq - hkv);
-        for (int j = 0; j < 4; ++j) store_elem<KV>(vc, vh, v[vh * 128 + lane + 32 * j], lane, j);
+        float vv[4];
+        for (int j = 0; j < 4; ++j) vv[j] = v[vh * 128 + lane + 32 * j];
+        for (int j = 0; j < 4; ++j) store_elem<KV>(vc, vh, vv[j], lane, j);
         return;
     }
-    bool is_q = r < hq;
     size_t idx = is_q ? (size_t)t * hq + r : (size_t)t * hkv + (r - hq);
     float *x = (is_q ? q : k) + idx * 128;
-    const float *w = is_q ? q_norm : k_norm;
     float xv[4], ss = 0.0f;
     for (int j = 0; j < 4; ++j) {
         xv[j] = x[lane + 32 * j];
@@ -446,14 +461,11 @@ __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, co
     ss = warp_sum(ss);
     float scale = 1.0f / sqrtf(ss / 128.0f + eps);
     float y[4];
-    for (int j = 0; j < 4; ++j) y[j] = xv[j] * scale * w[lane + 32 * j];
-    uint32_t pos = pos0 + t;
+    for (int j = 0; j < 4; ++j) y[j] = xv[j] * scale * wv[j];
     for (int j = 0; j < 2; ++j) {
-        int i = lane + 32 * j;
-        float c = cos_t[(size_t)pos * 64 + i], s = sin_t[(size_t)pos * 64 + i];
         float a = y[j], b = y[j + 2];
-        y[j] = a * c - b * s;
-        y[j + 2] = b * c + a * s;
+        y[j] = a * c[j] - b * s[j];
+        y[j + 2] = b * c[j] + a * s[j];
     }
     for (int j = 0; j < 4; ++j) {
         x[lane + 32 * j] = y[j];
@@ -576,15 +588,15 @@ static int32_t rms_norm_common(brasa_cmd *cmd, brasa_arg x, brasa_arg w, brasa_a
     uint64_t tot = (uint64_t)rows * n;
     BRASA_REQUIRE(ctx, n > 0 && arg_fits(x, tot * 4) && arg_fits(w, (uint64_t)n * 4) && arg_fits(out, tot * (half_out ? 2 : 4)), "rms_norm: buffers too small");
     if (rows == 0) return BRASA_OK;
+    if (rows >= 2 && n % 512 == 0 && n <= 512 * RMS_BLOCK_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
+        if (half_out) BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<true>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
+        else BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<false>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
+        return brasa_post_launch(cmd, "rms_norm");
+    }
     if (rows >= 256 && n % 128 == 0 && n <= 128 * RMS_MAX_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
         const unsigned blocks = (rows + 1) / 2;
         if (half_out) BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_rows_kernel<true>, dim3(blocks), dim3(64), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), rows, n, eps));
         else BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_rows_kernel<false>, dim3(blocks), dim3(64), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), rows, n, eps));
-        return brasa_post_launch(cmd, "rms_norm");
-    }
-    if (rows >= 2 && n % 512 == 0 && n <= 512 * RMS_BLOCK_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
-        if (half_out) BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<true>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
-        else BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<false>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
         return brasa_post_launch(cmd, "rms_norm");
     }
     unsigned threads = n >= 1024 ? 256 : (n >= 256 ? 128 : 32);
