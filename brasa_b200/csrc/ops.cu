@@ -61,7 +61,7 @@ __global__ void rms_norm_kernel(const float *x, const float *w, void *out, uint3
 }
 
 // The same with one warp per row and the row held in registers (n a multiple of 128, at most 128 * RMS_MAX_CHUNKS):
-// one pass over x with 16-byte loads, no shared memory, two rows per block. Used for many rows (prefill, batch steps).
+// one pass over x with 16-byte loads, no shared memory, two rows per block. Used from 256 rows on whose length is no multiple of 512.
 constexpr int RMS_MAX_CHUNKS = 20;
 template <bool HALF_OUT>
 __global__ void __launch_bounds__(64) rms_norm_rows_kernel(const float *x, const float *w, void *out, uint32_t rows, uint32_t n, float eps) {
@@ -99,8 +99,8 @@ __global__ void __launch_bounds__(64) rms_norm_rows_kernel(const float *x, const
 }
 
 // One block of 128 threads per row, the row in registers (n a multiple of 512, at most 512 * RMS_BLOCK_CHUNKS): one pass with
-// 16-byte loads and one block barrier. What bounds it is latency: a warp per row left 512 rows of 2 560 at 3 warps an SM (9.7 us a launch of a 512-token prompt; 3.7 a
-// launch at 1 024 tokens now).
+// 16-byte loads and one block barrier. What bounds it is latency: a warp per row left 512 rows of 2 560 at three warps an SM (9.7 us a
+// launch in a prompt of 512 tokens; 3.7 us now at 1 024).
 constexpr int RMS_BLOCK_CHUNKS = 10;
 template <bool HALF_OUT>
 __global__ void __launch_bounds__(128) rms_norm_block_kernel(const float *x, const float *w, void *out, uint32_t n, float eps) {

@@ -821,7 +821,7 @@ def test_sampler_for_many_rows_follows_the_reference_sampler(B, ctx, K, n):
             assert agree >= 0.97 * total, (agree, total)
 
 
-@pytest.mark.parametrize("n", [1, 2, 9, 513, 4097, 60_000])
+@pytest.mark.parametrize("n", [1, 2, 9, 513, 4097, 60_000, 600_001])
 @pytest.mark.parametrize("top_k,top_p", [(0, 1.0), (0, 0.9), (7, 1.0), (30, 0.8)])
 def test_device_sampler_against_64_bits(B, ctx, K, n, top_k, top_p):
     """The one-row sampler where its split can go wrong (fewer candidates than blocks or threads, every eighth one longer than the last;
