@@ -26,7 +26,7 @@ struct brasa_ctx {
     size_t gemv_partials_floats = 0;
     uint32_t *gemv_counters = nullptr;
     size_t gemv_counters_n = 0;
-    uint32_t *status = nullptr;  // device status word: non-zero after a bounded wait gave up
+    uint32_t *status = nullptr;  // status word (mapped host memory): non-zero after a bounded wait gave up
     uint32_t timeouts = 0;       // waits that gave up so far (kernels with state across launches compare it to what they last saw)
     bool pdl = true;             // programmatic dependent launch between decode kernels
     bool capturing = false;      // a stream capture is open (brasa_graph_capture_begin)

@@ -59,12 +59,14 @@ int32_t brasa_ctx_create(int32_t device, brasa_ctx **out) {
     cudaGetDeviceProperties(&prop, device);
     ctx->sm_count = prop.multiProcessorCount;
     ctx->smem_optin = prop.sharedMemPerBlockOptin;
-    if (cudaMalloc(&ctx->status, 256) != cudaSuccess) {
+    // The status word lies in host memory that kernels write only when a wait gave up: the host reads it after a synchronisation without a
+    // copy of its own, which was a quarter of a short command (one GEMV of 9 728 x 2 560: 40.8 us with the copy, 30.0 without).
+    if (cudaHostAlloc((void **)&ctx->status, 256, cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) {
         cudaStreamDestroy(ctx->stream);
         delete ctx;
         return BRASA_ENOMEM;
     }
-    cudaMemset(ctx->status, 0, 256);
+    memset(ctx->status, 0, 256);
     const char *env = getenv("BRASA_PDL");
     if (env && env[0] == '0') ctx->pdl = false;
 #ifdef BRASA_TRACE_BUILD
@@ -95,7 +97,7 @@ void brasa_ctx_destroy(brasa_ctx *ctx) {
     cudaFree(ctx->kv_expand);
     cudaFree(ctx->gemm_counters);
     cudaFree(ctx->gemv_trace);
-    cudaFree(ctx->status);
+    cudaFreeHost(ctx->status);
     cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -138,10 +140,9 @@ int32_t brasa_debug_trace_read(brasa_ctx *ctx, uint64_t *out, uint32_t n) {
 int32_t brasa_ctx_sync(brasa_ctx *ctx) {
     if (!ctx) return BRASA_EINVAL;
     BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    uint32_t st = 0;
-    BRASA_CUDA(ctx, cudaMemcpy(&st, ctx->status, 4, cudaMemcpyDeviceToHost));
+    const uint32_t st = *static_cast<volatile uint32_t *>(ctx->status);
     if (st != 0) {
-        cudaMemset(ctx->status, 0, 4);
+        *static_cast<volatile uint32_t *>(ctx->status) = 0;
         ++ctx->timeouts;
         if (ctx->gemm_counters) cudaMemset(ctx->gemm_counters, 0, GEMM_TC_COUNTERS * 4);  // a kernel that gave up may have left arrivals behind
         return brasa_fail(ctx, BRASA_ETIMEOUT, "a bounded device-side wait ran out (status %u)", st);
@@ -249,10 +250,9 @@ int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds) {
         float ms = 0;
         cudaEventElapsedTime(&ms, cmd->start, cmd->end);
         if (gpu_seconds) *gpu_seconds = ms * 1e-3;
-        uint32_t st = 0;
-        cudaMemcpy(&st, ctx->status, 4, cudaMemcpyDeviceToHost);
+        const uint32_t st = *static_cast<volatile uint32_t *>(ctx->status);
         if (st != 0) {
-            cudaMemset(ctx->status, 0, 4);
+            *static_cast<volatile uint32_t *>(ctx->status) = 0;
             ++ctx->timeouts;
             if (ctx->gemm_counters) cudaMemset(ctx->gemm_counters, 0, GEMM_TC_COUNTERS * 4);
             rc = brasa_fail(ctx, BRASA_ETIMEOUT, "a bounded device-side wait ran out (status %u)", st);
