@@ -22,6 +22,7 @@
 #include "attn_device.cuh"
 #include "brasa_internal.h"
 #include "gemv_device.cuh"
+#include "tc_device.cuh"
 
 using namespace brasa_dev;
 
@@ -811,34 +812,33 @@ __global__ void __launch_bounds__(32 * (FLASH_SW + 1), 1) flash_tc_f16_kernel(co
         }
         ok = wait_s(j);
         uint32_t hi[NCH][16], lo[NCH][16];
+        const uint32_t ts = tmem_s + 128 * (j & 1) + trow + chalf;
+        if (softmax) {  // this tile's largest score of the row: own 64 columns, then the other half's through shared memory
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float tmax = -INFINITY;
+#pragma unroll
+            for (int cc = 0; cc < NCH; ++cc) {
+                if (j < nfree) max_chunk<false>(ts + 32 * cc, 0, 0, tmax);
+                else max_chunk<true>(ts + 32 * cc, j * 128 + chalf + 32 * cc, qpos, tmax);
+            }
+            pair_max[cgrp][row] = __float2half_rn(tmax);
+            ok = tc_pair_agree(1 + (warp & 3), ok);
+        }
         if (ok) {
             if (issuer && !SPLITKV && j + 2 < nkt) fetch_k(j + 2);
             if (issuer && SPLITKV && j + 1 < nkt) fetch_k(j + 1);
             float rescale = 1.0f;
             bool move = false;
             if (softmax) {
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t ts = tmem_s + 128 * (j & 1) + trow + chalf;
-                {
-                    // this tile's largest score of the row: own 64 columns, then the other half's through shared memory
-                    float tmax = -INFINITY;
+                float tmax = -INFINITY;
 #pragma unroll
-                    for (int cc = 0; cc < NCH; ++cc) {
-                        if (j < nfree) max_chunk<false>(ts + 32 * cc, 0, 0, tmax);
-                        else max_chunk<true>(ts + 32 * cc, j * 128 + chalf + 32 * cc, qpos, tmax);
-                    }
-                    pair_max[cgrp][row] = __float2half_rn(tmax);
-                    asm volatile("bar.sync %0, %1;" ::"r"(1 + (warp & 3)), "r"(32 * NG) : "memory");  // the warps that share these rows
-                    tmax = -INFINITY;
-#pragma unroll
-                    for (int g = 0; g < NG; ++g) tmax = fmaxf(tmax, __half2float(pair_max[g][row]));
-                    if (tmax > m + ONEPASS_SLACK || (m == -INFINITY && tmax != -INFINITY)) {
-                        move = m != -INFINITY;
-                        rescale = move ? ex2_approx((m - tmax) * 1.4426950408889634f) : 1.0f;
-                        l *= rescale;
-                        m = tmax;
-                        mneg = -m * 1.4426950408889634f;
-                    }
+                for (int g = 0; g < NG; ++g) tmax = fmaxf(tmax, __half2float(pair_max[g][row]));
+                if (tmax > m + ONEPASS_SLACK || (m == -INFINITY && tmax != -INFINITY)) {
+                    move = m != -INFINITY;
+                    rescale = move ? ex2_approx((m - tmax) * 1.4426950408889634f) : 1.0f;
+                    l *= rescale;
+                    m = tmax;
+                    mneg = -m * 1.4426950408889634f;
                 }
 #pragma unroll
                 for (int cc = 0; cc < NCH; ++cc) {
@@ -1217,7 +1217,6 @@ __global__ void __launch_bounds__(576, 1) flash_tc_two_kernel(const __grid_const
             for (uint32_t j = j0; j < j1; ++j) {
                 ok = wait(&s_ready[x], (it0 + j - j0) & 1);  // S of this tile, and with it every product issued before: P V of the tile before
                 ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t v[2][32];
                 tmem_ld32(ts, v[0]);
@@ -1233,7 +1232,8 @@ __global__ void __launch_bounds__(576, 1) flash_tc_two_kernel(const __grid_const
                 for (int i = 0; i < 64; ++i) t[i & 3] = fmaxf(t[i & 3], __uint_as_float(v[i >> 5][i & 31]));
                 float tmax = fmaxf(fmaxf(t[0], t[1]), fmaxf(t[2], t[3]));
                 pair[x][h][row] = __float2half_rn(tmax);
-                asm volatile("bar.sync %0, 64;" ::"r"(both) : "memory");
+                ok = tc_pair_agree(both, ok);  // (after a wait that gave up, what was read of S counts for nothing)
+                if (!ok) break;
                 tmax = fmaxf(__half2float(pair[x][0][row]), __half2float(pair[x][1][row]));
                 float rescale = 1.0f;
                 bool move = false;
@@ -1280,7 +1280,7 @@ __global__ void __launch_bounds__(576, 1) flash_tc_two_kernel(const __grid_const
             ok = __all_sync(0xffffffffu, ok);
             float *sums = reinterpret_cast<float *>(smem + x * TILE_BYTES);  // [half][row], over the Q tile: its products are done
             if (ok) sums[h * 128 + row] = l0 + l1;
-            asm volatile("bar.sync %0, 64;" ::"r"(both) : "memory");
+            ok = tc_pair_agree(both, ok);
             if (ok && len < item.nkt) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 float *dst = fp.part + ((size_t)(2 * blockIdx.x + (j0 == 0)) * 2 + x) * FL2_TILE;

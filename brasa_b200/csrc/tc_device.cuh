@@ -32,6 +32,20 @@ __device__ __forceinline__ bool tc_elect_one() {
         : "=r"(pred));
     return pred != 0;
 }
+// The meeting of the two warps that hold the same rows of an attention tile: a barrier of their 64 threads that also tells each whether
+// both go on. A warp whose wait gave up comes here like the other and both leave together; one that left without coming would leave
+// the other at a barrier that nobody completes.
+__device__ __forceinline__ bool tc_pair_agree(uint32_t bar, bool ok) {
+    uint32_t both;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %2, 0;\n\t"
+        "bar.red.and.pred q, %1, 64, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(both)
+        : "r"(bar), "r"(ok ? 1u : 0u)
+        : "memory");
+    return both != 0;
+}
 // K-major operand: rows of 128 bytes, groups of 8 rows 1024 bytes apart, 128-byte swizzle
 __device__ __forceinline__ uint64_t tc_desc_kmajor(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);

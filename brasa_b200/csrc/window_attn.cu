@@ -330,13 +330,32 @@ __global__ void __launch_bounds__(288, 1) window_tc_kernel(const __grid_constant
         uint32_t hi[32], lo_[32];
         float rescale = 1.0f;
         bool move = false;
+        const uint32_t ts = tmem + 128 * (j & 1) + trow + c0;
+        const uint32_t k0 = a.key0 + (jbeg + j) * 128;  // position of the tile's first key
+        const bool free_tile = k0 + 127 <= qfirst && k0 + a.window > qfirst + 127;
+        // a key of column c is visible when lob <= c <= hib
+        const int hib = (int)qpos - (int)(k0 + c0), lob = hib - (int)a.window + 1;
+        if (!CAP && softmax) {  // the tile's largest score of the row: own 64 columns, then the other half's through shared memory
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            float tmax = -INFINITY;
+#pragma unroll
+            for (int cc = 0; cc < 2; ++cc) {
+                uint32_t v[32];
+                tc_ld32(ts + 32 * cc, v);
+                if (free_tile) {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i) tmax = fmaxf(tmax, __uint_as_float(v[i]) * sl);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        if (32 * cc + i <= hib && 32 * cc + i >= lob) tmax = fmaxf(tmax, __uint_as_float(v[i]) * sl);
+                }
+            }
+            pair_max[cgrp][row] = tmax;
+            ok = tc_pair_agree(1 + (warp & 3), ok);
+        }
         if (ok && softmax) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t ts = tmem + 128 * (j & 1) + trow + c0;
-            const uint32_t k0 = a.key0 + (jbeg + j) * 128;  // position of the tile's first key
-            const bool free_tile = k0 + 127 <= qfirst && k0 + a.window > qfirst + 127;
-            // a key of column c is visible when lob <= c <= hib
-            const int hib = (int)qpos - (int)(k0 + c0), lob = hib - (int)a.window + 1;
             if constexpr (CAP) {
 #pragma unroll
                 for (int cc = 0; cc < 2; ++cc) {
@@ -358,23 +377,7 @@ __global__ void __launch_bounds__(288, 1) window_tc_kernel(const __grid_constant
                     }
                 }
             } else {
-                float tmax = -INFINITY;
-#pragma unroll
-                for (int cc = 0; cc < 2; ++cc) {
-                    uint32_t v[32];
-                    tc_ld32(ts + 32 * cc, v);
-                    if (free_tile) {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) tmax = fmaxf(tmax, __uint_as_float(v[i]) * sl);
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 32; ++i)
-                            if (32 * cc + i <= hib && 32 * cc + i >= lob) tmax = fmaxf(tmax, __uint_as_float(v[i]) * sl);
-                    }
-                }
-                pair_max[cgrp][row] = tmax;
-                asm volatile("bar.sync %0, %1;" ::"r"(1 + (warp & 3)), "r"(64) : "memory");  // the two warps that share these rows
-                tmax = fmaxf(pair_max[0][row], pair_max[1][row]);
+                const float tmax = fmaxf(pair_max[0][row], pair_max[1][row]);
                 if (tmax > m + SLACK || (m == -INFINITY && tmax != -INFINITY)) {
                     move = m != -INFINITY;
                     rescale = move ? ex2(m - tmax) : 1.0f;

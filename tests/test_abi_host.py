@@ -198,3 +198,19 @@ def test_few_token_gemm_partition(B):
     assert L.brasa_gemm_few_tokens_plan(148, 1 << 20, 1 << 6, C.byref(blocks), C.byref(parts), C.byref(scratch)) != 0
     assert L.brasa_gemm_few_tokens_plan(148, 0, 4, C.byref(blocks), C.byref(parts), C.byref(scratch)) != 0
     assert L.brasa_gemm_few_tokens_owner(100, 10, 100) == 0xFFFFFFFF
+
+
+@pytest.mark.parametrize("name,kernels", [("flash_tc.cu", 2), ("window_attn.cu", 1)])
+def test_row_warps_of_the_attention_kernels_leave_together(name, kernels):
+    """The two warps that hold the same query rows meet at counted barriers, and each may give up a wait on its own. So a meeting has to tell
+    both whether they go on (tc_pair_agree), and neither may leave between a wait for scores and the meeting behind it: the other would
+    stand at a barrier that never fills, and the block would never end. Read from the source, since a GPU is not made to hang for it."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "brasa_b200" / "csrc" / name).read_text())
+    assert not re.search(r"\bbar(rier)?\.(cta\.)?sync", text)  # every meeting of fewer than all threads carries the verdict
+    score_waits = list(re.finditer(r"ok = (wait_s\(j\)|wait\(&s_ready\[x\]|wait\(&bar_s\[j & 1\])", text))
+    meetings = [m.start() for m in re.finditer(r"ok = tc_pair_agree\(", text)]
+    followed = [w for w in score_waits if any(w.start() < m < w.start() + 2500 for m in meetings)]
+    assert len(followed) == kernels
+    for w in followed:
+        between = text[w.end():min(m for m in meetings if m > w.start())]
+        assert not re.search(r"\b(break|return|continue)\b", between)
