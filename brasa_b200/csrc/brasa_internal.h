@@ -48,7 +48,15 @@ struct brasa_ctx {
     float *gemm_part = nullptr;      // partial output tiles of the split-K tensor-core GEMM
     size_t gemm_part_bytes = 0;
     uint32_t *gemm_counters = nullptr;  // arrivals per output tile of that GEMM (GEMM_TC_COUNTERS words, zero between launches)
+    bool recorded = false;              // a graph has been recorded: its kernels may hold the address of any workspace there was
+    std::vector<void *> outgrown;       // workspaces such a graph may still use, freed with the context (see brasa_workspace)
 };
+
+// Makes a workspace of the context at least `need` bytes large; its contents do not matter. A larger one takes its place behind everything
+// enqueued so far. The old one is freed, unless a graph has been recorded on the context: a replay writes where the recorded launch wrote, so
+// then the old one stays until the context goes, and the new one is at least half again as large, so that what stays is less than
+// twice what is in use. BRASA_EINVAL while a graph is being recorded, BRASA_ENOMEM (and no workspace) when memory runs out.
+int32_t brasa_workspace(brasa_ctx *ctx, void **p, size_t *bytes, size_t need);
 
 // Launches `kernel` as a programmatic dependent of the kernel before it on the context's stream: it may start while that
 // kernel is still running and must execute griddepcontrol.wait before it touches anything that kernel produces (and the

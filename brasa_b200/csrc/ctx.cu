@@ -96,6 +96,7 @@ void brasa_ctx_destroy(brasa_ctx *ctx) {
     cudaFree(ctx->flash_part);
     cudaFree(ctx->kv_expand);
     cudaFree(ctx->gemm_counters);
+    for (void *p : ctx->outgrown) cudaFree(p);
     cudaFree(ctx->gemv_trace);
     cudaFreeHost(ctx->status);
     cudaStreamDestroy(ctx->stream);
@@ -271,6 +272,7 @@ int32_t brasa_graph_capture_begin(brasa_ctx *ctx) {
     BRASA_REQUIRE(ctx, !ctx->capturing, "a capture is already open on this context");
     BRASA_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     ctx->capturing = true;
+    ctx->recorded = true;
     ctx->capture_launches = 0;
     return BRASA_OK;
 }
@@ -355,23 +357,39 @@ int32_t brasa_post_launch(brasa_cmd *cmd, const char *name) {
     return BRASA_OK;
 }
 
-int32_t brasa_gemv_scratch(brasa_ctx *ctx, size_t partial_floats, size_t counters) {
-    if (partial_floats > ctx->gemv_partials_floats) {
-        BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->gemv_partials);
-        ctx->gemv_partials = nullptr;
-        ctx->gemv_partials_floats = 0;
-        BRASA_CUDA(ctx, cudaMalloc(&ctx->gemv_partials, partial_floats * sizeof(float)));
-        ctx->gemv_partials_floats = partial_floats;
+int32_t brasa_workspace(brasa_ctx *ctx, void **p, size_t *bytes, size_t need) {
+    if (*bytes >= need) return BRASA_OK;
+    BRASA_REQUIRE(ctx, !ctx->capturing, "a workspace of %llu bytes is needed and none can be allocated while a graph is recorded", (unsigned long long)need);
+    BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    if (*p && ctx->recorded) {
+        ctx->outgrown.push_back(*p);
+        need = std::max(need, *bytes + *bytes / 2);
+    } else {
+        cudaFree(*p);
     }
+    *p = nullptr;
+    *bytes = 0;
+    if (cudaMalloc(p, need) != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+        return brasa_fail(ctx, BRASA_ENOMEM, "no memory for a workspace of %llu bytes", (unsigned long long)need);
+    }
+    *bytes = need;
+    return BRASA_OK;
+}
+
+int32_t brasa_gemv_scratch(brasa_ctx *ctx, size_t partial_floats, size_t counters) {
+    size_t bytes = ctx->gemv_partials_floats * sizeof(float);
+    const int32_t rc = brasa_workspace(ctx, (void **)&ctx->gemv_partials, &bytes, partial_floats * sizeof(float));
+    ctx->gemv_partials_floats = bytes / sizeof(float);
+    BRASA_TRY(rc);
     if (counters > ctx->gemv_counters_n) {
-        BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-        cudaFree(ctx->gemv_counters);
-        ctx->gemv_counters = nullptr;
-        ctx->gemv_counters_n = 0;
-        BRASA_CUDA(ctx, cudaMalloc(&ctx->gemv_counters, counters * sizeof(uint32_t)));
-        BRASA_CUDA(ctx, cudaMemset(ctx->gemv_counters, 0, counters * sizeof(uint32_t)));
-        ctx->gemv_counters_n = counters;
+        bytes = ctx->gemv_counters_n * sizeof(uint32_t);
+        const int32_t rc2 = brasa_workspace(ctx, (void **)&ctx->gemv_counters, &bytes, counters * sizeof(uint32_t));
+        ctx->gemv_counters_n = 0;  // (until they are zero)
+        BRASA_TRY(rc2);
+        BRASA_CUDA(ctx, cudaMemsetAsync(ctx->gemv_counters, 0, bytes, ctx->stream));
+        ctx->gemv_counters_n = bytes / sizeof(uint32_t);
     }
     return BRASA_OK;
 }

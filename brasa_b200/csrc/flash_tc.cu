@@ -1413,16 +1413,8 @@ int32_t brasa_flash_tc_launch(brasa_cmd *cmd, int32_t kv, const float *q, const 
         const uint8_t *kh = kc, *vh = vc, *kl = nullptr, *vl = nullptr;
         if (split) {  // q8_0: the rows seen by this call as f16 hi + lo arrays (exact), rebuilt on every call
             const size_t one = rows * 256, need = 4 * one;
-            if (ctx->kv_expand_bytes < need) {
-                BRASA_REQUIRE(ctx, !ctx->capturing, "flash attention: the q8_0 expansion buffer cannot grow while a graph is recorded");
-                BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-                if (ctx->kv_expand) cudaFree(ctx->kv_expand);
-                ctx->kv_expand = nullptr;
-                ctx->kv_expand_bytes = 0;
-                const size_t grow = need + need / 4;  // a prompt fed in chunks asks for a little more every call
-                BRASA_CUDA(ctx, cudaMalloc((void **)&ctx->kv_expand, grow));
-                ctx->kv_expand_bytes = grow;
-            }
+            if (ctx->kv_expand_bytes < need)  // (a prompt fed in chunks asks for a little more every call)
+                BRASA_TRY(brasa_workspace(ctx, (void **)&ctx->kv_expand, &ctx->kv_expand_bytes, need + need / 4));
             uint8_t *base = ctx->kv_expand;
             const uint32_t blocks = (uint32_t)((rows * 16 + 255) / 256);
             BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kv_q8_expand_kernel, dim3(blocks), dim3(256), 0, kc, (__half *)base, (__half *)(base + one), rows));
@@ -1472,15 +1464,9 @@ int32_t brasa_flash_tc_launch(brasa_cmd *cmd, int32_t kv, const float *q, const 
         }
         fp.units = (uint32_t)units;
         uint32_t runs = std::min<uint32_t>((uint32_t)ctx->sm_count, std::max(1u, fp.units / 2));
-        const size_t need = (size_t)runs * 4 * FL2_TILE * sizeof(float);
-        if (cut && ctx->flash_part_bytes < need && !ctx->capturing) {
-            BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (ctx->flash_part) cudaFree(ctx->flash_part);
-            ctx->flash_part = nullptr;
-            ctx->flash_part_bytes = 0;
-            if (cudaMalloc((void **)&ctx->flash_part, need) == cudaSuccess) ctx->flash_part_bytes = need;
-            else cudaGetLastError();
-        }
+        // the most that any launch asks for (39.4 MB on 148 SMs), so that prompts of growing length allocate and synchronise once
+        const size_t need = (size_t)runs * 4 * FL2_TILE * sizeof(float), most = (size_t)ctx->sm_count * 4 * FL2_TILE * sizeof(float);
+        if (cut && ctx->flash_part_bytes < need && !ctx->capturing) brasa_workspace(ctx, (void **)&ctx->flash_part, &ctx->flash_part_bytes, most);
         if (cut && ctx->flash_part_bytes >= need) fp.part = ctx->flash_part;
         else {  // (or no workspace: a graph is being recorded, no memory is left)
             fp.whole = 1;

@@ -1075,16 +1075,7 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
     p.trace = (unsigned long long *)ctx->gemv_trace;
 #endif
     if (max_parts > 1 || p.defer) {
-        const size_t need = (size_t)scratch;
-        if (ctx->gemm_part_bytes < need) {
-            BRASA_REQUIRE(ctx, !ctx->capturing, "gemm: the split-K workspace cannot grow while a graph is recorded");
-            BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (ctx->gemm_part) cudaFree(ctx->gemm_part);
-            ctx->gemm_part = nullptr;
-            ctx->gemm_part_bytes = 0;
-            BRASA_CUDA(ctx, cudaMalloc((void **)&ctx->gemm_part, need));
-            ctx->gemm_part_bytes = need;
-        }
+        BRASA_TRY(brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, (size_t)scratch));
         p.part = ctx->gemm_part;
     }
     const size_t smem = (size_t)SK_NCS * SK_X_CHUNK + (size_t)p.raw_slots * SK_RAW + 1024;
@@ -1273,16 +1264,7 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
     p.ksplit = ksplit;
     dim3 grid(ncta_n, (ntile + mt - 1) / mt, ksplit);
     if (ksplit > 1) {
-        const size_t need = (size_t)ksplit * grid.x * grid.y * mt * BM * nb * BN * sizeof(float);
-        if (ctx->gemm_part_bytes < need) {
-            BRASA_REQUIRE(ctx, !ctx->capturing, "gemm: the split-K workspace cannot grow while a graph is recorded");
-            BRASA_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-            if (ctx->gemm_part) cudaFree(ctx->gemm_part);
-            ctx->gemm_part = nullptr;
-            ctx->gemm_part_bytes = 0;
-            BRASA_CUDA(ctx, cudaMalloc((void **)&ctx->gemm_part, need));
-            ctx->gemm_part_bytes = need;
-        }
+        BRASA_TRY(brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, (size_t)ksplit * grid.x * grid.y * mt * BM * nb * BN * sizeof(float)));
         if (!ctx->gemm_counters) {
             BRASA_REQUIRE(ctx, !ctx->capturing, "gemm: the split-K counters cannot be created while a graph is recorded");
             BRASA_CUDA(ctx, cudaMalloc((void **)&ctx->gemm_counters, GEMM_TC_COUNTERS * 4));

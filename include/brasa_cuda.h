@@ -102,7 +102,8 @@ int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds);  /* Pending::wait -
 /* CUDA graphs. No counterpart call in the reference, whose two command buffers per forward play this
  * role (crates/models/src/qwen3.rs:781-797): kernels enqueued on the context between begin and end are
  * recorded instead of run, and brasa_graph_launch replays them in one submission. Nothing that
- * allocates or synchronises may be called while a capture is open. */
+ * allocates or synchronises may be called while a capture is open. Between replays any call may be made: workspaces of the
+ * library that recorded kernels use stay where they are until the context is destroyed. */
 typedef struct brasa_graph brasa_graph;
 int32_t brasa_graph_capture_begin(brasa_ctx *ctx);
 int32_t brasa_graph_capture_end(brasa_ctx *ctx, brasa_graph **out);

@@ -747,6 +747,42 @@ def test_flash_attention_tensor_core_many_query_tiles(B, ctx, K, tokens, pos0, k
     assert float(np.max(d / np.maximum(vmax, 1e-30))) <= 1e-5
 
 
+@pytest.mark.parametrize("what", ["gemm-few", "gemm-pair", "flash-F16", "flash-Q8_0"])
+def test_recorded_kernels_keep_their_workspace(B, K, what):
+    """A recorded launch has the address of its workspace in it. Calls behind the recording that need a larger one must leave the old one
+    allocated: a replay gives the recorded result again, and writes into nothing that was allocated since."""
+    ctx = B.Context(0)
+    K = B.Kernels(ctx)
+    rng = O.Rng(len(what))
+    if what.startswith("gemm"):  # 16 or 90 tokens, then 200: the K range is cut for all of them
+        rows, cols, tokens = 512, 9728, 16 if what == "gemm-few" else 90
+        w = tiled(B, ctx, K, "q4_0", rng.qmatrix(O.Q4_0, rows, cols), rows, cols)[0]
+        gx, gy, big = ctx.buffer_from(rng.vec(200 * cols, 1.0).astype(np.float16)), ctx.buffer(tokens * rows * 4), ctx.buffer(200 * rows * 4)
+        small = lambda c: K.gemm(c, w, gx, gy, tokens)
+        large = lambda c: K.gemm(c, w, gx, big, 200)
+    else:  # 100 queries behind 1 024 keys, whose key range is cut; then 600 behind 4 096
+        kvt = getattr(B.KvType, what[6:])
+        hq, hkv, keys = 32, 8, 4736
+        gk, gv, _, _ = make_cache(B, ctx, kvt, rng.vec(keys * hkv * 128, 2.0), rng.vec(keys * hkv * 128, 3.0))
+        gx, gy, big = ctx.buffer_from(rng.vec(600 * hq * 128, 2.0)), ctx.buffer(100 * hq * 128 * 2), ctx.buffer(600 * hq * 128 * 2)
+        small = lambda c: K.flash_attention(c, gx, gk, gv, gy, B.AttnShape(100, hq, hkv, 128, 1024, kvt))
+        large = lambda c: K.flash_attention(c, gx, gk, gv, big, B.AttnShape(600, hq, hkv, 128, 4096, kvt))
+    run(ctx, small)
+    want = gy.download(np.uint8).copy()
+    graph = ctx.capture(small)
+    run(ctx, large)
+    since = [ctx.buffer(n << 20) for n in (1, 1, 2, 2, 4, 4, 8, 16, 32)]  # what freed memory would be handed out for
+    for b in since:
+        b.fill(0xA5)
+    gy.fill(0xFF)
+    run(ctx, graph.launch)
+    assert np.array_equal(gy.download(np.uint8), want)
+    for b in since:
+        assert np.all(b.download(np.uint8) == 0xA5)
+    graph.free()
+    ctx.close()
+
+
 # ---- sampling ------------------------------------------------------------------------------------
 
 @pytest.mark.parametrize("n", [50, 5000, 151_936])
