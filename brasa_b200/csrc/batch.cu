@@ -586,6 +586,7 @@ int32_t encode_step(brasa_batch *b, brasa_cmd *cmd, uint32_t n) {
     brasa_model *m = b->m;
     brasa_ctx *ctx = b->ctx;
     const brasa_config &c = m->cfg;
+    const SettledOperands settled(ctx);
     const uint32_t H = c.hidden;
     const bool half_io = n > GEMV_MAX_TOKENS && m->prefill_precision == BRASA_PREFILL_F16;
     const int32_t prec = half_io ? BRASA_PREFILL_F16 : BRASA_PREFILL_F32;

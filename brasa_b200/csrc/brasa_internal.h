@@ -30,6 +30,7 @@ struct brasa_ctx {
     uint32_t timeouts = 0;       // waits that gave up so far (kernels with state across launches compare it to what they last saw)
     bool pdl = true;             // programmatic dependent launch between decode kernels
     bool capturing = false;      // a stream capture is open (brasa_graph_capture_begin)
+    bool settled = false;        // see SettledOperands
     unsigned long long *gemv_trace = nullptr;  // device buffer of phase timestamps when BRASA_TRACE=1
     struct {
         const uint8_t *w[3];
@@ -57,6 +58,18 @@ struct brasa_ctx {
 // then the old one stays until the context goes, and the new one is at least half again as large, so that what stays is less than
 // twice what is in use. BRASA_EINVAL while a graph is being recorded, BRASA_ENOMEM (and no workspace) when memory runs out.
 int32_t brasa_workspace(brasa_ctx *ctx, void **p, size_t *bytes, size_t need);
+
+// While one of these lives, weights, norms and RoPE tables given to the operators were written by commands that have ended (a model's,
+// written when it is loaded), so a kernel may read them ahead of its griddepcontrol.wait. An operator called from outside gets any
+// buffer, also one that the call before it writes, and reads everything behind the wait.
+struct SettledOperands {
+    brasa_ctx *ctx;
+    bool before;
+    explicit SettledOperands(brasa_ctx *c) : ctx(c), before(c->settled) { c->settled = true; }
+    ~SettledOperands() { ctx->settled = before; }
+    SettledOperands(const SettledOperands &) = delete;
+    SettledOperands &operator=(const SettledOperands &) = delete;
+};
 
 // Launches `kernel` as a programmatic dependent of the kernel before it on the context's stream: it may start while that
 // kernel is still running and must execute griddepcontrol.wait before it touches anything that kernel produces (and the

@@ -55,6 +55,7 @@ struct PairParams {
     uint32_t n, ntok;      // tokens per tile (a multiple of 32, at most 256), token tiles
     uint32_t units, gran;  // tiles x chunks; a run begins and ends at a multiple of gran units
     uint32_t *status;
+    uint32_t settled;      // the weights may be asked for ahead of the dependency wait (SettledOperands)
     const float *resid;
     float *part;           // [2 x pairs][n tokens][256 rows]: slot 2 b is run b's tile that began before it, 2 b + 1 the one it leaves open
     __half *glu;
@@ -141,9 +142,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             tma_load_2d(dst + GP_CODES + h * 1024, &maps.scales[m], sx, row, &raw_full[r]);
         }
     };
-    // Launched as a programmatic dependent: the set-up above and the first chunks of weights (weights never change) overlap the
-    // end of the kernel before this one; what that kernel wrote (X, the residual, the workspace) is touched after the wait.
-    const uint32_t early = min(GP_RAW_SLOTS, nc);
+    // Launched as a programmatic dependent: the set-up above and a model's first chunks of weights overlap the end of the kernel before
+    // this one; what that kernel wrote (X, the residual, the workspace) is touched after the wait.
+    const uint32_t early = p.settled ? min(GP_RAW_SLOTS, nc) : 0u;
     if (tid == 0) {
         for (uint32_t ci = 0; ci < early; ++ci) issue_raw(ci);
     }
@@ -165,7 +166,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
         if (lane == 0) {  // ---- raw weight chunks ----
             uint32_t issued = early;
             for (uint32_t ci = early; ci < nc; ++ci) {
-                if (!wait(&raw_empty[ci % GP_RAW_SLOTS], ((ci / GP_RAW_SLOTS) - 1) & 1)) break;
+                if (ci >= GP_RAW_SLOTS && !wait(&raw_empty[ci % GP_RAW_SLOTS], ((ci / GP_RAW_SLOTS) - 1) & 1)) break;
                 issue_raw(ci);
                 issued = ci + 1;
             }
@@ -513,6 +514,7 @@ int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatr
     p.gran = 1;
     uint32_t pairs = std::min(sm_pairs, p.units);  // no run is empty
     p.status = ctx->status;
+    p.settled = ctx->settled;
     p.resid = resid;
     p.glu = glu;
     BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x) & 15) == 0, "gemm: misaligned x");

@@ -209,6 +209,7 @@ int32_t residual_add(brasa_model *m, brasa_cmd *cmd, uint64_t n) {
 int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32_t tokens, uint32_t pos0) {
     const brasa_config &c = m->cfg;
     Layer &l = m->layers[li];
+    const SettledOperands settled(m->ctx);
     const bool half_io = precision_for(m, tokens) == BRASA_PREFILL_F16;
     const uint32_t H = c.hidden;
     brasa_arg xin;
@@ -423,6 +424,7 @@ int32_t decode_step(brasa_model *m, brasa_cmd *cmd, uint32_t pos0) {
 
 int32_t qwen3_forward(brasa_model *m, brasa_cmd *cmd, uint32_t tokens, uint32_t pos0, const uint32_t *rows, uint32_t n_rows) {
     const brasa_config &c = m->cfg;
+    const SettledOperands settled(m->ctx);
     BRASA_TRY(brasa_k_embed(cmd, m->embed.q, A(m->ids), A(m->x), tokens));
     for (uint32_t li = 0; li < c.layers; ++li) BRASA_TRY(encode_layer_prefill(m, cmd, li, tokens, pos0));
     if (n_rows == 0) return BRASA_OK;

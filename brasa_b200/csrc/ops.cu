@@ -100,17 +100,20 @@ __global__ void __launch_bounds__(64) rms_norm_rows_kernel(const float *x, const
 
 // One block of 128 threads per row, the row in registers (n a multiple of 512, at most 512 * RMS_BLOCK_CHUNKS): one pass with
 // 16-byte loads and one block barrier. What bounds it is latency: a warp per row left 512 rows of 2 560 at three warps an SM (9.7 us a
-// launch in a prompt of 512 tokens; 3.7 us now at 1 024).
+// launch in a prompt of 512 tokens; 3.7 us now at 1 024). AHEAD: w was written long before (SettledOperands) and is asked for ahead of the
+// wait, which is most of what the kernel itself takes.
 constexpr int RMS_BLOCK_CHUNKS = 10;
-template <bool HALF_OUT>
+template <bool HALF_OUT, bool AHEAD>
 __global__ void __launch_bounds__(128) rms_norm_block_kernel(const float *x, const float *w, void *out, uint32_t n, float eps) {
     __shared__ float red[4];
     const uint32_t t = threadIdx.x, chunks = n / 512;
     const float4 *wr = reinterpret_cast<const float4 *>(w);
-    float4 wv[RMS_BLOCK_CHUNKS];
+    float4 wv[AHEAD ? RMS_BLOCK_CHUNKS : 1];
+    if constexpr (AHEAD) {
 #pragma unroll
-    for (int c = 0; c < RMS_BLOCK_CHUNKS; ++c)
-        if (c < (int)chunks) wv[c] = wr[c * 128 + t];  // (a constant: ahead of the wait)
+        for (int c = 0; c < RMS_BLOCK_CHUNKS; ++c)
+            if (c < (int)chunks) wv[c] = wr[c * 128 + t];
+    }
     asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const float4 *xr = reinterpret_cast<const float4 *>(x + (size_t)blockIdx.x * n);
@@ -131,7 +134,7 @@ __global__ void __launch_bounds__(128) rms_norm_block_kernel(const float *x, con
 #pragma unroll
     for (int c = 0; c < RMS_BLOCK_CHUNKS; ++c) {
         if (c < (int)chunks) {
-            const float4 ww = wv[c];
+            const float4 ww = AHEAD ? wv[AHEAD ? c : 0] : wr[c * 128 + t];
             const float a = v[c].x * scale * ww.x, b = v[c].y * scale * ww.y, cc = v[c].z * scale * ww.z, d = v[c].w * scale * ww.w;
             if (HALF_OUT) {
                 const __half2 h0 = __floats2half2_rn(a, b), h1 = __floats2half2_rn(cc, d);
@@ -424,7 +427,7 @@ __device__ __forceinline__ void store_elem(uint8_t *cache, size_t row, float v, 
 }
 
 // One warp per row of 128: rows of a token are hq query heads, then hkv key heads, then hkv value heads.
-template <int KV>
+template <int KV, bool AHEAD>
 __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, const float *q_norm, const float *k_norm, const float *cos_t,
                                           const float *sin_t, uint8_t *kc, uint8_t *vc, uint32_t hq, uint32_t hkv, uint32_t pos0, float eps,
                                           uint32_t rows) {
@@ -433,7 +436,8 @@ __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, co
     uint32_t per_tok = hq + 2 * hkv, t = gr / per_tok, r = gr % per_tok;
     bool is_q = r < hq;
     float wv[4], c[2], s[2];
-    if (gr < rows && r < hq + hkv) {  // constants: ahead of the wait
+    if (!AHEAD) asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
+    if (gr < rows && r < hq + hkv) {  // a model's norms and tables (SettledOperands): ahead of the wait
         const float *w = is_q ? q_norm : k_norm;
         for (int j = 0; j < 4; ++j) wv[j] = w[lane + 32 * j];
         for (int j = 0; j < 2; ++j) {
@@ -441,7 +445,7 @@ __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, co
             s[j] = sin_t[(size_t)(pos0 + t) * 64 + lane + 32 * j];
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // (launched as a programmatic dependent: see brasa_launch_dependent)
+    if (AHEAD) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (gr >= rows) return;
     if (r >= hq + hkv) {
@@ -589,8 +593,9 @@ static int32_t rms_norm_common(brasa_cmd *cmd, brasa_arg x, brasa_arg w, brasa_a
     BRASA_REQUIRE(ctx, n > 0 && arg_fits(x, tot * 4) && arg_fits(w, (uint64_t)n * 4) && arg_fits(out, tot * (half_out ? 2 : 4)), "rms_norm: buffers too small");
     if (rows == 0) return BRASA_OK;
     if (rows >= 2 && n % 512 == 0 && n <= 512 * RMS_BLOCK_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
-        if (half_out) BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<true>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
-        else BRASA_CUDA(ctx, brasa_launch_dependent(ctx, rms_norm_block_kernel<false>, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
+        auto kernel = ctx->settled ? (half_out ? rms_norm_block_kernel<true, true> : rms_norm_block_kernel<false, true>)
+                                   : (half_out ? rms_norm_block_kernel<true, false> : rms_norm_block_kernel<false, false>);
+        BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernel, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
         return brasa_post_launch(cmd, "rms_norm");
     }
     if (rows >= 256 && n % 128 == 0 && n <= 128 * RMS_MAX_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
@@ -687,7 +692,7 @@ int32_t brasa_k_qk_norm_rope_store(brasa_cmd *cmd, int32_t kv, const brasa_arg q
     if (rows == 0) return BRASA_OK;
     unsigned grid = (rows + 3) / 4;
 #define LAUNCH_QK(KVT)                                                                                                                              \
-    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, qk_norm_rope_store_kernel<KVT>, dim3(grid), dim3(128), 0, (float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]), \
+    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, ctx->settled ? qk_norm_rope_store_kernel<KVT, true> : qk_norm_rope_store_kernel<KVT, false>, dim3(grid), dim3(128), 0, (float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]), \
                                            (const float *)arg_ptr(qkv[2]), (const float *)arg_ptr(norms[0]), (const float *)arg_ptr(norms[1]),           \
                                            (const float *)arg_ptr(cos_t), (const float *)arg_ptr(sin_t), arg_ptr(dst[0]), arg_ptr(dst[1]), sh.hq, sh.hkv, \
                                            sh.pos0, eps, rows))

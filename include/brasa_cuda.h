@@ -95,6 +95,10 @@ int32_t brasa_buf_fill(brasa_buf *buf, uint64_t offset, int32_t byte, uint64_t n
 uint64_t brasa_buf_bytes(brasa_buf *buf);
 void *brasa_buf_ptr(brasa_buf *buf); /* device address */
 
+/* The calls of a command see what the calls before them wrote. Weight matrices are the one exception: kernels of neighbouring calls
+ * overlap, and a product may ask for its weights (brasa_qmatrix.data; w and w2 of brasa_linear) while the call before it is still
+ * running. They are written by transfers, fills, brasa_k_quantize and brasa_k_repack, behind which a product waits, or by a
+ * command that has ended. */
 int32_t brasa_cmd_begin(brasa_ctx *ctx, brasa_cmd **out);     /* Context::command :237 */
 int32_t brasa_cmd_commit(brasa_cmd *cmd);                     /* Command::commit :379 */
 int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds);  /* Pending::wait -> GpuTiming :411; frees cmd */

@@ -354,6 +354,45 @@ def test_qk_norm_rope_store(B, ctx, K, kv, tokens, pos0):
     assert not kc.download(np.uint8, off).any()
 
 
+@pytest.mark.parametrize("what", ["norm", "norm16", "qk"])
+def test_operands_written_by_the_call_before(B, ctx, K, what):
+    """Operators overlap their neighbours' launches, and any buffer may be a norm weight or a RoPE table, one that the call before writes
+    in the same command too: the results are those of commands that end in between."""
+    rng = O.Rng(len(what))
+    rows, n, hq, hkv, dim = 200, 1024, 8, 2, 128
+    gx, gw, g1, g2 = ctx.buffer_from(rng.vec(rows * n, 3.0)), ctx.buffer_from(rng.vec(n, 2.0)), ctx.buffer(rows * n * 4), ctx.buffer(rows * n * 4)
+    before = lambda c: K.rms_norm(c, gx, gw, g1, rows, n, 1e-6)  # its last rows are the next call's weight, or its norms and tables
+    last = (rows - 1) * n * 4
+    if what == "qk":
+        q0, k0, v0 = (rng.vec(rows * h * dim, 2.0) for h in (hq, hkv, hkv))
+        gq, gk, gv, kc, vc = ctx.buffer_from(q0), ctx.buffer_from(k0), ctx.buffer_from(v0), ctx.buffer(rows * hkv * dim * 4), ctx.buffer(rows * hkv * dim * 4)
+        table = B.RopeTable(ctx, 1e6, dim, rows)
+        table.cos, table.sin = g1.at(last - 4 * rows * 64), g1.at(last - 8 * rows * 64)
+        shape = B.AttnShape(rows, hq, hkv, dim, 0, B.KvType.F32)
+        behind = lambda c: K.qk_norm_rope_store(c, B.KvType.F32, [gq, gk, gv], [g1.at(last), g1.at(last + 512)], 1e-6, table, [kc, vc], shape)
+        outs = [gq, gk, kc]
+    else:
+        behind = lambda c: (K.rms_norm if what == "norm" else K.rms_norm_f16)(c, gx, g1.at(last), g2, rows, n, 1e-6)
+        outs = [g2]
+
+    def result(together):
+        if what == "qk":
+            gq.upload(q0)
+            gk.upload(k0)
+        g1.fill(0)
+        if together:
+            run(ctx, lambda c: (before(c), behind(c)))
+        else:
+            run(ctx, before)
+            run(ctx, behind)
+        return [o.download(np.uint32) for o in outs]
+
+    want = result(False)
+    for _ in range(10):
+        for g, w in zip(result(True), want):
+            assert np.array_equal(g, w)
+
+
 @pytest.mark.parametrize("kv", ["F32", "F16", "Q8_0"])
 def test_paged_store_and_decode_attention(B, ctx, K, kv):
     """The kernel-level paged operators: three sequences of different lengths whose 16-position pages lie scattered in
