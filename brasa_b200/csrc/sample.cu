@@ -362,11 +362,11 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
     return cut;
 }
 
-// Row r: logits[r n ..], the PCG32 state at rng + 2 r, the token at out + r. `lone`: what a row whose largest logit is not
-// finite yields, the last of its candidates when set (the end of the reference's walk, which no comparison with NaN stops), else
-// the first infinite one, or token 0. keep_steps: the dynamic shared memory holds a byte per id of a block.
+// Row r: logits[r n ..], the PCG32 state at rng + 2 r, the token at out + r. keep_steps: the dynamic shared memory holds a byte per id of
+// a block. A kept candidate whose weight is NaN (a NaN among the logits, an infinite largest one, nothing but -inf) makes the reference's
+// sums NaN, which no comparison stops: its walk ends at the last of the top_k kept candidates, and that is the token here.
 __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS, 2)
-    sample_kernel(const float *logits, uint32_t n, float temperature, uint32_t top_k, float top_p, float fix, bool lone, bool keep_steps,
+    sample_kernel(const float *logits, uint32_t n, float temperature, uint32_t top_k, float top_p, float fix, bool keep_steps,
                   unsigned long long *rng, uint32_t *out) {
     extern __shared__ __align__(16) uint8_t step_bytes[];
     __shared__ SampleShared s;
@@ -381,39 +381,38 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
     row.per_step = 8.0f / temperature;
     row.fix = fix;
     if (tid == 0) s.pass = 0;
-    uint32_t kmax = 0;
+    uint32_t kmax = 0, kmin = 0xffffffffu;
 #pragma unroll 8
-    for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) kmax = max(kmax, order_key(row.l[i]));
-    for (int o = 16; o > 0; o >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-    if (lane == 0) s.wcnt[warp] = kmax;
+    for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) {
+        const uint32_t k = order_key(row.l[i]);
+        kmax = max(kmax, k);
+        kmin = min(kmin, k);
+    }
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    if (lane == 0) s.mass[warp] = ((unsigned long long)kmax << 32) | kmin;
     for (uint32_t i = tid; i < SM_WARPS * 256; i += SM_THREADS) (&s.wh[0][0])[i] = 0;
     __syncthreads();
-    for (uint32_t w = 0; w < SM_WARPS; ++w) kmax = max(kmax, s.wcnt[w]);
-    if (tid == 0) s.word[0] = kmax;
+    for (uint32_t w = 0; w < SM_WARPS; ++w) {
+        kmax = max(kmax, (uint32_t)(s.mass[w] >> 32));
+        kmin = min(kmin, (uint32_t)s.mass[w]);
+    }
+    if (tid == 0) s.word[0] = ((unsigned long long)kmax << 32) | kmin;
     cluster_sync();
-    for (uint32_t b = 0; b < SM_CLUSTER; ++b) kmax = max(kmax, (uint32_t)cluster_load(&s.word[0], b));
+    for (uint32_t b = 0; b < SM_CLUSTER; ++b) {
+        const unsigned long long v = cluster_load(&s.word[0], b);
+        kmax = max(kmax, (uint32_t)(v >> 32));
+        kmin = min(kmin, (uint32_t)v);
+    }
     if (tid == 0) s.pass = 1;
     __syncthreads();
     row.mx = key_value(kmax);
     const unsigned long long old = rng[2 * (size_t)r], inc = rng[2 * (size_t)r + 1];
-    if (!isfinite(row.mx)) {
-        cluster_sync();  // nobody's `word` or state is needed any more
-        if (me == 0 && warp == 0) {
-            unsigned long long best = lone ? ~0ull : ((unsigned long long)n << 1);
-            for (uint32_t i = lane; i < n; i += 32) {
-                const float v = row.l[i];
-                if (lone) best = min(best, ((unsigned long long)order_key(v) << 32) | (0xffffffffu - i));
-                else if (v == INFINITY) best = min(best, (unsigned long long)i);
-            }
-            for (int o = 16; o > 0; o >>= 1) best = min(best, __shfl_xor_sync(0xffffffffu, best, o));
-            if (lane == 0) {
-                out[r] = lone ? 0xffffffffu - (uint32_t)best : (best < n ? (uint32_t)best : 0u);
-                rng[2 * (size_t)r] = old * 6364136223846793005ULL + inc;
-            }
-        }
-        return;
-    }
-    const bool counted = top_k > 0 && top_k < n;
+    // below: every candidate whose key is smaller has a NaN for its weight. to_end: some kept candidate has, whatever top_k keeps. (Every
+    // step is 255 where the largest logit or the temperature is no number, so that the count below needs no other form.)
+    const uint32_t below = order_key(-INFINITY) + (isinf(temperature) ? 1u : 0u);
+    const bool keep_all = top_k == 0 || top_k >= n, to_end = !isfinite(row.mx) || isnan(temperature) || (keep_all && kmin < below);
+    const bool counted = !keep_all || to_end;
     // mass (and count) of every step
 #pragma unroll 4
     for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) {
@@ -442,9 +441,12 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
     const uint32_t x = (uint32_t)(((old >> 18) ^ old) >> 27), rot = (uint32_t)(old >> 59);
     const uint32_t u24 = ((x >> rot) | (x << ((32 - rot) & 31))) >> 8;  // one PCG32 draw
     Prefix kept{0u, 0xffffffffu};  // everything
-    if (counted) kept = select_prefix<BOUND_COUNT>(s, row, kept, top_k, 0.0f, 0u);
-    if (top_p < 1.0f) kept = select_prefix<BOUND_SHARE>(s, row, kept, 0u, top_p, 0u);
-    const Prefix pick = select_prefix<BOUND_DRAW>(s, row, kept, 0u, 0.0f, u24);
+    if (counted) kept = select_prefix<BOUND_COUNT>(s, row, kept, keep_all ? n : top_k, 0.0f, 0u);
+    Prefix pick = kept;  // (its last candidate)
+    if (!to_end && !(counted && kept.t < below)) {
+        if (top_p < 1.0f) kept = select_prefix<BOUND_SHARE>(s, row, kept, 0u, top_p, 0u);
+        pick = select_prefix<BOUND_DRAW>(s, row, kept, 0u, 0.0f, u24);
+    }
     cluster_sync();  // every block has read the state, and the others' shared memory
     if (me == 0 && tid == 0) {
         out[r] = pick.id;
@@ -468,7 +470,7 @@ __global__ void __launch_bounds__(1024) argmax_rows_kernel(const float *logits, 
 }  // namespace
 
 // Sampler::sample for `count` rows of n logits at once: row r uses the PCG32 state at rng + 2 r; out[r] receives its token.
-static int32_t sample_launch(brasa_cmd *cmd, const float *logits, uint32_t n, uint32_t count, float temperature, uint32_t top_k, float top_p, bool lone,
+static int32_t sample_launch(brasa_cmd *cmd, const float *logits, uint32_t n, uint32_t count, float temperature, uint32_t top_k, float top_p,
                              unsigned long long *rng, uint32_t *out) {
     brasa_ctx *ctx = cmd->ctx;
     int bits = 0;
@@ -476,8 +478,8 @@ static int32_t sample_launch(brasa_cmd *cmd, const float *logits, uint32_t n, ui
     const size_t bytes = (((size_t)n + SM_CLUSTER - 1) / SM_CLUSTER + 15) / 16 * 16;
     const bool keep_steps = bytes + sizeof(SampleShared) + 4096 <= ctx->smem_optin / 2;  // (two blocks on an SM: many rows at once)
     if (keep_steps) BRASA_TRY(brasa_smem_optin(ctx, (const void *)sample_kernel, bytes));
-    sample_kernel<<<count * SM_CLUSTER, SM_THREADS, keep_steps ? bytes : 0, ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), lone,
-                                                                                          keep_steps, rng, out);
+    sample_kernel<<<count * SM_CLUSTER, SM_THREADS, keep_steps ? bytes : 0, ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), keep_steps,
+                                                                                          rng, out);
     return brasa_post_launch(cmd, "sample_top_p");
 }
 
@@ -490,7 +492,7 @@ int32_t brasa_sample_batched_launch(brasa_cmd *cmd, const float *logits, uint32_
         return brasa_post_launch(cmd, "argmax_rows");
     }
     BRASA_REQUIRE(ctx, top_p > 0.0f, "sample_top_p: top_p must be positive");
-    return sample_launch(cmd, logits, n, count, temperature, top_k, top_p, count == 1, rng, out);
+    return sample_launch(cmd, logits, n, count, temperature, top_k, top_p, rng, out);
 }
 
 int32_t brasa_advance_launch(brasa_cmd *cmd, uint32_t *ids, const uint32_t *next, uint32_t *out_ids, uint32_t *out_count, uint32_t out_cap,
@@ -531,8 +533,7 @@ int32_t brasa_k_sample_top_p(brasa_cmd *cmd, brasa_arg logits, uint32_t n, float
                   "sample_top_p: buffers too small or misaligned");
     if (temperature <= 0.0f) return brasa_argmax_launch(cmd, (const float *)arg_ptr(logits), n, (uint32_t *)arg_ptr(out_u32));
     BRASA_REQUIRE(ctx, top_p > 0.0f, "sample_top_p: top_p must be positive");
-    return sample_launch(cmd, (const float *)arg_ptr(logits), n, 1, temperature, top_k, top_p, true, (unsigned long long *)arg_ptr(rng_state),
-                         (uint32_t *)arg_ptr(out_u32));
+    return sample_launch(cmd, (const float *)arg_ptr(logits), n, 1, temperature, top_k, top_p, (unsigned long long *)arg_ptr(rng_state), (uint32_t *)arg_ptr(out_u32));
 }
 
 int32_t brasa_k_sample_rows(brasa_cmd *cmd, brasa_arg logits, uint32_t n, uint32_t count, float temperature, uint32_t top_k, float top_p,

@@ -940,6 +940,50 @@ def test_device_sampler_against_64_bits(B, ctx, K, n, top_k, top_p):
     assert checked >= 4 or n <= 9
 
 
+@pytest.mark.parametrize("n", [1, 9, 5000, 600_001])
+def test_device_sampler_rows_without_a_finite_sum(B, ctx, K, n):
+    """NaN among the logits (either sign: the total order puts one first, the other last), an infinite largest one, nothing but -inf, a
+    temperature that is infinite or no number: the reference's sums are NaN and its walk ends at the last kept candidate. The same token
+    for a row alone and among others, with and without top-k, and the state moves on by one draw. One row's NaN is outside top-k."""
+    rng = np.random.default_rng(n)
+    base = (rng.standard_normal(n) * 3.0).astype(np.float32)
+    neg_nan = np.array([0xFFC00000], np.uint32).view(np.float32)[0]
+    place, other = n // 3, 2 * n // 3
+    rows = []
+    for v in (np.nan, neg_nan, np.inf, None, -np.inf):
+        l = np.full(n, -np.inf, np.float32) if v is None else base.copy()
+        if v is not None:
+            l[[place, other]] = v
+        rows.append(l)
+    finite = base.copy()
+    finite[other] = 90.0  # a certain choice among rows that have none
+    out, out3 = ctx.buffer(4), ctx.buffer(12)
+    for temperature in (0.8, np.inf, np.nan):
+        for top_k, top_p in ((0, 1.0), (0, 0.9), (5, 0.9), (1, 1.0), (n, 0.5)):
+            for i, l in enumerate(rows):
+                if i == 4 and temperature == 0.8:
+                    continue  # masked candidates of a finite row: an ordinary draw
+                if i == 1 and 1 < top_k < n and temperature == 0.8:
+                    continue  # its NaN is not kept: likewise
+                if i == 4 and temperature == np.inf and (0 < top_k < n or n < 4):
+                    continue  # likewise
+                want = O.Sampler(temperature, top_k, top_p, seed=7).sample(l)
+                state = ctx.buffer_from(B.pcg32_state(7))
+                g = ctx.buffer_from(l)
+                run(ctx, lambda c: K.sample_top_p(c, g, n, temperature, top_k, top_p, state, out))
+                assert int(out.download(np.uint32, 1)[0]) == want, (i, temperature, top_k, top_p)
+                old, inc = (int(v) for v in B.pcg32_state(7))
+                assert int(state.download(np.uint64, 2)[0]) == (old * 6364136223846793005 + inc) % 2 ** 64
+                if n <= 5000:
+                    g = ctx.buffer_from(np.concatenate([finite, l, finite]))
+                    states, scratch = ctx.buffer_from(np.tile(B.pcg32_state(7), 3)), ctx.buffer(3 * n * 8)
+                    run(ctx, lambda c: K.sample_rows(c, g, n, 3, temperature, top_k, top_p, states, scratch, out3))
+                    got = out3.download(np.uint32, 3)
+                    assert int(got[1]) == want, (i, temperature, top_k, top_p)
+                    if temperature == 0.8:
+                        assert got[0] == got[2] == other
+
+
 def test_device_sampler_frequency_and_greedy(B, ctx, K):
     """The reference's frequency check (sampler.rs:252-267): logits (0, ln 3) at temperature 1 pick token 1 three
     times out of four; temperature 0 is the greedy argmax."""
