@@ -61,7 +61,8 @@ __global__ void rms_norm_kernel(const float *x, const float *w, void *out, uint3
 }
 
 // The same with one warp per row and the row held in registers (n a multiple of 128, at most 128 * RMS_MAX_CHUNKS):
-// one pass over x with 16-byte loads, no shared memory, two rows per block. Used from 256 rows on whose length is no multiple of 512.
+// one pass over x with 16-byte loads, no shared memory, two rows per block. Used from 256 rows on where the block-per-row form
+// below does not take them (see rms_norm_common).
 constexpr int RMS_MAX_CHUNKS = 20;
 template <bool HALF_OUT>
 __global__ void __launch_bounds__(64) rms_norm_rows_kernel(const float *x, const float *w, void *out, uint32_t rows, uint32_t n, float eps) {
@@ -592,9 +593,13 @@ static int32_t rms_norm_common(brasa_cmd *cmd, brasa_arg x, brasa_arg w, brasa_a
     uint64_t tot = (uint64_t)rows * n;
     BRASA_REQUIRE(ctx, n > 0 && arg_fits(x, tot * 4) && arg_fits(w, (uint64_t)n * 4) && arg_fits(out, tot * (half_out ? 2 : 4)), "rms_norm: buffers too small");
     if (rows == 0) return BRASA_OK;
-    if (rows >= 2 && n % 512 == 0 && n <= 512 * RMS_BLOCK_CHUNKS && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
-        auto kernel = ctx->settled ? (half_out ? rms_norm_block_kernel<true, true> : rms_norm_block_kernel<false, true>)
-                                   : (half_out ? rms_norm_block_kernel<true, false> : rms_norm_block_kernel<false, false>);
+    // A block per row costs its start and its barrier, which many short rows cannot hide: 16 384 rows of 512 take it 21.6 us and a warp per row
+    // 14.1, of 1 024 25.6 and 20.8, of 1 536 29.5 and 29.7; fewer or longer rows are its own (2 048 of 512: 5.4 and 5.0; 4 096 of 1 024: 8.2 and
+    // 8.5; 512 of 2 560: 4.8 and 7.8). The weight ahead of the wait pays in registers what few blocks on an SM do not miss (512 rows of
+    // 2 560: 3.9 us against 4.8; 4 096: 11.0 against 9.9; 16 384 of 4 096: 83 against 62).
+    if (rows >= 2 && n % 512 == 0 && n <= 512 * RMS_BLOCK_CHUNKS && (n >= 2048 || rows < 8 * n) && x.offset % 16 == 0 && w.offset % 16 == 0 && out.offset % 16 == 0) {
+        auto kernel = ctx->settled && rows <= 1024 ? (half_out ? rms_norm_block_kernel<true, true> : rms_norm_block_kernel<false, true>)
+                                                   : (half_out ? rms_norm_block_kernel<true, false> : rms_norm_block_kernel<false, false>);
         BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernel, dim3(rows), dim3(128), 0, (const float *)arg_ptr(x), (const float *)arg_ptr(w), arg_ptr(out), n, eps));
         return brasa_post_launch(cmd, "rms_norm");
     }

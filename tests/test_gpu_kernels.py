@@ -124,6 +124,21 @@ def test_rms_norm(ctx, K, rows, n):
     assert np.array_equal(gh.download(np.uint16), O.f32_to_f16_array(got))
 
 
+@pytest.mark.parametrize("rows,n", [(2, 512), (255, 1024), (4095, 512), (4096, 512), (8193, 1024), (12_288, 1536), (4100, 2048), (300, 5120), (260, 5632)])
+def test_rms_norm_by_rows_and_length(ctx, K, rows, n):
+    """Either side of the lines between a block per row and a warp per row (1 536 columns at most from 8 n rows on), the shortest and longest
+    rows that are held in registers and one beyond; each row against the norm in 64 bits, within the rounding of a 32-bit sum of n."""
+    rng = np.random.default_rng(rows + n)
+    x, w = rng.standard_normal((rows, n), np.float32), rng.standard_normal(n, np.float32)
+    gx, gw, go, gh = ctx.buffer_from(x), ctx.buffer_from(w), ctx.buffer(rows * n * 4), ctx.buffer(rows * n * 2)
+    run(ctx, lambda c: (K.rms_norm(c, gx, gw, go, rows, n, 1e-6), K.rms_norm_f16(c, gx, gw, gh, rows, n, 1e-6)))
+    got = go.download(np.float32).reshape(rows, n)
+    xd = x.astype(np.float64)
+    want = xd / np.sqrt((xd * xd).mean(axis=1, keepdims=True) + 1e-6) * w
+    assert np.max(np.abs(got - want) / np.maximum(np.abs(want), 1e-6)) <= 1e-5
+    assert np.array_equal(gh.download(np.uint16), O.f32_to_f16_array(got.ravel()))
+
+
 def test_softmax(ctx, K):
     rng = O.Rng(12)
     for rows, n in [(4, 1000), (32, 129), (1, 16384)]:
