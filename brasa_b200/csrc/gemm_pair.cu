@@ -468,10 +468,41 @@ EncodeTiledFn encode_tiled() {
 
 }  // namespace
 
-// Tokens per tile and token tiles of a product of `tokens` tokens: as few tiles of up to 256 as hold them, of equal size.
-static void pair_tokens(uint32_t tokens, uint32_t *n, uint32_t *ntok) {
-    *ntok = (tokens + 255) / 256;
-    *n = ((tokens + *ntok - 1) / *ntok + 31) / 32 * 32;
+// How a product is cut: token tiles of equal size (as few of up to `most` as hold the tokens), runs of whole tiles or even ones.
+struct PairPlan {
+    uint32_t n, ntok, units, pairs, gran;
+    double cost;
+};
+static PairPlan pair_plan(uint32_t sm_pairs, uint32_t tiles, uint32_t cpt, uint32_t tokens, uint32_t most, bool glu) {
+    PairPlan p{};
+    p.ntok = (tokens + most - 1) / most;
+    p.n = ((tokens + p.ntok - 1) / p.ntok + 31) / 32 * 32;
+    p.units = tiles * p.ntok * cpt;
+    p.pairs = std::min(sm_pairs, p.units);  // no run is empty
+    p.gran = 1;
+    // Runs of whole tiles, or even ones that cut tiles: which is shorter, in chunks. Cut tiles cost their parts' way through memory and the
+    // kernel behind: 10 chunks' time for 256 tokens a tile, 7 for 128; 4 where that kernel also takes SwiGLU off the blocks. 3 584 tokens: qkv 99 us
+    // whole, 109 cut; o 70, 83; down 141, 156; gate / up 322, 320. 512 tokens: qkv 29, 35; gate / up 73, 66.
+    uint32_t chunks = (p.units + p.pairs - 1) / p.pairs;
+    const uint32_t whole = (tiles * p.ntok + p.pairs - 1) / p.pairs * cpt;
+    const bool cut = whole > chunks + 4 + (glu ? 0 : p.n / 42);
+    if (!cut) {
+        chunks = whole;
+        p.gran = cpt;
+        p.pairs = std::min(sm_pairs, p.units / cpt);
+    }
+    p.cost = chunks * (1.0 + p.n / 1280.0) + p.n / 60.0 + (cut ? 4.0 + p.n / 25.0 : 0.0);
+    return p;
+}
+
+// Tiles of up to 256 tokens, or of up to 128 where that is shorter by more than 3 %. A chunk takes 1.18 us with 256 tokens and 1.07 with 128 (the
+// conversion of its weights takes the most of both), the last tile's way out of tensor memory and the launch 10.8 and 8.0: a product of
+// few tiles, whose runs are a handful of chunks, is its way in and out, and twice the tiles cost it nothing while pairs are idle. us with
+// 256 and with 128: 256 x 256, 256 tokens 12.0, 9.1; 1 024 x 2 560 22.0, 16.6; 2 560 x 2 560, 512 tokens 22.6, 18.7; 1 000 tokens 25.0,
+// 27.9; 2 560 x 9 728, 256 tokens 30.0, 25.9; 512 tokens 34.2, 36.3. The costs are in chunks.
+static PairPlan pair_plan(uint32_t sm_pairs, uint32_t tiles, uint32_t cpt, uint32_t tokens, bool glu) {
+    const PairPlan wide = pair_plan(sm_pairs, tiles, cpt, tokens, 256, glu), narrow = pair_plan(sm_pairs, tiles, cpt, tokens, 128, glu);
+    return narrow.cost < 0.97 * wide.cost ? narrow : wide;
 }
 
 // True when brasa_gemm_pair_launch takes the product (every matrix q4_0 tiled and 16-byte aligned): rows in whole tiles (256; gate
@@ -486,7 +517,7 @@ bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tok
         if ((reinterpret_cast<uintptr_t>(arg_ptr(ws[i].data)) & 15) != 0) return false;
         tiles += ws[i].rows / (glu ? 128 : 256);
     }
-    return tiles * ((tokens + 255) / 256) * (ws[0].cols / GP_CHUNK) < (1ull << 31);
+    return tiles * ((tokens + 127) / 128) * (ws[0].cols / GP_CHUNK) < (1ull << 31);
 }
 
 // Y_i = W_i X (+ resid, one matrix), or out = f16(silu(W_0 X) * (W_1 X)): the arguments of brasa_gemm_tc_launch.
@@ -507,25 +538,19 @@ int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatr
         if (glu) tiles = ws[0].rows / 128;
         p.tile_end[i] = tiles;
     }
-    pair_tokens(tokens, &p.n, &p.ntok);
+    const PairPlan plan = pair_plan(sm_pairs, tiles, cpt, tokens, glu != nullptr);
+    uint32_t pairs = plan.pairs;
+    p.n = plan.n;
+    p.ntok = plan.ntok;
+    p.units = plan.units;
+    p.gran = plan.gran;
     p.cols = cols;
     p.tokens = tokens;
-    p.units = tiles * p.ntok * cpt;
-    p.gran = 1;
-    uint32_t pairs = std::min(sm_pairs, p.units);  // no run is empty
     p.status = ctx->status;
     p.settled = ctx->settled;
     p.resid = resid;
     p.glu = glu;
     BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x) & 15) == 0, "gemm: misaligned x");
-    // Runs of whole tiles, or even ones that cut tiles: which is shorter, in chunks. Cut tiles cost their parts' way through memory and the
-    // kernel behind: 10 chunks' time for 256 tokens a tile, 7 for 128; 4 where that kernel also takes SwiGLU off the blocks. 3 584 tokens: qkv 99 us
-    // whole, 109 cut; o 70, 83; down 141, 156; gate / up 322, 320. 512 tokens: qkv 29, 35; gate / up 73, 66.
-    const uint32_t whole = (tiles * p.ntok + pairs - 1) / pairs * cpt;
-    if (whole <= (p.units + pairs - 1) / pairs + 4 + (glu ? 0 : p.n / 42)) {
-        p.gran = cpt;
-        pairs = std::min(sm_pairs, p.units / cpt);
-    }
     bool shared = false;  // some run begins inside a tile
     for (uint32_t b = 1; b < pairs; ++b) shared = shared || pair_begin(b, pairs, p.units, p.gran) % cpt != 0;
     if (shared) {

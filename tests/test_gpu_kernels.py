@@ -756,6 +756,30 @@ def test_gemm_cta_pairs(B, ctx, K, rows, cols, tokens):
     assert np.all(np.abs(got - o) <= 1e-5 * (np.abs(wu) * 1.1 * s + np.abs(w) * su) + np.abs(o) * 2.0 ** -10 + 1e-7)
 
 
+@pytest.mark.parametrize("rows,cols,tokens", [(256, 256, 129), (256, 256, 1000), (1024, 2560, 256), (2560, 512, 700), (2560, 512, 1000), (512, 9728, 256), (512, 9728, 400),
+                                              (4096, 256, 1500)])
+def test_gemm_cta_pairs_with_narrow_token_tiles(B, ctx, K, rows, cols, tokens):
+    """Products of few tiles take their tokens in tiles of up to 128 instead of 256 (either side of that line, whole and cut runs), as do
+    their residual and SwiGLU forms: the oracle's sums within the bound of the reference's GEMM test."""
+    rng = O.Rng(rows + tokens)
+    raw, uraw = rng.qmatrix(O.Q4_0, rows, cols), rng.qmatrix(O.Q4_0, rows, cols)
+    w, up = (tiled(B, ctx, K, "q4_0", m, rows, cols)[0] for m in (raw, uraw))
+    x, acc0 = rng.vec(tokens * cols, 1.0), rng.vec(tokens * rows, 2.0)
+    gx, gy, gs, ga = ctx.buffer_from(x.astype(np.float16)), ctx.buffer(tokens * rows * 4), ctx.buffer(tokens * rows * 4), ctx.buffer_from(acc0)
+    gy.fill(0xFF)
+    run(ctx, lambda c: (K.gemm(c, w, gx, gy, tokens), K.gemm_add(c, w, gx, ga, gs, tokens)))
+    want, s = O.matmul(O.Q4_0, raw, rows, cols, x, f16_inputs=True)
+    assert np.max(np.abs(gy.download(np.float32).reshape(tokens, rows) - want) / s) <= 1e-5
+    d = np.abs(ga.download(np.float32).reshape(tokens, rows) - (want + acc0.reshape(tokens, rows)))
+    assert np.all(d <= 1e-5 * s + 2.0 ** -23 * (np.abs(want) + np.abs(acc0.reshape(tokens, rows))))
+    go = ctx.buffer(tokens * rows * 2)
+    run(ctx, lambda c: K.gemm_swiglu(c, w, up, gx, gy, gs, go, tokens))
+    wu, su = O.matmul(O.Q4_0, uraw, rows, cols, x, f16_inputs=True)
+    o = O.swiglu(want, wu).reshape(tokens, rows)
+    got = go.download(np.float16).astype(np.float32).reshape(tokens, rows)
+    assert np.all(np.abs(got - o) <= 1e-5 * (np.abs(wu) * 1.1 * s + np.abs(want) * su) + np.abs(o) * 2.0 ** -10 + 1e-7)
+
+
 @pytest.mark.parametrize("kv", ["F16", "Q8_0"])
 @pytest.mark.parametrize("hq,hkv,tokens,pos0", [(8, 2, 130, 3000), (3, 1, 300, 2100), (5, 5, 1, 1400), (32, 8, 700, 0), (32, 32, 333, 50), (6, 2, 257, 1000), (2, 1, 40, 5000)])
 def test_flash_attention_query_tile_pairs(B, ctx, K, kv, hq, hkv, tokens, pos0):
