@@ -498,18 +498,24 @@ static PairPlan pair_plan(uint32_t sm_pairs, uint32_t tiles, uint32_t cpt, uint3
         p.gran = cpt;
         p.pairs = std::min(sm_pairs, p.units / cpt);
     }
-    p.cost = chunks * (1.0 + p.n / 1280.0) + p.n / 60.0 + (cut ? 4.0 + p.n / 25.0 : 0.0);
+    p.cost = chunks * (1.0 + p.n / 1100.0) + p.n / 140.0 + (cut ? p.n / 20.0 : 0.0);
     return p;
 }
 
-// Tiles of up to 256 tokens, or of up to 128 where that is shorter by more than 3 %. A chunk takes 1.18 us with 256 tokens and 1.07 with 128 (the
-// conversion of its weights takes the most of both), the last tile's way out of tensor memory and the launch 10.8 and 8.0: a product of
-// few tiles, whose runs are a handful of chunks, is its way in and out, and twice the tiles cost it nothing while pairs are idle. us with
-// 256 and with 128: 256 x 256, 256 tokens 12.0, 9.1; 1 024 x 2 560 22.0, 16.6; 2 560 x 2 560, 512 tokens 22.6, 18.7; 1 000 tokens 25.0,
-// 27.9; 2 560 x 9 728, 256 tokens 30.0, 25.9; 512 tokens 34.2, 36.3. The costs are in chunks.
+// Token tiles of the width, 256 down to 64, that ends soonest. The costs are in chunks and follow 670 products of 14 matrices, of whose best width
+// they miss 0.3 % on average: a chunk takes a little longer the more tokens there are (the conversion of its weights takes the most of it), and
+// so does the last tile's way out, the more so through a workspace. A product of few tiles, whose runs are a handful of chunks, is its way in
+// and out, and more tiles cost it nothing while pairs are idle; one of little more than a wave of tiles gets by with a chunk less. us with 256,
+// 128 and 64: 256 x 256, 256 tokens 12.0, 9.1, 8.4; 1 024 x 2 560 22.0, 16.6, 14.5; 2 560 x 2 560, 512 tokens 22.6, 18.7, 25.4; 1 000 tokens
+// 25.0, 27.9, 38.4; 2 560 x 9 728, 256 tokens 30.0, 25.9, 33.4; 512 tokens 34.2, 36.3, 55.4; 2 560 x 512, 2 000 tokens 22.1, 20.7, 27.7, with
+// 160 19.4. Up to 96 tokens one tile holds them all (two of 64 cost 3 to 13 % more).
 static PairPlan pair_plan(uint32_t sm_pairs, uint32_t tiles, uint32_t cpt, uint32_t tokens, bool glu) {
-    const PairPlan wide = pair_plan(sm_pairs, tiles, cpt, tokens, 256, glu), narrow = pair_plan(sm_pairs, tiles, cpt, tokens, 128, glu);
-    return narrow.cost < 0.97 * wide.cost ? narrow : wide;
+    PairPlan best = pair_plan(sm_pairs, tiles, cpt, tokens, 256, glu);
+    for (uint32_t most = 224; most >= 64 && tokens > 96; most -= 32) {
+        const PairPlan p = pair_plan(sm_pairs, tiles, cpt, tokens, most, glu);
+        if (p.cost < best.cost) best = p;
+    }
+    return best;
 }
 
 // True when brasa_gemm_pair_launch takes the product (every matrix q4_0 tiled and 16-byte aligned): rows in whole tiles (256; gate
@@ -524,7 +530,7 @@ bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tok
         if ((reinterpret_cast<uintptr_t>(arg_ptr(ws[i].data)) & 15) != 0) return false;
         tiles += ws[i].rows / (glu ? 128 : 256);
     }
-    return tiles * ((tokens + 127) / 128) * (ws[0].cols / GP_CHUNK) < (1ull << 31);
+    return tiles * ((tokens + 63ull) / 64) * (ws[0].cols / GP_CHUNK) < (1ull << 31);
 }
 
 // Y_i = W_i X (+ resid, one matrix), or out = f16(silu(W_0 X) * (W_1 X)): the arguments of brasa_gemm_tc_launch.

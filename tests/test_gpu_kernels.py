@@ -757,10 +757,10 @@ def test_gemm_cta_pairs(B, ctx, K, rows, cols, tokens):
 
 
 @pytest.mark.parametrize("rows,cols,tokens", [(256, 256, 129), (256, 256, 1000), (1024, 2560, 256), (2560, 512, 700), (2560, 512, 1000), (512, 9728, 256), (512, 9728, 400),
-                                              (4096, 256, 1500)])
+                                              (4096, 256, 1500), (2560, 512, 2000), (512, 512, 70)])
 def test_gemm_cta_pairs_with_narrow_token_tiles(B, ctx, K, rows, cols, tokens):
-    """Products of few tiles take their tokens in tiles of up to 128 instead of 256 (either side of that line, whole and cut runs), as do
-    their residual and SwiGLU forms: the oracle's sums within the bound of the reference's GEMM test."""
+    """Products of few tiles take their tokens in narrower tiles (from 256 down to 64, whole and cut runs), as do their residual and SwiGLU
+    forms: the oracle's sums within the bound of the reference's GEMM test."""
     rng = O.Rng(rows + tokens)
     raw, uraw = rng.qmatrix(O.Q4_0, rows, cols), rng.qmatrix(O.Q4_0, rows, cols)
     w, up = (tiled(B, ctx, K, "q4_0", m, rows, cols)[0] for m in (raw, uraw))
