@@ -533,6 +533,23 @@ bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tok
     return tiles * ((tokens + 63ull) / 64) * (ws[0].cols / GP_CHUNK) < (1ull << 31);
 }
 
+// True when gemm_tc_kernel is ahead on a product that the pairs take: more than a wave of tiles of few K chunks. The conversion threads drain
+// a tile themselves, and behind a handful of chunks the products wait for that; gemm_tc_kernel has twice the blocks, each with a tile of its
+// own. Both sides in us by waves (of pairs, of SMs) and chunks a tile, plain and SwiGLU, from 250 products of 256 to 1 536 columns. us, pairs
+// and gemm_tc: SwiGLU of 4 096 x 256 at 1 024 tokens 25.6, 18.9; x 512 29.5, 22.9; x 1 024 34.2, 30.0; at 8 192 tokens 200, 193; 2 560 x 512 at
+// 3 584 52.2, 42.6; plain 4 096 x 256 at 2 048 18.8, 16.4; x 512 22.8, 20.3. A product with a residual is the pairs' everywhere (0.74 at most).
+bool brasa_gemm_pair_behind(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool resid, bool glu) {
+    const uint32_t sms = (uint32_t)ctx->sm_count, cpt = ws[0].cols / GP_CHUNK;
+    if (resid || (!glu && cpt > 3)) return false;
+    uint32_t tiles = 0;
+    for (uint32_t i = 0; i < (glu ? 1 : count); ++i) tiles += ws[i].rows / (glu ? 128 : 256);
+    const uint32_t units = tiles * ((tokens + 255) / 256), pair_waves = (units + sms / 2 - 1) / (sms / 2), sm_waves = (units + sms - 1) / sms;
+    if (pair_waves < 2) return false;
+    const double pairs = glu ? 6.6 + pair_waves * (8.4 + 1.3 * cpt) : 4.7 + 1.35 * cpt + pair_waves * (5.15 + 1.25 * cpt);
+    const double tc = glu ? 3.2 + sm_waves * (12.0 + 3.6 * cpt) : 3.7 + sm_waves * (9.05 + 3.7 * cpt);
+    return 1.05 * tc < pairs;
+}
+
 // Y_i = W_i X (+ resid, one matrix), or out = f16(silu(W_0 X) * (W_1 X)): the arguments of brasa_gemm_tc_launch.
 int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, const __half *x, float *const *ys, uint32_t tokens, const float *resid,
                                __half *glu) {

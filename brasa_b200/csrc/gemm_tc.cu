@@ -14,7 +14,7 @@
 //   * after the last stage warps 4-11 read the accumulators (tcgen05.ld, one token per lane) and store Y.
 // Up to three matrices that share X (q, k, v) go into one launch: the grid's x index walks their 128-row tiles.
 // More than 64 tokens of q4_0 matrices in whole tiles of 256 rows go to gemm_pair.cu, 9 to 64 to the few-token kernel below: this
-// kernel serves what is left (rows an odd number of 128; the q6_0 head).
+// kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
 // Every wait is bounded: a wait that runs out raises the context's status word and a CTA-wide flag, every role
 // leaves its loop, tensor memory is freed and the kernel returns.
 #include <cuda.h>
@@ -32,6 +32,7 @@
 using namespace brasa_dev;
 
 bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool glu);  // gemm_pair.cu
+bool brasa_gemm_pair_behind(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool resid, bool glu);
 int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, const __half *x, float *const *ys, uint32_t tokens, const float *resid,
                                __half *glu);
 
@@ -1177,7 +1178,8 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
                (uint64_t)tiles128 * (ws[0].cols / BK) * (uint64_t)(ctx->sm_count + 1) < (1ull << 32);
     for (uint32_t i = 0; i < count; ++i) few = few && ws[i].qtype == BRASA_Q4_0;
     if (few) return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
-    if (brasa_gemm_pair_takes(ws, count, tokens, glu != nullptr)) return brasa_gemm_pair_launch(cmd, count, ws, x, ys, tokens, resid, glu);
+    if (brasa_gemm_pair_takes(ws, count, tokens, glu != nullptr) && !brasa_gemm_pair_behind(ctx, ws, count, tokens, resid != nullptr, glu != nullptr))
+        return brasa_gemm_pair_launch(cmd, count, ws, x, ys, tokens, resid, glu);
     // Shape of a CTA: MT token tiles of 128 x NB weight tiles of 128 rows (MT x NB x 128 accumulator columns <= 512).
     // Every CTA reads its token tiles' X once per launch, so X crosses L2 -> SM (weight tiles / NB) times: the
     // estimate is the larger of that traffic at about 4.5 TB/s and waves x stages x cycles per stage of one CTA.

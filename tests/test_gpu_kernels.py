@@ -780,6 +780,29 @@ def test_gemm_cta_pairs_with_narrow_token_tiles(B, ctx, K, rows, cols, tokens):
     assert np.all(np.abs(got - o) <= 1e-5 * (np.abs(wu) * 1.1 * s + np.abs(want) * su) + np.abs(o) * 2.0 ** -10 + 1e-7)
 
 
+@pytest.mark.parametrize("rows,cols,tokens", [(4096, 256, 1024), (1024, 1024, 3584), (2560, 512, 2100), (9600, 256, 70), (640, 256, 8192), (4096, 1536, 1024)])
+def test_gemm_of_few_columns_and_many_tokens(B, ctx, K, rows, cols, tokens):
+    """Plain and SwiGLU products either side of the line between the pairs and gemm_tc_kernel: a bit more than a wave of tiles, several waves, few
+    tokens over many rows. 64 tokens of each (the first, the last, the tiles' edges) against the oracle's sums."""
+    rng = O.Rng(rows + tokens)
+    raw, uraw = rng.qmatrix(O.Q4_0, rows, cols), rng.qmatrix(O.Q4_0, rows, cols)
+    w, up = (tiled(B, ctx, K, "q4_0", m, rows, cols)[0] for m in (raw, uraw))
+    x = rng.vec(tokens * cols, 1.0)
+    gx, gy, gs, go = ctx.buffer_from(x.astype(np.float16)), ctx.buffer(tokens * rows * 4), ctx.buffer(tokens * rows * 4), ctx.buffer(tokens * rows * 2)
+    gy.fill(0xFF)
+    run(ctx, lambda c: K.gemm(c, w, gx, gy, tokens))
+    pick = np.unique(np.concatenate([np.arange(0, tokens, max(1, tokens // 40)), np.arange(127, tokens, 128)[:16], [tokens - 1, min(tokens - 1, 256)]]))
+    xs = np.ascontiguousarray(x.reshape(tokens, cols)[pick]).ravel()
+    want, s = O.matmul(O.Q4_0, raw, rows, cols, xs, f16_inputs=True)
+    y = gy.download(np.float32).reshape(tokens, rows)
+    assert np.all(np.isfinite(y)) and np.max(np.abs(y[pick] - want) / s) <= 1e-5
+    run(ctx, lambda c: K.gemm_swiglu(c, w, up, gx, gy, gs, go, tokens))
+    wu, su = O.matmul(O.Q4_0, uraw, rows, cols, xs, f16_inputs=True)
+    o = O.swiglu(want, wu).reshape(len(pick), rows)
+    got = go.download(np.float16).astype(np.float32).reshape(tokens, rows)[pick]
+    assert np.all(np.abs(got - o) <= 1e-5 * (np.abs(wu) * 1.1 * s + np.abs(want) * su) + np.abs(o) * 2.0 ** -10 + 1e-7)
+
+
 @pytest.mark.parametrize("kv", ["F16", "Q8_0"])
 @pytest.mark.parametrize("hq,hkv,tokens,pos0", [(8, 2, 130, 3000), (3, 1, 300, 2100), (5, 5, 1, 1400), (32, 8, 700, 0), (32, 32, 333, 50), (6, 2, 257, 1000), (2, 1, 40, 5000)])
 def test_flash_attention_query_tile_pairs(B, ctx, K, kv, hq, hkv, tokens, pos0):
