@@ -85,8 +85,8 @@ __global__ void advance_kernel(uint32_t *ids, const uint32_t *next, uint32_t *ou
 // Masses are 64-bit fixed point (weight x 2^k with n 2^k <= 2^62, truncated): sums do not depend on the order of the
 // additions, and what truncation loses is below 2^-26 of the largest weight for 2^18 candidates, a quarter of one rounding
 // of the f32 sums the reference forms.
-// A row is one cluster of eight blocks, each with an eighth of the ids; histograms meet through distributed shared memory, one cluster
-// barrier per histogram. The logits are read twice, for the maximum and for the first histogram, which also leaves every id's step as a
+// A row is one cluster of eight blocks, each with an eighth of the ids, or one block (see sample_launch); a cluster's histograms meet through
+// distributed shared memory, one cluster barrier per histogram. The logits are read twice, for the maximum and for the first histogram, which also leaves every id's step as a
 // byte in shared memory; the later passes look at four steps per word and touch the few logits that match (vocabularies too long for
 // that work the step out again). Bound: latency, some ten passes of a barrier each. One row of 151 936: 79 us (3 840 with one block a row
 // that bisected over the whole row, 158 with every pass over the logits); a step of 64 rows 113 us (240 as eleven launches).
@@ -107,18 +107,26 @@ __device__ __forceinline__ float key_value(uint32_t k) {  // inverse of order_ke
 }
 __device__ __forceinline__ bool in_prefix(uint32_t key, uint32_t id, Prefix p) { return key > p.t || (key == p.t && id <= p.id); }
 
-constexpr int SM_THREADS = 512, SM_WARPS = SM_THREADS / 32, SM_CLUSTER = 8;
+constexpr int SM_THREADS = 512, SM_WARPS = SM_THREADS / 32, SM_CLUSTER = 8;  // (a row's blocks: CL, 1 or SM_CLUSTER)
 
+template <int CL>
 __device__ __forceinline__ uint32_t cluster_rank() {
-    uint32_t r;
-    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    uint32_t r = 0;
+    if (CL > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
     return r;
 }
+template <int CL>
 __device__ __forceinline__ void cluster_sync() {
+    if (CL == 1) {
+        __syncthreads();
+        return;
+    }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+template <int CL>
 __device__ __forceinline__ unsigned long long cluster_load(const unsigned long long *local, uint32_t rank) {  // the same word of block `rank`
+    if (CL == 1) return *local;
     const uint32_t a = (uint32_t)__cvta_generic_to_shared(local);
     uint32_t remote;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(a), "r"(rank));
@@ -137,14 +145,15 @@ struct SampleShared {
 };
 
 // The sum over the cluster of one number per block, and the sum over the blocks before this one.
+template <int CL>
 __device__ unsigned long long cluster_sum(SampleShared &s, unsigned long long mine, unsigned long long &before) {
-    const uint32_t buf = s.pass & 1, me = cluster_rank();
+    const uint32_t buf = s.pass & 1, me = cluster_rank<CL>();
     if (threadIdx.x == 0) s.word[buf] = mine;
-    cluster_sync();
+    cluster_sync<CL>();
     unsigned long long all = 0;
     before = 0;
-    for (uint32_t r = 0; r < SM_CLUSTER; ++r) {
-        const unsigned long long v = cluster_load(&s.word[buf], r);
+    for (uint32_t r = 0; r < CL; ++r) {
+        const unsigned long long v = cluster_load<CL>(&s.word[buf], r);
         all += v;
         if (r < me) before += v;
     }
@@ -192,10 +201,11 @@ __device__ __forceinline__ void block_hist(SampleShared &s, uint32_t buf) {
         s.hist[buf][threadIdx.x] = a;
     }
 }
+template <int CL>
 __device__ __forceinline__ unsigned long long cluster_bin(const SampleShared &s, uint32_t buf) {  // thread < 256: its bin over the cluster
     unsigned long long h = 0;
 #pragma unroll
-    for (uint32_t r = 0; r < SM_CLUSTER; ++r) h += cluster_load(&s.hist[buf][threadIdx.x], r);
+    for (uint32_t r = 0; r < CL; ++r) h += cluster_load<CL>(&s.hist[buf][threadIdx.x], r);
     return h;
 }
 // The first bin at which `above` and the bins so far reach s.bound: into s.bin, what lies before it into s.above. h: thread's bin (thread
@@ -237,7 +247,7 @@ enum SampleBound { BOUND_COUNT, BOUND_SHARE, BOUND_DRAW };
 
 // Narrows `inside` to its shortest prefix whose mass reaches the bound (top_k candidates; top_p of its mass; u24 / 2^24 of
 // its mass, at least one unit). s.mass and s.count are those of `inside`, and of the narrowed one afterwards unless it is the draw.
-template <SampleBound KIND>
+template <SampleBound KIND, int CL>
 __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix inside, uint32_t top_k, float top_p, uint32_t u24) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, len = row.hi - row.lo;
     pick_bin(s, tid < 256 ? (KIND == BOUND_COUNT ? s.count[tid] : s.mass[tid]) : 0ull, true, [&](unsigned long long total) -> unsigned long long {
@@ -267,8 +277,8 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
             }
         }
         block_hist(s, buf);
-        cluster_sync();
-        const unsigned long long h = tid < 256 ? cluster_bin(s, buf) : 0ull;
+        cluster_sync<CL>();
+        const unsigned long long h = tid < 256 ? cluster_bin<CL>(s, buf) : 0ull;
         __syncthreads();
         if (tid == 0) ++s.pass;
         pick_bin(s, h, false, [](unsigned long long) { return 0ull; });
@@ -297,7 +307,7 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
         mine += s.wcnt[w];
     }
     unsigned long long before;
-    cluster_sum(s, mine, before);
+    cluster_sum<CL>(s, mine, before);
     before += before_warp;
     if (tid == 0) s.hit = 0;
     __syncthreads();
@@ -323,7 +333,7 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
     }
     __syncthreads();
     unsigned long long unused;
-    const unsigned long long id1 = cluster_sum(s, s.hit, unused);
+    const unsigned long long id1 = cluster_sum<CL>(s, s.hit, unused);
     const Prefix cut{pref, (uint32_t)id1 - 1};
     if (KIND != BOUND_DRAW) {  // what the narrowed prefix holds of each step
         unsigned long long c = 0, w = 0;
@@ -351,8 +361,8 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
             c += s.wh[k][0];
             w += s.wh[k][1];
         }
-        c = cluster_sum(s, c, unused);
-        w = cluster_sum(s, w, unused);
+        c = cluster_sum<CL>(s, c, unused);
+        w = cluster_sum<CL>(s, w, unused);
         if (tid < 256 && tid >= step) {
             s.count[tid] = tid == step ? c : 0ull;
             s.mass[tid] = tid == step ? w : 0ull;
@@ -365,13 +375,14 @@ __device__ Prefix select_prefix(SampleShared &s, const SampleRow &row, Prefix in
 // Row r: logits[r n ..], the PCG32 state at rng + 2 r, the token at out + r. keep_steps: the dynamic shared memory holds a byte per id of
 // a block. A kept candidate whose weight is NaN (a NaN among the logits, an infinite largest one, nothing but -inf) makes the reference's
 // sums NaN, which no comparison stops: its walk ends at the last of the top_k kept candidates, and that is the token here.
-__global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS, 2)
+template <int CL>
+__global__ void __cluster_dims__(CL, 1, 1) __launch_bounds__(SM_THREADS, 2)
     sample_kernel(const float *logits, uint32_t n, float temperature, uint32_t top_k, float top_p, float fix, bool keep_steps,
                   unsigned long long *rng, uint32_t *out) {
     extern __shared__ __align__(16) uint8_t step_bytes[];
     __shared__ SampleShared s;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.x / SM_CLUSTER, me = cluster_rank();
-    const uint32_t seg = (uint32_t)(((uint64_t)n + SM_CLUSTER - 1) / SM_CLUSTER);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = blockIdx.x / CL, me = cluster_rank<CL>();
+    const uint32_t seg = (uint32_t)(((uint64_t)n + CL - 1) / CL);
     SampleRow row;
     row.l = logits + (size_t)r * n;
     row.lo = (uint32_t)min((uint64_t)n, (uint64_t)me * seg);
@@ -398,9 +409,9 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
         kmin = min(kmin, (uint32_t)s.mass[w]);
     }
     if (tid == 0) s.word[0] = ((unsigned long long)kmax << 32) | kmin;
-    cluster_sync();
-    for (uint32_t b = 0; b < SM_CLUSTER; ++b) {
-        const unsigned long long v = cluster_load(&s.word[0], b);
+    cluster_sync<CL>();
+    for (uint32_t b = 0; b < CL; ++b) {
+        const unsigned long long v = cluster_load<CL>(&s.word[0], b);
         kmax = max(kmax, (uint32_t)(v >> 32));
         kmin = min(kmin, (uint32_t)v);
     }
@@ -423,8 +434,8 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
         if (w) atomicAdd(&s.wh[warp][at], w);
     }
     block_hist(s, 1);
-    cluster_sync();
-    if (tid < 256) s.mass[tid] = cluster_bin(s, 1);
+    cluster_sync<CL>();
+    if (tid < 256) s.mass[tid] = cluster_bin<CL>(s, 1);
     __syncthreads();
     if (tid == 0) s.pass = 2;
     if (counted) {
@@ -432,8 +443,8 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
         __syncthreads();
         for (uint32_t i = row.lo + tid; i < row.hi; i += SM_THREADS) atomicAdd(&s.wh[warp][keep_steps ? step_bytes[i - row.lo] : row.step(row.l[i])], 1ull);
         block_hist(s, 0);
-        cluster_sync();
-        if (tid < 256) s.count[tid] = cluster_bin(s, 0);
+        cluster_sync<CL>();
+        if (tid < 256) s.count[tid] = cluster_bin<CL>(s, 0);
         __syncthreads();
         if (tid == 0) s.pass = 3;
     }
@@ -441,13 +452,13 @@ __global__ void __cluster_dims__(SM_CLUSTER, 1, 1) __launch_bounds__(SM_THREADS,
     const uint32_t x = (uint32_t)(((old >> 18) ^ old) >> 27), rot = (uint32_t)(old >> 59);
     const uint32_t u24 = ((x >> rot) | (x << ((32 - rot) & 31))) >> 8;  // one PCG32 draw
     Prefix kept{0u, 0xffffffffu};  // everything
-    if (counted) kept = select_prefix<BOUND_COUNT>(s, row, kept, keep_all ? n : top_k, 0.0f, 0u);
+    if (counted) kept = select_prefix<BOUND_COUNT, CL>(s, row, kept, keep_all ? n : top_k, 0.0f, 0u);
     Prefix pick = kept;  // (its last candidate)
     if (!to_end && !(counted && kept.t < below)) {
-        if (top_p < 1.0f) kept = select_prefix<BOUND_SHARE>(s, row, kept, 0u, top_p, 0u);
-        pick = select_prefix<BOUND_DRAW>(s, row, kept, 0u, 0.0f, u24);
+        if (top_p < 1.0f) kept = select_prefix<BOUND_SHARE, CL>(s, row, kept, 0u, top_p, 0u);
+        pick = select_prefix<BOUND_DRAW, CL>(s, row, kept, 0u, 0.0f, u24);
     }
-    cluster_sync();  // every block has read the state, and the others' shared memory
+    cluster_sync<CL>();  // every block has read the state, and the others' shared memory
     if (me == 0 && tid == 0) {
         out[r] = pick.id;
         rng[2 * (size_t)r] = old * 6364136223846793005ULL + inc;
@@ -475,11 +486,19 @@ static int32_t sample_launch(brasa_cmd *cmd, const float *logits, uint32_t n, ui
     brasa_ctx *ctx = cmd->ctx;
     int bits = 0;
     while (bits < 32 && (1ull << bits) < n) ++bits;
-    const size_t bytes = (((size_t)n + SM_CLUSTER - 1) / SM_CLUSTER + 15) / 16 * 16;
-    const bool keep_steps = bytes + sizeof(SampleShared) + 4096 <= ctx->smem_optin / 2;  // (two blocks on an SM: many rows at once)
-    if (keep_steps) BRASA_TRY(brasa_smem_optin(ctx, (const void *)sample_kernel, bytes));
-    sample_kernel<<<count * SM_CLUSTER, SM_THREADS, keep_steps ? bytes : 0, ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), keep_steps,
-                                                                                          rng, out);
+    // A row in one block saves the cluster barriers and a wave of blocks for every 37 rows; in a cluster it saves seven eighths of the walks over
+    // the logits. us for one row, 64 and 200, one block and cluster: 50 logits 25, 39; 27, 84; 31, 254; 8 000 logits 39, 42; 43, 92; 52, 281;
+    // 32 768 logits 102, 48; 104, 109; 129, 333. The steps of a long row do not fit one block's memory: a cluster then.
+    auto step_bytes = [&](uint32_t blocks) { return (((size_t)n + blocks - 1) / blocks + 15) / 16 * 16; };
+    auto fits = [&](uint32_t blocks) { return step_bytes(blocks) + sizeof(SampleShared) + 4096 <= ctx->smem_optin / 2; };  // (two blocks on an SM: many rows at once)
+    const uint64_t waves = ((uint64_t)count * SM_CLUSTER + 2 * ctx->sm_count - 1) / (2 * ctx->sm_count);
+    const uint32_t blocks = fits(1) && 25.0 + n / 425.0 < waves * (38.0 + n / 2900.0) ? 1 : SM_CLUSTER;
+    const auto kernel = blocks == 1 ? sample_kernel<1> : sample_kernel<SM_CLUSTER>;
+    const size_t bytes = step_bytes(blocks);
+    const bool keep_steps = fits(blocks);
+    if (keep_steps) BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernel, bytes));
+    kernel<<<count * blocks, SM_THREADS, keep_steps ? bytes : 0, ctx->stream>>>(logits, n, temperature, top_k, top_p, ldexpf(1.0f, 62 - bits), keep_steps, rng,
+                                                                                out);
     return brasa_post_launch(cmd, "sample_top_p");
 }
 

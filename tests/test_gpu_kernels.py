@@ -1002,6 +1002,23 @@ def test_device_sampler_against_64_bits(B, ctx, K, n, top_k, top_p):
     assert checked >= 4 or n <= 9
 
 
+@pytest.mark.parametrize("n,count", [(8, 3), (1000, 70), (8192, 9), (20_000, 2), (20_000, 90), (69_000, 300), (80_000, 40)])
+@pytest.mark.parametrize("top_k,top_p", [(0, 0.9), (30, 0.8)])
+def test_sampler_rows_in_one_block_and_in_a_cluster(B, ctx, K, n, count, top_k, top_p):
+    """A row's token is the same whether it is sampled in one block or by a cluster: masses are whole numbers, whatever order they are added
+    in. Rows of a launch of many (either side of the rule, by length and by count) against each row alone."""
+    rng = np.random.default_rng(n + count)
+    l = (rng.standard_normal((count, n)) * 2.0).astype(np.float32)
+    l[:, ::7] = np.round(l[:, ::7])  # equal logits on either side of the cuts
+    gl, states, scratch, out = ctx.buffer_from(l), ctx.buffer_from(np.tile(B.pcg32_state(11), count)), ctx.buffer(8 * count * n), ctx.buffer(4 * count)
+    run(ctx, lambda c: K.sample_rows(c, gl, n, count, 0.9, top_k, top_p, states, scratch, out))
+    got = out.download(np.uint32, count)
+    for r in range(0, count, max(1, count // 8)):
+        state, one = ctx.buffer_from(B.pcg32_state(11)), ctx.buffer(4)
+        run(ctx, lambda c: K.sample_top_p(c, gl.at(4 * r * n), n, 0.9, top_k, top_p, state, one))
+        assert int(one.download(np.uint32, 1)[0]) == got[r], r
+
+
 @pytest.mark.parametrize("n", [1, 9, 5000, 600_001])
 def test_device_sampler_rows_without_a_finite_sum(B, ctx, K, n):
     """NaN among the logits (either sign: the total order puts one first, the other last), an infinite largest one, nothing but -inf, a
