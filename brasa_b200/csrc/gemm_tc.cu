@@ -1170,6 +1170,7 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
     for (uint32_t i = 0; i < count; ++i) {
         BRASA_REQUIRE(ctx, brasa_gemm_tc_supported(ws[i], tokens) && ws[i].cols == ws[0].cols, "gemm: shape not taken by the tensor-core kernel");
         BRASA_REQUIRE(ctx, glu || (reinterpret_cast<uintptr_t>(ys[i]) & 15) == 0, "gemm: misaligned y");
+        BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(arg_ptr(ws[i].data)) & 15) == 0, "gemm: misaligned weights");  // (TMA, 16-byte loads)
         rows256 = rows256 && ws[i].rows % 256 == 0;
         tiles128 += ws[i].rows / BN;
     }
@@ -1249,7 +1250,6 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
         const uint32_t rb = tiled_row_bytes(BRASA_Q4_0, wi.cols);
         cuuint64_t wdims[2] = {rb, wi.rows}, wstrides[1] = {rb};
         cuuint32_t wbox[2] = {32, BN * nb}, westr[2] = {1, 1};
-        BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(arg_ptr(wi.data)) & 15) == 0, "gemm: misaligned weights");
         CUresult wr = encode_tiled()(&wmaps.m[i], CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, arg_ptr(wi.data), wdims, wstrides, wbox, westr,
                                      CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                                      CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

@@ -848,6 +848,22 @@ def test_flash_attention_tensor_core_many_query_tiles(B, ctx, K, tokens, pos0, k
     assert float(np.max(d / np.maximum(vmax, 1e-30))) <= 1e-5
 
 
+@pytest.mark.parametrize("qtype", ["q4_0", "q6_0"])
+def test_gemm_refuses_misaligned_weights(B, ctx, K, qtype):
+    """Tiled weights that do not start on a 16-byte boundary are refused before anything is launched, whatever the token count."""
+    rows, cols = 256, 512
+    raw = O.Rng(3).qmatrix(QT[qtype][0], rows, cols)
+    buf, x, y = ctx.buffer(raw.nbytes + 16), ctx.buffer(600 * cols * 2), ctx.buffer(600 * rows * 4)
+    w = B.QMatrix(buf.at(8), B.WeightType(QT[qtype][1]), rows, cols, B.Layout.TILED)
+    for tokens in (16, 100, 600):
+        launches = ctx.launch_count()
+        cmd = ctx.command()
+        with pytest.raises(B.BrasaError, match="misaligned weights"):
+            K.gemm(cmd, w, x, y, tokens)
+        cmd.wait()
+        assert ctx.launch_count() == launches
+
+
 @pytest.mark.parametrize("what", ["gemm-few", "gemm-pair", "flash-F16", "flash-Q8_0"])
 def test_recorded_kernels_keep_their_workspace(B, K, what):
     """A recorded launch has the address of its workspace in it. Calls behind the recording that need a larger one must leave the old one
