@@ -636,7 +636,10 @@ template <> struct KvSeg<BRASA_KV_Q8_0> {
 // Every warp walks keys of its own, four at a time, with a running maximum, sum and output in registers: sixteen lanes hold two keys, a
 // lane 8 dims of them for four heads. Nothing is shared until a group of keys is done, so an item has two block barriers where a tile
 // form (K and V tiles in shared memory, 64 keys between barriers) had four per 64 keys, and the next keys' rows are on their
-// way while these are worked on. The bound is the multiply-adds (1 024 per key for four heads, 512 lanes): ATTN_MEASURED
+// way while these are worked on. The bound is the multiply-adds (1 024 per key for four heads, 512 lanes). us a
+// token of eight layers of 2 560 with 32 heads, the tile form's in brackets, behind 512 and 16 384 keys: f16 cache, 8 KV heads 238 (244), 366
+// (506); 32 KV heads 265 (291), 763 (1 401); 4 KV heads, whose eight heads walk the keys twice, 256 (258), 366 (430); q8_0, 8 KV heads 242
+// (249), 362 (571); 4 KV heads 259 (262), 373 (460).
 template <int KV>
 __device__ __forceinline__ void attention_op(const TokCtx &c, const TokOp &op, uint32_t oi, uint32_t epoch, uint32_t heads,
                                           uint32_t kv_heads, uint32_t max_chunks, const float *cos_t, const float *sin_t,

@@ -972,9 +972,9 @@ __global__ void __launch_bounds__(32 * (FLASH_SW + 1), 1) flash_tc_f16_kernel(co
 //     SPLITKV four are in use at a time, and the fifth covers the copies because the lo terms are needed last;
 //   * the work is a line of items and key tiles, cut into one run per SM where that ends sooner (see the launch): 448 items over 148 SMs
 //     would leave 144 SMs idle for the last four. A run's parts of items go to a workspace and are merged by a dependent kernel.
-// Measured (32 query heads over 8; us, one-tile kernel in brackets): f16 cache, 1 024 queries behind 4 096 keys 132 (195), 3 584 behind 12 800
-// 1 122 (1 775), 3 584 behind none 179 (298); q8_0 cache 207 (285), 1 855 (2 540), 267 (414). Tensor pipe active 63 % (f16) and 68 % (q8_0) of
-// a busy SM's cycles at 1 024 queries before the row threads were doubled; what is left is the way from S to P of one tile (16 MUFU.EX2
+// Measured (32 query heads over 8; us, one-tile kernel in brackets): f16 cache, 1 024 queries behind 4 096 keys 129 (195), 3 584 behind 12 800
+// 1 106 (1 775), 3 584 behind none 174 (298); q8_0 cache 208 (285), 1 816 (2 540), 260 (414). Tensor pipe active 50 % (f16) and 55 % (q8_0) of
+// the SMs' active cycles at 1 024 queries; what is left is the way from S to P of one tile (16 MUFU.EX2
 // lanes a clock: 1 024 cycles a tile) where the other tile's products are shorter.
 constexpr uint32_t FL2_SLOTS = 5;
 constexpr uint32_t FL2_START = 2;
