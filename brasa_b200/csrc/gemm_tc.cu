@@ -1127,7 +1127,7 @@ extern "C" uint32_t brasa_gemm_few_tokens_owner(uint32_t units, uint32_t blocks,
 
 // True when the tensor-core kernel takes this product (the caller falls back to the warp-MMA kernel otherwise).
 bool brasa_gemm_tc_supported(const brasa_qmatrix &w, uint32_t tokens) {
-    return (w.qtype == BRASA_Q4_0 || w.qtype == BRASA_Q6_0) && w.layout == BRASA_LAYOUT_TILED && w.rows % BN == 0 && w.cols % BK == 0 && w.cols >= BK && tokens > 0 &&
+    return (w.qtype == BRASA_Q4_0 || w.qtype == BRASA_Q6_0) && w.layout == BRASA_LAYOUT_TILED && w.rows > 0 && w.rows % BN == 0 && w.cols % BK == 0 && w.cols >= BK && tokens > 0 &&
            encode_tiled() != nullptr;
 }
 

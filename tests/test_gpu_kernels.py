@@ -864,6 +864,18 @@ def test_gemm_refuses_misaligned_weights(B, ctx, K, qtype):
         assert ctx.launch_count() == launches
 
 
+def test_products_refuse_a_matrix_without_rows(B, ctx, K):
+    """A tiled matrix of no rows is an error from every entry point of the products, never a division by the number of its tiles."""
+    buf, x = ctx.buffer(64), ctx.buffer(200 * 256 * 2)
+    w = B.QMatrix(buf, B.WeightType.Q4_0, 0, 256, B.Layout.TILED)
+    for call in (lambda c: K.gemm(c, w, x, buf, 200), lambda c: K.gemm_add(c, w, x, buf, buf, 200), lambda c: K.gemm_swiglu(c, w, w, x, buf, buf, buf, 200),
+                 lambda c: K.gemm_multi(c, [w, w], x, [buf, buf], 200, B.PrefillPrecision.F16)):
+        cmd = ctx.command()
+        with pytest.raises(B.BrasaError):
+            call(cmd)
+        cmd.wait()
+
+
 @pytest.mark.parametrize("what", ["gemm-few", "gemm-pair", "flash-F16", "flash-Q8_0"])
 def test_recorded_kernels_keep_their_workspace(B, K, what):
     """A recorded launch has the address of its workspace in it. Calls behind the recording that need a larger one must leave the old one
