@@ -1036,7 +1036,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
     # ---- dominant kernel: the whole-token decode kernel, one launch per token (timed above with CUDA events) ----
     t_token = total_s / (args.steps * steps_tokens)
     ach = bytes_per_token / t_token / 1e9
-    roof = {"bound": "hbm", "kernel": "decode_token_kernel<kv f16>: one launch = one token (36 layers, lm_head, argmax)",
+    roof = {"bound": "hbm", "kernel": "decode_token_mma_kernel<kv f16>: one launch = one token (36 layers, lm_head, argmax)",
             "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "peak_source": peak_kind, "us_per_launch": t_token * 1e6,
             "algorithmic_bytes_per_launch": bytes_per_token, "traffic": TOKEN_KERNEL_TRAFFIC_BYTES,
             "note": "weights 2 360 553 504 B + 147 456 B per cached position, mean position of the timed steps"}

@@ -375,6 +375,35 @@ def test_token_kernel_takes_wide_feed_forward_in_halves(ffn, monkeypatch, tmp_pa
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("hidden,heads,kv_heads,ffn,vocab,kv", [
+    (768, 6, 2, 1024, 512, "f16"),      # the narrowest; blocks without rows of an operation, one matrix after another inside a slot
+    (1024, 40, 8, 10240, 512, "q8_0"),  # slots of 16, 8 and 4 rows: o_proj and down_proj as wide as it takes
+    (1280, 16, 16, 3328, 40960, "f16"),  # a head of more slots than the ring, in tiles of two; a last tile of a few rows
+    (3072, 8, 1, 4096, 1024, "f16"),    # the widest hidden size
+    (2048, 8, 2, 2048, 20480, "q8_0"),  # rows of all widths in the same bank
+])
+def test_token_kernel_on_integer_products(hidden, heads, kv_heads, ffn, vocab, kv, monkeypatch, tmp_path):
+    """Models whose token runs on integer tensor products, against the kernel-per-operation path: slots of every number of rows, tiles that
+    are one slot or several, remainders. Same tolerance as for the other whole-token kernel (crates/models/tests/forward.rs:40-55)."""
+    import brasa_b200 as B
+    from brasa_b200 import synth
+    kvt, tol = {"f16": (B.KvType.F16, 1e-3), "q8_0": (B.KvType.Q8_0, 2e-2)}[kv]
+    cfg = dict(synth.QWEN3_4B, tie_word_embeddings=True, num_hidden_layers=2, hidden_size=hidden, intermediate_size=ffn, num_attention_heads=heads,
+               num_key_value_heads=kv_heads, vocab_size=vocab)
+    synth.write_synthetic_model(B.Context(0), tmp_path / "m.brasa", cfg, seed=4)
+    runs = []
+    for mode in ("0", "1"):
+        monkeypatch.setenv("BRASA_TOKEN_KERNEL", mode)
+        ctx = B.Context(0)
+        m = B.Qwen3.load(ctx, tmp_path / "m.brasa", B.Limits(ctx=64, max_tokens=16, max_logit_rows=1, kv=kvt))
+        m.forward(list(range(7)), 0, want_logits=False)
+        runs.append(np.stack([m.forward([11 * i + 5], 7 + i)[0][0].copy() for i in range(8)]))
+        m.free()
+    assert np.isfinite(runs[1]).all()
+    assert np.abs(runs[0] - runs[1]).max() <= tol * np.abs(runs[0]).max()
+
+
+@pytest.mark.gpu
 def test_token_kernel_long_cache_groups_chunks(monkeypatch, golden_dir):
     """Past (SMs / kv heads) attention chunks a block of the whole-token kernel walks several chunks with a running
     maximum and sum: 2 700 positions of an f32 cache (32-key chunks, 2 kv heads) are well beyond that point. Logits must
