@@ -545,8 +545,16 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_kernel(const __grid_constant__
 // that covers a tile's whole K range stores Y; any other writes a partial tile, and a second small kernel, launched as
 // this one's dependent, adds each shared tile's partial tiles in K order and the residual (every SM takes part; one block
 // doing it as the last to arrive took longer than the products themselves).
-constexpr uint32_t SK_TT = 64, SK_X_TILE = SK_TT * BK * 2;  // 8 KB of X per stage
-constexpr uint32_t SK_NCS = 3, SK_X_CHUNK = 4 * SK_X_TILE;  // ring of three chunks (four stages each): 32 KB of X per slot
+//
+// 65 to 128 tokens (an admitted prompt; see brasa_gemm_tc_few_tokens) go through the same kernel with N = 128: the weights are converted once for all of them and a
+// product of 128 tokens takes the tensor core about as long as a chunk's conversion takes the warps. Its X takes twice the room, so
+// there are two chunks of X and A and five of raw weights instead of three and seven.
+constexpr uint32_t SK_TT = 64, SK_TT_MOST = 128;  // tokens of the two forms
+template <uint32_t TT>
+struct Sk {
+    static constexpr uint32_t X_TILE = TT * BK * 2, X_CHUNK = 4 * X_TILE;  // 8 or 16 KB of X per stage; a slot of the ring holds four stages
+    static constexpr uint32_t NCS = TT == 64 ? 3 : 2, RAW_SLOTS = TT == 64 ? 7 : 5;
+};
 constexpr uint32_t SK_ACOL = 128, SK_TMEM = 512;  // A in tensor memory: 128 columns per chunk slot from column 128; accumulator at column 0
 constexpr uint32_t SK_CODES = BN * 128, SK_RAW = SK_CODES + BN * 16;                     // 16 KB of codes + 2 KB of scales per four stages
 
@@ -563,7 +571,8 @@ struct SkinnyParams {
     uint32_t max_parts;  // most blocks that share one tile
     uint32_t *status;
     const float *resid;
-    float *part;         // [tile][max_parts][64 tokens][128 rows]: what the blocks that share a tile leave for the kernel below
+    uint32_t tt;         // tokens of the form: 64 or 128
+    float *part;         // [tile][max_parts][tt tokens][128 rows]: what the blocks that share a tile leave for the kernel below
     __half *glu;         // when set (two matrices, gate then up): every tile goes to `part` and the kernel below writes f16(silu(gate) * up) here
     uint32_t defer;      // every tile goes to `part`: the kernel that follows forms Y (and more) from the partial tiles
     unsigned long long *trace;  // a developer's build only: phase time stamps
@@ -586,8 +595,10 @@ BRASA_HD static inline uint32_t skinny_owner(uint32_t u, uint32_t units, uint32_
     return c;
 }
 
+template <uint32_t TT>
 __global__ void __launch_bounds__(384, 1) gemm_tc_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ SkinnyMaps maps,
                                                                 SkinnyParams p) {
+    constexpr uint32_t SK_NCS = Sk<TT>::NCS, SK_X_CHUNK = Sk<TT>::X_CHUNK, SK_X_TILE = Sk<TT>::X_TILE;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full_x[SK_NCS], full_a[SK_NCS], empty[SK_NCS], raw_full[8], raw_empty[8], acc_full, acc_empty;
@@ -686,7 +697,7 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_skinny_kernel(const __grid_con
             }
         }
     } else if (warp == 2) {
-        if (lane == 0) {  // ---- X tiles: the chunk's stages, 64 tokens x 64 halves each, on one barrier ----
+        if (lane == 0) {  // ---- X tiles: the chunk's stages, TT tokens x 64 halves each, on one barrier ----
             uint32_t issued = 0, k = k_beg, left = nu, cs = 0, ph = 0;
             for (uint32_t c = 0; c < nc; ++c) {
                 const uint32_t n = chunk_len(k, left);
@@ -713,8 +724,8 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_skinny_kernel(const __grid_con
     } else if (warp == 1) {
         // ---- tensor core. The whole warp walks the chunks and waits; one lane issues. A chunk costs the issuing lane two
         // waits, up to sixteen products (operand addresses are constants of the unrolled slots) and one commit. ----
-        // instruction descriptor: D f32, A and B f16, both K-major, M = 128 weight rows, N = 64 tokens
-        const uint32_t idesc = (1u << 4) | ((uint32_t)(SK_TT >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
+        // instruction descriptor: D f32, A and B f16, both K-major, M = 128 weight rows, N = TT tokens
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(TT >> 3) << 17) | ((uint32_t)(BN >> 4) << 24);
         const uint64_t db_slot0 = smem_desc(smem_u32(smem));
         uint32_t seg = 0, k = k_beg, left = nu, ph = 0;  // seg: runs of one tile finished so far
         bool first = true, ok = true;
@@ -840,42 +851,47 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_skinny_kernel(const __grid_con
             ok = ok && wait(&acc_full, seg & 1);
             ok = __all_sync(0xffffffffu, ok);  // the tensor-memory load needs the whole warp
             if (tid == 128 && seg < 4) SKT(410 + seg * 8 + 1);
-            uint32_t v[32];
             if (ok) {
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                const uint32_t taddr = tmem_base + ((q * 32u) << 16) + 32 * th;
-                asm volatile(
-                    "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
-                    "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
-                      "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
-                      "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
-                      "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-                    : "r"(taddr)
-                    : "memory");
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&acc_empty);  // the next tile's products may overwrite the accumulator
                 const uint32_t row = 32 * q + lane;
-                if (whole) {
+                const uint32_t z = whole || k0 == 0 ? 0u : blockIdx.x - skinny_owner(t * nkst, p.units, P);  // (a tile begun here is this block's from its first stage)
+                float *ptile = p.part + ((size_t)t * p.max_parts + z) * (TT * BN);
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const uint32_t token = 32 * th + i;
-                        if (token < p.tokens) {
-                            const size_t at = (size_t)token * yrows + n0 + row;
-                            float o = __uint_as_float(v[i]);
-                            if (p.resid) o = p.resid[at] + o;
-                            ymat[at] = o;
-                        }
+                for (uint32_t h = 0; h < TT / 64; ++h) {  // 32 tokens at a time
+                    const uint32_t tok0 = TT / 2 * th + 32 * h, taddr = tmem_base + ((q * 32u) << 16) + tok0;
+                    uint32_t v[32];
+                    asm volatile(
+                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, "
+                        "%20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]),
+                          "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]),
+                          "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]),
+                          "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+                        : "r"(taddr)
+                        : "memory");
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (h + 1 == TT / 64) {
+                        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&acc_empty);  // the next tile's products may overwrite the accumulator
                     }
-                } else {
-                    const uint32_t z = k0 == 0 ? 0u : blockIdx.x - skinny_owner(t * nkst, p.units, P);  // (a tile begun here is this block's from its first stage)
-                    float *ptile = p.part + ((size_t)t * p.max_parts + z) * (SK_TT * BN);
+                    if (whole) {
 #pragma unroll
-                    for (int i = 0; i < 32; ++i) {
-                        const uint32_t token = 32 * th + i;
-                        if (token < p.tokens) ptile[token * BN + row] = __uint_as_float(v[i]);
+                        for (int i = 0; i < 32; ++i) {
+                            const uint32_t token = tok0 + i;
+                            if (token < p.tokens) {
+                                const size_t at = (size_t)token * yrows + n0 + row;
+                                float o = __uint_as_float(v[i]);
+                                if (p.resid) o = p.resid[at] + o;
+                                ymat[at] = o;
+                            }
+                        }
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            const uint32_t token = tok0 + i;
+                            if (token < p.tokens) ptile[token * BN + row] = __uint_as_float(v[i]);
+                        }
                     }
                 }
             }
@@ -903,13 +919,14 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_skinny_kernel(const __grid_con
 // Launched as its dependent: its blocks sit beside the GEMM's and start the moment the last partial tile is out, and
 // every SM takes part (one float4 of Y per thread, all of its partial tiles' loads in flight at once).
 __device__ __forceinline__ float4 skinny_tile_sum(const SkinnyParams &p, uint32_t t, uint32_t parts, uint32_t i) {
-    const float *p0 = p.part + (size_t)t * p.max_parts * (SK_TT * BN);
+    const uint32_t tile = p.tt * BN;
+    const float *p0 = p.part + (size_t)t * p.max_parts * tile;
     float4 a = __ldcg(reinterpret_cast<const float4 *>(p0) + i);
     for (uint32_t z0 = 1; z0 < parts; z0 += 8) {  // always in the order of the K ranges
         float4 b[8];
 #pragma unroll
         for (int dz = 0; dz < 8; ++dz)
-            b[dz] = z0 + dz < parts ? __ldcg(reinterpret_cast<const float4 *>(p0 + (size_t)(z0 + dz) * (SK_TT * BN)) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+            b[dz] = z0 + dz < parts ? __ldcg(reinterpret_cast<const float4 *>(p0 + (size_t)(z0 + dz) * tile) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int dz = 0; dz < 8; ++dz) {
             if (z0 + dz < parts) {
@@ -925,7 +942,7 @@ __global__ void __launch_bounds__(256) gemm_tc_skinny_sum_kernel(SkinnyParams p,
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const uint32_t t = blockIdx.x, nkst = p.cols / BK;
     const uint32_t parts = skinny_owner(t * nkst + nkst - 1, p.units, blocks) - skinny_owner(t * nkst, p.units, blocks) + 1;
-    const uint32_t live = min(SK_TT, p.tokens) * (BN / 4);  // float4s of the tile that hold tokens
+    const uint32_t live = min(p.tt, p.tokens) * (BN / 4);  // float4s of the tile that hold tokens
     if (p.glu) {  // tile t of gate and tile t of up: out = f16(silu(gate) * up), four rows of a token per thread
         const uint32_t tu = t + p.tile_end[0];
         const uint32_t parts_u = skinny_owner(tu * nkst + nkst - 1, p.units, blocks) - skinny_owner(tu * nkst, p.units, blocks) + 1;
@@ -1040,10 +1057,12 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
     uint64_t scratch = 0;
     BRASA_REQUIRE(ctx, brasa_gemm_few_tokens_plan((uint32_t)ctx->sm_count, tiles, nkst, &blocks, &max_parts, &scratch) == BRASA_OK, "gemm: shape outside the few-token kernel");
     BRASA_REQUIRE(ctx, (reinterpret_cast<uintptr_t>(x) & 15) == 0, "gemm: misaligned x");
+    p.tt = tokens <= SK_TT ? SK_TT : SK_TT_MOST;
+    scratch *= p.tt / SK_TT;
     CUtensorMap tmap;
     {
         cuuint64_t dims[2] = {cols, tokens}, strides[1] = {(cuuint64_t)cols * 2};
-        cuuint32_t box[2] = {BK, SK_TT}, estr[2] = {1, 1};
+        cuuint32_t box[2] = {BK, p.tt}, estr[2] = {1, 1};
         CUresult cr = encode_tiled()(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<__half *>(x), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                                      CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (cr != CUDA_SUCCESS) return brasa_fail(ctx, BRASA_ECUDA, "cuTensorMapEncodeTiled failed (%d)", (int)cr);
@@ -1065,7 +1084,7 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
     }
     p.cols = cols;
     p.tokens = tokens;
-    p.raw_slots = 7;
+    p.raw_slots = p.tt == SK_TT ? Sk<SK_TT>::RAW_SLOTS : Sk<SK_TT_MOST>::RAW_SLOTS;
     p.units = units;
     p.max_parts = max_parts;
     p.status = ctx->status;
@@ -1079,8 +1098,10 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
         BRASA_TRY(brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, (size_t)scratch));
         p.part = ctx->gemm_part;
     }
-    const size_t smem = (size_t)SK_NCS * SK_X_CHUNK + (size_t)p.raw_slots * SK_RAW + 1024;
-    BRASA_TRY(brasa_smem_optin(ctx, (const void *)gemm_tc_skinny_kernel, ctx->smem_optin - 2048));
+    const auto kernel = p.tt == SK_TT ? gemm_tc_skinny_kernel<SK_TT> : gemm_tc_skinny_kernel<SK_TT_MOST>;
+    const size_t ring = p.tt == SK_TT ? (size_t)Sk<SK_TT>::NCS * Sk<SK_TT>::X_CHUNK : (size_t)Sk<SK_TT_MOST>::NCS * Sk<SK_TT_MOST>::X_CHUNK;
+    const size_t smem = ring + (size_t)p.raw_slots * SK_RAW + 1024;
+    BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernel, ctx->smem_optin - 2048));
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(384);
@@ -1091,14 +1112,14 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
     attr[0].val.programmaticStreamSerializationAllowed = ctx->pdl ? 1 : 0;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, gemm_tc_skinny_kernel, tmap, maps, p));
+    BRASA_CUDA(ctx, cudaLaunchKernelEx(&cfg, kernel, tmap, maps, p));
     BRASA_TRY(brasa_post_launch(cmd, "gemm_tc_skinny"));
     if (norm_out) {  // one matrix, Y = the residual stream itself: sum, residual add and the norm behind it
         BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_tc_skinny_sum_norm_kernel, dim3(tokens), dim3(512), 0, p, blocks, norm_w, norm_out, eps));
         return brasa_post_launch(cmd, "gemm_tc_skinny_sum_norm");
     }
     if (max_parts == 1 && !glu) return BRASA_OK;
-    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_tc_skinny_sum_kernel, dim3(glu ? tiles / 2 : tiles, 8), dim3(256), 0, p, blocks));
+    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, gemm_tc_skinny_sum_kernel, dim3(glu ? tiles / 2 : tiles, p.tt / 8), dim3(256), 0, p, blocks));
     return brasa_post_launch(cmd, "gemm_tc_skinny_sum");
 }
 
@@ -1132,18 +1153,33 @@ bool brasa_gemm_tc_supported(const brasa_qmatrix &w, uint32_t tokens) {
 }
 
 // True when brasa_gemm_tc_launch takes these matrices with the few-token kernel (whose fused SwiGLU may write over X: its
-// output is stored by a kernel that starts after every product has been formed).
+// output is stored by a kernel that starts after every product has been formed). Above 64 tokens that asks for a workspace that can be had:
+// without one (a graph is being recorded, no memory is left) the product is another kernel's.
 bool brasa_gemm_tc_few_tokens(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens) {
-    if (tokens == 0 || tokens > SK_TT || count < 1 || count > 3) return false;
+    if (tokens == 0 || tokens > SK_TT_MOST || count < 1 || count > 3) return false;
     uint64_t tiles = 0;
     for (uint32_t i = 0; i < count; ++i) {
         if (!brasa_gemm_tc_supported(ws[i], tokens) || ws[i].qtype != BRASA_Q4_0 || ws[i].cols != ws[0].cols) return false;
         tiles += ws[i].rows / BN;
     }
-    return tiled_row_bytes(BRASA_Q4_0, ws[0].cols) % 16 == 0 && tiles * (ws[0].cols / BK) * (uint64_t)(ctx->sm_count + 1) < (1ull << 32);
+    const uint32_t nkst = ws[0].cols / BK;
+    if (tiled_row_bytes(BRASA_Q4_0, ws[0].cols) % 16 != 0 || tiles * nkst * (uint64_t)(ctx->sm_count + 1) >= (1ull << 32)) return false;
+    if (tokens <= SK_TT) return true;
+    // Above 64 tokens the pair kernel is ahead where a launch of several matrices is small (its tiles fill the SMs whole) or so large that
+    // the tensor core holds it. us at 100 tokens, this kernel and the pairs: q, k and v of 2 560 columns (15.7 M weights) 16.6, 17.8; of 1 536
+    // (4.7 M) 14.2, 13.1; gate and up of 1 536 (12.6 M) 18.3, 13.9; of 2 560 (50 M) 25.8, 28.0; of 5 120 (262 M) 76.2, 80.5, but at 128 tokens
+    // 81.8, 78.2. One matrix (o, down): 9.6 .. 38.7 against 12.0 .. 41.9.
+    const uint64_t weights = tiles * BN * ws[0].cols;
+    if (count > 1 && (weights < 14000000 || (weights > 200000000 && tokens > 100))) return false;
+    uint32_t blocks, parts;
+    uint64_t scratch;
+    if (brasa_gemm_few_tokens_plan((uint32_t)ctx->sm_count, (uint32_t)tiles, nkst, &blocks, &parts, &scratch) != BRASA_OK) return false;
+    const size_t need = (size_t)scratch * (SK_TT_MOST / SK_TT), most = (size_t)ctx->sm_count * 256 * 256 * sizeof(float);  // (the pair kernel's bound)
+    if (ctx->gemm_part_bytes < need && !ctx->capturing) brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, std::max(need, most));
+    return ctx->gemm_part_bytes >= need;
 }
 
-// acc = acc + W X and out = f16(rms_norm(acc) * norm_w) for at most 64 tokens (brasa_gemm_tc_few_tokens holds for w, its rows
+// acc = acc + W X and out = f16(rms_norm(acc) * norm_w) for at most 128 tokens (brasa_gemm_tc_few_tokens holds for w, its rows
 // are a multiple of 512 up to 5120, pointers 16-byte aligned): the few-token kernel, then one kernel for sum, add and norm.
 int32_t brasa_gemm_tc_add_norm(brasa_cmd *cmd, const brasa_qmatrix &w, const __half *x, float *acc, const float *norm_w, __half *out, uint32_t tokens,
                                float eps) {
@@ -1174,11 +1210,8 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
         rows256 = rows256 && ws[i].rows % 256 == 0;
         tiles128 += ws[i].rows / BN;
     }
-    // at most 64 tokens of q4_0 matrices: the persistent form whose accumulator rows are weight rows
-    bool few = tokens <= SK_TT && tiled_row_bytes(BRASA_Q4_0, ws[0].cols) % 16 == 0 &&
-               (uint64_t)tiles128 * (ws[0].cols / BK) * (uint64_t)(ctx->sm_count + 1) < (1ull << 32);
-    for (uint32_t i = 0; i < count; ++i) few = few && ws[i].qtype == BRASA_Q4_0;
-    if (few) return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
+    // at most 128 tokens of q4_0 matrices: the persistent form whose accumulator rows are weight rows
+    if (brasa_gemm_tc_few_tokens(ctx, ws, count, tokens)) return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
     if (brasa_gemm_pair_takes(ws, count, tokens, glu != nullptr) && !brasa_gemm_pair_behind(ctx, ws, count, tokens, resid != nullptr, glu != nullptr))
         return brasa_gemm_pair_launch(cmd, count, ws, x, ys, tokens, resid, glu);
     // Shape of a CTA: MT token tiles of 128 x NB weight tiles of 128 rows (MT x NB x 128 accumulator columns <= 512).

@@ -205,8 +205,9 @@ int32_t residual_add(brasa_model *m, brasa_cmd *cmd, uint64_t n) {
 }
 
 // Layer li for `tokens` > 1 tokens from pos0 (also used for a single token by run_layers when asked
-// for the unfused order). Input and output in ws.x.
-int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32_t tokens, uint32_t pos0) {
+// for the unfused order). Input and output in ws.x. Of several layers in order [l0, l1), every norm but the first is formed behind the
+// residual add before it (one kernel behind a product of few tokens; the two kernels otherwise, with the same bits).
+int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32_t tokens, uint32_t pos0, uint32_t l0, uint32_t l1) {
     const brasa_config &c = m->cfg;
     Layer &l = m->layers[li];
     const SettledOperands settled(m->ctx);
@@ -214,7 +215,7 @@ int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32
     const uint32_t H = c.hidden;
     brasa_arg xin;
     if (half_io) {
-        BRASA_TRY(brasa_k_rms_norm_f16(cmd, A(m->x), A(l.attn_norm), A(m->xh), tokens, H, c.eps));
+        if (li == l0 || m->tp) BRASA_TRY(brasa_k_rms_norm_f16(cmd, A(m->x), A(l.attn_norm), A(m->xh), tokens, H, c.eps));
         xin = A(m->xh);
     } else {
         BRASA_TRY(brasa_k_rms_norm(cmd, A(m->x), A(l.attn_norm), A(m->norm_out), tokens, H, c.eps));
@@ -239,14 +240,14 @@ int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32
     } else {
         BRASA_TRY(brasa_k_flash_attention_with(cmd, A(m->q), all.k, all.v, attn, sh, half_io ? BRASA_PREFILL_F16 : BRASA_PREFILL_F32));
     }
-    if (half_io && !m->tp) BRASA_TRY(brasa_k_gemm_add(cmd, l.wo.q, attn, A(m->x), A(m->h), tokens));  // x += Wo attn in the GEMM's epilogue
+    if (half_io && !m->tp) BRASA_TRY(brasa_k_gemm_add_rms_norm_f16(cmd, l.wo.q, attn, A(m->x), A(m->h), A(l.ffn_norm), A(m->xh), tokens, c.eps));  // x += Wo attn, its norm
     else {
         BRASA_TRY(matmul(m, cmd, l.wo, attn, A(m->h), tokens, half_io));
         BRASA_TRY(residual_add(m, cmd, (uint64_t)tokens * H));
     }
     brasa_arg act;
     if (half_io) {
-        BRASA_TRY(brasa_k_rms_norm_f16(cmd, A(m->x), A(l.ffn_norm), A(m->xh), tokens, H, c.eps));
+        if (m->tp) BRASA_TRY(brasa_k_rms_norm_f16(cmd, A(m->x), A(l.ffn_norm), A(m->xh), tokens, H, c.eps));
         // one fused launch writes the f16 activations while X is still being read: they go to the (then unused) up buffer
         act = brasa_gemm_swiglu_fuses(l.gate.q, l.up.q, tokens) ? A(m->up) : A(m->xh);
         BRASA_TRY(brasa_k_gemm_swiglu(cmd, l.gate.q, l.up.q, A(m->xh), A(m->gate), A(m->up), act, tokens));
@@ -257,6 +258,8 @@ int32_t encode_layer_prefill(brasa_model *m, brasa_cmd *cmd, uint32_t li, uint32
         BRASA_TRY(brasa_k_swiglu(cmd, A(m->gate), A(m->up), A(m->gate), (uint64_t)tokens * c.ffn));
         act = A(m->gate);
     }
+    if (half_io && !m->tp && li + 1 < l1)
+        return brasa_k_gemm_add_rms_norm_f16(cmd, l.down.q, act, A(m->x), A(m->h), A(m->layers[li + 1].attn_norm), A(m->xh), tokens, c.eps);
     if (half_io && !m->tp) return brasa_k_gemm_add(cmd, l.down.q, act, A(m->x), A(m->h), tokens);
     BRASA_TRY(matmul(m, cmd, l.down, act, A(m->h), tokens, half_io));
     return residual_add(m, cmd, (uint64_t)tokens * H);
@@ -426,7 +429,7 @@ int32_t qwen3_forward(brasa_model *m, brasa_cmd *cmd, uint32_t tokens, uint32_t 
     const brasa_config &c = m->cfg;
     const SettledOperands settled(m->ctx);
     BRASA_TRY(brasa_k_embed(cmd, m->embed.q, A(m->ids), A(m->x), tokens));
-    for (uint32_t li = 0; li < c.layers; ++li) BRASA_TRY(encode_layer_prefill(m, cmd, li, tokens, pos0));
+    for (uint32_t li = 0; li < c.layers; ++li) BRASA_TRY(encode_layer_prefill(m, cmd, li, tokens, pos0, 0, c.layers));
     if (n_rows == 0) return BRASA_OK;
     for (uint32_t i = 0, n; i < n_rows; i += n) {  // neighbouring places share a launch
         for (n = 1; i + n < n_rows && rows[i + n] == rows[i] + n;) ++n;
@@ -470,7 +473,7 @@ int32_t qwen3_run_layers(brasa_model *m, brasa_cmd *cmd, const uint32_t *, const
         BRASA_TRY(set_position(m, pos0));
         BRASA_TRY(encode_decode_token(m, cmd, l0, l1, false));
     } else {
-        for (uint32_t li = l0; li < l1; ++li) BRASA_TRY(encode_layer_prefill(m, cmd, li, tokens, pos0));
+        for (uint32_t li = l0; li < l1; ++li) BRASA_TRY(encode_layer_prefill(m, cmd, li, tokens, pos0, l0, l1));
     }
     return brasa_buf_download(m->x, 0, y, n);
 }

@@ -640,6 +640,38 @@ def test_gemm_few_tokens_persistent(B, ctx, K, rows, cols):
             assert np.array_equal(ga.download(np.float32), acc0 + first[0])
 
 
+@pytest.mark.parametrize("tokens", [65, 97, 128])
+@pytest.mark.parametrize("rows,cols,glu", [((2560,), 9728, False), ((1024,), 256, False), ((4096, 1024, 1024), 2560, False), ((9728, 9728), 2560, True)])
+def test_gemm_65_to_128_tokens(B, ctx, K, rows, cols, glu, tokens):
+    """The form of the few-token kernel for 65 to 128 tokens: one tile of 128 tokens, of which as many as there are are stored; partial tiles of
+    twice the size; SwiGLU and the residual and norm behind it. Same bounds as every GEMM; a second launch gives the same bits."""
+    rng = O.Rng(93)
+    raws = [rng.qmatrix(O.Q4_0, r, cols) for r in rows]
+    ms = [tiled(B, ctx, K, "q4_0", raw, r, cols)[0] for raw, r in zip(raws, rows)]
+    x = rng.vec(tokens * cols, 0.5)
+    gxh, gys = ctx.buffer_from(x.astype(np.float16)), [ctx.buffer(tokens * r * 4) for r in rows]
+    wants = [O.matmul(O.Q4_0, raw, r, cols, x, f16_inputs=True) for raw, r in zip(raws, rows)]
+    if glu:
+        go = ctx.buffer(tokens * rows[0] * 2)
+        for _ in range(2):
+            run(ctx, lambda c: K.gemm_swiglu(c, ms[0], ms[1], gxh, gys[0], gys[1], go, tokens))
+            got = go.download(np.float16).astype(np.float32)
+            (wg, sg), (wu, su) = wants
+            want = O.swiglu(wg, wu).ravel()
+            bound = 1e-5 * (np.abs(wu) * 1.1 * sg + np.abs(wg) * su).ravel() + np.abs(want) * 2.0 ** -10 + 1e-7  # as in the fused SwiGLU's test above
+            assert np.all(np.abs(got - want) <= bound)
+        return
+    for _ in range(2):
+        run(ctx, lambda c: K.gemm_multi(c, ms, gxh, gys, tokens, B.PrefillPrecision.F16))
+        for gy, (want, s16), r in zip(gys, wants, rows):
+            assert np.max(np.abs(gy.download(np.float32).reshape(tokens, r) - want) / s16) <= 1e-5, r
+    if len(rows) == 1:
+        first, acc0 = gys[0].download(np.float32), rng.vec(tokens * rows[0], 2.0)
+        ga, gs = ctx.buffer_from(acc0), ctx.buffer(tokens * rows[0] * 4)
+        run(ctx, lambda c: K.gemm_add(c, ms[0], gxh, ga, gs, tokens))
+        assert np.array_equal(ga.download(np.float32), acc0 + first)
+
+
 @pytest.mark.parametrize("rows,cols,tokens", [(2560, 4096, 40), (2560, 9728, 64), (5120, 512, 9), (1024, 512, 33), (2560, 4096, 100)])
 def test_gemm_add_rms_norm_equals_the_two_calls(B, ctx, K, rows, cols, tokens):
     """acc += W x followed by the RMS norm of acc, as one call: behind the few-token GEMM one kernel adds the blocks' partial
