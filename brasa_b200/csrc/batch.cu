@@ -143,7 +143,6 @@ __device__ __forceinline__ void split_h2(float x, float y, uint32_t &hi, uint32_
 __device__ __forceinline__ uint32_t piece(uint32_t r, uint32_t c) { return r * 256u + ((c ^ (r & 7u)) << 4); }
 
 constexpr uint32_t MMA_TILE = 128 * 256;  // one K or V tile
-constexpr int PAGED_MMA_TILES = 2;       // groups of 16 / G sequences a shared-prefix block serves with one pair of tiles
 constexpr size_t MMA_SMEM = 2 * MMA_TILE + (2 * 4 * 16 + 16) * sizeof(float);  // three blocks per SM
 
 __device__ __forceinline__ void mma_f16_full(float c[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
@@ -157,7 +156,7 @@ __device__ __forceinline__ void mma_f16_full(float c[4], uint32_t a0, uint32_t a
 // groups of 16 / G consecutive sequences (row = local sequence * G + head in group), so the shared K and V tiles are
 // fetched and multiplied once per 16 / G sequences; grid z = sequence group; the pages are those of the group's first
 // sequence (the prefix pages are the same for all).
-template <bool MULTI>
+template <bool MULTI, int RT>
 __global__ void __launch_bounds__(128) decode_partial_paged_mma_kernel(const float *q, Paged kp, Paged vp, const uint32_t *lens, float *partials,
                                                                        uint32_t hq, uint32_t max_chunks, float scale, uint32_t first_chunk, uint32_t nseq,
                                                                        uint32_t late_wait) {
@@ -167,9 +166,8 @@ __global__ void __launch_bounds__(128) decode_partial_paged_mma_kernel(const flo
     if (!late_wait) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     constexpr int RH = MULTI ? 2 : 1;  // row halves in use: rows g (and g + 8)
-    // MULTI: a block serves PAGED_MMA_TILES groups of 16 / G sequences with the same K and V tiles: all their scores first (K is
+    // MULTI: a block serves RT groups of 16 / G sequences with the same K and V tiles: all their scores first (K is
     // then done with), then group by group softmax, P V and the four warps' sum in shared memory over the K tile.
-    constexpr int RT = MULTI ? PAGED_MMA_TILES : 1;
     extern __shared__ __align__(128) uint8_t smem_b[];
     uint8_t *kt = smem_b, *vt = smem_b + MMA_TILE;
     float *osum = reinterpret_cast<float *>(kt);  // [4 warps][16 rows][128], over the K tile once every warp is done with it
@@ -581,6 +579,25 @@ int32_t choose_tokens(brasa_batch *b, brasa_cmd *cmd, brasa_buf *logits, uint32_
     return BRASA_OK;
 }
 
+// How many groups of 16 / G sequences a block of the shared-prefix attention serves with one pair of K and V tiles: 1 to 3, by the waves of
+// three blocks an SM. `tiles`: (chunk, KV head) pairs. us a launch with 1, 2 and 3, 8 KV heads and groups of four: 64 sequences behind
+// 256 positions 12, 20, 24; 512: 20, 21, 28; 1 024: 30, 34, 28; 2 048: 49, 54, 53; 4 096: 91, 89, 88; 32 behind 1 024: 19, 21, 27.
+uint32_t shared_groups(const brasa_ctx *ctx, uint32_t tiles, uint32_t groups) {
+    constexpr double FIXED[3] = {1.0, 3.3, 3.0}, WAVE[3] = {9.4, 17.0, 25.3};
+    const uint32_t slots = 3 * (uint32_t)ctx->sm_count;
+    uint32_t best = 1;
+    double least = 1e30;
+    for (uint32_t rt = 1; rt <= 3; ++rt) {
+        const uint64_t blocks = (uint64_t)tiles * ((groups + rt - 1) / rt);
+        const double us = FIXED[rt - 1] + WAVE[rt - 1] * (double)((blocks + slots - 1) / slots);
+        if (us < least) {
+            least = us;
+            best = rt;
+        }
+    }
+    return best;
+}
+
 // One decode step for the first n sequences: ids[n] -> logits[n][vocab]. Uses the model's workspace (n <= max_tokens).
 int32_t encode_step(brasa_batch *b, brasa_cmd *cmd, uint32_t n) {
     brasa_model *m = b->m;
@@ -637,8 +654,7 @@ int32_t encode_step(brasa_batch *b, brasa_cmd *cmd, uint32_t n) {
     } while (0)
         if (m->limits.kv == BRASA_KV_F32) LAUNCH_BATCH(BRASA_KV_F32);
         else if (m->limits.kv == BRASA_KV_F16) {
-                BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_partial_paged_mma_kernel<false>, MMA_SMEM));
-                BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_partial_paged_mma_kernel<true>, MMA_SMEM));
+                BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_partial_paged_mma_kernel<false, 1>, MMA_SMEM));
             // the step's kernels are programmatic dependents of one another: each sets itself up while the one before it ends
             BRASA_CUDA(ctx, brasa_launch_dependent(ctx, qk_norm_rope_store_paged_kernel<BRASA_KV_F16>, dim3((rows + 3) / 4), dim3(128), 0, F(m->q), F(m->k_new),
                                                    F(m->v_new), F(l.q_norm), F(l.k_norm), F(m->rope_cos), F(m->rope_sin), kl, vl, table, b->max_pages, lens,
@@ -648,15 +664,17 @@ int32_t encode_step(brasa_batch *b, brasa_cmd *cmd, uint32_t n) {
             const uint32_t G = c.heads / c.kv_heads;
             const uint32_t shared_chunks = (n > 1 && 16 % G == 0 && G < 16) ? b->common_pages * PAGE / 128 : 0;
             if (shared_chunks) {
-                const uint32_t spb = 16 / G;
-                BRASA_CUDA(ctx, brasa_launch_dependent(ctx, decode_partial_paged_mma_kernel<true>,
-                                                       dim3(shared_chunks, c.kv_heads, (n + spb * PAGED_MMA_TILES - 1) / (spb * PAGED_MMA_TILES)), dim3(128), MMA_SMEM,
-                                                       F(m->q), kp, vp, lens, F(b->partials), c.heads, (uint32_t)b->max_chunks, scale, 0u, n, 0u));
+                const uint32_t groups = (n + 16 / G - 1) / (16 / G), rt = shared_groups(ctx, shared_chunks * c.kv_heads, groups);
+                static void (*const kernels[3])(const float *, Paged, Paged, const uint32_t *, float *, uint32_t, uint32_t, float, uint32_t, uint32_t, uint32_t) = {
+                    decode_partial_paged_mma_kernel<true, 1>, decode_partial_paged_mma_kernel<true, 2>, decode_partial_paged_mma_kernel<true, 3>};
+                BRASA_TRY(brasa_smem_optin(ctx, (const void *)kernels[rt - 1], MMA_SMEM));
+                BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernels[rt - 1], dim3(shared_chunks, c.kv_heads, (groups + rt - 1) / rt), dim3(128), MMA_SMEM, F(m->q), kp, vp,
+                                                       lens, F(b->partials), c.heads, (uint32_t)b->max_chunks, scale, 0u, n, 0u));
                 BRASA_TRY(brasa_post_launch(cmd, "decode_partial_paged_mma_shared"));
             }
             if ((uint32_t)b->max_chunks > shared_chunks) {
                 // (behind the shared-prefix form it runs beside it and waits for it at its end)
-                BRASA_CUDA(ctx, brasa_launch_dependent(ctx, decode_partial_paged_mma_kernel<false>, dim3((uint32_t)b->max_chunks - shared_chunks, c.kv_heads, n),
+                BRASA_CUDA(ctx, brasa_launch_dependent(ctx, decode_partial_paged_mma_kernel<false, 1>, dim3((uint32_t)b->max_chunks - shared_chunks, c.kv_heads, n),
                                                        dim3(128), MMA_SMEM, F(m->q), kp, vp, lens, F(b->partials), c.heads, (uint32_t)b->max_chunks, scale,
                                                        shared_chunks, n, shared_chunks ? 1u : 0u));
                 BRASA_TRY(brasa_post_launch(cmd, "decode_partial_paged_mma"));
@@ -763,8 +781,8 @@ int32_t brasa_k_decode_attention_paged(brasa_cmd *cmd, brasa_arg q, brasa_paged_
     float *pp = (float *)arg_ptr(partials);
     dim3 agrid(max_chunks, hkv, pg.seqs), rgrid(hq, pg.seqs);
     if (pg.kv == BRASA_KV_F16) {  // tensor-core partials (one block per chunk, kv head and sequence)
-        BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_partial_paged_mma_kernel<false>, MMA_SMEM));
-        decode_partial_paged_mma_kernel<false><<<agrid, 128, MMA_SMEM, ctx->stream>>>(qp, kp, vp, lens, pp, hq, max_chunks, scale, 0, pg.seqs, 0);
+        BRASA_TRY(brasa_smem_optin(ctx, (const void *)decode_partial_paged_mma_kernel<false, 1>, MMA_SMEM));
+        decode_partial_paged_mma_kernel<false, 1><<<agrid, 128, MMA_SMEM, ctx->stream>>>(qp, kp, vp, lens, pp, hq, max_chunks, scale, 0, pg.seqs, 0);
     } else {
         const size_t smem = (128 * TS + 8 * D + 8 * 128 + 16) * sizeof(float);
         if (pg.kv == BRASA_KV_F32) {

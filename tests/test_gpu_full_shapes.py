@@ -116,6 +116,37 @@ def test_serving_batch_of_64_sequences_matches_each_sequence_alone(B, ctx, group
         m.free()
 
 
+@pytest.mark.parametrize("nseq,prefix", [(62, 1024), (63, 3456)])
+def test_shared_prefix_blocks_of_two_and_three_groups(B, ctx, tmp_path_factory, nseq, prefix):
+    """Enough shared-prefix work that a block of its attention takes three groups of sequences (1 024 positions) or two (3 456) with one pair
+    of K and V tiles, the last group and the last block ragged. The first step's logits against the sequences alone; tolerance as above."""
+    d = tmp_path_factory.mktemp("groups")
+    cfg = BF.tiny_config(layers=1, hidden=512, heads=32, kv_heads=8, ffn=512, vocab=512)
+    BF.write_brasa(d / "model.brasa", cfg, BF.synth_weights(cfg, seed=12, std=0.04, norm_jitter=0.1))
+    rng = np.random.default_rng(65)
+    shared = rng.integers(0, 512, prefix).astype(np.uint32)
+    own = [rng.integers(0, 512, int(n)).astype(np.uint32) for n in rng.integers(3, 40, nseq)]
+    m = B.Qwen3.load(ctx, d / "model.brasa", B.Limits(ctx=prefix + 128, max_tokens=512, max_logit_rows=1, kv=B.KvType.F16))
+    try:
+        bt = B.Batch(m, max_seqs=nseq, num_pages=prefix // 16 + nseq * 4, max_positions=prefix + 64)
+        try:
+            bt.set_prefix(shared)
+            for x in own:
+                bt.add_sequence(x)
+            first = bt.peek_logits()
+            ids, _ = bt.decode(1)
+        finally:
+            bt.free()
+        for s in range(nseq):
+            prompt = np.concatenate([shared, own[s]])
+            for off in range(0, prompt.size, 512):
+                m.forward(prompt[off:off + 512], off, want_logits=False)
+            lg, _ = m.forward([int(ids[s, 0])], prompt.size)
+            assert np.abs(first[s] - lg[0]).max() <= 5e-3 * np.abs(lg[0]).max(), s
+    finally:
+        m.free()
+
+
 def test_serving_batch_sampled_tokens_follow_the_reference_sampler(B, ctx, group4_model):
     """Temperature 0.7 / top-p 0.95 with one PCG32 stream per sequence: every step's token of every sequence against
     the oracle's Sampler::sample (sampler.rs:60-146) fed the logits the GPU itself produced for that step."""
