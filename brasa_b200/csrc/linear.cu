@@ -428,7 +428,8 @@ struct TcParams {
 template <int BN>
 struct TcShape {
     static constexpr uint32_t STAGE = BM * BK * 2 + BN * BK * 2;
-    static constexpr uint32_t NS = BN == 256 ? 4 : (BN == 128 ? 6 : 8);
+    static constexpr uint32_t NS = BN == 256 ? 4 : (BN == 192 ? 5 : (BN == 128 ? 6 : 8));
+    static constexpr uint32_t ACC = BN == 192 ? 256 : BN;  // columns from one accumulator to the other (tensor memory is had in powers of two)
     static constexpr size_t SMEM = (size_t)NS * STAGE + EPI_BYTES + 1024;
 };
 
@@ -523,7 +524,7 @@ __device__ __forceinline__ void tile_out(const TcProblem &p, uint32_t acc, float
 
 template <int BN>
 __global__ void __launch_bounds__(256, 1) linear_tc_kernel(const __grid_constant__ TcParams tp) {
-    constexpr uint32_t NS = TcShape<BN>::NS, STAGE = TcShape<BN>::STAGE;
+    constexpr uint32_t NS = TcShape<BN>::NS, STAGE = TcShape<BN>::STAGE, ACC = TcShape<BN>::ACC;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     __shared__ uint64_t full[NS], empty[NS], acc_full[2], acc_empty[2];
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_kernel(const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 2) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(2u * BN) : "memory");
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base_s)), "r"(2u * ACC) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -611,7 +612,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_kernel(const __grid_constant
                     const uint32_t a0 = smem_u32(smem + s * STAGE), b0 = a0 + BM * BK * 2;
 #pragma unroll
                     for (uint32_t ks = 0; ks < BK / 16; ++ks)
-                        tc_mma(tmem + buf * BN, tc_desc_kmajor(a0 + ks * 32), tc_desc_kmajor(b0 + ks * 32), tc_idesc_bf16(BM, BN), (j > 0 || ks > 0) ? 1u : 0u);
+                        tc_mma(tmem + buf * ACC, tc_desc_kmajor(a0 + ks * 32), tc_desc_kmajor(b0 + ks * 32), tc_idesc_bf16(BM, BN), (j > 0 || ks > 0) ? 1u : 0u);
                     tc_commit(&empty[s]);
                     if (j + 1 == ns) tc_commit(&acc_full[buf]);
                 }
@@ -630,7 +631,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_kernel(const __grid_constant
             ok = __all_sync(0xffffffffu, wait(&acc_full[buf], (seq >> 1) & 1));
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const uint32_t ncol = min((uint32_t)BN, p.rows - row0), acc = tmem + buf * BN + ((q * 32u) << 16);
+            const uint32_t ncol = min((uint32_t)BN, p.rows - row0), acc = tmem + buf * ACC + ((q * 32u) << 16);
             if (tok0 + 32 * q < p.tokens) {
                 const bool bare = !p.bias && !p.resid && p.scale == 1.0f && p.cap == 0.0f;
                 if (p.act == LINEAR_ACT_GELU_TANH && p.mul && bare) tile_out<EPI_GELU_MUL>(p, acc, stage, row0, ncol, tok0 + 32 * q, lane);
@@ -647,7 +648,7 @@ __global__ void __launch_bounds__(256, 1) linear_tc_kernel(const __grid_constant
     __syncthreads();
     if (warp == 2) {
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * BN) : "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2u * ACC) : "memory");
     }
 }
 
@@ -757,14 +758,32 @@ int32_t brasa_linear_launch(brasa_cmd *cmd, const LinearProblem *ps, uint32_t co
         linear_f32_kernel<<<tiles, 256, 0, ctx->stream>>>(sp);
         return brasa_post_launch(cmd, "linear_f32");
     }
-    // the widest tile that still gives every SM work
-    auto tiles_of = [&](uint32_t bn) {
-        uint32_t t = 0;
-        for (uint32_t i = 0; i < n; ++i) t += (p[i].rows + bn - 1) / bn * ((p[i].tokens + BM - 1) / BM);
-        return t;
-    };
-    if (tiles_of(256) >= (uint32_t)ctx->sm_count) return launch_tc<256>(cmd, p, n);
-    if (tiles_of(128) >= (uint32_t)ctx->sm_count) return launch_tc<128>(cmd, p, n);
+    // The width whose busiest CTA (the first: tiles are dealt out in order) ends soonest. us a K stage of 64 columns where a CTA has several
+    // tiles; a quarter more where it has one, whose first stages nothing covers (but for the narrowest, whose stages are short). What bounds
+    // a stage is its operands' way from L2 (48 KB at the widest), for narrow tiles the chain of waits. us with widths of 64, 128, 192 and 256:
+    // 2 560 rows of 13 824 columns at 2 048 tokens 430, 307, 252, 262; at 1 000 275, 223, 162, 172; at 500 184, 135, 145, 160.
+    constexpr uint32_t WIDTH[4] = {64, 128, 192, 256};
+    constexpr double STAGE_US[4] = {0.40, 0.49, 0.56, 0.62}, ALONE[4] = {1.0, 1.25, 1.25, 1.25};
+    uint32_t best = 0;
+    double least = 1e30;
+    for (uint32_t w = 0; w < 4; ++w) {
+        uint64_t end = 0, stages = 0, mine = 0;  // tiles so far; stages and tiles of the first CTA
+        for (uint32_t i = 0; i < n; ++i) {
+            const uint64_t begin = end, sms = (uint32_t)ctx->sm_count;
+            end += (uint64_t)((p[i].rows + WIDTH[w] - 1) / WIDTH[w]) * ((p[i].tokens + BM - 1) / BM);
+            const uint64_t t = (end + sms - 1) / sms - (begin + sms - 1) / sms;
+            mine += t;
+            stages += t * ((p[i].seg[0].cols + BK - 1) / BK + (p[i].seg[1].cols + BK - 1) / BK);
+        }
+        const double us = (double)stages * STAGE_US[w] * (mine == 1 ? ALONE[w] : 1.0);
+        if (us < least) {
+            least = us;
+            best = w;
+        }
+    }
+    if (best == 3) return launch_tc<256>(cmd, p, n);
+    if (best == 2) return launch_tc<192>(cmd, p, n);
+    if (best == 1) return launch_tc<128>(cmd, p, n);
     return launch_tc<64>(cmd, p, n);
 }
 

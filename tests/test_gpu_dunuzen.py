@@ -119,6 +119,12 @@ def test_linear_group(ctx, tokens_n, shapes, f32):
         assert np.abs(got[:, :want.shape[1]] - want).max() <= tol
 
 
+def test_linear_group_in_tiles_of_192_rows(ctx):
+    """Shapes whose estimate names tiles of 192 rows: the last one of 74, the last tokens' of 103; then several tiles to a CTA."""
+    test_linear_group(ctx, 999, [(2570, 72, 24)], False)
+    test_linear_group(ctx, 2040, [(2570, 136, 0)], False)
+
+
 WINDOWS = [  # heads, dim, rot, vdim, window, pos0, tokens
     (2, 32, 16, 32, 5, 0, 40), (3, 64, 8, 64, 128, 0, 300), (1, 96, 32, 128, 129, 200, 131), (2, 128, 64, 128, 1000, 0, 257), (1, 192, 64, 64, 127, 1000, 2),
     (2, 16, 8, 72, 1, 3, 130), (1, 136, 16, 200, 33, 77, 65), (2, 64, 24, 128, 256, 255, 256)]

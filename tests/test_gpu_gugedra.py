@@ -131,6 +131,11 @@ def test_linear_epilogues(ctx, n, rows, cols, f32):
         assert np.abs(got[:, :rows] - r).max() <= 1e-5 * np.abs(r).max() and not got[:, rows:].any()
 
 
+def test_linear_epilogues_in_tiles_of_192_rows(ctx):
+    """The same out of tiles of 192 rows: three pairs of gate and up blocks a tile, ragged ends."""
+    test_linear_epilogues(ctx, 999, 640, 72, False)
+
+
 WINDOWS = [  # heads, kv_heads, dim, vdim, rot_dims, window, pos0, tokens, ring, softcap
     (4, 2, 32, 32, 32, 5, 0, 40, 0, 8.0), (6, 2, 64, 64, 16, 128, 0, 300, 384, 30.0), (3, 1, 96, 128, 24, 129, 200, 131, 384, 5.0), (2, 2, 128, 64, 128, 1000, 0, 257, 0, 0.0),
     (8, 1, 192, 128, 64, 127, 1000, 2, 128, 50.0), (2, 1, 16, 72, 6, 1, 3, 130, 256, 12.0), (1, 1, 200, 200, 10, 33, 77, 65, 128, 20.0), (4, 4, 64, 128, 32, 256, 255, 256, 512, 0.0),
