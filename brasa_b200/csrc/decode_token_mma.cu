@@ -169,30 +169,34 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
     }
     const bool save = op.save_resid != 0;
 #pragma unroll 1
-    for (uint32_t u0 = tid; u0 < nu; u0 += 2 * TK_THREADS) {
+    for (uint32_t u0 = tid; u0 < nu; u0 += 3 * TK_THREADS) {
         uint32_t u = u0, e = (u >> 2) * 32 + 4 * (u & 3);
-        bool two = u + TK_THREADS < nu;
+        uint32_t passes = min(3u, (nu - u + TK_THREADS - 1) / TK_THREADS);
         constexpr uint32_t FAR = TK_THREADS * 8;  // elements from a thread's unit to its next
-        uint4 a, b, a2 = make_uint4(0, 0, 0, 0), b2 = a2;
+        uint4 a, b, a2 = make_uint4(0, 0, 0, 0), b2 = a2, a3 = a2, b3 = a2;
         if (op.in_kind == IN_EMBED) {
             const bool in_table = c.token < vocab;
             const float4 z = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             const float4 va = in_table ? embed_quad(embed, c.token, cols, e / 4) : z, vb = in_table ? embed_quad(embed, c.token, cols, e / 4 + 4) : z;
             a = make_uint4(__float_as_uint(va.x), __float_as_uint(va.y), __float_as_uint(va.z), __float_as_uint(va.w));
             b = make_uint4(__float_as_uint(vb.x), __float_as_uint(vb.y), __float_as_uint(vb.z), __float_as_uint(vb.w));
-            u0 -= TK_THREADS;  // one pass at a time
-            two = false;
+            u0 -= 2 * TK_THREADS;  // one pass at a time
+            passes = 1;
         } else {
             const uint32_t *src = in + e;
 #pragma unroll 1
             for (uint32_t it = 0;; ++it) {
                 a = vs_load4(src);
                 b = vs_load4(src + 16);
-                if (two) {
+                if (passes > 1) {
                     a2 = vs_load4(src + FAR);
                     b2 = vs_load4(src + FAR + 16);
                 }
-                if ((vs_there(a) && vs_there(b) && vs_there(a2) && vs_there(b2)) || *c.abort_flag()) break;
+                if (passes > 2) {
+                    a3 = vs_load4(src + 2 * FAR);
+                    b3 = vs_load4(src + 2 * FAR + 16);
+                }
+                if ((vs_there(a) && vs_there(b) && vs_there(a2) && vs_there(b2) && vs_there(a3) && vs_there(b3)) || *c.abort_flag()) break;
                 if (it >= POLL_LIMIT) {
                     give_up(c, 3);
                     break;
@@ -227,10 +231,11 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
                 v[4] *= n1.x; v[5] *= n1.y; v[6] *= n1.z; v[7] *= n1.w;
             }
             x_eighth_to_planes(c.xfb(), tk_smem + op.meta_off, u >> 2, u & 3, v, bias);
-            if (!two) break;
-            two = false;
+            if (--passes == 0) break;
             a = a2;
             b = b2;
+            a2 = a3;
+            b2 = b3;
             u += TK_THREADS;
             e += FAR;
         }
