@@ -50,6 +50,8 @@ struct brasa_ctx {
     size_t gemm_part_bytes = 0;
     uint32_t *gemm_counters = nullptr;  // arrivals per output tile of that GEMM (GEMM_TC_COUNTERS words, zero between launches)
     bool recorded = false;              // a graph has been recorded: its kernels may hold the address of any workspace there was
+    std::mutex events_lock;
+    std::vector<std::pair<cudaEvent_t, cudaEvent_t>> events;  // timing events of finished commands for the next ones, at most 16 pairs
     std::vector<void *> outgrown;       // workspaces such a graph may still use, freed with the context (see brasa_workspace)
 };
 

@@ -97,6 +97,10 @@ void brasa_ctx_destroy(brasa_ctx *ctx) {
     cudaFree(ctx->kv_expand);
     cudaFree(ctx->gemm_counters);
     for (void *p : ctx->outgrown) cudaFree(p);
+    for (const auto &e : ctx->events) {
+        cudaEventDestroy(e.first);
+        cudaEventDestroy(e.second);
+    }
     cudaFree(ctx->gemv_trace);
     cudaFreeHost(ctx->status);
     cudaStreamDestroy(ctx->stream);
@@ -224,7 +228,16 @@ int32_t brasa_cmd_begin(brasa_ctx *ctx, brasa_cmd **out) {
     *out = nullptr;
     BRASA_CUDA(ctx, cudaSetDevice(ctx->device));
     brasa_cmd *c = new brasa_cmd{ctx, nullptr, nullptr, false};
-    if (cudaEventCreate(&c->start) != cudaSuccess || cudaEventCreate(&c->end) != cudaSuccess) {
+    {
+        const std::lock_guard<std::mutex> hold(ctx->events_lock);
+        if (!ctx->events.empty()) {
+            c->start = ctx->events.back().first;
+            c->end = ctx->events.back().second;
+            ctx->events.pop_back();
+        }
+    }
+    if (!c->start && (cudaEventCreate(&c->start) != cudaSuccess || cudaEventCreate(&c->end) != cudaSuccess)) {
+        if (c->start) cudaEventDestroy(c->start);
         delete c;
         return brasa_fail(ctx, BRASA_ECUDA, "cudaEventCreate failed");
     }
@@ -259,8 +272,15 @@ int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds) {
             rc = brasa_fail(ctx, BRASA_ETIMEOUT, "a bounded device-side wait ran out (status %u)", st);
         }
     }
-    cudaEventDestroy(cmd->start);
-    cudaEventDestroy(cmd->end);
+    {
+        const std::lock_guard<std::mutex> hold(ctx->events_lock);
+        if (rc == BRASA_OK && ctx->events.size() < 16) {
+            ctx->events.emplace_back(cmd->start, cmd->end);
+        } else {
+            cudaEventDestroy(cmd->start);
+            cudaEventDestroy(cmd->end);
+        }
+    }
     delete cmd;
     return rc;
 }
