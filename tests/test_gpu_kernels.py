@@ -369,6 +369,27 @@ def test_qk_norm_rope_store(B, ctx, K, kv, tokens, pos0):
     assert not kc.download(np.uint8, off).any()
 
 
+@pytest.mark.parametrize("kv", ["F16", "Q8_0"])
+@pytest.mark.parametrize("hq,hkv,tokens", [(4, 4, 5), (16, 4, 3), (8, 4, 5), (6, 2, 9), (12, 6, 1)])
+def test_qk_norm_rope_store_rows_per_warp(B, ctx, K, kv, hq, hkv, tokens):
+    """Four rows to a warp where both head counts allow it, one otherwise (and for 8-bit caches of few query heads to a KV head): the last
+    block ragged, the same bounds as above."""
+    kvt, rng, dim, pos0 = B.KvType[kv], O.Rng(28), 128, 5
+    q, k, v = (rng.vec(tokens * h * dim, 2.0) for h in (hq, hkv, hkv))
+    qn, kn = rng.vec(dim, 1.5), rng.vec(dim, 1.5)
+    table, (cos, sin) = B.RopeTable(ctx, 1e6, dim, pos0 + tokens), O.rope_table(1e6, dim, pos0 + tokens)
+    gq, gk, gv, gqn, gkn = (ctx.buffer_from(a) for a in (q, k, v, qn, kn))
+    n = tokens * hkv * dim
+    kc, vc = ctx.buffer(kvt.bytes(n)), ctx.buffer(kvt.bytes(n))
+    run(ctx, lambda c: K.qk_norm_rope_store(c, kvt, [gq, gk, gv], [gqn, gkn], 1e-6, table, [kc, vc], B.AttnShape(tokens, hq, hkv, dim, pos0, kvt)))
+    for got, x, w, h in ((gq, q, qn, hq), (gk, k, kn, hkv)):
+        want = O.rope_neox(O.rms_norm(x, w, dim, 1e-6), h, dim, pos0, cos, sin)
+        assert np.max(np.abs(got.download(np.float32) - want)) <= 2e-5 * np.max(np.abs(want))
+    for cache, x in ((kc, gk.download(np.float32)), (vc, v)):
+        want = O.quantize_kv_q8(x) if kv == "Q8_0" else O.f32_to_f16_array(x).view(np.uint8)
+        assert np.array_equal(cache.download(np.uint8, kvt.bytes(n)), want)
+
+
 @pytest.mark.parametrize("what", ["norm", "norm16", "qk"])
 def test_operands_written_by_the_call_before(B, ctx, K, what):
     """Operators overlap their neighbours' launches, and any buffer may be a norm weight or a RoPE table, one that the call before writes
