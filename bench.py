@@ -53,7 +53,7 @@ PROMPT, GENERATE, CTX = 512, 256, 2048
 SEED = 20251
 # dram__bytes_read + dram__bytes_write of one gate/up + SwiGLU GEMV launch under ncu (algorithmic bytes: 28 065 792)
 GATE_UP_TRAFFIC_BYTES = 28_130_000
-# dram__bytes_read + dram__bytes_write of one decode_token_kernel launch at position 512 under ncu (algorithmic bytes at
+# dram__bytes_read + dram__bytes_write of one decode_token_mma_kernel launch at position 512 under ncu (algorithmic bytes at
 # that position: 2 436 050 976)
 TOKEN_KERNEL_TRAFFIC_BYTES = 2_452_740_000
 # dram__bytes_read + dram__bytes_write of one serving decode step of 64 sequences (all its kernels, summed) under ncu,

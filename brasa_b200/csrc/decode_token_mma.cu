@@ -10,7 +10,7 @@
 // Bound: the exchanges and, in the rows phase, shared-memory bandwidth (a unit of 16 rows x 128 columns takes 22 wavefronts, 8 of
 // them the codes). Each operation ends with a block barrier although nothing there needs one: without it the warps that have no
 // rows to store poll for the next input beside those that do, and hold up their stores (1.24 against 1.10 ms a token).
-// us a token, one B200, decode_token.cu's in brackets: 4B architecture at 512 positions, f16 1 010 (1 118); at 16 384, q8_0 1 713 (1 845).
+// us a token, one B200, decode_token.cu's in brackets: 4B architecture at 512 positions, f16 1 006 (1 118); at 16 384, q8_0 1 713 (1 845).
 #include <memory>
 
 #include "decode_token_mma.h"

@@ -13,8 +13,8 @@
 //   * warp 1, one lane: tcgen05.mma for the stage, then tcgen05.commit to hand the stage back.
 //   * after the last stage warps 4-11 read the accumulators (tcgen05.ld, one token per lane) and store Y.
 // Up to three matrices that share X (q, k, v) go into one launch: the grid's x index walks their 128-row tiles.
-// More than 64 tokens of q4_0 matrices in whole tiles of 256 rows go to gemm_pair.cu, 9 to 64 to the few-token kernel below: this
-// kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
+// q4_0 matrices go to the few-token kernel below with up to 64 tokens, and up to 128 where it is ahead (brasa_gemm_tc_few_tokens), with
+// more, in whole tiles of 256 rows, to gemm_pair.cu: this kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
 // Every wait is bounded: a wait that runs out raises the context's status word and a CTA-wide flag, every role
 // leaves its loop, tensor memory is freed and the kernel returns.
 #include <cuda.h>
@@ -546,9 +546,9 @@ __global__ void __launch_bounds__(384, 1) gemm_tc_kernel(const __grid_constant__
 // this one's dependent, adds each shared tile's partial tiles in K order and the residual (every SM takes part; one block
 // doing it as the last to arrive took longer than the products themselves).
 //
-// 65 to 128 tokens (an admitted prompt; see brasa_gemm_tc_few_tokens) go through the same kernel with N = 128: the weights are converted once for all of them and a
-// product of 128 tokens takes the tensor core about as long as a chunk's conversion takes the warps. Its X takes twice the room, so
-// there are two chunks of X and A and five of raw weights instead of three and seven.
+// 65 to 128 tokens (an admitted prompt; see brasa_gemm_tc_few_tokens) go through the same kernel with N = 128: the weights are
+// converted once for all of them and a product of 128 tokens takes the tensor core about as long as a chunk's conversion takes the
+// warps. Its X takes twice the room, so there are two chunks of X and A and five of raw weights instead of three and seven.
 constexpr uint32_t SK_TT = 64, SK_TT_MOST = 128;  // tokens of the two forms
 template <uint32_t TT>
 struct Sk {
@@ -1125,7 +1125,7 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
 
 }  // namespace
 
-// How a product of up to 64 tokens is cut over the SMs (include/brasa_cuda.h): the (tile, stage) units in order, `blocks`
+// How a few-token product is cut over the SMs (include/brasa_cuda.h; scratch_bytes is that of 64 tokens, up to 128 take twice as much): the (tile, stage) units in order, `blocks`
 // equal runs, run b = units [b units / blocks, (b + 1) units / blocks).
 extern "C" int32_t brasa_gemm_few_tokens_plan(uint32_t sm_count, uint32_t tiles, uint32_t stages, uint32_t *blocks, uint32_t *max_parts,
                                               uint64_t *scratch_bytes) {
