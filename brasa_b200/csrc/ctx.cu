@@ -51,6 +51,7 @@ int32_t brasa_ctx_create(int32_t device, brasa_ctx **out) {
     if (cudaSetDevice(device) != cudaSuccess) return BRASA_ECUDA;
     brasa_ctx *ctx = new brasa_ctx();
     ctx->device = device;
+    ctx->events.reserve(16);  // (giving a pair back allocates nothing)
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) {
         delete ctx;
         return BRASA_ECUDA;
