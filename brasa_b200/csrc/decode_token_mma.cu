@@ -544,8 +544,8 @@ bool slot_rows(int qtype, uint32_t cols, uint32_t *lrps) {
 // cut into `slices` of its columns. The warps' first tiles are waited for before the input is (tile_begin), so the ring must hold them
 // all: row_warps x slots of a tile <= ring; where the block has more slots than the ring, a tile of several takes a third of it at most, so that
 // slots are asked for while a tile is worked on. Among what fits, the split whose busiest warp has the least shared-memory traffic (a group of
-// 128 columns: 10 wavefronts of x, 12 of sixteen rows), then the one with fewer partial sums. An lm_head's partial sums (sum_room floats
-// at most) take the ring's place in shared memory.
+// 128 columns: 10 wavefronts of x, 12 of sixteen rows), then the one with fewer partial sums. More than one slice asks for at most sum_room
+// partial sums; one slice's are as many as the block has rows, however many that is (ring_layout).
 constexpr uint32_t SUM_ROOM = 6144, MAX_COLS = 10240;  // (wider rows are fewer than four to a slot: a tile would hold most of the ring)
 // Hidden sizes this kernel takes; us a token against decode_token.cu's (4 layers, f16, 100 positions): 512 55.6 (57.4), but a short chat of
 // it 1 052 (1 023); 768 73.5 (75.4), 1 024 77.7 (83.8), 1 536 83.7 (90.3), 2 048 161 (167), 2 560 173 (201), 4 096 193 (182): rows of 4 096
@@ -572,6 +572,76 @@ Split gemv_split(uint32_t rows, uint32_t lrps, uint32_t cols, uint32_t ring, uin
     return best;
 }
 
+// Splits for a ring of `ring` slots and where things lie in shared memory then; bytes of it. op_rows: the most rows a block has of an
+// operation. Beside the ring lie x in fixed point from the bottom of one area, partial sums at its top, and the norm weight, over whose place
+// the attention's area goes on: it is staged during o_proj and down only.
+size_t ring_layout(std::vector<OpRecord> &ops, const std::vector<uint32_t> &op_rows, uint32_t G, uint32_t hidden, uint32_t ring, TokParams &p) {
+    uint32_t sums = 0, last_sums = 0, max_cols = 0, max_op_slots = 0;  // sums: of the layers' operations, of the lm_head
+    for (size_t i = 0; i < ops.size(); ++i) {
+        TokOp &o = ops[i].op;
+        if (o.type != OP_GEMV) continue;
+        const Split split = gemv_split(op_rows[i], o.lrps, o.cols, ring, SUM_ROOM);
+        o.tile = split.tile;
+        o.slices = split.slices;
+        o.step = split.row_warps * split.tile;
+        uint32_t &most = o.epilogue == EPI_LOGITS ? last_sums : sums;
+        most = std::max(most, op_rows[i] * o.slices);
+        max_cols = std::max(max_cols, o.cols);
+        max_op_slots = std::max(max_op_slots, (op_rows[i] + (1u << o.lrps) - 1) >> o.lrps);
+        const uint32_t groups = o.cols / 128;
+        for (uint32_t w = 0; w < TK_WARPS; ++w) {
+            const uint32_t place = w / o.slices, slice = w % o.slices;
+            ops[i].plan[w] = WarpPlan{place < split.row_warps ? place * o.tile : NO_ROWS, slice, groups * slice / o.slices, groups * (slice + 1) / o.slices};
+        }
+    }
+    const size_t nw_bytes = (size_t)hidden * 4;
+    size_t at = (size_t)ring * SLOT_CAP;
+    auto take = [&](size_t bytes) {
+        const size_t o = at;
+        at = (at + bytes + 15) / 16 * 16;
+        return (uint32_t)o;
+    };
+    const size_t x_bytes = (size_t)max_cols / 32 * X_BLOCK_BYTES, last_x = (size_t)hidden / 32 * X_BLOCK_BYTES;
+    const size_t area = std::max(x_bytes + (size_t)sums * 4, last_x + (size_t)last_sums * 4) + 16;
+    const size_t xf_bytes = (std::max(area, ATTN_AREA_BYTES > nw_bytes ? ATTN_AREA_BYTES - nw_bytes : 0) + 127) / 128 * 128;
+    p.nslot = ring;
+    p.nslot_mul = (uint32_t)(((1ull << 32) + ring - 1) / ring);
+    p.off_xf = take(xf_bytes);
+    p.off_nw = take(nw_bytes);
+    p.off_resid = take(((size_t)(hidden + G - 1) / G + 1) * 4);
+    p.off_sdesc = take((size_t)max_op_slots * sizeof(SlotDesc));
+    p.off_full = take(((size_t)ring + 1) * 8);
+    p.off_done = take((size_t)ring * 8);
+    p.off_red = take(48 * 4);
+    p.off_ops = take(OP_BUFFERS * sizeof(OpBuffer));
+    p.off_zeros = take(32 + 32 + 4) / 32 * 32 + 16;  // off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
+    for (OpRecord &r : ops) {
+        r.op.meta_off = p.off_xf + r.op.cols / 32 * X_PLANE_BYTES;
+        r.op.part_off = (uint32_t)(p.off_xf + xf_bytes - (size_t)(r.op.epilogue == EPI_LOGITS ? last_sums : sums) * 4) & ~15u;
+    }
+    return at;
+}
+// The ring's length and the operations' splits want each other: the longest ring that the splits it allows leave room for (p and smem are its
+// layout), 0 where there is none. A ring of one slot counts as none: 2^32 / 1 does not fit nslot_mul, and a block that waits for its
+// only slot's next rows keeps no weights coming. An lm_head of millions of rows, whose partial sums lie beside the ring, shortens it that far.
+uint32_t fit_ring(std::vector<OpRecord> &ops, const std::vector<uint32_t> &op_rows, uint32_t G, uint32_t hidden, uint32_t smem_optin, TokParams &p, size_t &smem) {
+    for (uint32_t ring = smem_optin / SLOT_CAP; ring >= 2; --ring) {
+        smem = ring_layout(ops, op_rows, G, hidden, ring, p);
+        if (smem <= smem_optin) return ring;
+    }
+    return 0;
+}
+// The most rows that one of G blocks has of an operation, over its matrices.
+uint32_t most_rows(const TokOp &o, uint32_t G) {
+    uint32_t most = 0;
+    for (uint32_t b = 0; b < G; ++b) {
+        uint32_t r0, r1, first[3], nrows[3];
+        block_rows(o.total_rows, o.nmat, o.rows, o.epilogue == EPI_SWIGLU, b, G, r0, r1, first, nrows);
+        most = std::max(most, nrows[0] + nrows[1] + nrows[2]);
+    }
+    return most;
+}
+
 }  // namespace
 
 struct brasa_token_mma {
@@ -584,6 +654,36 @@ struct brasa_token_mma {
     size_t vector_bytes = 0;
     uint32_t timeouts_seen = 0;  // the context's count of abandoned waits when the vectors were last known clean
 };
+
+extern "C" uint32_t brasa_token_ring_slots(uint32_t sm_count, uint32_t smem_bytes, uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t ffn, uint32_t vocab,
+                                           int32_t head_qtype, int32_t kv) {
+    brasa_token_model m{};
+    m.hidden = hidden;
+    m.heads = heads;
+    m.ffn = ffn;
+    m.kv = kv;
+    if (sm_count == 0 || heads == 0 || kv_heads == 0 || vocab == 0 || (head_qtype != BRASA_Q4_0 && head_qtype != BRASA_Q6_0) || !brasa_token_mma_takes(m)) return 0;
+    std::vector<OpRecord> ops;
+    std::vector<uint32_t> op_rows;
+    auto add = [&](int32_t qtype, uint32_t cols, std::initializer_list<uint32_t> rows, uint32_t epilogue) {
+        OpRecord r{};
+        r.op.type = OP_GEMV;
+        r.op.cols = cols;
+        r.op.epilogue = epilogue;
+        for (uint32_t n : rows) r.op.total_rows += r.op.rows[r.op.nmat++] = n;
+        if (epilogue == EPI_SWIGLU) r.op.total_rows = r.op.rows[0];
+        if (!slot_rows(qtype, cols, &r.op.lrps)) return false;
+        op_rows.push_back(most_rows(r.op, sm_count));
+        ops.push_back(r);
+        return true;
+    };
+    if (!add(BRASA_Q4_0, hidden, {heads * 128, kv_heads * 128, kv_heads * 128}, EPI_SCALE) || !add(BRASA_Q4_0, heads * 128, {hidden}, EPI_RESID) ||
+        !add(BRASA_Q4_0, hidden, {ffn, ffn}, EPI_SWIGLU) || !add(BRASA_Q4_0, ffn, {hidden}, EPI_RESID) || !add(head_qtype, hidden, {vocab}, EPI_LOGITS))
+        return 0;
+    TokParams p{};
+    size_t smem = 0;
+    return fit_ring(ops, op_rows, sm_count, hidden, smem_bytes, p, smem);
+}
 
 bool brasa_token_mma_takes(const brasa_token_model &m) {
     if (m.kv == BRASA_KV_F32 || m.tp.world > 1 || m.hidden < MIN_HIDDEN || m.hidden > MAX_HIDDEN) return false;
@@ -685,10 +785,9 @@ int32_t brasa_token_mma_create(brasa_ctx *ctx, const brasa_token_model &m, brasa
     gemv_op(1, &m.head, EPI_LOGITS, true, m.final_norm, x_op, false);
     BRASA_REQUIRE(ctx, (size_t)(vs_next - (uint32_t *)vs_base) <= par_words, "token program: activation vectors overran their area");
     BRASA_REQUIRE(ctx, ops.size() + 2 < EPOCH_SPAN, "token program: too many operations");
-    uint32_t staged = 0, max_cols = 0;
+    uint32_t staged = 0;
     for (size_t i = 0; i < ops.size(); ++i) {
         TokOp &o = ops[i].op;
-        max_cols = std::max(max_cols, o.cols);
         if (o.normw) o.nw_use = ++staged;
         if (i + 1 < ops.size() && ops[i + 1].op.normw) {
             BRASA_REQUIRE(ctx, !o.normw, "token program: two operations in a row with a norm weight");
@@ -701,7 +800,6 @@ int32_t brasa_token_mma_create(brasa_ctx *ctx, const brasa_token_model &m, brasa
     std::vector<SlotDesc> slots;
     std::vector<uint32_t> slot_begin(G + 1, 0), op_rows(ops.size(), 0);  // op_rows: the most rows a block has of an operation
     std::vector<BlockRows> block_ops(ops.size() * G, BlockRows{});
-    uint32_t max_op_slots = 0;
     for (uint32_t b = 0; b < G; ++b) {
         slot_begin[b] = (uint32_t)slots.size();
         for (size_t oi = 0; oi < ops.size(); ++oi) {
@@ -728,63 +826,13 @@ int32_t brasa_token_mma_create(brasa_ctx *ctx, const brasa_token_model &m, brasa
                 slots.push_back(d);
             }
             op_rows[oi] = std::max(op_rows[oi], items);
-            max_op_slots = std::max(max_op_slots, (items + rps - 1) / rps);
         }
     }
     slot_begin[G] = (uint32_t)slots.size();
 
-    // The ring's length and the operations' splits want each other: the longest ring that the splits it allows leave room for. Beside it lie
-    // x in fixed point from the bottom of one area, partial sums at its top, and the norm weight, over whose place the attention's area
-    // goes on: it is staged during o_proj and down only.
     TokParams &p = prog->params;
-    const size_t nw_bytes = (size_t)H * 4;
-    auto layout = [&](uint32_t ring) -> size_t {  // splits for a ring of this many slots; bytes of shared memory
-        uint32_t sums = 0, last_sums = 0;         // of the layers' operations, of the lm_head
-        for (size_t i = 0; i < ops.size(); ++i) {
-            TokOp &o = ops[i].op;
-            if (o.type != OP_GEMV) continue;
-            const Split split = gemv_split(op_rows[i], o.lrps, o.cols, ring, SUM_ROOM);
-            o.tile = split.tile;
-            o.slices = split.slices;
-            o.step = split.row_warps * split.tile;
-            uint32_t &most = o.epilogue == EPI_LOGITS ? last_sums : sums;
-            most = std::max(most, op_rows[i] * o.slices);
-            const uint32_t groups = o.cols / 128;
-            for (uint32_t w = 0; w < TK_WARPS; ++w) {
-                const uint32_t place = w / o.slices, slice = w % o.slices;
-                ops[i].plan[w] = WarpPlan{place < split.row_warps ? place * o.tile : NO_ROWS, slice, groups * slice / o.slices, groups * (slice + 1) / o.slices};
-            }
-        }
-        size_t at = (size_t)ring * SLOT_CAP;
-        auto take = [&](size_t bytes) {
-            const size_t o = at;
-            at = (at + bytes + 15) / 16 * 16;
-            return (uint32_t)o;
-        };
-        const size_t x_bytes = (size_t)max_cols / 32 * X_BLOCK_BYTES, last_x = (size_t)H / 32 * X_BLOCK_BYTES;
-        const size_t area = std::max(x_bytes + (size_t)sums * 4, last_x + (size_t)last_sums * 4) + 16;
-        const size_t xf_bytes = (std::max(area, ATTN_AREA_BYTES > nw_bytes ? ATTN_AREA_BYTES - nw_bytes : 0) + 127) / 128 * 128;
-        p.nslot = ring;
-        p.nslot_mul = (uint32_t)(((1ull << 32) + ring - 1) / ring);
-        p.off_xf = take(xf_bytes);
-        p.off_nw = take(nw_bytes);
-        p.off_resid = take(((size_t)(H + G - 1) / G + 1) * 4);
-        p.off_sdesc = take((size_t)max_op_slots * sizeof(SlotDesc));
-        p.off_full = take(((size_t)ring + 1) * 8);
-        p.off_done = take((size_t)ring * 8);
-        p.off_red = take(48 * 4);
-        p.off_ops = take(OP_BUFFERS * sizeof(OpBuffer));
-        p.off_zeros = take(32 + 32 + 4) / 32 * 32 + 16;  // off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
-        for (OpRecord &r : ops) {
-            r.op.meta_off = p.off_xf + r.op.cols / 32 * X_PLANE_BYTES;
-            r.op.part_off = (uint32_t)(p.off_xf + xf_bytes - (size_t)(r.op.epilogue == EPI_LOGITS ? last_sums : sums) * 4) & ~15u;
-        }
-        return at;
-    };
-    uint32_t ring = (uint32_t)(ctx->smem_optin / SLOT_CAP);
-    while (ring > 0 && layout(ring) > ctx->smem_optin) --ring;
+    const uint32_t ring = fit_ring(ops, op_rows, G, H, (uint32_t)ctx->smem_optin, p, prog->smem);
     if (ring == 0) return BRASA_OK;  // (the vectors leave no room for weights)
-    prog->smem = layout(ring);
 
     void *d_ops, *d_slots, *d_begin, *d_bops;
     BRASA_TRY(upload(ops.data(), ops.size() * sizeof(OpRecord), &d_ops));

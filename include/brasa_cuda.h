@@ -178,6 +178,11 @@ int32_t brasa_k_gemm_add(brasa_cmd *cmd, brasa_qmatrix w, brasa_arg x_f16, brasa
 int32_t brasa_gemm_few_tokens_plan(uint32_t sm_count, uint32_t tiles, uint32_t stages, uint32_t *blocks, uint32_t *max_parts, uint64_t *scratch_bytes);
 /* the block whose run holds `unit` (UINT32_MAX for arguments outside a plan) */
 uint32_t brasa_gemm_few_tokens_owner(uint32_t units, uint32_t blocks, uint32_t unit);
+/* Slots of the weight ring with which the whole-token decode kernel on integer products (decode_token_mma.cu) runs such a model on a
+ * GPU of sm_count SMs with smem_bytes of shared memory per block: at least 2, or 0 where another path runs its tokens. No counterpart in
+ * the reference, whose decode step is one dispatch per operation. head_qtype: of the lm_head; kv: BRASA_KV_*. */
+uint32_t brasa_token_ring_slots(uint32_t sm_count, uint32_t smem_bytes, uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t ffn, uint32_t vocab,
+                                int32_t head_qtype, int32_t kv);
 /* acc += W x, then out_f16 = f16(rms_norm(acc) * norm_w): a layer's residual add and the norm that opens the next block
  * (qwen3.rs:810-826 then :700-712 as one call). One GEMM and one kernel behind it for up to 64 tokens; otherwise the two calls. */
 int32_t brasa_k_gemm_add_rms_norm_f16(brasa_cmd *cmd, brasa_qmatrix w, brasa_arg x_f16, brasa_arg acc, brasa_arg scratch, brasa_arg norm_w,

@@ -200,6 +200,36 @@ def test_few_token_gemm_partition(B):
     assert L.brasa_gemm_few_tokens_owner(100, 10, 100) == 0xFFFFFFFF
 
 
+def test_token_ring_is_one_the_kernel_can_index(B):
+    """The weight ring of the whole-token kernel on integer products over models up to vocabularies of 2^23: none, or at least two slots (one
+    would make the kernel's reciprocal of their number 2^32, which its 32-bit word holds as 0: every slot but the first would lie behind
+    the ring), never more for a larger vocabulary; and that reciprocal gives the list index of every slot exactly."""
+    L = B.lib()
+    L.brasa_token_ring_slots.argtypes = [C.c_uint32] * 7 + [C.c_int32] * 2
+    L.brasa_token_ring_slots.restype = C.c_uint32
+    SMS, SMEM, Q4, Q6 = 148, 232448, int(B.WeightType.Q4_0), int(B.WeightType.Q6_0)
+    f16, q8, f32 = int(B.KvType.F16), int(B.KvType.Q8_0), int(B.KvType.F32)
+    assert L.brasa_token_ring_slots(SMS, SMEM, 2560, 32, 8, 9728, 151936, Q6, f16) >= 4  # the 4B architecture
+    assert L.brasa_token_ring_slots(SMS, SMEM, 2560, 32, 8, 9728, 151936, Q6, f32) == 0  # decode_token.cu's
+    assert L.brasa_token_ring_slots(SMS, SMEM, 512, 8, 2, 1536, 1024, Q6, f16) == 0
+    seen = set()
+    for hidden, heads, ffn in [(768, 6, 1024), (1024, 16, 3072), (1024, 40, 10240), (1536, 8, 4096), (2048, 16, 6144), (2560, 32, 9728), (3072, 24, 8192), (3072, 80, 10240)]:
+        for head in (Q4, Q6):
+            for kv in (f16, q8):
+                last = 1 << 30
+                for vocab in [*range(1 << 17, (1 << 23) + 1, 1 << 17)]:
+                    ring = L.brasa_token_ring_slots(SMS, SMEM, hidden, heads, heads // 2, ffn, vocab, head, kv)
+                    assert ring != 1 and ring <= last, (hidden, vocab, ring)
+                    last = ring
+                    seen.add(ring)
+    assert 0 in seen and 2 in seen and max(seen) >= 7
+    for ring in seen - {0}:
+        mul = ((1 << 32) + ring - 1) // ring
+        assert mul < 1 << 32
+        k = np.concatenate([np.arange(4096, dtype=np.uint64), np.random.default_rng(1).integers(0, 1 << 24, 4096).astype(np.uint64)])
+        assert np.array_equal((k * np.uint64(mul)) >> np.uint64(32), k // np.uint64(ring)), ring
+
+
 @pytest.mark.parametrize("name,kernels", [("flash_tc.cu", 2), ("window_attn.cu", 1)])
 def test_row_warps_of_the_attention_kernels_leave_together(name, kernels):
     """The two warps that hold the same query rows meet at counted barriers, and each may give up a wait on its own. So a meeting has to tell
