@@ -457,11 +457,11 @@ __device__ __forceinline__ void gemv_epilogue(const TokCtx &c, const TokOp &op, 
             Best other{__shfl_xor_sync(0xffffffffu, bst.v, o), __shfl_xor_sync(0xffffffffu, bst.i, o)};
             bst = better(bst, other);
         }
-        if (lane == 0) { c.red[16 + warp] = bst.v; c.red[32 + warp] = __uint_as_float(bst.i); }
+        if (lane == 0) { c.red[RED_BEST + warp] = bst.v; c.red[RED_INDEX + warp] = __uint_as_float(bst.i); }
         __syncthreads();
         if (tid == 0) {
 #pragma unroll 1
-            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red[16 + w], __float_as_uint(c.red[32 + w])});
+            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red[RED_BEST + w], __float_as_uint(c.red[RED_INDEX + w])});
             ll_store(cand + 2 * c.b, __float_as_uint(bst.v), epoch);
             ll_store(cand + 2 * c.b + 1, bst.i, epoch);
         }
@@ -483,8 +483,8 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
     c.sdesc = reinterpret_cast<uint4 *>(c.nwbuf + p.nw_floats);      // descriptors of the slots this operation refills
     c.full = reinterpret_cast<uint64_t *>(c.sdesc + p.sdesc_n);
     c.done = reinterpret_cast<uint32_t *>(c.full + p.nslot);
-    c.red = reinterpret_cast<float *>(c.done + p.nslot);             // [48]
-    uint32_t *ops_s = reinterpret_cast<uint32_t *>(c.red + 48);      // [2][OPS_WORDS]: operation, then this block's rows
+    c.red = reinterpret_cast<float *>(c.done + p.nslot);             // [RED_WORDS]
+    uint32_t *ops_s = reinterpret_cast<uint32_t *>(c.red + RED_WORDS);      // [2][OPS_WORDS]: operation, then this block's rows
     c.s_abort = ops_s + 2 * OPS_WORDS;
     c.status = p.status;
     c.trace = p.trace;
@@ -576,7 +576,7 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
                 if (warp == TK_WARPS - 1) {  // 1 / rms of the whole input from the warps' sums, parked for the epilogue
                     float tot = c.red[lane & (TK_WARPS - 1)];
                     for (int o = TK_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-                    if (lane == 0) c.red[47] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
+                    if (lane == 0) c.red[RED_SCALE] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
                 }
                 if (op.qtype == BRASA_Q4_0) {
                     if (op.fast && op.nact == 5) wr = gemv_rows<BRASA_Q4_0, PLANES, 5>(c, op, bo, gslot, half, wr);
@@ -592,7 +592,7 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
                 __syncthreads();
                 TRACE(8);
             }
-            gemv_epilogue(c, op, bo, c.red[47], epoch, p.logits, p.cand, p);
+            gemv_epilogue(c, op, bo, c.red[RED_SCALE], epoch, p.logits, p.cand, p);
         } else {
             attention_op<KV>(AttnCtx{c.xfb, c.s_abort, c.status, c.G, c.b, c.pos, c.par_cur, c.par_alt}, op, oi, epoch, p.heads, p.kv_heads, p.max_chunks, p.cos_t, p.sin_t, p.partials, p.attn_scale);
         }
@@ -617,11 +617,11 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
             Best other{__shfl_xor_sync(0xffffffffu, bst.v, o), __shfl_xor_sync(0xffffffffu, bst.i, o)};
             bst = better(bst, other);
         }
-        if (lane == 0) { c.red[16 + warp] = bst.v; c.red[32 + warp] = __uint_as_float(bst.i); }
+        if (lane == 0) { c.red[RED_BEST + warp] = bst.v; c.red[RED_INDEX + warp] = __uint_as_float(bst.i); }
         __syncthreads();
         if (tid == 0) {
 #pragma unroll 1
-            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red[16 + w], __float_as_uint(c.red[32 + w])});
+            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red[RED_BEST + w], __float_as_uint(c.red[RED_INDEX + w])});
             if (p.tp_world > 1) {
                 // this rank's best (logit, vocabulary row) to every rank, then the best of all: largest logit, lowest row
                 // among equals (NaN never wins: it never became a candidate)
@@ -911,7 +911,7 @@ int32_t brasa_token_program_create(brasa_ctx *ctx, const brasa_token_model &m, b
     p.resid_floats = ((H + G - 1) / G + 4) & ~3u;
     p.sdesc_n = max_op_slots;
     p.nw_floats = (nw_floats + 3) & ~3u;
-    const size_t fixed = p.xf_bytes + (size_t)(p.part_floats + p.resid_floats + p.nw_floats) * 4 + (size_t)p.sdesc_n * 16 + 48 * 4 + 2 * OPS_WORDS * 4 + 16;
+    const size_t fixed = p.xf_bytes + (size_t)(p.part_floats + p.resid_floats + p.nw_floats) * 4 + (size_t)p.sdesc_n * 16 + RED_WORDS * 4 + 2 * OPS_WORDS * 4 + 16;
     BRASA_REQUIRE(ctx, fixed + 2 * (SLOT_CAP + 12) + 1024 <= ctx->smem_optin, "token program: the model's vectors do not fit shared memory");
     uint32_t nslot = (uint32_t)((ctx->smem_optin - 1024 - fixed) / (SLOT_CAP + 12));
     nslot &= ~1u;  // even: a ring slot always serves the same half of the warps

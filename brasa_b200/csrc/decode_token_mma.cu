@@ -120,7 +120,7 @@ struct TokCtx {
     __device__ __forceinline__ uint64_t *nw_full() const { return full(p.nslot); }
     __device__ __forceinline__ uint32_t *done(uint32_t s) const { return reinterpret_cast<uint32_t *>(tk_smem + p.off_done) + s; }  // warps that are done with a slot
     __device__ __forceinline__ uint32_t *gen(uint32_t s) const { return done(p.nslot + s); }                                       // how often it has been reused
-    __device__ __forceinline__ float *red() const { return reinterpret_cast<float *>(tk_smem + p.off_red); }                       // [48]
+    __device__ __forceinline__ float *red() const { return reinterpret_cast<float *>(tk_smem + p.off_red); }                       // [RED_WORDS]
     __device__ __forceinline__ OpBuffer *ops() const { return reinterpret_cast<OpBuffer *>(tk_smem + p.off_ops); }                 // [OP_BUFFERS]
     __device__ __forceinline__ uint32_t *zeros() const { return reinterpret_cast<uint32_t *>(tk_smem + p.off_zeros); }               // [8]
     __device__ __forceinline__ volatile uint32_t *abort_flag() const { return zeros() + 8; }
@@ -379,11 +379,11 @@ __device__ __forceinline__ void gemv_epilogue(const TokCtx &c, const TokOp &op, 
             Best other{__shfl_xor_sync(0xffffffffu, bst.v, o), __shfl_xor_sync(0xffffffffu, bst.i, o)};
             bst = better(bst, other);
         }
-        if (lane == 0) { c.red()[16 + warp] = bst.v; c.red()[32 + warp] = __uint_as_float(bst.i); }
+        if (lane == 0) { c.red()[RED_BEST + warp] = bst.v; c.red()[RED_INDEX + warp] = __uint_as_float(bst.i); }
         __syncthreads();
         if (tid == 0) {
 #pragma unroll 1
-            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red()[16 + w], __float_as_uint(c.red()[32 + w])});
+            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red()[RED_BEST + w], __float_as_uint(c.red()[RED_INDEX + w])});
             ll_store(cand + 2 * c.b, __float_as_uint(bst.v), epoch);
             ll_store(cand + 2 * c.b + 1, bst.i, epoch);
         }
@@ -476,13 +476,13 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
             if (warp == TK_WARPS - 1) {  // 1 / rms of the whole input from the warps' sums, parked for the epilogue
                 float tot = c.red()[lane & (TK_WARPS - 1)];
                 for (int o = TK_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
-                if (lane == 0) c.red()[47] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
+                if (lane == 0) c.red()[RED_SCALE] = op.scaled ? 1.0f / sqrtf(tot / (float)op.cols + op.eps) : 1.0f;
             }
             if (op.qtype == BRASA_Q4_0) gemv_rows<BRASA_Q4_0>(c, op, job, rec.plan[warp], nrows, gslot);
             else gemv_rows<BRASA_Q6_0>(c, op, job, rec.plan[warp], nrows, gslot);
             gslot += total_slots;
             __syncthreads();
-            gemv_epilogue(c, op, bo, c.red()[47], epoch, p.logits, p.cand);
+            gemv_epilogue(c, op, bo, c.red()[RED_SCALE], epoch, p.logits, p.cand);
         } else {
             if (warp == TK_WARPS - 2) cp_async_wait();
             attention_op<KV>(AttnCtx{c.xfb(), c.abort_flag(), p.status, c.G, c.b, c.pos, c.par_cur, c.par_alt}, op, oi, epoch, p.heads, p.kv_heads, p.max_chunks, p.cos_t, p.sin_t, p.partials, p.attn_scale);
@@ -507,11 +507,11 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
             Best other{__shfl_xor_sync(0xffffffffu, bst.v, o), __shfl_xor_sync(0xffffffffu, bst.i, o)};
             bst = better(bst, other);
         }
-        if (lane == 0) { c.red()[16 + warp] = bst.v; c.red()[32 + warp] = __uint_as_float(bst.i); }
+        if (lane == 0) { c.red()[RED_BEST + warp] = bst.v; c.red()[RED_INDEX + warp] = __uint_as_float(bst.i); }
         __syncthreads();
         if (tid == 0) {
 #pragma unroll 1
-            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red()[16 + w], __float_as_uint(c.red()[32 + w])});
+            for (int w = 1; w < TK_WARPS; ++w) bst = better(bst, Best{c.red()[RED_BEST + w], __float_as_uint(c.red()[RED_INDEX + w])});
             const uint32_t tok = (bst.v == -INFINITY || bst.i == 0xffffffffu) ? 0u : bst.i;
             *p.next_id = tok;
             p.ids[0] = tok;
@@ -612,7 +612,7 @@ size_t ring_layout(std::vector<OpRecord> &ops, const std::vector<uint32_t> &op_r
     p.off_sdesc = take((size_t)max_op_slots * sizeof(SlotDesc));
     p.off_full = take(((size_t)ring + 1) * 8);
     p.off_done = take((size_t)ring * 8);
-    p.off_red = take(48 * 4);
+    p.off_red = take(RED_WORDS * 4);
     p.off_ops = take(OP_BUFFERS * sizeof(OpBuffer));
     p.off_zeros = take(32 + 32 + 4) / 32 * 32 + 16;  // off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
     for (OpRecord &r : ops) {

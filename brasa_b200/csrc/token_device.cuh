@@ -12,6 +12,12 @@ constexpr uint32_t POLL_LIMIT = 1u << 20;  // polls of an activation word before
 constexpr uint32_t EPOCH_SPAN = 1024;      // epochs of one launch; operations + 2 must stay below it
 constexpr uint32_t VS_EMPTY = 0xffffffffu;  // an activation word nobody has written in this launch
 
+// Words of a block's reduction area: the warps' sums of x^2 from word 0, each warp's best logit and its index, and the scale of the operation's
+// outputs. The scale has a word of its own: every warp reads it behind the rows' barrier, and a warp without rows of the lm_head stores its best
+// without another barrier.
+constexpr uint32_t RED_BEST = TK_WARPS, RED_INDEX = 2 * TK_WARPS, RED_SCALE = 3 * TK_WARPS, RED_WORDS = RED_SCALE + 4;
+static_assert(RED_WORDS % 4 == 0, "what follows the area is copied in 16-byte words");
+
 enum { OP_GEMV = 0, OP_ATTN = 1 };
 enum { IN_LL = 0, IN_EMBED = 1 };
 enum { EPI_SCALE = 0, EPI_SWIGLU = 1, EPI_RESID = 2, EPI_LOGITS = 3 };

@@ -230,6 +230,23 @@ def test_token_ring_is_one_the_kernel_can_index(B):
         assert np.array_equal((k * np.uint64(mul)) >> np.uint64(32), k // np.uint64(ring)), ring
 
 
+@pytest.mark.parametrize("name", ["decode_token.cu", "decode_token_mma.cu"])
+def test_token_kernels_keep_the_output_scale_in_a_word_of_its_own(name):
+    """Behind the rows' barrier every warp of a whole-token kernel reads the scale of the operation's outputs; a warp without rows of the lm_head
+    then stores its best logit with no barrier in between. So no word of that store, whatever the warp, may be the scale's. Read from the source:
+    the window is some hundred cycles."""
+    words = dict(TK_WARPS=16)
+    for a, b in re.findall(r"\b(RED_\w+) = ([^,;]+)", (ROOT / "brasa_b200" / "csrc" / "token_device.cuh").read_text()):
+        words[a] = eval(b, {}, words)
+    text = (ROOT / "brasa_b200" / "csrc" / name).read_text()
+    stores = [(i, [eval(i, {}, dict(words, warp=w)) for w in range(16)] if "warp" in i else [eval(i, {}, words)])
+              for i in re.findall(r"\bred(?:\(\))?\[([^\]&]+)\] = ", text)]
+    best, scale = [w for i, ws in stores if "warp" in i and i != "warp" for w in ws], [ws[0] for i, ws in stores if "warp" not in i]
+    assert len(best) == 64 and len(scale) == 1  # a block's best, the choice among the blocks: logit and index each
+    assert scale[0] not in best and scale[0] >= 16 and max(best + scale) < words["RED_WORDS"]
+    assert re.findall(r"gemv_epilogue\(c, op, bo, c\.red(?:\(\))?\[(\w+)\]", text) == ["RED_SCALE"]
+
+
 @pytest.mark.parametrize("name,kernels", [("flash_tc.cu", 2), ("window_attn.cu", 1)])
 def test_row_warps_of_the_attention_kernels_leave_together(name, kernels):
     """The two warps that hold the same query rows meet at counted barriers, and each may give up a wait on its own. So a meeting has to tell
