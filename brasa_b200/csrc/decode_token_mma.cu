@@ -124,6 +124,7 @@ struct TokCtx {
     __device__ __forceinline__ OpBuffer *ops() const { return reinterpret_cast<OpBuffer *>(tk_smem + p.off_ops); }                 // [OP_BUFFERS]
     __device__ __forceinline__ uint32_t *zeros() const { return reinterpret_cast<uint32_t *>(tk_smem + p.off_zeros); }               // [8]
     __device__ __forceinline__ volatile uint32_t *abort_flag() const { return zeros() + 8; }
+    __device__ __forceinline__ volatile uint32_t *norms_asked() const { return zeros() + 9; }  // norm weights whose copy has been asked for
     __device__ __forceinline__ uint32_t *status_word() const { return p.status; }
 };
 
@@ -417,7 +418,10 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
         for (uint32_t i = lane; i <= REC_WORDS; i += 32)
             cp_async16(dst + i, i < REC_WORDS ? reinterpret_cast<const uint4 *>(p.ops + oi) + i : reinterpret_cast<const uint4 *>(p.block_ops + (size_t)oi * G + b));
     };
+    // (not after a wait that gave up: the norm weight before this one may be on its way still, and its barrier must not be armed anew)
     auto stage_norm = [&](const float *w, uint32_t cols) {
+        if (*c.abort_flag()) return;
+        *c.norms_asked() = *c.norms_asked() + 1;
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_expect_tx(c.nw_full(), cols * 4);
         bulk_g2s(c.nwbuf(), w, cols * 4, c.nw_full());
@@ -431,6 +435,7 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
         }
         mbar_init(c.nw_full(), 1);
         *c.abort_flag() = 0;
+        *c.norms_asked() = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (tid < 8) c.zeros()[tid] = 0;
@@ -491,7 +496,10 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
     }
 
     // a block that has given up waits (again with a limit) for its copies before it leaves
-    if (*c.abort_flag() && tid < (int)min(p.nslot, c.my_slots)) mbar_wait(c.full(tid), *c.gen(tid) & 1);
+    if (*c.abort_flag()) {
+        if (tid < (int)min(p.nslot, c.my_slots)) mbar_wait(c.full(tid), *c.gen(tid) & 1);
+        if (tid == TK_THREADS - 1 && *c.norms_asked()) mbar_wait(c.nw_full(), (*c.norms_asked() - 1) & 1);
+    }
 
     // ---- greedy choice and the step's bookkeeping: block 0 gathers every block's best logit ----
     if (b == 0) {
@@ -614,7 +622,7 @@ size_t ring_layout(std::vector<OpRecord> &ops, const std::vector<uint32_t> &op_r
     p.off_done = take((size_t)ring * 8);
     p.off_red = take(RED_WORDS * 4);
     p.off_ops = take(OP_BUFFERS * sizeof(OpBuffer));
-    p.off_zeros = take(32 + 32 + 4) / 32 * 32 + 16;  // off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
+    p.off_zeros = take(16 + 32 + 8) / 32 * 32 + 16;  // zeros, two words; off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
     for (OpRecord &r : ops) {
         r.op.meta_off = p.off_xf + r.op.cols / 32 * X_PLANE_BYTES;
         r.op.part_off = (uint32_t)(p.off_xf + xf_bytes - (size_t)(r.op.epilogue == EPI_LOGITS ? last_sums : sums) * 4) & ~15u;

@@ -247,6 +247,23 @@ def test_token_kernels_keep_the_output_scale_in_a_word_of_its_own(name):
     assert re.findall(r"gemv_epilogue\(c, op, bo, c\.red(?:\(\))?\[(\w+)\]", text) == ["RED_SCALE"]
 
 
+def test_token_kernel_that_gave_up_waits_for_every_copy_it_asked_for():
+    """A block of the whole-token kernel on integer products has two kinds of bulk copies in flight, ring slots and the next norm weight. Once a
+    wait has given up, nobody waits for either any more, so neither may be asked for again (its barrier may be armed still), and the block
+    waits for both before it leaves: shared memory that a copy still writes is the next block's. Read from the source, since no wait is made
+    to run out on a GPU here."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "brasa_b200" / "csrc" / "decode_token_mma.cu").read_text())
+    asks = re.findall(r"\b(issue_slot|stage_norm)\((?!const)", text)
+    assert asks.count("issue_slot") == 2 and asks.count("stage_norm") == 2  # the first ones; one refill, one norm an operation
+    refill = text.index("issue_slot(c, c.sdesc()")
+    assert "!*c.abort_flag()" in text[text.rindex("if (", 0, refill):refill]
+    norm = text[text.index("auto stage_norm = "):]
+    assert norm.index("if (*c.abort_flag()) return;") < norm.index("*c.norms_asked() = *c.norms_asked() + 1;") < norm.index("mbar_expect_tx")
+    leave = text[text.index("gemv_epilogue(c, op, bo, c.red()"):text.index("if (b == 0)")]
+    leave = leave[leave.index("if (*c.abort_flag()"):]
+    assert "mbar_wait(c.full(tid), *c.gen(tid) & 1)" in leave and "mbar_wait(c.nw_full(), (*c.norms_asked() - 1) & 1)" in leave
+
+
 @pytest.mark.parametrize("name,kernels", [("flash_tc.cu", 2), ("window_attn.cu", 1)])
 def test_row_warps_of_the_attention_kernels_leave_together(name, kernels):
     """The two warps that hold the same query rows meet at counted barriers, and each may give up a wait on its own. So a meeting has to tell
