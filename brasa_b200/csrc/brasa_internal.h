@@ -60,6 +60,11 @@ struct brasa_ctx {
 // then the old one stays until the context goes, and the new one is at least half again as large, so that what stays is less than
 // twice what is in use. BRASA_EINVAL while a graph is being recorded, BRASA_ENOMEM (and no workspace) when memory runs out.
 int32_t brasa_workspace(brasa_ctx *ctx, void **p, size_t *bytes, size_t need);
+// The same for a caller that has another way when there is none: false then, and no error message stays behind.
+bool brasa_workspace_had(brasa_ctx *ctx, void **p, size_t *bytes, size_t need);
+// What the GEMMs' partial tiles are given: the most that the pair kernel asks for (38.8 MB on 148 SMs). It is there before a graph is recorded,
+// so that a recorded product goes the same way as one that is not.
+static inline size_t brasa_gemm_part_most(const brasa_ctx *ctx) { return (size_t)ctx->sm_count * 256 * 256 * sizeof(float); }
 
 // While one of these lives, weights, norms and RoPE tables given to the operators were written by commands that have ended (a model's,
 // written when it is loaded), so a kernel may read them ahead of its griddepcontrol.wait. An operator called from outside gets any

@@ -291,6 +291,7 @@ int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds) {
 int32_t brasa_graph_capture_begin(brasa_ctx *ctx) {
     if (!ctx) return BRASA_EINVAL;
     BRASA_REQUIRE(ctx, !ctx->capturing, "a capture is already open on this context");
+    if (ctx->gemm_part_bytes < brasa_gemm_part_most(ctx)) brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, brasa_gemm_part_most(ctx));
     BRASA_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     ctx->capturing = true;
     ctx->recorded = true;
@@ -397,6 +398,13 @@ int32_t brasa_workspace(brasa_ctx *ctx, void **p, size_t *bytes, size_t need) {
     }
     *bytes = need;
     return BRASA_OK;
+}
+
+bool brasa_workspace_had(brasa_ctx *ctx, void **p, size_t *bytes, size_t need) {
+    const std::string before = ctx->last_error;
+    if (brasa_workspace(ctx, p, bytes, need) == BRASA_OK) return true;
+    ctx->last_error = before;
+    return false;
 }
 
 int32_t brasa_gemv_scratch(brasa_ctx *ctx, size_t partial_floats, size_t counters) {

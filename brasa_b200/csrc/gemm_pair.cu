@@ -585,8 +585,8 @@ int32_t brasa_gemm_pair_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatr
     for (uint32_t b = 1; b < pairs; ++b) shared = shared || pair_begin(b, pairs, p.units, p.gran) % cpt != 0;
     if (shared) {
         // the most that any product asks for (38.8 MB on 148 SMs), so that prompts of growing length allocate and synchronise once
-        const size_t need = (size_t)2 * pairs * p.n * 256 * sizeof(float), most = (size_t)2 * sm_pairs * 256 * 256 * sizeof(float);
-        if (ctx->gemm_part_bytes < need && !ctx->capturing) brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, most);
+        const size_t need = (size_t)2 * pairs * p.n * 256 * sizeof(float);
+        if (ctx->gemm_part_bytes < need && !ctx->capturing) brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, brasa_gemm_part_most(ctx));
         if (ctx->gemm_part_bytes >= need) p.part = ctx->gemm_part;
         else {  // no workspace (a graph is being recorded, or no memory is left): runs of whole tiles
             p.gran = cpt;

@@ -1152,10 +1152,20 @@ bool brasa_gemm_tc_supported(const brasa_qmatrix &w, uint32_t tokens) {
            encode_tiled() != nullptr;
 }
 
+// Bytes of the partial tiles of 65 to 128 tokens, for matrices that brasa_gemm_tc_few_tokens has looked at; the most blocks that share a tile.
+static size_t few_tokens_scratch(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t *max_parts = nullptr) {
+    uint32_t tiles = 0, blocks = 0, parts = 0;
+    uint64_t scratch = 0;
+    for (uint32_t i = 0; i < count; ++i) tiles += ws[i].rows / BN;
+    if (brasa_gemm_few_tokens_plan((uint32_t)ctx->sm_count, tiles, ws[0].cols / BK, &blocks, &parts, &scratch) != BRASA_OK) return ~(size_t)0;
+    if (max_parts) *max_parts = parts;
+    return (size_t)scratch * (SK_TT_MOST / SK_TT);
+}
+
 // True when brasa_gemm_tc_launch takes these matrices with the few-token kernel (whose fused SwiGLU may write over X: its
-// output is stored by a kernel that starts after every product has been formed). Above 64 tokens that asks for a workspace that can be had:
-// without one (a graph is being recorded, no memory is left) the product is another kernel's.
-bool brasa_gemm_tc_few_tokens(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens) {
+// output is stored by a kernel that starts after every product has been formed). Shapes and tokens decide, not what earlier calls have left
+// behind; above 64 tokens a product whose partial tiles outgrow what a recording is given (brasa_gemm_part_most) is another kernel's in it.
+bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens) {
     if (tokens == 0 || tokens > SK_TT_MOST || count < 1 || count > 3) return false;
     uint64_t tiles = 0;
     for (uint32_t i = 0; i < count; ++i) {
@@ -1165,21 +1175,27 @@ bool brasa_gemm_tc_few_tokens(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t 
     const uint32_t nkst = ws[0].cols / BK;
     if (tiled_row_bytes(BRASA_Q4_0, ws[0].cols) % 16 != 0 || tiles * nkst * (uint64_t)(ctx->sm_count + 1) >= (1ull << 32)) return false;
     if (tokens <= SK_TT) return true;
+    if (ctx->capturing && few_tokens_scratch(ctx, ws, count) > brasa_gemm_part_most(ctx)) return false;
     // Above 64 tokens the pair kernel is ahead where a launch of several matrices is small (its tiles fill the SMs whole) or so large that
     // the tensor core holds it. us at 100 tokens, this kernel and the pairs: q, k and v of 2 560 columns (15.7 M weights) 16.6, 17.8; of 1 536
     // (4.7 M) 14.2, 13.1; gate and up of 1 536 (12.6 M) 18.3, 13.9; of 2 560 (50 M) 25.8, 28.0; of 5 120 (262 M) 76.2, 80.5, but at 128 tokens
     // 81.8, 78.2. One matrix (o, down): 9.6 .. 38.7 against 12.0 .. 41.9.
     const uint64_t weights = tiles * BN * ws[0].cols;
-    if (count > 1 && (weights < 14000000 || (weights > 200000000 && tokens > 100))) return false;
-    uint32_t blocks, parts;
-    uint64_t scratch;
-    if (brasa_gemm_few_tokens_plan((uint32_t)ctx->sm_count, (uint32_t)tiles, nkst, &blocks, &parts, &scratch) != BRASA_OK) return false;
-    const size_t need = (size_t)scratch * (SK_TT_MOST / SK_TT), most = (size_t)ctx->sm_count * 256 * 256 * sizeof(float);  // (the pair kernel's bound)
-    if (ctx->gemm_part_bytes < need && !ctx->capturing) brasa_workspace(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, std::max(need, most));
-    return ctx->gemm_part_bytes >= need;
+    return count == 1 || (weights >= 14000000 && (weights <= 200000000 || tokens <= 100));
 }
 
-// acc = acc + W X and out = f16(rms_norm(acc) * norm_w) for at most 128 tokens (brasa_gemm_tc_few_tokens holds for w, its rows
+// Behind brasa_gemm_tc_few_tokens, when nothing else keeps the product from it: whether its partial tiles have room (deferred: all of them, for
+// the kernel that forms SwiGLU or a norm). False above 64 tokens where no memory is left: the product is another kernel's then. Up to 64
+// there is none as good, and the launch reports what is missing.
+bool brasa_gemm_tc_few_tokens_room(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool deferred) {
+    if (tokens <= SK_TT) return true;
+    uint32_t parts;
+    const size_t need = few_tokens_scratch(ctx, ws, count, &parts);
+    if ((parts == 1 && !deferred) || ctx->gemm_part_bytes >= need) return true;
+    return !ctx->capturing && brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, std::max(need, brasa_gemm_part_most(ctx)));
+}
+
+// acc = acc + W X and out = f16(rms_norm(acc) * norm_w) for at most 128 tokens (brasa_gemm_tc_few_tokens and its room hold for w, its rows
 // are a multiple of 512 up to 5120, pointers 16-byte aligned): the few-token kernel, then one kernel for sum, add and norm.
 int32_t brasa_gemm_tc_add_norm(brasa_cmd *cmd, const brasa_qmatrix &w, const __half *x, float *acc, const float *norm_w, __half *out, uint32_t tokens,
                                float eps) {
@@ -1211,7 +1227,8 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
         tiles128 += ws[i].rows / BN;
     }
     // at most 128 tokens of q4_0 matrices: the persistent form whose accumulator rows are weight rows
-    if (brasa_gemm_tc_few_tokens(ctx, ws, count, tokens)) return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
+    if (brasa_gemm_tc_few_tokens(ctx, ws, count, tokens) && brasa_gemm_tc_few_tokens_room(ctx, ws, count, tokens, glu != nullptr))
+        return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
     if (brasa_gemm_pair_takes(ws, count, tokens, glu != nullptr) && !brasa_gemm_pair_behind(ctx, ws, count, tokens, resid != nullptr, glu != nullptr))
         return brasa_gemm_pair_launch(cmd, count, ws, x, ys, tokens, resid, glu);
     // Shape of a CTA: MT token tiles of 128 x NB weight tiles of 128 rows (MT x NB x 128 accumulator columns <= 512).

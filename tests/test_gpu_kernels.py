@@ -693,6 +693,38 @@ def test_gemm_65_to_128_tokens(B, ctx, K, rows, cols, glu, tokens):
         assert np.array_equal(ga.download(np.float32), acc0 + first)
 
 
+def test_recorded_product_does_not_depend_on_earlier_calls(B, K):
+    """A product of 65 to 128 tokens recorded into a graph gives the bits of the call that is not recorded, whether or not an earlier call has left
+    a workspace large enough for the few-token kernel's partial tiles."""
+    ctx, rows, cols, tokens = B.Context(0), 9472, 1024, 100
+    k = B.Kernels(ctx)
+    rng = O.Rng(97)
+    raw = rng.qmatrix(O.Q4_0, rows, cols)
+    m, _ = tiled(B, ctx, k, "q4_0", raw, rows, cols)
+    x = rng.vec(tokens * cols, 0.5)
+    gx, gy = ctx.buffer_from(x.astype(np.float16)), ctx.buffer(tokens * rows * 4)
+    want, s16 = O.matmul(O.Q4_0, raw, rows, cols, x, f16_inputs=True)
+
+    def result(call):
+        gy.fill(0)
+        run(ctx, call)
+        got = gy.download(np.float32)
+        assert np.max(np.abs(got.reshape(tokens, rows) - want) / s16) <= 1e-5
+        return got
+
+    def record():
+        return ctx.capture(lambda c: k.gemm(c, m, gx, gy, tokens))
+
+    before = record()
+    first = result(before.launch)
+    assert np.array_equal(result(lambda c: k.gemm(c, m, gx, gy, tokens)), first)
+    after = record()
+    assert np.array_equal(result(after.launch), first)
+    assert np.array_equal(result(before.launch), first)
+    before.free()
+    after.free()
+
+
 @pytest.mark.parametrize("rows,cols,tokens", [(2560, 4096, 40), (2560, 9728, 64), (5120, 512, 9), (1024, 512, 33), (2560, 4096, 100)])
 def test_gemm_add_rms_norm_equals_the_two_calls(B, ctx, K, rows, cols, tokens):
     """acc += W x followed by the RMS norm of acc, as one call: behind the few-token GEMM one kernel adds the blocks' partial
