@@ -176,6 +176,7 @@ def lib() -> C.CDLL:
         L.brasa_plan_buffer_bytes.restype = C.c_uint64
         L.brasa_session_model.restype = C.c_void_p
         L.brasa_ctx_launch_count.restype = C.c_uint64
+        L.brasa_ctx_last_launch.restype = C.c_char_p
         L.brasa_ctx_destroy.restype = None
         L.brasa_model_free.restype = None
         L.brasa_session_free.restype = None
@@ -281,6 +282,10 @@ class Context:
     def launch_count(self) -> int:
         """Kernels enqueued on this context so far (graph replays count their kernels)."""
         return int(lib().brasa_ctx_launch_count(self._h))
+
+    def last_launch(self) -> str:
+        """Name of the kernel enqueued last on this context."""
+        return lib().brasa_ctx_last_launch(self._h).decode()
 
     def mem_info(self) -> tuple[int, int]:
         f, t = C.c_uint64(), C.c_uint64()

@@ -41,6 +41,7 @@ struct brasa_ctx {
     bool token_kernel = true;    // run a decode token as one persistent kernel (BRASA_TOKEN_KERNEL=0 turns it off)
     uint64_t launches = 0;       // kernels enqueued on this context (graph replays count their nodes)
     uint64_t capture_launches = 0;
+    const char *last_launch = "";  // name of the last one (a literal)
     void *argmax_scratch = nullptr;  // arrival counter + per-block partial maxima
     uint8_t *kv_expand = nullptr;    // f16 hi/lo expansion of a q8_0 KV cache for the tensor-core prefill attention (K hi, K lo, V hi, V lo)
     size_t kv_expand_bytes = 0;
@@ -65,6 +66,9 @@ bool brasa_workspace_had(brasa_ctx *ctx, void **p, size_t *bytes, size_t need);
 // What the GEMMs' partial tiles are given: the most that the pair kernel asks for (38.8 MB on 148 SMs). It is there before a graph is recorded,
 // so that a recorded product goes the same way as one that is not.
 static inline size_t brasa_gemm_part_most(const brasa_ctx *ctx) { return (size_t)ctx->sm_count * 256 * 256 * sizeof(float); }
+
+// What the kernel that adds up the few-token GEMM's partial tiles makes of them (gemm_tc.cu): Y or Y + residual; that and a norm; SwiGLU.
+enum FewTokensUse { FEW_TOKENS_PLAIN, FEW_TOKENS_NORM, FEW_TOKENS_SWIGLU };
 
 // While one of these lives, weights, norms and RoPE tables given to the operators were written by commands that have ended (a model's,
 // written when it is loaded), so a kernel may read them ahead of its griddepcontrol.wait. An operator called from outside gets any

@@ -123,6 +123,7 @@ int32_t brasa_ctx_mem_info(brasa_ctx *ctx, uint64_t *free_bytes, uint64_t *total
 }
 
 uint64_t brasa_ctx_launch_count(brasa_ctx *ctx) { return ctx ? ctx->launches : 0; }
+const char *brasa_ctx_last_launch(brasa_ctx *ctx) { return ctx ? ctx->last_launch : ""; }
 
 #ifdef BRASA_TRACE_BUILD
 int32_t brasa_debug_gemv_trace(brasa_ctx *ctx, uint64_t out[16]) {
@@ -374,6 +375,7 @@ int32_t brasa_rope_table(double theta, uint32_t dim, uint32_t max_pos, float *co
 int32_t brasa_post_launch(brasa_cmd *cmd, const char *name) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return brasa_fail(cmd->ctx, BRASA_ECUDA, "launch of %s: %s", name, cudaGetErrorString(e));
+    cmd->ctx->last_launch = name;
     if (cmd->ctx->capturing) cmd->ctx->capture_launches += 1;
     else cmd->ctx->launches += 1;
     return BRASA_OK;

@@ -11,8 +11,8 @@
 
 bool brasa_gemm_tc_supported(const brasa_qmatrix &w, uint32_t tokens);
 bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool glu);
-bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens);
-bool brasa_gemm_tc_few_tokens_room(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool deferred);
+bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, FewTokensUse use);
+bool brasa_gemm_tc_few_tokens_room(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, FewTokensUse use);
 int32_t brasa_gemm_tc_add_norm(brasa_cmd *cmd, const brasa_qmatrix &w, const __half *x, float *acc, const float *norm_w, __half *out, uint32_t tokens,
                                float eps);
 int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, const __half *x, float *const *ys, uint32_t tokens,
@@ -240,10 +240,10 @@ int32_t brasa_k_gemm_add_rms_norm_f16(brasa_cmd *cmd, brasa_qmatrix w, brasa_arg
     if (!cmd) return BRASA_EINVAL;
     brasa_ctx *ctx = cmd->ctx;
     const uint64_t n = (uint64_t)tokens * w.rows;
-    if (tc_enabled() && tokens >= 2 && tokens > 8 && qm_fits(w) && brasa_gemm_tc_few_tokens(ctx, &w, 1, tokens) && w.rows % 512 == 0 && w.rows <= 5120 &&
+    if (tc_enabled() && tokens >= 2 && tokens > 8 && qm_fits(w) && brasa_gemm_tc_few_tokens(ctx, &w, 1, tokens, FEW_TOKENS_NORM) && w.rows % 512 == 0 && w.rows <= 5120 &&
         arg_fits(x_f16, (uint64_t)tokens * w.cols * 2) && arg_fits(acc, n * 4) && arg_fits(out_f16, n * 2) && arg_fits(norm_w, (uint64_t)w.rows * 4) &&
         x_f16.offset % 16 == 0 && acc.offset % 16 == 0 && out_f16.offset % 16 == 0 && norm_w.offset % 16 == 0 &&
-        brasa_gemm_tc_few_tokens_room(ctx, &w, 1, tokens, true))
+        brasa_gemm_tc_few_tokens_room(ctx, &w, 1, tokens, FEW_TOKENS_NORM))
         return brasa_gemm_tc_add_norm(cmd, w, (const __half *)arg_ptr(x_f16), (float *)arg_ptr(acc), (const float *)arg_ptr(norm_w),
                                       (__half *)arg_ptr(out_f16), tokens, eps);
     BRASA_TRY(brasa_k_gemm_add(cmd, w, x_f16, acc, scratch, tokens));
@@ -290,9 +290,9 @@ int32_t brasa_k_gemm_swiglu(brasa_cmd *cmd, brasa_qmatrix wg, brasa_qmatrix wu, 
     }
     // (few tokens: gate and up in one launch when the tensor-core kernel takes both, so that its runs cover all the SMs)
     const brasa_qmatrix both[2] = {wg, wu};
-    if (tc_enabled() && tokens > 8 && qm_fits(wg) && qm_fits(wu) && brasa_gemm_tc_few_tokens(cmd->ctx, both, 2, tokens) &&
+    if (tc_enabled() && tokens > 8 && qm_fits(wg) && qm_fits(wu) && brasa_gemm_tc_few_tokens(cmd->ctx, both, 2, tokens, FEW_TOKENS_SWIGLU) &&
         arg_fits(x_f16, (uint64_t)tokens * wg.cols * 2) && arg_fits(out_f16, (uint64_t)tokens * wg.rows * 2) && x_f16.offset % 16 == 0 &&
-        out_f16.offset % 16 == 0 && brasa_gemm_tc_few_tokens_room(cmd->ctx, both, 2, tokens, true))
+        out_f16.offset % 16 == 0 && brasa_gemm_tc_few_tokens_room(cmd->ctx, both, 2, tokens, FEW_TOKENS_SWIGLU))
         // its SwiGLU is formed by the kernel that adds up the blocks' partial tiles (the output may be X itself)
         return brasa_gemm_tc_launch(cmd, 2, both, (const __half *)arg_ptr(x_f16), nullptr, tokens, nullptr, (__half *)arg_ptr(out_f16));
     const brasa_arg outs[2] = {gate, up};

@@ -1,4 +1,5 @@
-// Prefill GEMM over CTA pairs (more than 64 tokens; those up to 128 that the few-token kernel leaves): Y[t, :] = W X[t, :], W q4_0 in the tiled layout, X f16, f32 accumulation
+// Prefill GEMM over CTA pairs (more than 64 tokens; those up to 128 that the few-token kernel leaves): Y[t, :] = W X[t, :],
+// W q4_0 in the tiled layout, X f16, f32 accumulation
 // (crates/kernels/src/lib.rs:842-970 and matmul_tiled.metal:35-53: each dequantised weight is rounded to f16 before it meets X).
 //
 // What bounds it: the tensor cores, once both operands reach them. A 128 x 256 product out of two shared-memory operands asks
@@ -520,8 +521,8 @@ static PairPlan pair_plan(uint32_t sm_pairs, uint32_t tiles, uint32_t cpt, uint3
 
 // True when brasa_gemm_pair_launch takes the product (every matrix q4_0 tiled and 16-byte aligned): rows in whole tiles (256; gate
 // and up 128 each) and more tokens than the few-token kernel's tile of 64; up to 128 tokens that kernel has the first choice
-// (brasa_gemm_tc_few_tokens: 77 us for a 4B layer's products at 100 tokens, 85 here). gemm_tc_kernel keeps the shapes whose rows are an odd
-// number of 128: a 4B layer's products at 200 tokens take 159 us here and 174 there, at 1 024 1.6 times as long there.
+// (brasa_gemm_tc_few_tokens). gemm_tc_kernel keeps the shapes whose rows are an odd number of 128: a 4B layer's products at 200 tokens take
+// 159 us here and 174 there, at 1 024 1.6 times as long there.
 bool brasa_gemm_pair_takes(const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool glu) {
     if (tokens <= 64 || encode_tiled() == nullptr) return false;
     uint64_t tiles = 0;

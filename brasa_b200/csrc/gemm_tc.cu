@@ -13,8 +13,8 @@
 //   * warp 1, one lane: tcgen05.mma for the stage, then tcgen05.commit to hand the stage back.
 //   * after the last stage warps 4-11 read the accumulators (tcgen05.ld, one token per lane) and store Y.
 // Up to three matrices that share X (q, k, v) go into one launch: the grid's x index walks their 128-row tiles.
-// q4_0 matrices go to the few-token kernel below with up to 64 tokens, and up to 128 where it is ahead (brasa_gemm_tc_few_tokens), with
-// more, in whole tiles of 256 rows, to gemm_pair.cu: this kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
+// q4_0 matrices go to the few-token kernel below with up to 64 tokens, and up to 128 where it is ahead (brasa_gemm_tc_few_tokens),
+// with more, in whole tiles of 256 rows, to gemm_pair.cu: this kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
 // Every wait is bounded: a wait that runs out raises the context's status word and a CTA-wide flag, every role
 // leaves its loop, tensor memory is freed and the kernel returns.
 #include <cuda.h>
@@ -1165,7 +1165,24 @@ static size_t few_tokens_scratch(const brasa_ctx *ctx, const brasa_qmatrix *ws, 
 // True when brasa_gemm_tc_launch takes these matrices with the few-token kernel (whose fused SwiGLU may write over X: its
 // output is stored by a kernel that starts after every product has been formed). Shapes and tokens decide, not what earlier calls have left
 // behind; above 64 tokens a product whose partial tiles outgrow what a recording is given (brasa_gemm_part_most) is another kernel's in it.
-bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens) {
+//
+// Above 64 tokens gemm_pair.cu is the other kernel. It runs whole tiles of 256 rows side by side on 74 CTA pairs and pays when a few of them have to
+// be cut; this one cuts every tile into even runs and pays for adding the parts up. Both sides in us, this kernel first, at 65, 100 and
+// 128 tokens, weights out of HBM, from 520 products of 256 to 16 384 columns:
+//   * a norm behind the sum takes that kernel's place, up to 5 120 rows: 2 560 x 4 096 13.4, 13.8, 14.3 : 17.1, 18.7, 19.1; 5 120 x 25 600
+//     38.9, 39.8, 40.3 : 43.0, 45.8, 46.9; 512 x 1 024 7.0, 7.1, 7.4 : 12.3, 11.8, 12.1.
+//   * gate and up: ahead where their 128-row tiles fill the SMs, 0.71 to 0.95 of the pairs' time (2 x 9 728 x 2 560 24.5, 24.9, 26.5 : 29.2, 30.3,
+//     31.4; 2 x 25 600 x 5 120 69.3, 72.5, 76.0 : 79.0, 82.5, 82.6); below that the pairs' tiles are one wave and whole (2 x 9 216 x 3 072 25.9, 26.1, 26.7 :
+//     24.1, 24.9, 24.3; 2 x 6 144 x 2 048 20.2, 20.5, 20.9 : 19.1, 19.8, 19.4), but for a few MB of weights (2 x 1 536 x 512 7.6 : 12.3).
+//   * otherwise by the shape: rows of up to two and a half times the columns leave the pairs few tiles to cut (2 560 x 9 728 16.9, 17.5, 17.9 : 18.2, 19.5,
+//     20.6; q, k and v of 2 560 columns, 6 144 rows, 14.3, 14.6, 15.1 : 15.7, 15.9, 16.0), more of them fill the pairs with whole ones (17 408 x
+//     5 120 29.5, 30.8, 32.5 : 26.2, 26.8, 27.0; 2 x 8 192 x 3 072 22.3, 23.6, 25.0 : 18.5, 19.3, 19.4). Several matrices of less than 14 M
+//     weights are the pairs' (3 x 2 048 x 2 048 13.9, 14.2, 14.6 : 13.7, 13.9, 14.2), one of less than 5 M never (1 536 x 512 6.1, 6.7, 6.9 : 7.6, 7.6, 7.7).
+//     From a tile of one matrix per SM on, blocks have whole tiles, whose residual they read with one row to a lane (18 944 x 5 120 with a
+//     residual 40.2, 40.3, 43.4 : 28.0, 28.9, 29.3).
+// What the pairs do not take (rows an odd number of 128) is this kernel's: 0.40 to 1.04 of gemm_tc_kernel's time (2 688 x 9 728 17.4, 17.8, 18.2 :
+// 23.7, 25.7, 26.4).
+bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, FewTokensUse use) {
     if (tokens == 0 || tokens > SK_TT_MOST || count < 1 || count > 3) return false;
     uint64_t tiles = 0;
     for (uint32_t i = 0; i < count; ++i) {
@@ -1176,22 +1193,21 @@ bool brasa_gemm_tc_few_tokens(const brasa_ctx *ctx, const brasa_qmatrix *ws, uin
     if (tiled_row_bytes(BRASA_Q4_0, ws[0].cols) % 16 != 0 || tiles * nkst * (uint64_t)(ctx->sm_count + 1) >= (1ull << 32)) return false;
     if (tokens <= SK_TT) return true;
     if (ctx->capturing && few_tokens_scratch(ctx, ws, count) > brasa_gemm_part_most(ctx)) return false;
-    // Above 64 tokens the pair kernel is ahead where a launch of several matrices is small (its tiles fill the SMs whole) or so large that
-    // the tensor core holds it. us at 100 tokens, this kernel and the pairs: q, k and v of 2 560 columns (15.7 M weights) 16.6, 17.8; of 1 536
-    // (4.7 M) 14.2, 13.1; gate and up of 1 536 (12.6 M) 18.3, 13.9; of 2 560 (50 M) 25.8, 28.0; of 5 120 (262 M) 76.2, 80.5, but at 128 tokens
-    // 81.8, 78.2. One matrix (o, down): 9.6 .. 38.7 against 12.0 .. 41.9.
-    const uint64_t weights = tiles * BN * ws[0].cols;
-    return count == 1 || (weights >= 14000000 && (weights <= 200000000 || tokens <= 100));
+    if (use == FEW_TOKENS_NORM || !brasa_gemm_pair_takes(ws, count, tokens, use == FEW_TOKENS_SWIGLU)) return true;
+    if (use == FEW_TOKENS_SWIGLU) return tiles >= (uint64_t)ctx->sm_count;
+    const uint64_t rows = tiles * BN, cols = ws[0].cols, weights = rows * cols;
+    const bool wide = 2 * rows > 5 * cols;
+    if (count > 1) return !wide && weights >= 14000000;
+    return (!wide || weights < 5000000) && tiles < (uint64_t)ctx->sm_count;
 }
 
-// Behind brasa_gemm_tc_few_tokens, when nothing else keeps the product from it: whether its partial tiles have room (deferred: all of them, for
-// the kernel that forms SwiGLU or a norm). False above 64 tokens where no memory is left: the product is another kernel's then. Up to 64
-// there is none as good, and the launch reports what is missing.
-bool brasa_gemm_tc_few_tokens_room(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, bool deferred) {
+// Behind brasa_gemm_tc_few_tokens, when nothing else keeps the product from it: whether its partial tiles have room. False above 64 tokens where
+// no memory is left: the product is another kernel's then. Up to 64 there is none as good, and the launch reports what is missing.
+bool brasa_gemm_tc_few_tokens_room(brasa_ctx *ctx, const brasa_qmatrix *ws, uint32_t count, uint32_t tokens, FewTokensUse use) {
     if (tokens <= SK_TT) return true;
     uint32_t parts;
     const size_t need = few_tokens_scratch(ctx, ws, count, &parts);
-    if ((parts == 1 && !deferred) || ctx->gemm_part_bytes >= need) return true;
+    if ((parts == 1 && use == FEW_TOKENS_PLAIN) || ctx->gemm_part_bytes >= need) return true;
     return !ctx->capturing && brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, std::max(need, brasa_gemm_part_most(ctx)));
 }
 
@@ -1227,7 +1243,8 @@ int32_t brasa_gemm_tc_launch(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix
         tiles128 += ws[i].rows / BN;
     }
     // at most 128 tokens of q4_0 matrices: the persistent form whose accumulator rows are weight rows
-    if (brasa_gemm_tc_few_tokens(ctx, ws, count, tokens) && brasa_gemm_tc_few_tokens_room(ctx, ws, count, tokens, glu != nullptr))
+    const FewTokensUse use = glu ? FEW_TOKENS_SWIGLU : FEW_TOKENS_PLAIN;
+    if (brasa_gemm_tc_few_tokens(ctx, ws, count, tokens, use) && brasa_gemm_tc_few_tokens_room(ctx, ws, count, tokens, use))
         return launch_skinny(cmd, count, ws, x, ys, tokens, resid, glu);
     if (brasa_gemm_pair_takes(ws, count, tokens, glu != nullptr) && !brasa_gemm_pair_behind(ctx, ws, count, tokens, resid != nullptr, glu != nullptr))
         return brasa_gemm_pair_launch(cmd, count, ws, x, ys, tokens, resid, glu);

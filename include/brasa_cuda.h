@@ -84,6 +84,8 @@ int32_t brasa_ctx_mem_info(brasa_ctx *ctx, uint64_t *free_bytes, uint64_t *total
 int32_t brasa_ctx_sync(brasa_ctx *ctx);
 /* Kernels enqueued on this context so far; a graph replay counts every kernel it holds. */
 uint64_t brasa_ctx_launch_count(brasa_ctx *ctx);
+/* Name of the kernel enqueued (or recorded) last on this context, "" before the first: which of several an entry point took. */
+const char *brasa_ctx_last_launch(brasa_ctx *ctx);
 /* cudaStream_t of the context, for callers that order their own work (NCCL, torch) against it. */
 void *brasa_ctx_stream(brasa_ctx *ctx);
 

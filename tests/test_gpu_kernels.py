@@ -693,6 +693,42 @@ def test_gemm_65_to_128_tokens(B, ctx, K, rows, cols, glu, tokens):
         assert np.array_equal(ga.download(np.float32), acc0 + first)
 
 
+@pytest.mark.parametrize("rows,cols,what,few", [
+    ((2560,), 4096, "plain", True), ((2560,), 4096, "add", True), ((7168,), 2304, "plain", False), ((7168,), 2304, "add", False), ((3072,), 1024, "plain", True),
+    ((2688,), 512, "plain", True), ((2048, 512, 512), 2560, "plain", False), ((4096, 1024, 1024), 2560, "plain", True), ((4096, 4096), 1792, "plain", False),
+    ((3072, 3072), 512, "swiglu", False), ((9472, 9472), 256, "swiglu", True), ((512,), 256, "norm", True), ((5120,), 256, "norm", True)])
+@pytest.mark.parametrize("tokens", [65, 128])
+def test_kernel_for_65_to_128_tokens(B, ctx, K, rows, cols, what, few, tokens):
+    """Which products of 65 to 128 tokens the few-token kernel takes, by shape and by what becomes of them, each side of every line of the rule with
+    the bounds of the tests around it."""
+    rng = O.Rng(95)
+    raws = [rng.qmatrix(O.Q4_0, r, cols) for r in rows]
+    ms = [tiled(B, ctx, K, "q4_0", raw, r, cols)[0] for raw, r in zip(raws, rows)]
+    x = rng.vec(tokens * cols, 0.5)
+    gx, gys = ctx.buffer_from(x.astype(np.float16)), [ctx.buffer(tokens * r * 4) for r in rows]
+    wants = [O.matmul(O.Q4_0, raw, r, cols, x, f16_inputs=True) for raw, r in zip(raws, rows)]
+    acc0, out = rng.vec(tokens * rows[0], 2.0), ctx.buffer(tokens * rows[0] * 2)
+    acc, w = ctx.buffer_from(acc0), ctx.buffer_from(np.ones(rows[0], np.float32))
+    run(ctx, {"plain": lambda c: K.gemm_multi(c, ms, gx, gys, tokens, B.PrefillPrecision.F16), "add": lambda c: K.gemm_add(c, ms[0], gx, acc, gys[0], tokens),
+              "norm": lambda c: K.gemm_add_rms_norm_f16(c, ms[0], gx, acc, gys[0], w, out, tokens, 1e-6),
+              "swiglu": lambda c: K.gemm_swiglu(c, ms[0], ms[1], gx, gys[0], gys[1], out, tokens)}[what])
+    assert ctx.last_launch().startswith("gemm_tc_skinny" if few else "gemm_pair"), ctx.last_launch()
+    if what == "swiglu":
+        (wg, sg), (wu, su) = wants
+        want = O.swiglu(wg, wu).ravel()
+        bound = 1e-5 * (np.abs(wu) * 1.1 * sg + np.abs(wg) * su).ravel() + np.abs(want) * 2.0 ** -10 + 1e-7  # as in the fused SwiGLU's test above
+        assert np.all(np.abs(out.download(np.float16).astype(np.float32) - want) <= bound)
+        return
+    for i, (want, s16) in enumerate(wants):
+        got = gys[i].download(np.float32).reshape(tokens, -1) if what == "plain" else (acc.download(np.float32) - acc0).reshape(tokens, -1)
+        rounding = 0.0 if what == "plain" else 2.0 ** -22 * np.abs(acc0.reshape(tokens, -1)) + 2.0 ** -22 * np.abs(want)  # of the sum, and of taking acc0 off again
+        assert np.all(np.abs(got - want) <= 1e-5 * s16 + rounding), i
+    if what == "norm":
+        y = acc.download(np.float32)
+        want = O.rms_norm(y, np.ones(rows[0], np.float32), rows[0], 1e-6)
+        assert np.all(np.abs(out.download(np.float16).astype(np.float32) - want) <= 2.0 ** -10 * np.abs(want) + 1e-6)
+
+
 def test_recorded_product_does_not_depend_on_earlier_calls(B, K):
     """A product of 65 to 128 tokens recorded into a graph gives the bits of the call that is not recorded, whether or not an earlier call has left
     a workspace large enough for the few-token kernel's partial tiles."""
