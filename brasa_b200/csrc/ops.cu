@@ -429,7 +429,7 @@ __device__ __forceinline__ void store_elem(uint8_t *cache, size_t row, float v, 
 
 // One warp per R rows of 128: rows of a token are hq query heads, then hkv key heads, then hkv value heads. With R = 4 (hq and hkv multiples
 // of four, so that the rows are of one token and one kind) the rows' loads go out together and share the norm weights and angles. Bound: HBM and
-// L2 (every row is read and written once), and with one row to a warp the bytes in flight.
+// L2 (every row is read and written once), and with one row to a warp the bytes in flight; for few rows the chain of one warp.
 template <int KV, bool AHEAD, int R>
 __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, const float *q_norm, const float *k_norm, const float *cos_t,
                                           const float *sin_t, uint8_t *kc, uint8_t *vc, uint32_t hq, uint32_t hkv, uint32_t pos0, float eps,
@@ -451,21 +451,24 @@ __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, co
     if (AHEAD) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     if (gr >= rows) return;
-    const bool is_v = r >= hq + hkv;
-    const size_t idx = is_q ? (size_t)t * hq + r : (size_t)t * hkv + (is_v ? r - hq - hkv : r - hq);
-    float *dst = is_q ? q : k;
-    const float *x = (is_v ? v : dst) + idx * 128;
     float xv[R][4];
+    if (r >= hq + hkv) {
+        const size_t idx = (size_t)t * hkv + (r - hq - hkv);
 #pragma unroll
-    for (int i = 0; i < R; ++i)
+        for (int i = 0; i < R; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) xv[i][j] = x[i * 128 + lane + 32 * j];
-    if (is_v) {
+            for (int j = 0; j < 4; ++j) xv[i][j] = v[(idx + i) * 128 + lane + 32 * j];
 #pragma unroll
         for (int i = 0; i < R; ++i)
             for (int j = 0; j < 4; ++j) store_elem<KV>(vc, idx + i, xv[i][j], lane, j);
         return;
     }
+    const size_t idx = is_q ? (size_t)t * hq + r : (size_t)t * hkv + (r - hq);
+    float *x = (is_q ? q : k) + idx * 128;
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) xv[i][j] = x[i * 128 + lane + 32 * j];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         float ss = 0.0f;
@@ -480,7 +483,7 @@ __global__ void qk_norm_rope_store_kernel(float *q, float *k, const float *v, co
             y[j + 2] = b * c[j] + a * s[j];
         }
         for (int j = 0; j < 4; ++j) {
-            dst[(idx + i) * 128 + lane + 32 * j] = y[j];
+            x[i * 128 + lane + 32 * j] = y[j];
             if (!is_q) store_elem<KV>(kc, idx + i, y[j], lane, j);
         }
     }
@@ -703,10 +706,13 @@ int32_t brasa_k_qk_norm_rope_store(brasa_cmd *cmd, int32_t kv, const brasa_arg q
     BRASA_REQUIRE(ctx, arg_fits(dst[0], brasa_kv_bytes(kv, tk)) && arg_fits(dst[1], brasa_kv_bytes(kv, tk)), "qk_norm_rope_store: cache too small");
     uint32_t rows = sh.tokens * (sh.hq + 2 * sh.hkv);
     if (rows == 0) return BRASA_OK;
-    // (8-bit rows are stored by way of their largest magnitudes, a chain that four rows of one warp walk one after the other: fewer than four
-    // query heads to a KV head are better off a row to a warp, 17.9 against 20.3 us below.) us at 3 584 tokens, four rows and one: 32 and 8
-    // heads f16 28.2, 46.9, q8_0 41.3, 47.9, f32 31.9, 46.9; 8 and 4 heads f16 9.9, 17.2, q8_0 20.3, 17.9. At 1 024 tokens f16 11.3, 15.2.
-    const bool four = sh.hq % 4 == 0 && sh.hkv % 4 == 0 && (kv != BRASA_KV_Q8_0 || sh.hq >= 4 * sh.hkv);
+    // Four rows to a warp once there are enough warps without it: from 48 rows an SM on. 8-bit rows are stored by way of their largest magnitudes, a
+    // chain that four rows of one warp walk one after the other, so they want eight query heads to a KV head, which are not stored, and many more
+    // rows. us, four rows and one: f16, 32 and 8 heads, 37 tokens 2.1, 1.8; 128 tokens (6 144 rows) 2.5, 2.2; 16 and 4 heads, 300 (7 200 rows) 2.4, 2.5;
+    // 32 and 8 heads, 512 4.2, 7.1; 3 584 26.7, 44.9; f32 there 30.2, 45.0; q8_0, 32 and 8 heads, 37 tokens 6.5, 2.5; 3 584 48.5, 46.5; 64 and
+    // 8 heads, 512 (40 960 rows) 12.2, 12.0; 1 024 20.3, 22.6; 3 584 66.3, 75.7.
+    const bool four = sh.hq % 4 == 0 && sh.hkv % 4 == 0 &&
+                      (kv != BRASA_KV_Q8_0 ? rows >= 48u * (uint32_t)ctx->sm_count : sh.hq >= 8 * sh.hkv && rows >= 440u * (uint32_t)ctx->sm_count);
     unsigned grid = four ? (rows + 15) / 16 : (rows + 3) / 4;
 #define LAUNCH_QK(KVT)                                                                                                                              \
     do {                                                                                                                                            \
@@ -721,7 +727,7 @@ int32_t brasa_k_qk_norm_rope_store(brasa_cmd *cmd, int32_t kv, const brasa_arg q
     else if (kv == BRASA_KV_F16) LAUNCH_QK(BRASA_KV_F16);
     else LAUNCH_QK(BRASA_KV_Q8_0);
 #undef LAUNCH_QK
-    return brasa_post_launch(cmd, "qk_norm_rope_store");
+    return brasa_post_launch(cmd, four ? "qk_norm_rope_store_four" : "qk_norm_rope_store");
 }
 
 int32_t brasa_k_store_kv(brasa_cmd *cmd, int32_t kv, brasa_arg src, brasa_arg dst, uint64_t n) {
