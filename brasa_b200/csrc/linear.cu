@@ -697,7 +697,7 @@ int32_t launch_tc(brasa_cmd *cmd, const LinearProblem *p, uint32_t n) {
     const size_t smem = TcShape<BN>::SMEM;
     BRASA_TRY(brasa_smem_optin(ctx, (const void *)linear_tc_kernel<BN>, smem));
     BRASA_CUDA(ctx, brasa_launch_dependent(ctx, linear_tc_kernel<BN>, dim3(std::min<uint32_t>(tiles, ctx->sm_count)), dim3(256), smem, tp));
-    return brasa_post_launch(cmd, "linear_tc");
+    return brasa_post_launch(cmd, BN == 256 ? "linear_tc_256" : (BN == 192 ? "linear_tc_192" : (BN == 128 ? "linear_tc_128" : "linear_tc_64")));
 }
 
 }  // namespace
@@ -759,24 +759,32 @@ int32_t brasa_linear_launch(brasa_cmd *cmd, const LinearProblem *ps, uint32_t co
         return brasa_post_launch(cmd, "linear_f32");
     }
     // The width whose busiest CTA (the first: tiles are dealt out in order) ends soonest. us a K stage of 64 columns where a CTA has several
-    // tiles; a quarter more where it has one, whose first stages nothing covers (but for the narrowest, whose stages are short). What bounds
-    // a stage is its operands' way from L2 (48 KB at the widest), for narrow tiles the chain of waits. us with widths of 64, 128, 192 and 256:
-    // 2 560 rows of 13 824 columns at 2 048 tokens 430, 307, 252, 262; at 1 000 275, 223, 162, 172; at 500 184, 135, 145, 160.
+    // tiles; more where it has one, whose first stages nothing covers (but for the narrowest, whose stages are short), most at the widest with
+    // one tile of tokens, when its weights come from HBM and half its time is the way in and out. What bounds a stage is its operands' way from L2
+    // (48 KB at the widest), for narrow tiles the chain of waits; rows beyond a matrix's end are not fetched. A narrower width has to save
+    // 2 %. us with widths of 64, 128, 192 and 256: 2 560 rows of 13 824 columns at 2 048 tokens 430, 307, 252, 262; at 1 000 275, 223,
+    // 162, 172; at 500 184, 135, 145, 160; 32 768 of 2 560 at 128 60, 42, 54, 45; 6 144, 576 and 32 of 2 560 in one launch at 2 048 168, 98, 75, 69.
+    // Over 465 launches of 31 shapes, 17 to 4 096 tokens, 0.2 % behind the best width on average.
     constexpr uint32_t WIDTH[4] = {64, 128, 192, 256};
-    constexpr double STAGE_US[4] = {0.40, 0.49, 0.56, 0.62}, ALONE[4] = {1.0, 1.25, 1.25, 1.25};
-    uint32_t best = 0;
+    constexpr double STAGE_US[4] = {0.40, 0.49, 0.56, 0.62}, ALONE[4] = {1.0, 1.25, 1.25, 1.25}, ALONE_ONE_PASS = 1.75;
+    bool one_pass = true;  // every weight is read by one CTA
+    for (uint32_t i = 0; i < n; ++i) one_pass = one_pass && p[i].tokens <= BM;
+    uint32_t best = 3;
     double least = 1e30;
-    for (uint32_t w = 0; w < 4; ++w) {
-        uint64_t end = 0, stages = 0, mine = 0;  // tiles so far; stages and tiles of the first CTA
+    for (uint32_t w = 4; w-- > 0;) {
+        uint64_t end = 0, mine = 0;  // tiles so far; tiles of the first CTA
+        double us = 0.0;             // its stages
         for (uint32_t i = 0; i < n; ++i) {
             const uint64_t begin = end, sms = (uint32_t)ctx->sm_count;
             end += (uint64_t)((p[i].rows + WIDTH[w] - 1) / WIDTH[w]) * ((p[i].tokens + BM - 1) / BM);
             const uint64_t t = (end + sms - 1) / sms - (begin + sms - 1) / sms;
+            uint32_t holds = w;  // the width that holds a matrix of few rows
+            while (holds > 0 && p[i].rows <= WIDTH[holds - 1]) --holds;
             mine += t;
-            stages += t * ((p[i].seg[0].cols + BK - 1) / BK + (p[i].seg[1].cols + BK - 1) / BK);
+            us += (double)(t * ((p[i].seg[0].cols + BK - 1) / BK + (p[i].seg[1].cols + BK - 1) / BK)) * STAGE_US[holds];
         }
-        const double us = (double)stages * STAGE_US[w] * (mine == 1 ? ALONE[w] : 1.0);
-        if (us < least) {
+        if (mine == 1) us *= w == 3 && one_pass ? ALONE_ONE_PASS : ALONE[w];
+        if (us < least * 0.98) {
             least = us;
             best = w;
         }

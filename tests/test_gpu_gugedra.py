@@ -134,6 +134,7 @@ def test_linear_epilogues(ctx, n, rows, cols, f32):
 def test_linear_epilogues_in_tiles_of_192_rows(ctx):
     """The same out of tiles of 192 rows: three pairs of gate and up blocks a tile, ragged ends."""
     test_linear_epilogues(ctx, 999, 640, 72, False)
+    assert ctx.last_launch() == "linear_tc_192"
 
 
 WINDOWS = [  # heads, kv_heads, dim, vdim, rot_dims, window, pos0, tokens, ring, softcap
