@@ -37,6 +37,7 @@ using namespace brasa_dev;
 namespace {
 
 constexpr uint32_t SLOT_CAP = 24 * 1024;   // bytes of one ring slot
+constexpr uint32_t DONE_PARITY = 1u << 31; // of a slot's count of warps that are done with it: whether it has been refilled an odd number of times
 constexpr int R = 2;                       // rows a warp works on at a time
 constexpr int NMAX = 5;                    // half blocks of x a lane keeps per column slice
 
@@ -359,8 +360,9 @@ __device__ __forceinline__ WarpRing gemv_rows(const TokCtx &c, const TokOp &op, 
         __syncwarp();
         if (lane == 0 && kk + c.nslot < c.my_slots) {
             // (the warp's reads of the slot are complete: their values went into the sums stored above)
-            if (atomicAdd(&c.done[rs], 1u) == TK_WARPS / 2 - 1) {  // last of the eight: the slot is free, refill it
-                c.done[rs] = 0;
+            // last of the eight: the slot is free, refill it (not after a wait that gave up: the slot's last copy may be on its way still)
+            if ((atomicAdd(&c.done[rs], 1u) & ~DONE_PARITY) == TK_WARPS / 2 - 1 && !*c.abort_flag()) {
+                c.done[rs] = (c.done[rs] & DONE_PARITY) ^ DONE_PARITY;
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 issue_slot(c, c.sdesc[j], rs);
             }
@@ -601,6 +603,13 @@ __global__ void __maxnreg__(128) decode_token_kernel(TokParams p) {
         __syncthreads();
         TRACE(12);
         TRACEB(3);
+    }
+
+    // a block that has given up waits (again with a limit) for its copies before it leaves
+    if (*c.s_abort) {
+        uint32_t s;  // worked out anew: what is kept for here from before the loop over the operations is spilled in it
+        asm volatile("mov.u32 %0, %%tid.x;" : "=r"(s));
+        if (s < min(p.nslot, p.slot_begin[b + 1] - p.slot_begin[b])) mbar_wait(&c.full[s], c.done[s] >> 31);
     }
 
     // ---- greedy choice and the step's bookkeeping: block 0 gathers every block's best logit ----

@@ -264,6 +264,18 @@ def test_token_kernel_that_gave_up_waits_for_every_copy_it_asked_for():
     assert "mbar_wait(c.full(tid), *c.gen(tid) & 1)" in leave and "mbar_wait(c.nw_full(), (*c.norms_asked() - 1) & 1)" in leave
 
 
+def test_dp4a_token_kernel_that_gave_up_waits_for_its_ring():
+    """The same of decode_token.cu, whose only bulk copies are the ring's: no refill once a wait has given up, and the last copy of every slot is
+    waited for in the phase that the slot's refills have come to."""
+    text = re.sub(r"//[^\n]*", "", (ROOT / "brasa_b200" / "csrc" / "decode_token.cu").read_text())
+    assert len(re.findall(r"\bissue_slot\((?!const)", text)) == 2 and len(re.findall(r"\bbulk_g2s\(", text)) == text[text.index("void issue_slot("):text.index("gemv_input(")].count("bulk_g2s(")
+    refill = text.index("issue_slot(c, c.sdesc[j], rs)")
+    ask = text[text.rindex("atomicAdd(&c.done[rs], 1u)", 0, refill):refill]
+    assert "!*c.abort_flag()" in ask and "c.done[rs] = (c.done[rs] & DONE_PARITY) ^ DONE_PARITY;" in ask
+    leave = text[text.index("gemv_epilogue(c, op, bo, c.red["):text.index("if (b == 0)")]
+    assert "if (*c.s_abort)" in leave and "mbar_wait(&c.full[s], c.done[s] >> 31)" in leave
+
+
 @pytest.mark.parametrize("name,kernels", [("flash_tc.cu", 2), ("window_attn.cu", 1)])
 def test_row_warps_of_the_attention_kernels_leave_together(name, kernels):
     """The two warps that hold the same query rows meet at counted barriers, and each may give up a wait on its own. So a meeting has to tell
