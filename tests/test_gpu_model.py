@@ -398,9 +398,95 @@ def test_token_kernel_on_integer_products(hidden, heads, kv_heads, ffn, vocab, k
         m = B.Qwen3.load(ctx, tmp_path / "m.brasa", B.Limits(ctx=64, max_tokens=16, max_logit_rows=1, kv=kvt))
         m.forward(list(range(7)), 0, want_logits=False)
         runs.append(np.stack([m.forward([11 * i + 5], 7 + i)[0][0].copy() for i in range(8)]))
+        assert (ctx.last_launch() == "decode_token_mma") == (mode == "1")
         m.free()
     assert np.isfinite(runs[1]).all()
     assert np.abs(runs[0] - runs[1]).max() <= tol * np.abs(runs[0]).max()
+
+
+@pytest.mark.parametrize("kv", ["F16", "Q8_0"])
+@pytest.mark.parametrize("position", [150, 1300])
+def test_token_on_integer_products_against_oracle(B, ctx, tmp_path, kv, position):
+    """Tokens of that kernel behind keys of several chunks (150: three to a head, merged) and of more than there are blocks for (1 300: a block
+    walks several), whose area in shared memory lies over the norm weight's, against the oracle over the GPU's own cache; then greedy tokens, which
+    the kernel chooses itself. A vocabulary of seven rows to a block: most warps come to its end without rows. Tolerance as in
+    crates/models/tests/forward.rs:40-55."""
+    cfg = BF.tiny_config(layers=2, hidden=768, heads=16, kv_heads=8, ffn=1024, vocab=1024)
+    BF.write_brasa(tmp_path / "m.brasa", cfg, BF.synth_weights(cfg, seed=21, std=0.03, norm_jitter=0.2))
+    ids = np.random.default_rng(6).integers(0, 1024, position + 4).astype(np.uint32)
+    m = B.Qwen3.load(ctx, tmp_path / "m.brasa", B.Limits(ctx=position + 16, max_tokens=256, max_logit_rows=1, kv=B.KvType[kv]))
+    try:
+        for off in range(0, position, 256):
+            m.forward(ids[off:min(off + 256, position)], off, want_logits=False)
+        orc = O.Qwen3Oracle(BF.BrasaFile(tmp_path / "m.brasa"), kv=kv.lower(), ctx=position + 16)
+        for layer in range(2):
+            for which, rows in (("k", orc.k), ("v", orc.v)):
+                raw = m.read_kv(layer, which, 0, position)
+                rows[layer, :position] = (raw.view(np.float16).astype(np.float32) if kv == "F16" else O.dequantize_kv_q8(raw)).reshape(position, -1)
+        want = []
+        for i in range(4):
+            got, _ = m.forward(ids[position + i:position + i + 1], position + i)
+            assert ctx.last_launch() == "decode_token_mma"
+            want.append(orc.forward(ids[position + i:position + i + 1], position + i)[0])
+            assert rel(got[0], want[i]) <= LOGIT_TOL[kv], i
+        got, _ = m.decode_greedy(int(ids[position]), position, 4)  # the first token's cache row is written anew
+        fed = int(ids[position])
+        for i in range(4):
+            lg = orc.forward([fed], position + i)[0]
+            assert lg[got[i]] >= lg.max() - 2 * LOGIT_TOL[kv] * np.abs(lg).max(), i
+            fed = int(got[i])
+    finally:
+        m.free()
+
+
+@pytest.mark.parametrize("what", ["plain", "outliers", "zeros", "inf", "nan"])
+def test_token_on_integer_products_input_planes(B, ctx, tmp_path, what):
+    """x as that kernel holds it, two bytes against the largest magnitude of 32 columns, seen through a model whose layers add nothing: the logits are
+    one product of the embedding row times the final norm's weight. Outliers stand in one half of a block, in the other, in both, in none; zeros
+    fill halves and whole blocks. Bound: half a step for every column, and f32 rounding. An infinity or a NaN leaves no finite logit
+    and token 0, and nothing behind for the next launch."""
+    cfg = BF.tiny_config(layers=1, hidden=1024, heads=8, kv_heads=2, ffn=1024, vocab=640)
+    w = BF.synth_weights(cfg, seed=22, std=0.05)
+    for name in w:
+        if name.endswith("proj.weight"):
+            w[name][:] = 0
+    rng, H = np.random.default_rng(7), 1024
+    norm = (1.0 + 0.2 * rng.standard_normal(H)).astype(np.float32)
+    blocks = norm.reshape(32, 2, 16)
+    if what == "outliers":
+        for b in range(32):
+            for half in range(2):
+                if b >> half & 1:
+                    blocks[b, half, rng.integers(16)] = (-1.0) ** b * 10.0 ** rng.uniform(1, 5)
+    elif what == "zeros":
+        blocks[::4] = 0
+        blocks[1::4, 0] = 0
+        blocks[2::4, 1] = 0
+        blocks[3, :, 3:] = 1e-42  # denormal
+    elif what != "plain":
+        norm[777] = {"inf": np.inf, "nan": np.nan}[what]
+    w["model.norm.weight"] = norm
+    BF.write_brasa(tmp_path / "m.brasa", cfg, w)
+    f = BF.BrasaFile(tmp_path / "m.brasa")
+    table = O.dequantize(O.Q6_0, f.raw("model.embed_tokens.weight"), 640 * H).reshape(640, H).astype(np.float64)
+    m = B.Qwen3.load(ctx, tmp_path / "m.brasa", B.Limits(ctx=32, max_tokens=16, max_logit_rows=1, kv=B.KvType.F16))
+    try:
+        for i, tok in enumerate((3, 639, 100)):
+            got, _ = m.forward([tok], i)
+            assert ctx.last_launch() == "decode_token_mma"
+            if what in ("inf", "nan"):
+                assert not np.isfinite(got[0]).any()
+                continue
+            x = table[tok] * norm
+            scale = 1.0 / np.sqrt(np.mean(table[tok] ** 2) + cfg["rms_norm_eps"])
+            half_step = np.repeat(np.abs(x).reshape(-1, 32).max(1) / 32639 / 2, 32)
+            bound = (np.abs(table) @ half_step) * 1.01 + 2e-6 * (np.abs(table) @ np.abs(x))
+            assert np.all(np.abs(got[0] - table @ x * scale) <= bound * scale)
+        ids, _ = m.decode_greedy(5, 3, 3)
+        if what in ("inf", "nan"):
+            assert not ids.any()
+    finally:
+        m.free()
 
 
 @pytest.mark.gpu
