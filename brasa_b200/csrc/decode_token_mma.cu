@@ -23,6 +23,11 @@ namespace {
 
 constexpr uint32_t SLOT_CAP = 23040;  // bytes of one ring slot: sixteen rows of 2 560 columns, eight of 5 120, four of 10 240
 constexpr uint32_t TILE = 16;         // rows of a warp's products
+constexpr uint32_t MAX_COLS = 10240;  // (wider rows are fewer than four to a slot: a tile would hold most of the ring)
+// Hidden sizes this kernel takes; us a token against decode_token.cu's (4 layers, f16, 100 positions): 512 55.6 (57.4), but a short chat of
+// it 1 052 (1 023); 768 73.5 (75.4), 1 024 77.7 (83.8), 1 536 83.7 (90.3), 2 048 161 (167), 2 560 173 (201), 4 096 193 (182): rows of 4 096
+// columns all begin in the same shared-memory bank and fill four fifths of a slot.
+constexpr uint32_t MIN_HIDDEN = 768, MAX_HIDDEN = 3072;
 
 struct SlotDesc {
     const uint8_t *src[2];  // the rows of one matrix, and of the next one where the slot reaches into it
@@ -152,8 +157,9 @@ __device__ __forceinline__ void issue_slot(const TokCtx &c, const uint4 *desc, u
 
 // ---- GEMV, phase 1: wait for the input, fold the norm weight, convert to fixed point. A thread takes eight values at a
 // time (values 4 j .. and 16 + 4 j .. of a block of 32, so that its words of the planes are neighbours), four lanes share a
-// block. Up to 4 096 columns that is one pass of the block, all its polls in flight at once; two passes' are where there are
-// more. Returns the warp's share of sum x^2.
+// block. Up to 4 096 columns, an input with a norm and an embedding row among them, that is one pass of the block, up to MAX_COLS three; the polls of
+// all of them are in flight at once. Returns the warp's share of sum x^2.
+static_assert(MAX_HIDDEN <= TK_THREADS * 8 && MAX_COLS <= 3 * TK_THREADS * 8, "passes of gemv_input");
 __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, const uint8_t *embed, uint32_t vocab) {
     const uint32_t cols = op.cols;
     const uint32_t tid = phase_tid(), nu = cols / 8;  // a multiple of 32: a warp is inside or outside as a whole
@@ -162,17 +168,17 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
     float ssq = 0.0f;
     const bool normed = op.normw != nullptr;
     float4 n0 = make_float4(1.0f, 1.0f, 1.0f, 1.0f), n1 = n0;
-    if (normed && tid < nu) {  // the norm weight, a bulk copy asked for one operation ahead: of the thread's first values before the input is there
+    if (normed && tid < nu) {  // the norm weight, a bulk copy asked for one operation ahead: of the thread's values before the input is there
         if (!slot_wait(c, c.nw_full(), (op.nw_use - 1) & 1)) give_up(c, 2);
         const uint32_t e = (tid >> 2) * 32 + 4 * (tid & 3);
         n0 = *reinterpret_cast<const float4 *>(c.nwbuf() + e);
         n1 = *reinterpret_cast<const float4 *>(c.nwbuf() + e + 16);
     }
     const bool save = op.save_resid != 0;
+    // (one round for every width taken; written as a branch, a token behind 16 384 keys of an 8-bit cache takes 1 709 us for 1 698)
 #pragma unroll 1
     for (uint32_t u0 = tid; u0 < nu; u0 += 3 * TK_THREADS) {
-        uint32_t u = u0, e = (u >> 2) * 32 + 4 * (u & 3);
-        uint32_t passes = min(3u, (nu - u + TK_THREADS - 1) / TK_THREADS);
+        uint32_t u = u0, e = (u >> 2) * 32 + 4 * (u & 3), passes = (nu - u + TK_THREADS - 1) / TK_THREADS;
         constexpr uint32_t FAR = TK_THREADS * 8;  // elements from a thread's unit to its next
         uint4 a, b, a2 = make_uint4(0, 0, 0, 0), b2 = a2, a3 = a2, b3 = a2;
         if (op.in_kind == IN_EMBED) {
@@ -181,8 +187,6 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
             const float4 va = in_table ? embed_quad(embed, c.token, cols, e / 4) : z, vb = in_table ? embed_quad(embed, c.token, cols, e / 4 + 4) : z;
             a = make_uint4(__float_as_uint(va.x), __float_as_uint(va.y), __float_as_uint(va.z), __float_as_uint(va.w));
             b = make_uint4(__float_as_uint(vb.x), __float_as_uint(vb.y), __float_as_uint(vb.z), __float_as_uint(vb.w));
-            u0 -= 2 * TK_THREADS;  // one pass at a time
-            passes = 1;
         } else {
             const uint32_t *src = in + e;
 #pragma unroll 1
@@ -224,10 +228,6 @@ __device__ __forceinline__ float gemv_input(const TokCtx &c, const TokOp &op, co
                 }
             }
             if (normed) {
-                if (e != (tid >> 2) * 32 + 4 * (tid & 3)) {
-                    n0 = *reinterpret_cast<const float4 *>(c.nwbuf() + e);
-                    n1 = *reinterpret_cast<const float4 *>(c.nwbuf() + e + 16);
-                }
                 v[0] *= n0.x; v[1] *= n0.y; v[2] *= n0.z; v[3] *= n0.w;
                 v[4] *= n1.x; v[5] *= n1.y; v[6] *= n1.z; v[7] *= n1.w;
             }
@@ -554,11 +554,7 @@ bool slot_rows(int qtype, uint32_t cols, uint32_t *lrps) {
 // slots are asked for while a tile is worked on. Among what fits, the split whose busiest warp has the least shared-memory traffic (a group of
 // 128 columns: 10 wavefronts of x, 12 of sixteen rows), then the one with fewer partial sums. More than one slice asks for at most sum_room
 // partial sums; one slice's are as many as the block has rows, however many that is (ring_layout).
-constexpr uint32_t SUM_ROOM = 6144, MAX_COLS = 10240;  // (wider rows are fewer than four to a slot: a tile would hold most of the ring)
-// Hidden sizes this kernel takes; us a token against decode_token.cu's (4 layers, f16, 100 positions): 512 55.6 (57.4), but a short chat of
-// it 1 052 (1 023); 768 73.5 (75.4), 1 024 77.7 (83.8), 1 536 83.7 (90.3), 2 048 161 (167), 2 560 173 (201), 4 096 193 (182): rows of 4 096
-// columns all begin in the same shared-memory bank and fill four fifths of a slot.
-constexpr uint32_t MIN_HIDDEN = 768, MAX_HIDDEN = 3072;
+constexpr uint32_t SUM_ROOM = 6144;
 struct Split {
     uint32_t tile, slices, row_warps;
 };
