@@ -91,7 +91,17 @@ struct TokParams {
     unsigned long long *partials;  // [heads][max_chunks][130]
     float attn_scale;
     uint32_t *status;
+#ifdef BRASA_TRACE_BUILD
+    unsigned long long *trace;  // block 0 stamps the phases of 16 operations from trace_op on, as in decode_token.cu
+    uint32_t trace_op;
+#endif
 };
+
+#ifdef BRASA_TRACE_BUILD
+#define TRACE(i) do { if (p.trace && blockIdx.x == 0 && threadIdx.x == 0 && oi >= p.trace_op && oi < p.trace_op + 16) p.trace[16 + (oi - p.trace_op) * 16 + (i)] = (unsigned long long)clock64(); } while (0)
+#else
+#define TRACE(i) do { } while (0)
+#endif
 
 // Values 4 qi .. 4 qi + 3 of row `row` of a tiled q6_0 table (embed_kernel's arithmetic).
 __device__ __forceinline__ float4 embed_quad(const uint8_t *table, uint32_t row, uint32_t cols, uint32_t qi) {
@@ -462,6 +472,7 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
         if (warp == TK_WARPS - 2 && oi + 1 < p.nops) fetch_op(oi + 1, buf);
         const uint32_t epoch = c.seq * EPOCH_SPAN + oi + 1;
 
+        TRACE(0);
         if (tid == TK_THREADS - 1 && op.next_normw) stage_norm(op.next_normw, op.next_cols);
         if (op.type == OP_GEMV) {
             const uint32_t nrows = bo.nrows, total_slots = bo.slots;
@@ -474,10 +485,13 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
                 }
             }
             RowsJob job = rows_begin(c, op, rec.plan[warp], nrows, gslot, tiled_row_bytes((int)op.qtype, op.cols));
+            TRACE(1);
             const float ssq = gemv_input(c, op, p.embed, p.vocab);
+            TRACE(3);
             if (lane == 0) c.red()[warp] = ssq;
             if (warp >= TK_WARPS - 2) cp_async_wait();  // the descriptors, the next operation: asked for before the input was waited for
             __syncthreads();
+            TRACE(4);
             if (warp == TK_WARPS - 1) {  // 1 / rms of the whole input from the warps' sums, parked for the epilogue
                 float tot = c.red()[lane & (TK_WARPS - 1)];
                 for (int o = TK_WARPS / 2; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
@@ -485,14 +499,18 @@ __global__ void __maxnreg__(128) decode_token_mma_kernel(const __grid_constant__
             }
             if (op.qtype == BRASA_Q4_0) gemv_rows<BRASA_Q4_0>(c, op, job, rec.plan[warp], nrows, gslot);
             else gemv_rows<BRASA_Q6_0>(c, op, job, rec.plan[warp], nrows, gslot);
+            TRACE(7);
             gslot += total_slots;
             __syncthreads();
+            TRACE(8);
             gemv_epilogue(c, op, bo, c.red()[RED_SCALE], epoch, p.logits, p.cand);
         } else {
             if (warp == TK_WARPS - 2) cp_async_wait();
             attention_op<KV>(AttnCtx{c.xfb(), c.abort_flag(), p.status, c.G, c.b, c.pos, c.par_cur, c.par_alt}, op, oi, epoch, p.heads, p.kv_heads, p.max_chunks, p.cos_t, p.sin_t, p.partials, p.attn_scale);
         }
+        TRACE(11);
         __syncthreads();
+        TRACE(12);
     }
 
     // a block that has given up waits (again with a limit) for its copies before it leaves
@@ -867,6 +885,11 @@ int32_t brasa_token_mma_create(brasa_ctx *ctx, const brasa_token_model &m, brasa
     p.par_words = (uint32_t)par_words;
     p.attn_scale = 1.0f / sqrtf(128.0f);
     p.status = ctx->status;
+#ifdef BRASA_TRACE_BUILD
+    p.trace = ctx->gemv_trace;
+    const char *env = getenv("BRASA_TRACE_OP");
+    p.trace_op = env ? (uint32_t)atoi(env) : 5;
+#endif
 
     const TokenKernel fn = token_kernel(m.kv);
     BRASA_TRY(brasa_smem_optin(ctx, (const void *)fn, prog->smem));
