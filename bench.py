@@ -28,8 +28,8 @@ size, and nothing else.
 
 With --gpus N > 1 (launched by torch.distributed.run) every rank serves its own replica: the path has
 no exchange step at batch 1, so the ranks share nothing and the aggregate is the sum ("replicas only").
---impl reference times the reference's CPU path alone (rank 0 only): tools/qwen3_ref.py from oracle/_ref/ when that was
-made (oracle/make_ref.py), else the oracle's C port.
+--impl reference times the reference's CPU path alone (rank 0 only): tools/qwen3_ref.py from oracle/_ref/ (oracle/make_ref.py). Where
+that was not made it says so ("unavailable") and times nothing: the oracle's C port is this repository's code and not the reference.
 """
 
 from __future__ import annotations
@@ -282,6 +282,9 @@ def time_qwen3_ref(path, cfg: dict, ids: np.ndarray, warmup: int, steps: int):
 def run_reference(args, rank: int):
     if rank != 0:
         return
+    if not (ROOT / "oracle" / "_ref" / "qwen3_ref.py").exists():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's tools/qwen3_ref.py is not on this machine (oracle/make_ref.py copies it from a checkout)"}))
+        return
     import oracle
     from brasa_b200 import synth
     oracle.build()
@@ -289,27 +292,16 @@ def run_reference(args, rank: int):
     path = model_path("qwen3-4b")
     if not path.exists():
         write_model_cpu(path, cfg)
-    cores = use_all_host_cores()
-    ids = prompt_ids(cfg["vocab_size"])
-    if (ROOT / "oracle" / "_ref" / "qwen3_ref.py").exists():
-        sec, cores, _ = time_qwen3_ref(path, cfg, ids, args.warmup, args.steps)
-        kind = "reference"
-        sample = (f"{args.steps} greedy decode tokens at positions {PROMPT}.. of this workload after a CPU prefill of its {PROMPT}-token prompt: the "
-                  f"reference's tools/qwen3_ref.py (torch CPU, {cores} threads, KV rounded to f16, dequantised layers kept in RAM), same model file "
-                  f"as the GPU arm when that file is already on the machine")
-    else:
-        total = args.warmup + args.steps
-        times, _ = cpu_decode_sample(path, None, ids[:total], PROMPT, total)
-        timed = times[args.warmup:]
-        sec = sum(timed) / len(timed)
-        kind = "port"
-        sample = (f"{args.steps} decode tokens at positions {PROMPT}.. of this workload, oracle C port (dequantise a row, f64 dot; OpenMP over rows), "
-                  f"KV cache of {PROMPT} zero rows (no CPU prefill: the reference's own Python forward was not staged on this machine)")
+    use_all_host_cores()
+    sec, cores, _ = time_qwen3_ref(path, cfg, prompt_ids(cfg["vocab_size"]), args.warmup, args.steps)
+    sample = (f"{args.steps} greedy decode tokens at positions {PROMPT}.. of this workload after a CPU prefill of its {PROMPT}-token prompt: the "
+              f"reference's tools/qwen3_ref.py (torch CPU, {cores} threads, KV rounded to f16, dequantised layers kept in RAM), same model file "
+              f"as the GPU arm when that file is already on the machine")
     value = 1.0 / sec
     line = {"impl": "reference", "metric": METRIC, "value": value, "unit": "tok/s", "n_gpus": args.gpus, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": sec * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
             "dtype": "f32 activations and accumulation, q4_0/q6_0 weights, f16 KV", "data": "synthetic", "config": workload_config(args.gpus),
-            "cpu_baseline": {"value": value, "unit": "tok/s", "cores": cores, "kind": kind, "sample": sample},
+            "cpu_baseline": {"value": value, "unit": "tok/s", "cores": cores, "kind": "reference", "sample": sample},
             "e2e": {"value": value, "unit": "tok/s", "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
     print(json.dumps(line))
 

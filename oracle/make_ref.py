@@ -5,8 +5,8 @@
 The reference's CPU implementation of the token loop is three Python files (tools/qwen3_ref.py, tools/brasa_file.py,
 tools/convert_brasa.py: torch and numpy only). They are copied, unmodified, from the checkout into oracle/_ref/, which
 is ignored by git (nothing of the reference enters the history) but travels with a working copy to the machine that
-runs the benchmark. `bench.py --impl reference` times Qwen3Ref from there when it is present and falls back to the C
-port of this directory otherwise. Nothing else reads oracle/_ref/.
+runs the benchmark. `bench.py --impl reference` times Qwen3Ref from there and says "unavailable" where it is not.
+Nothing else reads oracle/_ref/.
 """
 
 from __future__ import annotations
