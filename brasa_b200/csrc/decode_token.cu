@@ -22,7 +22,8 @@
 // decode_token_mma.cu takes the models whose products are worth integer tensor instructions (f16 and q8_0 caches, one GPU, hidden sizes
 // of 768 to 3 072; brasa_token_mma_takes); this kernel has the narrower ones (bound by the exchanges either way), the wider ones (32B: rows that a tile
 // of sixteen cannot hold in a slot), f32 caches and the shards of a tensor-parallel model.
-// GEMV arithmetic, x conversion and epilogues are those of gemv.cu (same rounding); attention works on 64-key
+// GEMV arithmetic, x conversion and epilogues are those of gemv.cu (with two byte planes of x for f16 and q8_0 caches, three there and
+// for f32 caches); attention works on 64-key
 // chunks (32 for an f32 cache) shared out over the blocks and is merged per head by the blocks at the far end of
 // the grid.
 #include <stdlib.h>

@@ -10,7 +10,7 @@
 // Bound: the exchanges and, in the rows phase, shared-memory bandwidth (a unit of 16 rows x 128 columns takes 22 wavefronts, 8 of
 // them the codes). Each operation ends with a block barrier although nothing there needs one: without it the warps that have no
 // rows to store poll for the next input beside those that do, and hold up their stores (1.24 against 1.10 ms a token).
-// us a token, one B200, decode_token.cu's in brackets: 4B architecture at 512 positions, f16 1 006 (1 118); at 16 384, q8_0 1 713 (1 845).
+// us a token, one B200, decode_token.cu's in brackets: 4B architecture at 512 positions, f16 992 (1 118); at 16 384, q8_0 1 698 (1 845).
 #include <memory>
 
 #include "decode_token_mma.h"
@@ -636,7 +636,8 @@ size_t ring_layout(std::vector<OpRecord> &ops, const std::vector<uint32_t> &op_r
     p.off_done = take((size_t)ring * 8);
     p.off_red = take(RED_WORDS * 4);
     p.off_ops = take(OP_BUFFERS * sizeof(OpBuffer));
-    p.off_zeros = take(16 + 32 + 8) / 32 * 32 + 16;  // zeros, two words; off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
+    // zeros, two words; off the banks that the lanes with a share of x read at the same time (its words begin at 32 bytes)
+    p.off_zeros = take(16 + 32 + 8) / 32 * 32 + 16;
     for (OpRecord &r : ops) {
         r.op.meta_off = p.off_xf + r.op.cols / 32 * X_PLANE_BYTES;
         r.op.part_off = (uint32_t)(p.off_xf + xf_bytes - (size_t)(r.op.epilogue == EPI_LOGITS ? last_sums : sums) * 4) & ~15u;

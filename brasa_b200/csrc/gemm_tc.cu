@@ -14,7 +14,8 @@
 //   * after the last stage warps 4-11 read the accumulators (tcgen05.ld, one token per lane) and store Y.
 // Up to three matrices that share X (q, k, v) go into one launch: the grid's x index walks their 128-row tiles.
 // q4_0 matrices go to the few-token kernel below with up to 64 tokens, and up to 128 where it is ahead (brasa_gemm_tc_few_tokens),
-// with more, in whole tiles of 256 rows, to gemm_pair.cu: this kernel serves what is left (rows an odd number of 128; the q6_0 head) and many tokens over few columns (brasa_gemm_pair_behind).
+// with more, in whole tiles of 256 rows, to gemm_pair.cu: this kernel serves what is left (rows an odd number of 128; the q6_0 head)
+// and many tokens over few columns (brasa_gemm_pair_behind).
 // Every wait is bounded: a wait that runs out raises the context's status word and a CTA-wide flag, every role
 // leaves its loop, tensor memory is freed and the kernel returns.
 #include <cuda.h>
@@ -1125,8 +1126,8 @@ int32_t launch_skinny(brasa_cmd *cmd, uint32_t count, const brasa_qmatrix *ws, c
 
 }  // namespace
 
-// How a few-token product is cut over the SMs (include/brasa_cuda.h; scratch_bytes is that of 64 tokens, up to 128 take twice as much): the (tile, stage) units in order, `blocks`
-// equal runs, run b = units [b units / blocks, (b + 1) units / blocks).
+// How a few-token product is cut over the SMs (include/brasa_cuda.h; scratch_bytes is that of 64 tokens, up to 128 take twice as
+// much): the (tile, stage) units in order, `blocks` equal runs, run b = units [b units / blocks, (b + 1) units / blocks).
 extern "C" int32_t brasa_gemm_few_tokens_plan(uint32_t sm_count, uint32_t tiles, uint32_t stages, uint32_t *blocks, uint32_t *max_parts,
                                               uint64_t *scratch_bytes) {
     if (!blocks || !max_parts || !scratch_bytes || sm_count == 0 || tiles == 0 || stages == 0) return BRASA_EINVAL;

@@ -9,7 +9,9 @@
 //   * x is fixed point per block of 32 columns, in two signed bytes (digits of base 256) against the block's largest magnitude / 32 639.
 //     The sums are exact integers; one conversion and one multiply by (block scale x step) per row and block follow. x is off by at
 //     most half a step, 1.5e-5 of the block's largest magnitude (the powers of two of gemv_device.cuh, P = 2: 1.5e-5 .. 3.1e-5 of
-//     that of 16 values).
+//     that of 16 values). An outlier coarsens twice as many values here, with a finer step. Relative error of a product of 2 560
+//     columns, here and with P = 2: normal x 2.1e-5, 2.9e-5; one column of 64 times 30 4.6e-5, 4.9e-5, times 300 4.7e-5, 5.1e-5, and
+//     for rows that have no weight on those columns 1.8e-3, 1.9e-3; Student's t of 1.5 degrees 4.7e-5, 5.2e-5.
 // mma.sync m16n8k32 takes 8 cycles of an SM's quarter here, twice the rate of dp4a (which takes 2 for 128 weights and one plane).
 #pragma once
 #include "gemv_device.cuh"
