@@ -706,26 +706,24 @@ int32_t brasa_k_qk_norm_rope_store(brasa_cmd *cmd, int32_t kv, const brasa_arg q
     BRASA_REQUIRE(ctx, arg_fits(dst[0], brasa_kv_bytes(kv, tk)) && arg_fits(dst[1], brasa_kv_bytes(kv, tk)), "qk_norm_rope_store: cache too small");
     uint32_t rows = sh.tokens * (sh.hq + 2 * sh.hkv);
     if (rows == 0) return BRASA_OK;
-    // Four rows to a warp once there are enough warps without it: from 48 rows an SM on. 8-bit rows are stored by way of their largest magnitudes, a
-    // chain that four rows of one warp walk one after the other, so they want eight query heads to a KV head, which are not stored, and many more
-    // rows. us, four rows and one: f16, 32 and 8 heads, 37 tokens 2.1, 1.8; 128 tokens (6 144 rows) 2.5, 2.2; 16 and 4 heads, 300 (7 200 rows) 2.4, 2.5;
-    // 32 and 8 heads, 512 4.2, 7.1; 3 584 26.7, 44.9; f32 there 30.2, 45.0; q8_0, 32 and 8 heads, 37 tokens 6.5, 2.5; 3 584 48.5, 46.5; 64 and
-    // 8 heads, 512 (40 960 rows) 12.2, 12.0; 1 024 20.3, 22.6; 3 584 66.3, 75.7.
-    const bool four = sh.hq % 4 == 0 && sh.hkv % 4 == 0 &&
-                      (kv != BRASA_KV_Q8_0 ? rows >= 48u * (uint32_t)ctx->sm_count : sh.hq >= 8 * sh.hkv && rows >= 440u * (uint32_t)ctx->sm_count);
+    // Four rows to a warp for f16 and f32 caches from 20 rows an SM on. us a layer of a prompt, four rows and one, f16: 4B shape, 37 tokens (12 rows an
+    // SM) 79.7, 79.1; 64 (21) 82.4, 83.8; 100 92.7, 96.7; 512 177, 184; 3 584 944, 968; 2 048 wide with 16 and 8 heads, 100 tokens (22) 77.9, 77.2; 512
+    // 126, 128; 2 048 314, 325; with 16 and 16, 200 (65) 97.6, 96.1; 300 110, 112; 512 wide with 8 and 4, 64 (7) 40.6, 40.1; 1 024 89, 91. 8-bit rows are
+    // stored by way of their largest magnitudes, a chain that four rows of one warp walk one after the other: 4B, 37 tokens 89.1, 85.7; 512
+    // 196, 193; 2 048 592, 587; 3 584 1 061, 1 051; 64 and 8 heads, 37 tokens 185, 182; 2 048 2 077, 2 103.
+    const bool four = kv != BRASA_KV_Q8_0 && sh.hq % 4 == 0 && sh.hkv % 4 == 0 && rows > 20u * (uint32_t)ctx->sm_count;
     unsigned grid = four ? (rows + 15) / 16 : (rows + 3) / 4;
-#define LAUNCH_QK(KVT)                                                                                                                              \
-    do {                                                                                                                                            \
-        const auto kernel = ctx->settled ? (four ? qk_norm_rope_store_kernel<KVT, true, 4> : qk_norm_rope_store_kernel<KVT, true, 1>)              \
-                                         : (four ? qk_norm_rope_store_kernel<KVT, false, 4> : qk_norm_rope_store_kernel<KVT, false, 1>);           \
-        BRASA_CUDA(ctx, brasa_launch_dependent(ctx, kernel, dim3(grid), dim3(128), 0, (float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]),          \
-                                               (const float *)arg_ptr(qkv[2]), (const float *)arg_ptr(norms[0]), (const float *)arg_ptr(norms[1]), \
-                                               (const float *)arg_ptr(cos_t), (const float *)arg_ptr(sin_t), arg_ptr(dst[0]), arg_ptr(dst[1]),     \
-                                               sh.hq, sh.hkv, sh.pos0, eps, rows));                                                                \
-    } while (0)
-    if (kv == BRASA_KV_F32) LAUNCH_QK(BRASA_KV_F32);
-    else if (kv == BRASA_KV_F16) LAUNCH_QK(BRASA_KV_F16);
-    else LAUNCH_QK(BRASA_KV_Q8_0);
+#define LAUNCH_QK(KVT, R)                                                                                                                           \
+    BRASA_CUDA(ctx, brasa_launch_dependent(ctx, ctx->settled ? qk_norm_rope_store_kernel<KVT, true, R> : qk_norm_rope_store_kernel<KVT, false, R>,     \
+                                           dim3(grid), dim3(128), 0, (float *)arg_ptr(qkv[0]), (float *)arg_ptr(qkv[1]),                              \
+                                           (const float *)arg_ptr(qkv[2]), (const float *)arg_ptr(norms[0]), (const float *)arg_ptr(norms[1]),        \
+                                           (const float *)arg_ptr(cos_t), (const float *)arg_ptr(sin_t), arg_ptr(dst[0]), arg_ptr(dst[1]), sh.hq,     \
+                                           sh.hkv, sh.pos0, eps, rows))
+    if (kv == BRASA_KV_Q8_0) LAUNCH_QK(BRASA_KV_Q8_0, 1);
+    else if (kv == BRASA_KV_F16 && four) LAUNCH_QK(BRASA_KV_F16, 4);
+    else if (kv == BRASA_KV_F16) LAUNCH_QK(BRASA_KV_F16, 1);
+    else if (four) LAUNCH_QK(BRASA_KV_F32, 4);
+    else LAUNCH_QK(BRASA_KV_F32, 1);
 #undef LAUNCH_QK
     return brasa_post_launch(cmd, four ? "qk_norm_rope_store_four" : "qk_norm_rope_store");
 }

@@ -370,10 +370,10 @@ def test_qk_norm_rope_store(B, ctx, K, kv, tokens, pos0):
 
 
 @pytest.mark.parametrize("kv", ["F16", "Q8_0"])
-@pytest.mark.parametrize("hq,hkv,tokens", [(4, 4, 5), (16, 4, 3), (8, 4, 5), (6, 2, 9), (12, 6, 1), (16, 4, 295), (16, 4, 297), (6, 2, 801), (32, 4, 1627), (32, 4, 1629)])
+@pytest.mark.parametrize("hq,hkv,tokens", [(4, 4, 5), (16, 4, 3), (8, 4, 5), (6, 2, 9), (12, 6, 1), (16, 4, 123), (16, 4, 124), (6, 2, 301), (16, 4, 700)])
 def test_qk_norm_rope_store_rows_per_warp(B, ctx, K, kv, hq, hkv, tokens):
-    """Four rows to a warp where both head counts allow it and there are rows enough (for 8-bit caches also eight query heads to a KV head), one
-    otherwise: the last block ragged, the same bounds as above."""
+    """Four rows to a warp where both head counts allow it, the cache is not an 8-bit one and there are rows enough, one otherwise: the last
+    block ragged, the same bounds as above."""
     kvt, rng, dim, pos0 = B.KvType[kv], O.Rng(28), 128, 5
     q, k, v = (rng.vec(tokens * h * dim, 2.0) for h in (hq, hkv, hkv))
     qn, kn = rng.vec(dim, 1.5), rng.vec(dim, 1.5)
@@ -383,7 +383,7 @@ def test_qk_norm_rope_store_rows_per_warp(B, ctx, K, kv, hq, hkv, tokens):
     kc, vc = ctx.buffer(kvt.bytes(n)), ctx.buffer(kvt.bytes(n))
     run(ctx, lambda c: K.qk_norm_rope_store(c, kvt, [gq, gk, gv], [gqn, gkn], 1e-6, table, [kc, vc], B.AttnShape(tokens, hq, hkv, dim, pos0, kvt)))
     sms, rows = 148, tokens * (hq + 2 * hkv)
-    four = hq % 4 == 0 and hkv % 4 == 0 and (rows >= 48 * sms if kv == "F16" else hq >= 8 * hkv and rows >= 440 * sms)
+    four = kv == "F16" and hq % 4 == 0 and hkv % 4 == 0 and rows > 20 * sms
     assert ctx.last_launch() == ("qk_norm_rope_store_four" if four else "qk_norm_rope_store")
     for got, x, w, h in ((gq, q, qn, hq), (gk, k, kn, hkv)):
         want = O.rope_neox(O.rms_norm(x, w, dim, 1e-6), h, dim, pos0, cos, sin)
