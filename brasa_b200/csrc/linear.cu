@@ -760,15 +760,16 @@ int32_t brasa_linear_launch(brasa_cmd *cmd, const LinearProblem *ps, uint32_t co
     }
     // The width whose busiest CTA (the first: tiles are dealt out in order) ends soonest. us a K stage of 64 columns where a CTA has several
     // tiles; more where it has one, whose first stages nothing covers (but for the narrowest, whose stages are short), most at the widest with
-    // one tile of tokens, when its weights come from HBM and half its time is the way in and out. What bounds a stage is its operands' way from L2
+    // one tile of tokens, when its weights come from HBM and half its time is the way in and out (up to 32 tokens one warp's way out: 32 768 rows
+    // of 2 560 columns at 17 tokens 70, 49, 49, 44 us, at 37 60, 40, 51, 43). What bounds a stage is its operands' way from L2
     // (48 KB at the widest), for narrow tiles the chain of waits; rows beyond a matrix's end are not fetched. A narrower width has to save
     // 2 %. us with widths of 64, 128, 192 and 256: 2 560 rows of 13 824 columns at 2 048 tokens 430, 307, 252, 262; at 1 000 275, 223,
     // 162, 172; at 500 184, 135, 145, 160; 32 768 of 2 560 at 128 60, 42, 54, 45; 6 144, 576 and 32 of 2 560 in one launch at 2 048 168, 98, 75, 69.
     // Over 465 launches of 31 shapes, 17 to 4 096 tokens, 0.2 % behind the best width on average.
     constexpr uint32_t WIDTH[4] = {64, 128, 192, 256};
     constexpr double STAGE_US[4] = {0.40, 0.49, 0.56, 0.62}, ALONE[4] = {1.0, 1.25, 1.25, 1.25}, ALONE_ONE_PASS = 1.75;
-    bool one_pass = true;  // every weight is read by one CTA
-    for (uint32_t i = 0; i < n; ++i) one_pass = one_pass && p[i].tokens <= BM;
+    bool one_pass = true;  // every weight is read by one CTA, for tokens of several warps
+    for (uint32_t i = 0; i < n; ++i) one_pass = one_pass && p[i].tokens > 32 && p[i].tokens <= BM;
     uint32_t best = 3;
     double least = 1e30;
     for (uint32_t w = 4; w-- > 0;) {

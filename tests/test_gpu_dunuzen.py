@@ -129,7 +129,7 @@ def test_linear_group_in_tiles_of_192_rows(ctx):
 
 @pytest.mark.parametrize("tokens_n, shapes, width", [
     (2, [(7, 40, 0)], 64), (130, [(65, 72, 0), (300, 72, 24), (1, 8, 0)], 64), (2000, [(6140, 72, 0)], 256), (1999, [(6140, 8, 0), (576, 8, 0), (32, 8, 0)], 256),
-    (17, [(33000, 8, 0)], 128), (128, [(28500, 8, 0)], 128), (127, [(28000, 8, 0)], 192), (300, [(9000, 16, 0)], 192),
+    (32, [(33000, 8, 0)], 256), (33, [(33000, 8, 0)], 128), (128, [(28500, 8, 0)], 128), (127, [(28000, 8, 0)], 192), (300, [(9000, 16, 0)], 192),
     (300, [(9500, 16, 0)], 256), (999, [(1280, 72, 0)], 128)])
 def test_linear_tile_width(ctx, tokens_n, shapes, width):
     """Tile widths on both sides of the estimate's lines: one tile to a CTA or several, with one tile of tokens or more, a matrix of few rows
