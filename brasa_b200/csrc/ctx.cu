@@ -292,7 +292,12 @@ int32_t brasa_cmd_wait(brasa_cmd *cmd, double *gpu_seconds) {
 int32_t brasa_graph_capture_begin(brasa_ctx *ctx) {
     if (!ctx) return BRASA_EINVAL;
     BRASA_REQUIRE(ctx, !ctx->capturing, "a capture is already open on this context");
-    if (ctx->gemm_part_bytes < brasa_gemm_part_most(ctx)) brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, brasa_gemm_part_most(ctx));
+    if (ctx->gemm_part_bytes < brasa_gemm_part_most(ctx)) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (the caller may be recording on a stream of its own)
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        brasa_workspace_had(ctx, (void **)&ctx->gemm_part, &ctx->gemm_part_bytes, brasa_gemm_part_most(ctx));
+        cudaThreadExchangeStreamCaptureMode(&mode);
+    }
     BRASA_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
     ctx->capturing = true;
     ctx->recorded = true;
