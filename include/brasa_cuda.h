@@ -188,7 +188,8 @@ uint32_t brasa_gemm_few_tokens_owner(uint32_t units, uint32_t blocks, uint32_t u
 uint32_t brasa_token_ring_slots(uint32_t sm_count, uint32_t smem_bytes, uint32_t hidden, uint32_t heads, uint32_t kv_heads, uint32_t ffn, uint32_t vocab,
                                 int32_t head_qtype, int32_t kv);
 /* acc += W x, then out_f16 = f16(rms_norm(acc) * norm_w): a layer's residual add and the norm that opens the next block
- * (qwen3.rs:810-826 then :700-712 as one call). One GEMM and one kernel behind it for up to 64 tokens; otherwise the two calls. */
+ * (qwen3.rs:810-826 then :700-712 as one call). One GEMM and one kernel behind it for up to 64 tokens,
+ * mostly up to 128; otherwise the two calls. */
 int32_t brasa_k_gemm_add_rms_norm_f16(brasa_cmd *cmd, brasa_qmatrix w, brasa_arg x_f16, brasa_arg acc, brasa_arg scratch, brasa_arg norm_w,
                                       brasa_arg out_f16, uint32_t tokens, float eps);
 int32_t brasa_k_gemm_multi(brasa_cmd *cmd, const brasa_qmatrix *ws, uint32_t count, brasa_arg x, const brasa_arg *ys, uint32_t tokens, int32_t precision); /* :872 */
